@@ -11,6 +11,16 @@
 // early exit changes only when it stops, not its answer: it returns the full
 // count when that reaches `need` and nothing otherwise, so the full count
 // settles it.
+//
+// What bounds it: FP64. A residual is about 70 f64 operations at 2 per clock
+// and SM; all of them in f64 took 8.1 ms for 77 M residuals (100 pairs, 2000
+// hypotheses each). So a match is first tested in FP32 with an error bound:
+// the test |dot| < th * den holds or fails for certain unless the two sides
+// come within the bound (a few matches in 10^5 of a wrong hypothesis, a few in
+// 10^3 of a near-true one), and only then is the f64 residual formed. The
+// counts and masks stay the f64 residual's, since a certain answer is its
+// answer whatever the roundings. The same call from host arrays went from 8.8
+// to 0.90 ms, most of which now is the upload of the 14 MB of hypotheses.
 #include <cuda_runtime.h>
 
 #include <cstdint>
@@ -54,9 +64,53 @@ __device__ __forceinline__ double residual(const double (&e)[9], double ax, doub
 
 constexpr int kWarpsPerBlock = 8;
 
+// Whether |r| < th, decided in FP32 where that is certain: 1 yes, 0 no, -1 not
+// decided. e is the hypothesis scaled by a power of two to a largest entry in
+// [1/2, 1) (the residual does not change), q the match, both rounded to f32,
+// th in [2^-60, 2^60]. With u = 2^-24, P = |ax| + |ay| + 1 and Q likewise of b:
+//   each component of e p is within 4.01 u P of its real value (two rounded
+//   inputs, two fused roundings), each of e^T q within 4.01 u Q, the dot product
+//   within 8 u P Q, and den, a Euclidean norm of four of them, within
+//   6 u (P + Q) + 5 u den (its sum, sqrt.approx at 2^-23).
+// The constants below also cover the roundings of the test itself and those of
+// the f64 residual (2^-53 relative to the same magnitudes). den must be
+// certainly positive for a "no": the residual of a zero den is 0, an inlier.
+// NaN and coordinates above 2^60 decide nothing.
+__device__ __forceinline__ int certain_inlier(const float (&e)[9], const float4 q, float th) {
+    constexpr float u = 0x1p-24f;
+    const float P = fabsf(q.x) + fabsf(q.y) + 1.0f, Q = fabsf(q.z) + fabsf(q.w) + 1.0f;
+    const float ep0 = fmaf(e[0], q.x, fmaf(e[1], q.y, e[2]));
+    const float ep1 = fmaf(e[3], q.x, fmaf(e[4], q.y, e[5]));
+    const float ep2 = fmaf(e[6], q.x, fmaf(e[7], q.y, e[8]));
+    const float et0 = fmaf(e[0], q.z, fmaf(e[3], q.w, e[6]));
+    const float et1 = fmaf(e[1], q.z, fmaf(e[4], q.w, e[7]));
+    const float dot = fabsf(fmaf(q.z, ep0, fmaf(q.w, ep1, ep2)));
+    float den;
+    asm("sqrt.approx.f32 %0, %1;"
+        : "=f"(den)
+        : "f"(fmaf(ep0, ep0, fmaf(ep1, ep1, fmaf(et0, et0, et1 * et1)))));
+    const float PQ = P * Q, ed = 12.0f * u * PQ, eg = 7.0f * u * (P + Q);
+    const float lo = fmaf(den, 1.0f - 16.0f * u, -eg), hi = fmaf(den, 1.0f + 16.0f * u, eg);
+    if (!(PQ < 0x1p60f)) return -1;
+    if (dot + ed < th * lo) return 1;
+    if (lo > 0.0f && dot - ed >= th * hi) return 0;
+    return -1;
+}
+
+// The matches rounded to f32, once a call: a conversion in the scoring loop
+// would go through the FP64 pipe for every hypothesis.
+__global__ void __launch_bounds__(256) sampson_round_kernel(const double4 *pts, float4 *pts32, uint64_t m) {
+    const uint64_t i = (uint64_t)blockIdx.x * blockDim.x + threadIdx.x;
+    if (i >= m) return;
+    const double4 q = pts[i];
+    pts32[i] = make_float4((float)q.x, (float)q.y, (float)q.z, (float)q.w);
+}
+
 // One warp per hypothesis: its pair's matches 32 at a time, the inlier bits
 // of each group of 32 by ballot (one mask word, written by lane 0 when the
-// hypothesis asks for its mask), the count by population count.
+// hypothesis asks for its mask), the count by population count. A hypothesis
+// whose entries or threshold leave the range of the FP32 test (2^-200..2^200
+// for the largest entry) is scored in f64 throughout.
 __global__ void __launch_bounds__(32 * kWarpsPerBlock) sampson_kernel(SampsonArgs a) {
     const uint32_t lane = threadIdx.x & 31;
     const uint64_t h = (uint64_t)blockIdx.x * kWarpsPerBlock + (threadIdx.x >> 5);
@@ -64,23 +118,39 @@ __global__ void __launch_bounds__(32 * kWarpsPerBlock) sampson_kernel(SampsonArg
     const uint32_t p = a.hyp_pair[h];
     const uint64_t m0 = a.pair_off[p], m1 = a.pair_off[p + 1];
     const double th = a.thresh[p];
-    double e[9];
+    // lane k < 9 holds entry k; the scaling moves its exponent field
+    const long long bits = lane < 9 ? __double_as_longlong(a.E[9 * h + lane]) : 0;
+    const int ex = (int)((bits >> 52) & 0x7ff);
+    const int top = __reduce_max_sync(0xffffffffu, ex);
+    const bool fast = top >= 1023 - 200 && top <= 1023 + 200 && th >= 0x1p-60 && th <= 0x1p60;
+    const int scaled = ex + (1022 - top);  // entries below 2^-900 of the largest become 0
+    const float mine = ex > 0 && scaled > 0 && fast
+                           ? (float)__longlong_as_double((bits & ~(0x7ffll << 52)) | ((long long)scaled << 52))
+                           : 0.0f;
+    float e32[9];
 #pragma unroll
-    for (int k = 0; k < 9; ++k) e[k] = a.E[9 * h + k];
+    for (int k = 0; k < 9; ++k) e32[k] = __shfl_sync(0xffffffffu, mine, k);
+    const float th32 = (float)th;
     uint32_t *mk = nullptr;
     if (a.masks && a.mask_off && a.mask_off[h] != ~0ull) mk = a.masks + a.mask_off[h];
     uint32_t c = 0;
     for (uint64_t i0 = m0; i0 < m1; i0 += 32) {
         const uint64_t i = i0 + lane;
-        bool in = false;
+        int in = 0;
         if (i < m1) {
-            const double4 q = a.pts[i];
-            // inliers_of / count_at_least: |r| < th, strict (two_view.rs:806, :812)
-            in = fabs(residual(e, q.x, q.y, q.z, q.w)) < th;
+            in = fast ? certain_inlier(e32, a.pts32[i], th32) : -1;
+            if (in < 0) {
+                double e[9];
+#pragma unroll
+                for (int k = 0; k < 9; ++k) e[k] = a.E[9 * h + k];
+                const double4 q = a.pts[i];
+                // inliers_of / count_at_least: |r| < th, strict (two_view.rs:806, :812)
+                in = fabs(residual(e, q.x, q.y, q.z, q.w)) < th;
+            }
         }
-        const uint32_t bits = __ballot_sync(0xffffffffu, in);
-        c += __popc(bits);
-        if (mk && lane == 0) mk[(i0 - m0) >> 5] = bits;
+        const uint32_t word = __ballot_sync(0xffffffffu, in > 0);
+        c += __popc(word);
+        if (mk && lane == 0) mk[(i0 - m0) >> 5] = word;
     }
     if (lane == 0) a.counts[h] = c;
 }
@@ -89,6 +159,7 @@ __global__ void __launch_bounds__(32 * kWarpsPerBlock) sampson_kernel(SampsonArg
 
 void launch_sampson(const SampsonArgs &a, cudaStream_t s) {
     if (!a.nh) return;
+    if (a.n_pts) sampson_round_kernel<<<(unsigned)((a.n_pts + 255) / 256), 256, 0, s>>>(a.pts, a.pts32, a.n_pts);
     const uint64_t blocks = (a.nh + kWarpsPerBlock - 1) / kWarpsPerBlock;
     sampson_kernel<<<(unsigned)blocks, 32 * kWarpsPerBlock, 0, s>>>(a);
 }

@@ -2315,7 +2315,7 @@ extern "C" slm_status slm_sampson_score(slm_ctx *c, const double *pts, const uin
                  o_e = al(o_th + 8 * (uint64_t)np), o_hp = al(o_e + 72 * (uint64_t)nh),
                  o_cnt = al(o_hp + 4 * (uint64_t)nh), o_moff = al(o_cnt + 4 * (uint64_t)nh),
                  o_mask = al(o_moff + (mask_off ? 8 * (uint64_t)nh : 0)),
-                 bytes = al(o_mask + (mask_off ? 4 * mask_words : 0));
+                 o_p32 = al(o_mask + (mask_off ? 4 * mask_words : 0)), bytes = al(o_p32 + 16 * m);
     slm_status st = w->score.ensure(c, bytes);
     if (st == SLM_OK) {
         unsigned char *d = w->score.as<unsigned char>();
@@ -2333,6 +2333,8 @@ extern "C" slm_status slm_sampson_score(slm_ctx *c, const double *pts, const uin
         if (e == cudaSuccess) {
             SampsonArgs a{};
             a.pts = reinterpret_cast<const double4 *>(d + o_pts);
+            a.n_pts = m;
+            a.pts32 = reinterpret_cast<float4 *>(d + o_p32);
             a.pair_off = reinterpret_cast<const uint64_t *>(d + o_off);
             a.thresh = reinterpret_cast<const double *>(d + o_th);
             a.E = reinterpret_cast<const double *>(d + o_e);

@@ -146,6 +146,8 @@ cudaError_t single_exact_enqueue(unsigned char *scratch, const SingleLayout &L, 
 // ~0, the inlier bits at masks[mask_off[h] ..].
 struct SampsonArgs {
     const double4 *pts;
+    uint64_t n_pts;
+    float4 *pts32;             // scratch of n_pts: the matches in f32
     const uint64_t *pair_off;
     const double *thresh;
     const double *E;

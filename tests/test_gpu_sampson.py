@@ -91,3 +91,49 @@ def test_bad_arguments_are_refused(matcher):
                              hp.ctypes.data_as(P(ctypes.c_uint32)), len(hyps), counts.ctypes.data_as(P(ctypes.c_uint32)),
                              mo.ctypes.data_as(P(ctypes.c_uint64)), counts.ctypes.data_as(P(ctypes.c_uint32)), 0)
     assert st == 1  # SLM_INVALID_ARG
+
+
+@pytest.mark.parametrize("scale", [0, 190, -190, 199, 201, -201, 300, -300, 500])
+@pytest.mark.parametrize("what", ["ulp", "huge", "nonfinite", "th"])
+def test_the_fp32_test_never_decides_otherwise_than_f64(matcher, scale, what):
+    """Hypotheses scaled by powers of two through the FP32 test's range and
+    beyond it; thresholds on a match's residual and one ulp either side of it;
+    coordinates that are huge, tiny, infinite or NaN; thresholds that are zero,
+    negative, infinite or outside the FP32 test's range: the f64 answer each time."""
+    rng = np.random.default_rng(1000 + scale)
+    n = 97
+    n1, n2, e = synth.two_view(rng, n, inlier_frac=0.6)
+    pts = np.concatenate([n1, n2], 1)
+    hyps = synth.essential_hypotheses(rng, e, 60)
+    hyps[10] = np.diag([0.0, 0.0, 1.0])  # den is 0 for every match: all inliers
+    hyps[11] = [[0, 0, 0], [0, 0, 0], [0, 1e-9, 1]]
+    hyps[12, 1] *= 2.0 ** -1000          # rows that vanish beside the others
+    ths = [1.5 / 800]
+    if what == "ulp":
+        for h, i in ((0, 3), (0, 50), (6, 7), (7, 90)):
+            r = abs(O.sampson_residual(hyps[h], pts[i, :2], pts[i, 2:]))
+            ths += [r, np.nextafter(r, 1), np.nextafter(r, 0)]
+    elif what == "huge":
+        pts[::3] *= 10.0 ** rng.uniform(-40, 40, (len(pts[::3]), 1))
+        pts[1] = [1e18, 1e18, 1e18, 1e18]
+        pts[2] = [1e300, 1, 1, 1]
+        ths += [1e15, 1e-12]
+    elif what == "nonfinite":
+        pts[5, 0], pts[6, 1], pts[7, 2], pts[8, 3] = np.nan, np.inf, -np.inf, np.nan
+        hyps[20, 0, 0], hyps[21, 2, 2], hyps[22, 1, 1] = np.nan, np.inf, -np.inf
+    else:
+        ths += [0.0, -1.0, np.inf, -np.inf, np.nan, 1e-30, 2.0 ** -60, 2.0 ** -61, 2.0 ** 60, 2.0 ** 61, 1e300]
+    hyps = hyps * 2.0 ** scale
+    npair = len(ths)
+    off = np.arange(npair + 1, dtype=np.uint64) * n
+    hp = np.repeat(np.arange(npair, dtype=np.uint32), len(hyps))
+    all_h, all_p = np.tile(hyps, (npair, 1, 1)), np.tile(pts, (npair, 1))
+    masks_for = list(range(0, len(hp), 7))
+    mo = np.full(len(hp), 2**64 - 1, np.uint64)
+    mo[masks_for] = np.arange(len(masks_for)) * ((n + 31) // 32)
+    got, gm = matcher.sampson_score(all_p, off, np.asarray(ths), all_h, hp, masks_for=masks_for)
+    want, wm = O.sampson_score(all_p, off, np.asarray(ths), all_h, hp, mask_off=mo, threads=8)
+    assert np.array_equal(got, want)
+    for h in masks_for:
+        w = wm[int(mo[h]):int(mo[h]) + (n + 31) // 32]
+        assert np.array_equal(gm[h], np.unpackbits(w.view(np.uint8), bitorder="little")[:n].astype(bool)), h
