@@ -77,7 +77,8 @@ typedef struct {
     float kernel_ms;            /* device time of the main matching kernel, last launch */
     float max_abs_err;          /* max |approx - exact| seen on rescored pairs */
     uint64_t kernel_launches;   /* kernels one launch of the batch runs */
-    float pass_ms[2];           /* BF16/FP8: tensor-core passes 1 and 2; FP32: [0] = exact kernel */
+    float pass_ms[2];           /* BF16: the tensor-core pass (both directions), and the undecided
+                                   rows' rescoring; FP8: passes 1 and 2; FP32: [0] = exact kernel */
     uint64_t pairs_routed;      /* BF16/FP8: pairs whose error bound was too loose to certify
                                    their rows, matched whole by the exact FP32 kernel */
     uint64_t pairs_rescued;     /* FP8: pairs whose FP8 bound was too loose for their distances,
@@ -214,9 +215,10 @@ uint32_t slm_store_num_views(slm_store *st);
 
 /* Tuning knobs; zero fields take the autotuned or default values. */
 typedef struct {
-    uint32_t items_per_sm;  /* FP32: target work items per SM when splitting columns */
-    uint32_t shortlist_k;   /* BF16/FP8: shortlist capacity, records of 4-column hit groups per
-                               row, column range and column half, 1..32 (0: 16) */
+    uint32_t items_per_sm;  /* FP32, FP8: target work items per SM when splitting columns */
+    uint32_t shortlist_k;   /* shortlist capacity, 1..32 (0: 16). BF16: a row whose bounds decide
+                               nothing is rescored over up to 2 shortlist_k columns; FP8: records
+                               of 4-column hit groups per row, column range and column half */
     uint32_t use_graph;     /* 1: replay a captured CUDA graph (default), 2: plain launches */
     uint32_t variant;       /* FP32: 0 packed f32x2 arithmetic (default), 1 all
                                scalar; both IEEE, bit-exact.
@@ -228,8 +230,8 @@ typedef struct {
 } slm_tune;
 
 /* Time a grid of settings on this batch with CUDA events (FP32: items per SM
- * {2, 4, 8} x arithmetic variant; BF16/FP8: items per SM {2, 4, 8} x row tiles
- * per work item {1, 2} x shortlist_k {8, 12, 16}) and return the fastest in
+ * {2, 4, 8} x arithmetic variant; FP8: items per SM {2, 4, 8} x row tiles
+ * per work item {1, 2} x shortlist_k {8, 12, 16}; BF16: the latter two) and return the fastest in
  * *best (and its time in *best_ms). The result is cached in the context under
  * the batch's shape (precision, mean rows per pair, pair count), which plans
  * with slm_tune.autotune = 1 use. Launches the batch several times. */

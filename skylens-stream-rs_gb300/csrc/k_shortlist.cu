@@ -1,21 +1,21 @@
-// k_shortlist.cu — BF16 / FP8 tcgen05 shortlist path of ratio_match.
+// k_shortlist.cu — the FP8 shortlist tier of ratio_match, the store's operand
+// images, and what both precisions share after their passes: routing to the
+// exact kernel, exact scans, compaction. (The BF16 pass is in k_top2.cu.)
 //
 // Reference: crates/core/src/matching.rs:144-215. See slm_shortlist.h for the
 // passes and the certification rules. Every match decision is either proven
 // by the per-pair error bound eps or settled with exact spec-order FP32
 // distances (matching.rs:146-155), so results equal the reference's.
 //
-// Tensor-core kernel (sl_pass_kernel, one persistent CTA per SM, 18 warps):
+// FP8 tensor-core kernel (sl_pass_kernel, one persistent CTA per SM, 18 warps):
 //   warp 0      TMA producer: per item the a tiles (1 or 2 x 128 rows, K-major,
-//               128B-swizzled operand images copied verbatim from the store;
-//               FP8 also norms and scales); per 128-column b tile the operand
-//               tile (and, in pass 2, column thresholds) through a ring of 3
-//               (BF16) or 4 (FP8) slots.
+//               128B-swizzled operand images copied verbatim from the store)
+//               with their norms and scales; per 128-column b tile the operand
+//               tile, norms and scales (and, in pass 2, column thresholds)
+//               through a ring of 4 slots.
 //   warp 1      allocates 512 TMEM columns; one thread issues tcgen05.mma
-//               (M=128, N=128, K=16 bf16 / K=32 e4m3) into a double-buffered
-//               pair of 128x128 f32 accumulators per a tile. BF16 adds a ninth
-//               K step over the norm extension (slm_shortlist.h), so the
-//               accumulator is d~ / 2.
+//               (M=128, N=128, K=32 e4m3) into a double-buffered pair of
+//               128x128 f32 accumulators per a tile.
 //   warps 2-17  epilogue: warp w reads TMEM lane quarter w % 4 of a tile
 //               ((w - 2) / 4) % 2, column half (w - 2) / 8 of every b tile,
 //               one thread per row, 16 columns per tcgen05.ld. Row minima use
@@ -24,103 +24,18 @@
 //               memory (by the epilogue warps of sub-partitions 2 and 3) and
 //               across CTAs with one atomicMin per column and tile. Pass 2
 //               looks for row-candidate and column-window hits in groups of 4
-//               columns behind the chunk minimum. BF16 pass 1 never reads the
-//               b stage: the MMA's commit alone frees it.
+//               columns behind the chunk minimum.
 #include <cuda_fp8.h>
 #include <cuda_bf16.h>
 #include <cuda_runtime.h>
 
 #include <cstdint>
 
-#include "ptx.cuh"
-#include "slm_shortlist.h"
+#include "shortlist.cuh"
 
 namespace slm {
 
 // ------------------------------------------------------------ small helpers
-
-// Order-preserving map of f32 to u32 (unsigned order == float order).
-SLM_DEV uint32_t f2ord(float f) {
-    const uint32_t b = __float_as_uint(f);
-    return (b & 0x80000000u) ? ~b : (b | 0x80000000u);
-}
-SLM_DEV float ord2f(uint32_t u) { return __uint_as_float((u & 0x80000000u) ? (u & 0x7fffffffu) : ~u); }
-
-SLM_DEV float min3f(float a, float b, float c) {
-    float d;
-    asm("min.f32 %0, %1, %2, %3;" : "=f"(d) : "f"(a), "f"(b), "f"(c));
-    return d;
-}
-
-SLM_DEV float warp_min_f32(float v) {
-    float r;
-    asm volatile("redux.sync.min.f32 %0, %1, 0xffffffff;" : "=f"(r) : "f"(v));
-    return r;
-}
-
-SLM_DEV uint64_t globaltimer() {
-    uint64_t t;
-    asm volatile("mov.u64 %0, %%globaltimer;" : "=l"(t));
-    return t;
-}
-
-// Minimum of 32 values (NaN inputs are ignored by min.f32).
-SLM_DEV float min32(const float (&d)[32]) {
-    float m[11];
-#pragma unroll
-    for (int k = 0; k < 10; ++k) m[k] = min3f(d[3 * k], d[3 * k + 1], d[3 * k + 2]);
-    m[10] = fminf(d[30], d[31]);
-    const float x = min3f(m[0], m[1], m[2]);
-    const float y = min3f(m[3], m[4], m[5]);
-    const float z = min3f(m[6], m[7], m[8]);
-    return fminf(min3f(x, y, z), fminf(m[9], m[10]));
-}
-
-typedef unsigned long long u64x;
-SLM_DEV u64x f2_pack(float lo, float hi) {
-    u64x d;
-    asm("mov.b64 %0, {%1, %2};" : "=l"(d) : "f"(lo), "f"(hi));
-    return d;
-}
-SLM_DEV float f2_lo(u64x v) { return __uint_as_float(static_cast<uint32_t>(v)); }
-SLM_DEV float f2_hi(u64x v) { return __uint_as_float(static_cast<uint32_t>(v >> 32)); }
-SLM_DEV u64x f2_add(u64x a, u64x b) {
-    u64x d;
-    asm("add.rn.f32x2 %0, %1, %2;" : "=l"(d) : "l"(a), "l"(b));
-    return d;
-}
-SLM_DEV u64x f2_sub(u64x a, u64x b) {
-    u64x d;
-    asm("sub.rn.f32x2 %0, %1, %2;" : "=l"(d) : "l"(a), "l"(b));
-    return d;
-}
-// Approximate-path arithmetic: one rounding, covered by the error bound.
-SLM_DEV u64x f2_fma(u64x a, u64x b, u64x c) {
-    u64x d;
-    asm("fma.rn.f32x2 %0, %1, %2, %3;" : "=l"(d) : "l"(a), "l"(b), "l"(c));
-    return d;
-}
-
-// 32 lanes x 16 consecutive 32-bit TMEM columns (asynchronous until the wait).
-SLM_DEV void tmem_ld16(uint32_t taddr, uint32_t (&r)[16]) {
-    asm volatile(
-        "tcgen05.ld.sync.aligned.32x32b.x16.b32 "
-        "{%0,%1,%2,%3,%4,%5,%6,%7,%8,%9,%10,%11,%12,%13,%14,%15}, [%16];"
-        : "=r"(r[0]), "=r"(r[1]), "=r"(r[2]), "=r"(r[3]), "=r"(r[4]), "=r"(r[5]), "=r"(r[6]), "=r"(r[7]),
-          "=r"(r[8]), "=r"(r[9]), "=r"(r[10]), "=r"(r[11]), "=r"(r[12]), "=r"(r[13]), "=r"(r[14]), "=r"(r[15])
-        : "r"(taddr)
-        : "memory");
-}
-// Waits for this thread's TMEM loads; the registers are operands so no use
-// of them can be scheduled before the wait.
-SLM_DEV void tmem_wait_ld16(uint32_t (&r)[16]) {
-    asm volatile("tcgen05.wait::ld.sync.aligned;"
-                 : "+r"(r[0]), "+r"(r[1]), "+r"(r[2]), "+r"(r[3]), "+r"(r[4]), "+r"(r[5]), "+r"(r[6]),
-                   "+r"(r[7]), "+r"(r[8]), "+r"(r[9]), "+r"(r[10]), "+r"(r[11]), "+r"(r[12]), "+r"(r[13]),
-                   "+r"(r[14]), "+r"(r[15])
-                 :
-                 : "memory");
-}
 
 // Column-window counts of 4 consecutive columns (16-byte aligned): adds 1.0
 // to each column whose x <= 0 (not for NaN) with one vector reduction, issued
@@ -139,18 +54,6 @@ SLM_DEV void red_add4_le0(float *p, float x0, float x1, float x2, float x3, bool
         "@q red.relaxed.gpu.global.add.v4.f32 [%0], {a, b, c, d};\n"
         "}\n" ::"l"(p),
         "f"(x0), "f"(x1), "f"(x2), "f"(x3), "r"((uint32_t)pred)
-        : "memory");
-}
-
-// st.global.v2 of (a, b) when pred holds, without a branch.
-SLM_DEV void st_pair_if(uint2 *p, uint32_t a, uint32_t b, bool pred) {
-    asm volatile(
-        "{\n"
-        ".reg .pred q;\n"
-        "setp.ne.u32 q, %3, 0;\n"
-        "@q st.global.v2.u32 [%0], {%1, %2};\n"
-        "}\n" ::"l"(p),
-        "r"(a), "r"(b), "r"((uint32_t)pred)
         : "memory");
 }
 
@@ -180,29 +83,6 @@ SLM_DEV float min16q(const float (&d)[16], float (&g4)[4]) {
 #pragma unroll
     for (int q = 0; q < 4; ++q) g4[q] = min3f(d[4 * q], d[4 * q + 1], fminf(d[4 * q + 2], d[4 * q + 3]));
     return min3f(g4[0], g4[1], fminf(g4[2], g4[3]));
-}
-
-// Exact reference distance (matching.rs:146-155): lane k = components 8c+k.
-SLM_DEV float sq_dist_spec(const float *__restrict__ p, const float *__restrict__ r) {
-    float acc[8] = {0.f, 0.f, 0.f, 0.f, 0.f, 0.f, 0.f, 0.f};
-    const float4 *p4 = reinterpret_cast<const float4 *>(p);
-    const float4 *r4 = reinterpret_cast<const float4 *>(r);
-#pragma unroll 4
-    for (int c = 0; c < 16; ++c) {
-        const float4 x0 = p4[2 * c], x1 = p4[2 * c + 1];
-        const float4 y0 = r4[2 * c], y1 = r4[2 * c + 1];
-        const float xs[8] = {x0.x, x0.y, x0.z, x0.w, x1.x, x1.y, x1.z, x1.w};
-        const float ys[8] = {y0.x, y0.y, y0.z, y0.w, y1.x, y1.y, y1.z, y1.w};
-#pragma unroll
-        for (int k = 0; k < 8; ++k) {
-            const float t = __fsub_rn(xs[k], ys[k]);
-            acc[k] = __fadd_rn(acc[k], __fmul_rn(t, t));
-        }
-    }
-    float s = 0.f;
-#pragma unroll
-    for (int k = 0; k < 8; ++k) s = __fadd_rn(s, acc[k]);
-    return s;
 }
 
 // ------------------------------------------------------------ store packing
@@ -293,21 +173,19 @@ __global__ void __launch_bounds__(128) pack_lowp_kernel(const uint4 *__restrict_
         }
     }
     if constexpr (!FP8) {
-        // norm extension (slm_shortlist.h): |a|^2 / 2 = hi + lo (the difference
+        // norm extension (slm_shortlist.h): |a|^2 / 4 = hi + lo (the difference
         // of a float and its bf16 rounding is exact in f32). Padding rows get
         // hi = NaN: every product with a padding row or column is NaN, which
-        // min.f32 and redux.min ignore and no threshold admits, so the pass
-        // kernels need no masks for ragged tiles
-        const float half = valid ? 0.5f * nrm : 0.f;
-        const __nv_bfloat16 hi = __float2bfloat16_rn(half);
-        const __nv_bfloat16 lo = __float2bfloat16_rn(half - __bfloat162float(hi));
+        // the minima ignore, so the pass needs no masks for ragged tiles
+        const float quarter = valid ? 0.25f * nrm : 0.f;
+        const __nv_bfloat16 hi = __float2bfloat16_rn(quarter);
+        const __nv_bfloat16 lo = __float2bfloat16_rn(quarter - __bfloat162float(hi));
         const uint32_t hl = valid ? ((uint32_t)__bfloat16_as_ushort(hi) | ((uint32_t)__bfloat16_as_ushort(lo) << 16))
                                   : 0x00007fc0u;  // padding rows: hi = NaN, lo = 0
         const uint32_t ones = 0x3f803f80u;  // two bf16 1.0
-        uint8_t *ext = dst + kBf16TileBytes + (r >> 3) * 384 + (r & 7) * 16;
+        uint8_t *ext = dst + kBf16TileBytes + (r >> 3) * 256 + (r & 7) * 16;
         *reinterpret_cast<uint4 *>(ext) = make_uint4(hl, ones, 0u, 0u);        // kc0: hi lo 1 1
         *reinterpret_cast<uint4 *>(ext + 128) = make_uint4(ones, hl, 0u, 0u);  // kc1: 1 1 hi lo
-        *reinterpret_cast<uint4 *>(ext + 256) = make_uint4(0u, 0u, 0u, 0u);    // kc2
     }
     norms[row0 + row] = valid ? nrm : __int_as_float(0x7fc00000);  // FP8: NaN distances to padding rows too
     if constexpr (FP8) qscale[row0 + row] = inv;
@@ -342,48 +220,13 @@ void launch_pack_lowp(const uint4 *tab, uint32_t ntiles, const float *raw, int f
 
 // ------------------------------------------------------------ tcgen05 pieces
 
-// Shared-memory matrix descriptor (tcgen05): K-major, 128B swizzle, 8-row
-// groups 1024 bytes apart (stride byte offset), version 1, base offset 0.
-SLM_DEV uint64_t umma_desc(uint32_t saddr) {
-    uint64_t d = 0;
-    d |= (uint64_t)((saddr >> 4) & 0x3fffu);   // start address
-    d |= (uint64_t)1 << 16;                    // leading byte offset (unused for swizzled K-major)
-    d |= (uint64_t)(1024 >> 4) << 32;          // stride byte offset
-    d |= (uint64_t)1 << 46;                    // descriptor version
-    d |= (uint64_t)2 << 61;                    // SWIZZLE_128B
-    return d;
-}
-
-// Shared-memory matrix descriptor: K-major without swizzle. Core matrices of
-// 8 rows x 16 bytes (rows 16 bytes apart); lbo = bytes between core matrices
-// along K, sbo = bytes between 8-row groups.
-SLM_DEV uint64_t umma_desc_plain(uint32_t saddr, uint32_t lbo, uint32_t sbo) {
-    uint64_t d = 0;
-    d |= (uint64_t)((saddr >> 4) & 0x3fffu);
-    d |= (uint64_t)((lbo >> 4) & 0x3fffu) << 16;
-    d |= (uint64_t)((sbo >> 4) & 0x3fffu) << 32;
-    d |= (uint64_t)1 << 46;  // descriptor version; layout type 0 = no swizzle
-    return d;
-}
-
-// Instruction descriptor: f32 accumulate, K-major A and B, M=128, N=128.
-// kind::f16 with bf16 inputs (format 1) or kind::f8f6f4 with e4m3 (format 0);
-// negate_b (bit 14) negates operand B.
-__host__ __device__ constexpr uint32_t umma_idesc(bool fp8, bool negate_b = false) {
-    return (1u << 4) | ((fp8 ? 0u : 1u) << 7) | ((fp8 ? 0u : 1u) << 10) | ((negate_b ? 1u : 0u) << 14) |
-           ((128u >> 3) << 17) | ((128u >> 4) << 24);
-}
-
-template <bool FP8>
 struct SlSmem {
-    static constexpr uint32_t kOp = FP8 ? kFp8TileBytes : kBf16TileStride;  // bytes per operand tile
-    static constexpr int kStages = FP8 ? kSlStages : 3;                      // b-tile ring depth
-    uint8_t A[2][kOp];
-    uint8_t B[kStages][kOp];
-    float bnorm[kStages][128];  // FP8 only (BF16 carries the norms in the operands)
-    float bthr[kStages][128];
-    float bthr2[kStages][128];  // pass 2, items of two pairs: the second pair's column thresholds
-    float bscale[kStages][128];
+    uint8_t A[2][kFp8TileBytes];
+    uint8_t B[kSlStages][kFp8TileBytes];
+    float bnorm[kSlStages][128];
+    float bthr[kSlStages][128];
+    float bthr2[kSlStages][128];  // pass 2, items of two pairs: the second pair's column thresholds
+    float bscale[kSlStages][128];
     float anorm[256];
     float athr[256];
     float ascale[256];
@@ -391,45 +234,22 @@ struct SlSmem {
     float2 rowx[256];          // pass 1: the second column half's row state
     uint32_t rownear[256];     // pass 1: the second column half's near-chunk count
     uint64_t a_full, a_empty;
-    uint64_t b_full[kStages], b_empty[kStages];
+    uint64_t b_full[kSlStages], b_empty[kSlStages];
     uint64_t t_full[2], t_empty[2];
     uint64_t ep_bar;  // epilogue warps: column partials of a tile are stored
     uint32_t tmem_base;
     uint32_t abort_flag;
 };
-
-template <bool FP8>
-constexpr size_t sl_smem_bytes() {
-    return sizeof(SlSmem<FP8>) + 1024;  // slack for 1024-byte alignment
-}
-
-// Bounded wait (about 2 s of wall time); on timeout raises the CTA abort flag
-// and records an error so every role leaves its loop.
-SLM_DEV bool sl_wait(uint64_t *bar, uint32_t parity, volatile uint32_t *abort_flag, uint32_t *err) {
-    uint64_t t0 = 0;
-    for (uint32_t it = 0;; ++it) {
-        if (mbar_try_wait(bar, parity)) return true;
-        if ((it & 63) == 63) {
-            if (*abort_flag) return false;
-            const uint64_t now = globaltimer();
-            if (t0 == 0) t0 = now;
-            else if (now - t0 > 2000000000ull) {
-                *abort_flag = 1;
-                atomicCAS(err, 0u, (uint32_t)DERR_TIMEOUT_MMA);
-                return false;
-            }
-        }
-    }
-}
+constexpr size_t kSlSmemBytes = sizeof(SlSmem) + 1024;  // slack for 1024-byte alignment
 
 // Items of two pairs (odd row-tile counts sharing a b view).
 SLM_DEV bool item_two_pairs(const SlItem &it) { return it.nat == 2 && it.pair[1] != it.pair[0]; }
 
-// Whether a pass works on a pair: tier 0's pass 1 on every pair, otherwise
-// the pairs of the tier (sl_pair_on).
+// Whether a pass works on a pair: pass 1 on every pair, pass 2 on those
+// neither routed nor rescued after it.
 template <int PASS>
 SLM_DEV bool pass_pair_on(const SlArgs &g, const SlPair &sp) {
-    return (PASS == 1 && !g.tier) || sl_pair_on(g, sp);
+    return PASS == 1 || sl_pair_on(g, sp);
 }
 // A pass skips an item when none of its pairs is on (all roles read the same
 // flags: earlier kernels wrote them).
@@ -445,27 +265,23 @@ constexpr int kSlWarpsPerQuarter = (kSlThreads / 32 + 3) / 4;
 constexpr int kSlMaxRegs = (16384 / (32 * kSlWarpsPerQuarter)) & ~7;
 static_assert(kSlMaxRegs == 96, "register budget of the 18-warp pass kernel");
 
-template <int PASS, bool FP8, bool DUMP>
+template <int PASS, bool DUMP>
 __global__ void __maxnreg__(kSlMaxRegs) sl_pass_kernel(SlArgs g) {
     extern __shared__ uint8_t sl_smem_raw[];
     const uint32_t pad = (1024u - (smem_u32(sl_smem_raw) & 1023u)) & 1023u;
-    SlSmem<FP8> &S = *reinterpret_cast<SlSmem<FP8> *>(sl_smem_raw + pad);
-    constexpr uint32_t kOp = SlSmem<FP8>::kOp;
-    constexpr int kStg = SlSmem<FP8>::kStages;
+    SlSmem &S = *reinterpret_cast<SlSmem *>(sl_smem_raw + pad);
+    constexpr uint32_t kOp = kFp8TileBytes;
+    constexpr int kStg = kSlStages;
     const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
     uint32_t *err = g.ctl + 1;
     volatile uint32_t *abort_flag = &S.abort_flag;
-    // the epilogue reads the b stage in pass 2 (thresholds) and for FP8 (norms, scales)
-    constexpr bool kEpReadsB = PASS == 2 || FP8;
 
     if (threadIdx.x == 0) {
         mbar_init(&S.a_full, 1);
         mbar_init(&S.a_empty, 1 + kSlEpWarps);
         for (int s = 0; s < kStg; ++s) {
             mbar_init(&S.b_full[s], 1);
-            // BF16 pass 1's epilogue reads nothing of the b stage (norms are in the
-            // product): the MMA's commit alone frees it, one use earlier
-            mbar_init(&S.b_empty[s], kEpReadsB ? 1 + kSlEpWarps : 1);
+            mbar_init(&S.b_empty[s], 1 + kSlEpWarps);
         }
         for (int b = 0; b < 2; ++b) {
             mbar_init(&S.t_full[b], 1);
@@ -498,7 +314,7 @@ __global__ void __maxnreg__(kSlMaxRegs) sl_pass_kernel(SlArgs g) {
                 const uint32_t cbase1 = two ? g.spairs[item.pair[1]].cbase : 0;
                 uint32_t bytes = item.nat * kOp;
                 if (PASS == 2) bytes += item.nat * 512;
-                if (FP8) bytes += item.nat * 1024;  // norms and scales
+                bytes += item.nat * 1024;  // norms and scales
                 mbar_arrive_expect_tx(&S.a_full, bytes);
 #pragma unroll
                 for (uint32_t a = 0; a < 2; ++a) {  // static indices keep the item in registers
@@ -506,23 +322,23 @@ __global__ void __maxnreg__(kSlMaxRegs) sl_pass_kernel(SlArgs g) {
                     const uint32_t pa = item.pair[a];
                     const uint32_t arow = g.pairs[pa].a_row0 + item.rt[a] * kTile;  // store row of the tile
                     bulk_g2s(S.A[a], g.optiles + (size_t)(arow / kTile) * kOp, kOp, &S.a_full);
-                    if (FP8) bulk_g2s(&S.anorm[a * 128], g.norms + arow, 512, &S.a_full);
+                    bulk_g2s(&S.anorm[a * 128], g.norms + arow, 512, &S.a_full);
                     if (PASS == 2)
                         bulk_g2s(&S.athr[a * 128], g.rowthr + g.spairs[pa].rbase + item.rt[a] * kTile, 512, &S.a_full);
-                    if (FP8) bulk_g2s(&S.ascale[a * 128], g.qscale + arow, 512, &S.a_full);
+                    bulk_g2s(&S.ascale[a * 128], g.qscale + arow, 512, &S.a_full);
                 }
                 for (uint32_t t = item.ct0; t < item.ct1; ++t) {
                     if (!sl_wait(&S.b_empty[st], sph ^ 1, abort_flag, err)) break;
                     const uint32_t brow = pm.b_row0 + t * kTile;
-                    uint32_t bb = kOp + (PASS == 2 ? (two ? 1024 : 512) : 0) + (FP8 ? 1024 : 0);
+                    uint32_t bb = kOp + (PASS == 2 ? (two ? 1024 : 512) : 0) + 1024;
                     mbar_arrive_expect_tx(&S.b_full[st], bb);
                     bulk_g2s(S.B[st], g.optiles + (size_t)(brow / kTile) * kOp, kOp, &S.b_full[st]);
-                    if (FP8) bulk_g2s(S.bnorm[st], g.norms + brow, 512, &S.b_full[st]);
+                    bulk_g2s(S.bnorm[st], g.norms + brow, 512, &S.b_full[st]);
                     if (PASS == 2) {
                         bulk_g2s(S.bthr[st], g.colthr + cbase0 + t * kTile, 512, &S.b_full[st]);
                         if (two) bulk_g2s(S.bthr2[st], g.colthr + cbase1 + t * kTile, 512, &S.b_full[st]);
                     }
-                    if (FP8) bulk_g2s(S.bscale[st], g.qscale + brow, 512, &S.b_full[st]);
+                    bulk_g2s(S.bscale[st], g.qscale + brow, 512, &S.b_full[st]);
                     if (++st == kStg) st = 0, sph ^= 1;
                 }
                 ++iter;
@@ -531,16 +347,13 @@ __global__ void __maxnreg__(kSlMaxRegs) sl_pass_kernel(SlArgs g) {
         }
     } else if (warp == 1) {
         // ---------------------------------------------------------- MMA issue
-        constexpr uint32_t idesc = umma_idesc(FP8);
-        constexpr uint32_t idesc_neg = umma_idesc(FP8, true);
+        constexpr uint32_t idesc = fp8_idesc();
         // Every operand tile has a fixed shared-memory address for the whole
         // kernel: the descriptors are made once, and a tile, stage or K step
         // adds its byte offset / 16 to the 14-bit start-address field (all
         // shared addresses lie below 256 KiB, so the field never carries).
         constexpr uint32_t kOp16 = kOp >> 4;
         const uint64_t adesc0 = umma_desc(smem_u32(S.A[0])), bdesc0 = umma_desc(smem_u32(S.B[0]));
-        const uint64_t aext0 = umma_desc_plain(smem_u32(S.A[0]) + kBf16TileBytes, 128, 384);
-        const uint64_t bext0 = umma_desc_plain(smem_u32(S.B[0]) + kBf16TileBytes + 128, 128, 384);
         uint32_t st = 0, sph = 0, tb = 0, tph = 0, iter = 0;
         for (uint32_t it = blockIdx.x; it < g.n_items; it += gridDim.x) {
             const SlItem item = g.items[it];
@@ -561,19 +374,9 @@ __global__ void __maxnreg__(kSlMaxRegs) sl_pass_kernel(SlArgs g) {
                         if (a >= item.nat) break;
                         const uint32_t d_tmem = tmem + (tb * 2 + a) * 128;
                         const uint64_t ad = adesc0 + (uint64_t)(a * kOp16);
-                        if constexpr (FP8) {
 #pragma unroll
-                            for (int k = 0; k < 4; ++k)  // K = 32 e4m3 = 32 bytes per step
-                                mma_f8(d_tmem, ad + 2 * k, bd + 2 * k, idesc, k > 0);
-                        } else {
-#pragma unroll
-                            for (int k = 0; k < 8; ++k) {  // K = 16 bf16 = 32 bytes per step; -a.b
-                                const uint32_t off16 = (k >> 2) * (16384 >> 4) + (k & 3) * 2;
-                                mma_f16(d_tmem, ad + off16, bd + off16, idesc_neg, k > 0);
-                            }
-                            // + (|a|^2 + |b|^2) / 2: A from kc0, B from kc1 of the norm extension
-                            mma_f16(d_tmem, aext0 + (uint64_t)(a * kOp16), bext0 + (uint64_t)(st * kOp16), idesc, true);
-                        }
+                        for (int k = 0; k < 4; ++k)  // K = 32 e4m3 = 32 bytes per step
+                            mma_f8(d_tmem, ad + 2 * k, bd + 2 * k, idesc, k > 0);
                     }
                     mma_commit(&S.b_empty[st]);
                     mma_commit(&S.t_full[tb]);
@@ -602,10 +405,6 @@ __global__ void __maxnreg__(kSlMaxRegs) sl_pass_kernel(SlArgs g) {
         const uint32_t lane_addr = (uint32_t)(q * 32) << 16;
         uint32_t st = 0, sph = 0, tb = 0, tph = 0, iter = 0, eph = 0;
         const float kInf = __int_as_float(0x7f800000);
-        // BF16 accumulators hold d~ / 2 (norms folded into the product): the
-        // epilogue compares in that domain and scales by 2 (exact) where values
-        // leave the kernel; FP8 computes d~ itself
-        constexpr float kDom = FP8 ? 1.f : 2.f;
         for (uint32_t it = blockIdx.x; it < g.n_items; it += gridDim.x) {
             const SlItem item = g.items[it];
             if (item_off<PASS>(g, item)) continue;
@@ -633,9 +432,9 @@ __global__ void __maxnreg__(kSlMaxRegs) sl_pass_kernel(SlArgs g) {
             const bool qvalid = active && rt * kTile + q * 32 < pm.na;
             const uint32_t i = rt * kTile + q * 32 + lane;    // row within the pair
             const bool rvalid = active && i < pm.na;
-            const float na_i = (FP8 && active) ? S.anorm[r] : 0.f;
-            const float thr_i = (PASS == 2 && active) ? S.athr[r] * (1.f / kDom) : -kInf;
-            const float sa_i = (FP8 && active) ? S.ascale[r] : 1.f;
+            const float na_i = active ? S.anorm[r] : 0.f;
+            const float thr_i = (PASS == 2 && active) ? S.athr[r] : -kInf;
+            const float sa_i = active ? S.ascale[r] : 1.f;
             __syncwarp();
             if (lane == 0) mbar_arrive(&S.a_empty);
             float m1 = kInf, m2 = kInf;
@@ -652,12 +451,7 @@ __global__ void __maxnreg__(kSlMaxRegs) sl_pass_kernel(SlArgs g) {
             uint32_t ncand = 0;
             bool ok = true;
             for (uint32_t t = item.ct0; t < item.ct1; ++t) {
-                // without the epilogue's b_empty arrivals the producer may refill a
-                // stage twice before this warp would wait on it (its parity would be
-                // ambiguous): an epilogue that does not read the stage waits on t_full
-                // only, which implies the MMA consumed the stage
-                if ((kEpReadsB && !sl_wait(&S.b_full[st], sph, abort_flag, err)) ||
-                    !sl_wait(&S.t_full[tb], tph, abort_flag, err)) {
+                if (!sl_wait(&S.b_full[st], sph, abort_flag, err) || !sl_wait(&S.t_full[tb], tph, abort_flag, err)) {
                     ok = false;
                     break;
                 }
@@ -670,32 +464,25 @@ __global__ void __maxnreg__(kSlMaxRegs) sl_pass_kernel(SlArgs g) {
                         const uint32_t cb = h * 64 + c * 16;   // column within the tile
                         const uint32_t j0 = t * kTile + cb;    // column within the pair
                         float d[16];
-                        if constexpr (FP8) {
-                            const float4 *bn4 = reinterpret_cast<const float4 *>(&S.bnorm[st][cb]);
-                            const float4 *bs4 = reinterpret_cast<const float4 *>(&S.bscale[st][cb]);
-                            const float m2sa = -2.f * sa_i;
+                        const float4 *bn4 = reinterpret_cast<const float4 *>(&S.bnorm[st][cb]);
+                        const float4 *bs4 = reinterpret_cast<const float4 *>(&S.bscale[st][cb]);
+                        const float m2sa = -2.f * sa_i;
 #pragma unroll
-                            for (int k4 = 0; k4 < 4; ++k4) {
-                                const float4 nb = bn4[k4], sb = bs4[k4];
-                                const float nbv[4] = {nb.x, nb.y, nb.z, nb.w}, sbv[4] = {sb.x, sb.y, sb.z, sb.w};
+                        for (int k4 = 0; k4 < 4; ++k4) {
+                            const float4 nb = bn4[k4], sb = bs4[k4];
+                            const float nbv[4] = {nb.x, nb.y, nb.z, nb.w}, sbv[4] = {sb.x, sb.y, sb.z, sb.w};
 #pragma unroll
-                                for (int e = 0; e < 4; ++e)
-                                    d[4 * k4 + e] = fmaf(__uint_as_float(vc[4 * k4 + e]), m2sa * sbv[e], na_i + nbv[e]);
-                            }
-                        } else {
-#pragma unroll
-                            for (int k = 0; k < 16; ++k) d[k] = __uint_as_float(vc[k]);  // d~ / 2
+                            for (int e = 0; e < 4; ++e)
+                                d[4 * k4 + e] = fmaf(__uint_as_float(vc[4 * k4 + e]), m2sa * sbv[e], na_i + nbv[e]);
                         }
                         if constexpr (PASS == 1) {
                             if (DUMP && pid == 0 && rvalid) {
 #pragma unroll
                                 for (int k = 0; k < 16; ++k)
-                                    if (j0 + k < pm.nb) g.dump[(size_t)i * pm.nb + j0 + k] = kDom * d[k];
+                                    if (j0 + k < pm.nb) g.dump[(size_t)i * pm.nb + j0 + k] = d[k];
                             }
                             const float cm = min16(d);
-                            // FP8 only: the bf16 bound is too tight for rows to go wide
-                            // (the overflow count after pass 2 still routes such pairs)
-                            if constexpr (FP8) near += (cm >= m1 && cm <= m1 + w2) ? 1u : 0u;
+                            near += (cm >= m1 && cm <= m1 + w2) ? 1u : 0u;
                             m2 = fminf(m2, fmaxf(m1, cm));
                             m1 = fminf(m1, cm);
 
@@ -713,19 +500,13 @@ __global__ void __maxnreg__(kSlMaxRegs) sl_pass_kernel(SlArgs g) {
                             // both tests' group minima first (independent chains), then
                             // the rare bodies. Row candidates: d~ <= T (rows certain to
                             // have no match carry T = -inf); column window: d~ <= c1 + 2 eps,
-                            // x = d - thr in the accumulator domain (the sign is exact)
+                            // x = d - thr (the sign is exact)
                             float x[16];
 #pragma unroll
                             for (int k4 = 0; k4 < 4; ++k4) {
                                 u64x x0, x1;
-                                if constexpr (FP8) {
-                                    x0 = f2_sub(f2_pack(d[4 * k4], d[4 * k4 + 1]), tt[k4].x);
-                                    x1 = f2_sub(f2_pack(d[4 * k4 + 2], d[4 * k4 + 3]), tt[k4].y);
-                                } else {
-                                    const u64x mhalf = f2_pack(-0.5f, -0.5f);
-                                    x0 = f2_fma(tt[k4].x, mhalf, f2_pack(d[4 * k4], d[4 * k4 + 1]));
-                                    x1 = f2_fma(tt[k4].y, mhalf, f2_pack(d[4 * k4 + 2], d[4 * k4 + 3]));
-                                }
+                                x0 = f2_sub(f2_pack(d[4 * k4], d[4 * k4 + 1]), tt[k4].x);
+                                x1 = f2_sub(f2_pack(d[4 * k4 + 2], d[4 * k4 + 3]), tt[k4].y);
                                 x[4 * k4 + 0] = f2_lo(x0);
                                 x[4 * k4 + 1] = f2_hi(x0);
                                 x[4 * k4 + 2] = f2_lo(x1);
@@ -735,7 +516,7 @@ __global__ void __maxnreg__(kSlMaxRegs) sl_pass_kernel(SlArgs g) {
                             const float cm = min16q(d, gr);
                             const float xm = rvalid ? min16q(x, gc) : kInf;
                             if (cm <= thr_i) {
-                                // a hit group: one record of its 4 values (accumulator domain)
+                                // a hit group: one record of its 4 values
 #pragma unroll
                                 for (int qq = 0; qq < 4; ++qq) {
                                     if (gr[qq] <= thr_i) {
@@ -813,11 +594,11 @@ __global__ void __maxnreg__(kSlMaxRegs) sl_pass_kernel(SlArgs g) {
                         }
                         const uint32_t j = t * kTile + col;
                         if (j < pm.nb && m < kInf && (grp ? on1 : on0))
-                            atomicMin(&g.colmin[(grp ? cb1 : cb0) + j], f2ord(kDom * m));
+                            atomicMin(&g.colmin[(grp ? cb1 : cb0) + j], f2ord(m));
                     }
                 }
                 __syncwarp();
-                if (kEpReadsB && lane == 0) mbar_arrive(&S.b_empty[st]);
+                if (lane == 0) mbar_arrive(&S.b_empty[st]);
                 if (++st == kStg) st = 0, sph ^= 1;
                 tb ^= 1;
                 if (tb == 0) tph ^= 1;
@@ -839,7 +620,7 @@ __global__ void __maxnreg__(kSlMaxRegs) sl_pass_kernel(SlArgs g) {
                     m1 = fminf(m1, o.x);
                     // slot = row within its 256-row group (items of one 128-row tile start mid-group)
                     const size_t slot = (size_t)mypart * 256 + (i & 255u);
-                    g.rowpart[slot] = make_float2(kDom * m1, kDom * m2);
+                    g.rowpart[slot] = make_float2(m1, m2);
                     g.rownear[slot] = near + S.rownear[r];
                 }
             } else {
@@ -866,28 +647,6 @@ __global__ void __maxnreg__(kSlMaxRegs) sl_pass_kernel(SlArgs g) {
 // Per pair, before pass 1: the error bound eps from the two views'
 // statistics. A pair with non-finite or huge inputs cannot be certified and is
 // routed to the exact kernel.
-// The per-pair error bound of this launch's precision (g.fp8) from the two
-// views' statistics; false when the pair cannot be certified (non-finite or
-// huge inputs).
-SLM_DEV bool pair_eps(const SlArgs &g, const SlPair &sp, float *eps_out) {
-    const ViewStat va = g.vstats[sp.view_a], vb = g.vstats[sp.view_b];
-    const double A = __uint_as_float(va.nmax), B = __uint_as_float(vb.nmax);
-    const double Ra = __uint_as_float(va.rho), Rb = __uint_as_float(vb.rho);
-    const double Qa = __uint_as_float(va.nqmax), Qb = __uint_as_float(vb.nqmax);
-    bool unsafe = va.bad || vb.bad || !(A <= 64.0) || !(B <= 64.0);
-    // |d~ - d| <= 2 |a.b - q(a).q(b)| + accumulation and rounding terms, with
-    // |a.b - q(a).q(b)| <= |a - q(a)| |b| + |q(a)| |b - q(b)| (Cauchy-Schwarz).
-    double eps = 2.0 * (Ra * B + Qa * Rb) * (1.0 + 1e-3);
-    eps += 5e-4 * Qa * Qb + 5e-5 * (A * A + B * B) + 2e-5 * (A + B) * (A + B) + 1e-6;
-    // BF16: the tensor core also accumulates the folded norms (|a|^2 + |b|^2) / 2
-    // and their bf16 split (relative 2^-17); the accumulation is taken as no
-    // better than 2^-11 relative to that magnitude, doubled with d~
-    if (!g.fp8) eps += 5e-4 * (A * A + B * B);
-    if (!(eps < 1e30)) unsafe = true;
-    *eps_out = unsafe ? __int_as_float(0x7f800000) : (float)(eps * (1.0 + 1e-6));
-    return !unsafe;
-}
-
 __global__ void __launch_bounds__(256) sl_eps_kernel(SlArgs g) {
     const uint32_t p = blockIdx.x * blockDim.x + threadIdx.x;
     if (p >= g.npairs) return;
@@ -902,66 +661,26 @@ __global__ void __launch_bounds__(256) sl_eps_kernel(SlArgs g) {
     if (sp.routed) atomicAdd(&g.ctl[kCtlRouteMarks], 1u);
 }
 
-// Tier 1 (the BF16 rescue of an FP8 plan), one CTA per pair and block of
-// kSlRowBlock columns: for each rescued pair, the BF16 bound (block 0), its
-// column minima back to +inf and its per-pair counters back to 0 (tier 0's
-// pass 1 and mid wrote them; its pass 2 skipped the pair, so the records and
-// window counts are still clear).
+// Tier 1 (the BF16 rescue of an FP8 plan), one thread per pair: for each
+// rescued pair, the BF16 bound and its counters back to 0 (tier 0's mid wrote
+// them).
 __global__ void __launch_bounds__(256) sl_rescue_prep_kernel(SlArgs g) {
-    const uint32_t p = blockIdx.x, blk = blockIdx.y;
-    const PairMeta pm = g.pairs[p];
+    const uint32_t p = blockIdx.x * blockDim.x + threadIdx.x;
+    if (p >= g.npairs) return;
     const SlPair sp = g.spairs[p];
-    if (!sl_pair_on(g, sp)) return;  // block-uniform
-    const uint32_t nb_pad = (pm.nb + kTile - 1) / kTile * kTile;
-    const uint32_t c0 = blk * kSlRowBlock, c1 = min(c0 + kSlRowBlock, nb_pad);
-    for (uint32_t j = c0 + threadIdx.x; j < c1; j += blockDim.x) g.colmin[sp.cbase + j] = 0xff800000u;  // +inf
-    if (blk == 0 && threadIdx.x < 4) g.pairctl[4 * (size_t)p + threadIdx.x] = 0;
-    if (blk == 0 && threadIdx.x == 0) {
-        float eps;
-        if (!pair_eps(g, sp, &eps)) {  // cannot happen after tier 0 (unsafe pairs are routed there)
-            g.spairs[p].routed = 1;
-            atomicAdd(&g.ctl[kCtlRouteMarks], 1u);
-        }
-        g.spairs[p].eps = eps;
-        atomicAdd(&g.ctl[kCtlRescuedPairs], 1u);
-        atomicAdd(&g.ctl[kCtlRescuedRows], pm.na);
+    if (!sl_pair_on(g, sp)) return;
+    for (int k = 0; k < 4; ++k) g.pairctl[4 * (size_t)p + k] = 0;
+    float eps;
+    if (!pair_eps(g, sp, &eps)) {  // cannot happen after tier 0 (unsafe pairs are routed there)
+        g.spairs[p].routed = 1;
+        atomicAdd(&g.ctl[kCtlRouteMarks], 1u);
     }
-}
-
-// ------------------------------------------------------- certified tests
-
-// The decisions below are proved in f32 with directed rounding: each side of
-// a comparison is rounded toward the weaker claim, so a true comparison of the
-// rounded values implies it for the real numbers. The factors cover the
-// reference's own rounding of (r*r)*d2 (at most 2^-24 relative).
-constexpr float kUp = 1.000001f;    // > 1 + 2^-24
-constexpr float kDown = 0.999999f;  // < 1 - 2^-24
-
-// No match for the row: d1 >= m1 - eps >= r^2 (m2 + eps) kUp >= fl(r^2 d2),
-// where m1 - eps bounds d1 from below and m2 + eps bounds d2 from above.
-SLM_DEV bool certain_no_match(float m1, float m2, float eps, float r2) {
-    return __fsub_rd(m1, eps) >= __fmul_ru(__fmul_ru(r2, __fadd_ru(m2, eps)), kUp);
-}
-
-// The ratio test passes: d1 <= a1 + eps < r^2 (a2 - eps) kDown <= fl(r^2 d2).
-SLM_DEV bool certain_ratio_pass(float a1, float a2, float eps, float r2) {
-    return __fadd_ru(a1, eps) < __fmul_rd(__fmul_rd(r2, __fsub_rd(a2, eps)), kDown);
-}
-
-// Window x + 2 eps, rounded up (a larger threshold only admits more); NaN
-// becomes +inf (admit everything).
-SLM_DEV float window_up(float x, float eps) {
-    const float t = __fmul_ru(__fadd_ru(x, 2.f * eps), kUp);
-    return t == t ? t : __int_as_float(0x7f800000);
+    g.spairs[p].eps = eps;
+    atomicAdd(&g.ctl[kCtlRescuedPairs], 1u);
+    atomicAdd(&g.ctl[kCtlRescuedRows], g.pairs[p].na);
 }
 
 // ------------------------------------------------------------------ mid
-
-// Row blocks of a pair: enough for its rows and its columns.
-SLM_DEV uint32_t pair_blocks(const PairMeta &pm) {
-    const uint32_t n = max(pm.na, pm.nb);
-    return max(1u, (n + kSlRowBlock - 1) / kSlRowBlock);
-}
 
 // One CTA per pair and block of kSlRowBlock rows and columns: row thresholds
 // from the pass-1 partials, column thresholds from the column minima, and the
@@ -1061,40 +780,14 @@ __global__ void __launch_bounds__(kThreads) sl_mid_kernel(SlArgs g) {
         const uint32_t w = atomicAdd(const_cast<uint32_t *>(&pc[kPcWide]), 0u);
         const uint32_t o = atomicAdd(const_cast<uint32_t *>(&pc[kPcOpen]), 0u);
         // more than 1/8 of the undecided rows are expected to overflow their
-        // shortlist: settle the whole pair with the BF16 passes (tier 0 of an
-        // FP8 plan) or with the exact kernel
+        // shortlist: settle the whole pair with the BF16 pass
         if (w * 8 > o && o) {
-            if (g.rescue) {
-                g.spairs[p].rescued = 1;
-            } else {
-                g.spairs[p].routed = 1;
-                atomicAdd(&g.ctl[kCtlRouteMarks], 1u);
-            }
+            g.spairs[p].rescued = 1;
         }
     }
 }
 
 // ------------------------------------------------------------- finalize
-
-SLM_DEV void sl_push(SlQueue *q, uint32_t *len, uint32_t cap, uint32_t *err, uint32_t pair, uint32_t kind, uint32_t i,
-                     uint32_t j) {
-    const uint32_t s = atomicAdd(len, 1u);
-    if (s < cap) {
-        SlQueue e;
-        e.pair = pair;
-        e.kind = kind;
-        e.i = i;
-        e.j = j;
-        q[s] = e;
-    } else {
-        atomicCAS(err, 0u, (uint32_t)DERR_BAD_ITEM);
-    }
-}
-
-SLM_DEV void push_scan(const SlArgs &g, uint32_t pair, uint32_t kind, uint32_t i, uint32_t j) {
-    sl_push(g.queue, &g.ctl[kCtlScanLen], g.queue_cap, g.ctl + 1, pair, kind, i, j);
-    atomicAdd(&g.ctl[kind == 0 ? kCtlQueueRows : kCtlQueueCols], 1u);
-}
 
 // Mutual check of a candidate (i, j) from the column window counts: a row
 // whose d~ lies above the window (c1 + 2 eps) is provably not the column's
@@ -1139,7 +832,6 @@ __global__ void __launch_bounds__(kThreads, 1) sl_finalize_kernel(SlArgs g) {
             // padding columns, are not in S); a half with more hit groups than
             // records overflowed and the row is scanned exactly instead
             const float T = g.rowthr[ridx];
-            const float dom = g.fp8 ? 1.f : 2.f;
             float a1 = kInf, a2 = kInf;
             uint32_t j1 = 0xffffffffu, n = 0;
             bool over = false;
@@ -1158,7 +850,7 @@ __global__ void __launch_bounds__(kThreads, 1) sl_finalize_kernel(SlArgs g) {
                     const float vs[8] = {v0.x, v0.y, v0.z, v0.w, v1.x, v1.y, v1.z, v1.w};
 #pragma unroll
                     for (int q = 0; q < 8; ++q) {
-                        const float v = dom * vs[q];
+                        const float v = vs[q];
                         const uint32_t j = (q < 4 ? jb0 : jb1) + (q & 3);
                         if (!(v <= T)) continue;
                         ++n;
@@ -1198,23 +890,6 @@ __global__ void __launch_bounds__(kThreads, 1) sl_finalize_kernel(SlArgs g) {
 
 // ------------------------------------------------------------- exact work
 
-// Exact distance by 8 lanes: lane k of the group accumulates components
-// 8c+k for c = 0..15 (matching.rs:146-155), then the lane sums are added in
-// order 0..7. p and r may differ per group; the result is valid in all 8 lanes.
-SLM_DEV float dist8(const float *__restrict__ p, const float *__restrict__ r) {
-    const uint32_t lane = threadIdx.x & 31, k = lane & 7, base = lane & ~7u;
-    float acc = 0.f;
-#pragma unroll
-    for (int c = 0; c < 16; ++c) {
-        const float t = __fsub_rn(p[8 * c + k], r[8 * c + k]);
-        acc = __fadd_rn(acc, __fmul_rn(t, t));
-    }
-    float s = 0.f;
-#pragma unroll
-    for (int q = 0; q < 8; ++q) s = __fadd_rn(s, __shfl_sync(0xffffffffu, acc, base + q));
-    return s;
-}
-
 // One warp per row of the rescore queue: exact distances of S (4 at a time),
 // the reference's row rule (matching.rs:182-187, 204-206), then the mutual
 // check from the column window counts.
@@ -1238,8 +913,6 @@ __global__ void __launch_bounds__(256) sl_rescore_kernel(SlArgs g) {
         // S = the records' columns with d~ <= T, four entries at a time: lane group
         // grp computes queued entry grp, every lane merges the results in order
         const float T = g.rowthr[ridx];
-        // records of FP8 pairs hold d~, those of BF16 (and rescued) pairs d~ / 2
-        const float dom = g.fp8 && !sp.rescued ? 1.f : 2.f;
         uint32_t qj = 0, nq = 0;  // this lane group's queued column (0: a valid placeholder)
         float qv = kInf;
         auto flush = [&](uint32_t cnt) {
@@ -1272,7 +945,7 @@ __global__ void __launch_bounds__(256) sl_rescore_kernel(SlArgs g) {
                 const float vs[4] = {v4.x, v4.y, v4.z, v4.w};
 #pragma unroll
                 for (uint32_t q = 0; q < 4; ++q) {
-                    const float v = dom * vs[q];
+                    const float v = vs[q];
                     if (!(v <= T)) continue;  // warp-uniform: every lane reads the same record
                     if (grp == nq) {
                         qj = jb + q;
@@ -1341,6 +1014,8 @@ __global__ void __launch_bounds__(256) sl_scan_kernel(SlArgs g) {
         const SlQueue qe = g.queue[e];
         const PairMeta pm = g.pairs[qe.pair];
         const SlPair sp = g.spairs[qe.pair];
+        if (sp.routed) continue;  // block-uniform: the exact kernel settled the whole pair
+        if (threadIdx.x == 0) atomicAdd(&g.ctl[qe.kind == 0 ? kCtlQueueRows : kCtlQueueCols], 1u);
         const float *A = g.raw + (size_t)pm.a_row0 * kDesc;
         const float *B = g.raw + (size_t)pm.b_row0 * kDesc;
         uint32_t dec = kDecNone, col = qe.j;
@@ -1640,14 +1315,10 @@ void launch_gather_blocks(const SlArgs &a, const uint64_t *slot_off, const uint6
 // ---------------------------------------------------------------- launch
 
 cudaError_t init_shortlist_kernels() {
-    const int sb = (int)sl_smem_bytes<false>(), s8 = (int)sl_smem_bytes<true>();
     const cudaFuncAttribute at = cudaFuncAttributeMaxDynamicSharedMemorySize;
-    cudaError_t e = cudaFuncSetAttribute(sl_pass_kernel<1, false, false>, at, sb);
-    if (e == cudaSuccess) e = cudaFuncSetAttribute(sl_pass_kernel<1, false, true>, at, sb);
-    if (e == cudaSuccess) e = cudaFuncSetAttribute(sl_pass_kernel<2, false, false>, at, sb);
-    if (e == cudaSuccess) e = cudaFuncSetAttribute(sl_pass_kernel<1, true, false>, at, s8);
-    if (e == cudaSuccess) e = cudaFuncSetAttribute(sl_pass_kernel<1, true, true>, at, s8);
-    if (e == cudaSuccess) e = cudaFuncSetAttribute(sl_pass_kernel<2, true, false>, at, s8);
+    cudaError_t e = cudaFuncSetAttribute(sl_pass_kernel<1, false>, at, (int)kSlSmemBytes);
+    if (e == cudaSuccess) e = cudaFuncSetAttribute(sl_pass_kernel<1, true>, at, (int)kSlSmemBytes);
+    if (e == cudaSuccess) e = cudaFuncSetAttribute(sl_pass_kernel<2, false>, at, (int)kSlSmemBytes);
     return e;
 }
 
@@ -1660,20 +1331,11 @@ int launch_shortlist_eps(const SlArgs &a, cudaStream_t s) {
 int launch_shortlist_pass(const SlArgs &a, int pass, int sms, cudaStream_t s) {
     const int grid = (int)(a.n_items < (uint32_t)sms ? a.n_items : (uint32_t)sms);
     if (!grid) return 0;
-    const size_t sb = sl_smem_bytes<false>(), s8 = sl_smem_bytes<true>();
-    if (pass == 1) {
-        if (a.fp8)
-            a.dump ? sl_pass_kernel<1, true, true><<<grid, kSlThreads, s8, s>>>(a)
-                   : sl_pass_kernel<1, true, false><<<grid, kSlThreads, s8, s>>>(a);
-        else
-            a.dump ? sl_pass_kernel<1, false, true><<<grid, kSlThreads, sb, s>>>(a)
-                   : sl_pass_kernel<1, false, false><<<grid, kSlThreads, sb, s>>>(a);
-    } else {
-        if (a.fp8)
-            sl_pass_kernel<2, true, false><<<grid, kSlThreads, s8, s>>>(a);
-        else
-            sl_pass_kernel<2, false, false><<<grid, kSlThreads, sb, s>>>(a);
-    }
+    if (pass == 1)
+        a.dump ? sl_pass_kernel<1, true><<<grid, kSlThreads, kSlSmemBytes, s>>>(a)
+               : sl_pass_kernel<1, false><<<grid, kSlThreads, kSlSmemBytes, s>>>(a);
+    else
+        sl_pass_kernel<2, false><<<grid, kSlThreads, kSlSmemBytes, s>>>(a);
     return 1;
 }
 
@@ -1698,7 +1360,7 @@ int launch_shortlist_finalize(const SlArgs &a, cudaStream_t s) {
 
 int launch_shortlist_rescue_prep(const SlArgs &a, cudaStream_t s) {
     if (!a.npairs) return 0;
-    sl_rescue_prep_kernel<<<dim3(a.npairs, a.row_blocks), 256, 0, s>>>(a);
+    sl_rescue_prep_kernel<<<(a.npairs + 255) / 256, 256, 0, s>>>(a);
     return 1;
 }
 
@@ -1728,10 +1390,10 @@ int launch_shortlist_tail(const SlArgs &a, int sms, cudaStream_t s) {
         launch_pack_routed(a.pairs, a.xlist, a.ctl + kCtlRoutedPairs, a.raw, const_cast<float *>(a.tiled), 2 * sms, s);
     launch_exact(x, sms, s);
     sl_route_finalize_kernel<<<dim3(rgrid, a.row_blocks), 256, 0, s>>>(a);
-    sl_rescore_kernel<<<5 * sms, 256, 0, s>>>(a);  // 40 warps per SM: latency-bound gathers
+    if (a.fp8) sl_rescore_kernel<<<5 * sms, 256, 0, s>>>(a);  // 40 warps per SM: latency-bound gathers
     sl_scan_kernel<<<2 * sms, 256, 0, s>>>(a);
     sl_compact_kernel<<<per_block, 256, 0, s>>>(a);
-    return a.fp8 ? 7 : 8;
+    return 7;
 }
 
 }  // namespace slm

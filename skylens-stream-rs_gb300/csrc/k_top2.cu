@@ -1,0 +1,664 @@
+// k_top2.cu — the BF16 shortlist: one tensor-core pass per direction that
+// leaves, for every row, its nearest column and its two smallest distance
+// estimates; then the decisions they certify, and the rows they do not.
+//
+// Reference: crates/core/src/matching.rs:144-215. ratio_match needs a row's two
+// smallest distances and its nearest column, and, for the cross-check, the
+// nearest row of that column. Pass (a, b) gives the first for every row of a,
+// pass (b, a) the second for every row of b; both are the same kernel.
+//
+// sl_top2_kernel (persistent, one CTA per SM, 18 warps):
+//   warp 0      TMA producer: 1 or 2 a tiles of 128 rows, kept while
+//               consecutive segments share them; b tiles two at a time (256
+//               columns, 72 KiB) through two stages.
+//   warp 1      one thread issues tcgen05.mma, M = 128, N = 256, K = 16: per a
+//               tile 8 steps over the components (B negated) and one over the
+//               norm extension, so the accumulator is d~ / 2. Two accumulators
+//               of 256 TMEM columns take turns.
+//   warps 2-17  epilogue: warp w reads TMEM lane quarter w % 4, every fourth
+//               16-column chunk, one thread per row.
+// What a row keeps, exactly, at 13 instructions per 16 columns:
+//   - the minimum of each chunk comes with the load (tcgen05.ld.red); running
+//     best, second best and best chunk of these minima;
+//   - the running minimum of each of the 16 column classes (column mod 16).
+//   The best column is (best chunk, best class). The second smallest distance
+//   lies in another chunk or, if in the same, in another class: it is the
+//   smaller of the second best chunk minimum and the second best class
+//   minimum. (Equal minima give a second best equal to the best, which
+//   certifies nothing, so their column does not matter.)
+//
+// Why this shape. N = 256: with N = 128 every MMA reads as many bytes of A as
+// of B from shared memory, 128 bytes per clock for 64 clocks of tensor work;
+// N = 256 reads 12 KiB per 128 clocks. A second pass in the other direction
+// costs one more run over the tensor cores, but rows only: minima over the 32
+// lanes of a warp (redux) for the column side took more issue slots than the
+// whole row epilogue does. The epilogue takes 29 clocks per 32 x 16 chunk and
+// sub-partition (measured alone; 43 with a min tree instead of ld.red) where
+// the MMA takes 72, so the tensor pipe is the bound: 1.73 ms for both
+// directions of a 240-view zone (3663 pairs, 2 x 4.87 G distances), 94 % of the
+// measured BF16 rate with the padding of ragged tiles counted. The two passes
+// before (N = 128; row and column minima, then the candidates of each row
+// recomputed against a threshold) took 1.33 and 1.64 ms, and the zone's batch
+// with its lists read back 3.50 ms; now 2.29.
+#include <cuda_runtime.h>
+
+#include <cstdint>
+
+#include "shortlist.cuh"
+
+namespace slm {
+
+namespace {
+
+constexpr uint32_t kKb = 16384;                              // one K block (64 components) of a 128-row tile
+constexpr uint32_t kStageBytes = 2 * kBf16TileStride;        // two b tiles, K block by K block
+constexpr uint32_t kStageExt = 4 * kKb;                      // their norm extensions, after the four K blocks
+constexpr int kTopStages = 2;
+static_assert(kStageExt + 2 * kBf16ExtBytes == kStageBytes, "stage layout");
+
+struct TopSmem {
+    uint8_t A[2][kBf16TileStride];
+    uint8_t B[kTopStages][kStageBytes];
+    float2 mm[2][3][128];  // [a tile][other column group][row]: (m1, m2) to merge
+    uint32_t mj[2][3][128];
+    uint64_t a_full, a_empty;
+    uint64_t b_full[kTopStages], b_empty[kTopStages];
+    uint64_t t_full[2], t_empty[2];
+    uint32_t tmem_base;
+    uint32_t abort_flag;
+};
+constexpr size_t kTopSmemBytes = sizeof(TopSmem) + 1024;  // slack for 1024-byte alignment
+static_assert(kTopSmemBytes <= 232448, "shared memory of one CTA");
+
+// 32 lanes x 16 TMEM columns and their minimum (asynchronous until the wait);
+// NaN columns are ignored unless all 16 are NaN.
+SLM_DEV void tmem_ld16_min(uint32_t taddr, uint32_t (&r)[16], uint32_t &mn) {
+    asm volatile(
+        "tcgen05.ld.red.sync.aligned.32x32b.x16.min.f32 "
+        "{%0,%1,%2,%3,%4,%5,%6,%7,%8,%9,%10,%11,%12,%13,%14,%15}, %16, [%17];"
+        : "=r"(r[0]), "=r"(r[1]), "=r"(r[2]), "=r"(r[3]), "=r"(r[4]), "=r"(r[5]), "=r"(r[6]), "=r"(r[7]),
+          "=r"(r[8]), "=r"(r[9]), "=r"(r[10]), "=r"(r[11]), "=r"(r[12]), "=r"(r[13]), "=r"(r[14]), "=r"(r[15]),
+          "=r"(mn)
+        : "r"(taddr)
+        : "memory");
+}
+
+// Per row of one a tile and column group, over a segment's columns.
+struct RowTop {
+    float cls[16];      // minimum of each column class
+    float m1, m2;       // two smallest chunk minima
+    uint32_t chunk;     // chunk of m1
+    SLM_DEV void reset() {
+        const float inf = __int_as_float(0x7f800000);
+#pragma unroll
+        for (int k = 0; k < 16; ++k) cls[k] = inf;
+        m1 = m2 = inf;
+        chunk = 0;
+    }
+    SLM_DEV void add_min(float cm, uint32_t c) {
+        m2 = fminf(m2, fmaxf(m1, cm));
+        chunk = cm < m1 ? c : chunk;
+        m1 = fminf(m1, cm);
+    }
+    // The row's best column (relative to the segment) and exact second smallest.
+    SLM_DEV void close(uint32_t &j, float &second) {
+        uint32_t k1 = 0;
+        float lo[8], hi[8];
+#pragma unroll
+        for (int k = 15; k >= 0; --k) k1 = cls[k] == m1 ? k : k1;
+#pragma unroll
+        for (int k = 0; k < 8; ++k) {
+            lo[k] = fminf(cls[k], cls[k + 8]);
+            hi[k] = fmaxf(cls[k], cls[k + 8]);
+        }
+#pragma unroll
+        for (int n = 4; n; n >>= 1)
+#pragma unroll
+            for (int k = 0; k < n; ++k) {
+                hi[k] = min3f(hi[k], hi[k + n], fmaxf(lo[k], lo[k + n]));
+                lo[k] = fminf(lo[k], lo[k + n]);
+            }
+        j = chunk * 16 + k1;
+        second = fminf(m2, hi[0]);
+    }
+};
+
+// bar.sync of `n` threads that also returns the AND of ok over them.
+SLM_DEV bool bar_and(int id, int n, bool ok) {
+    uint32_t r;
+    asm volatile(
+        "{\n"
+        ".reg .pred p, q;\n"
+        "setp.ne.u32 p, %3, 0;\n"
+        "bar.red.and.pred q, %1, %2, p;\n"
+        "selp.u32 %0, 1, 0, q;\n"
+        "}\n"
+        : "=r"(r)
+        : "r"(id), "r"(n), "r"((uint32_t)ok)
+        : "memory");
+    return r != 0;
+}
+
+// Instruction descriptor: bf16 inputs, f32 accumulate, K-major A and B, M = 128.
+__host__ __device__ constexpr uint32_t top_idesc(uint32_t n, bool negate_b) {
+    return (1u << 4) | (1u << 7) | (1u << 10) | ((negate_b ? 1u : 0u) << 14) | ((n >> 3) << 17) | ((128u >> 4) << 24);
+}
+
+// Tier 1 (the BF16 rescue of an FP8 plan) works on the rescued pairs only.
+SLM_DEV bool top_item_off(const SlArgs &g, const TopItem &it) {
+    return g.tier && !sl_pair_on(g, g.spairs[it.pair]);
+}
+
+template <bool DUMP>
+__global__ void __maxnreg__(96) sl_top2_kernel(SlArgs g) {
+    extern __shared__ uint8_t top_smem_raw[];
+    const uint32_t pad = (1024u - (smem_u32(top_smem_raw) & 1023u)) & 1023u;
+    TopSmem &S = *reinterpret_cast<TopSmem *>(top_smem_raw + pad);
+    const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
+    uint32_t *err = g.ctl + 1;
+    volatile uint32_t *abort_flag = &S.abort_flag;
+
+    if (threadIdx.x == 0) {
+        mbar_init(&S.a_full, 1);
+        mbar_init(&S.a_empty, 1);
+        for (int s = 0; s < kTopStages; ++s) {
+            mbar_init(&S.b_full[s], 1);
+            mbar_init(&S.b_empty[s], 1);
+        }
+        for (int b = 0; b < 2; ++b) {
+            mbar_init(&S.t_full[b], 1);
+            mbar_init(&S.t_empty[b], kTopEpWarps);
+        }
+        S.abort_flag = 0;
+        fence_mbar_init();
+    }
+    if (warp == 1) {
+        tmem_alloc(&S.tmem_base, 512);
+        tmem_relinquish();
+        tc_fence_before();
+    }
+    __syncthreads();
+    tc_fence_after();
+    const uint32_t tmem = S.tmem_base;
+    const uint32_t it0 = g.tstart[blockIdx.x], it1 = g.tstart[blockIdx.x + 1];
+
+    if (warp == 0) {
+        // ---------------------------------------------------------- producer
+        if (lane == 0) {
+            uint32_t st = 0, sph = 0, loads = 0, cur = 0xffffffffu;
+            bool ok = true;
+            for (uint32_t it = it0; it < it1 && ok; ++it) {
+                const TopItem item = g.titems[it];
+                if (top_item_off(g, item)) continue;
+                if (item.a_tile != cur) {
+                    if (loads && !(ok = sl_wait(&S.a_empty, (loads - 1) & 1, abort_flag, err))) break;
+                    cur = item.a_tile;
+                    ++loads;
+                    mbar_arrive_expect_tx(&S.a_full, item.nat * kBf16TileStride);
+                    for (uint32_t a = 0; a < item.nat; ++a)
+                        bulk_g2s(S.A[a], g.optiles + (size_t)(item.a_tile + a) * kBf16TileStride, kBf16TileStride,
+                                 &S.a_full);
+                }
+                for (uint32_t t = 0; t < item.nt; t += 2) {
+                    if (!(ok = sl_wait(&S.b_empty[st], sph ^ 1, abort_flag, err))) break;
+                    const uint32_t n = min(2u, item.nt - t);
+                    mbar_arrive_expect_tx(&S.b_full[st], n * kBf16TileStride);
+                    for (uint32_t u = 0; u < n; ++u) {
+                        const uint8_t *src = g.optiles + (size_t)(item.b_tile + t + u) * kBf16TileStride;
+                        bulk_g2s(S.B[st] + u * kKb, src, kKb, &S.b_full[st]);
+                        bulk_g2s(S.B[st] + (2 + u) * kKb, src + kKb, kKb, &S.b_full[st]);
+                        bulk_g2s(S.B[st] + kStageExt + u * kBf16ExtBytes, src + 2 * kKb, kBf16ExtBytes, &S.b_full[st]);
+                    }
+                    if (++st == kTopStages) st = 0, sph ^= 1;
+                }
+            }
+        }
+    } else if (warp == 1) {
+        // ---------------------------------------------------------- MMA issue
+        // descriptors of fixed shared-memory addresses; a tile, stage or K step
+        // adds its byte offset / 16 (all addresses lie below 256 KiB: no carry).
+        // The norm extension of a row is one 16-byte core matrix row per operand
+        // role; leading offset 0 reads it twice along K, and it holds |v|^2 / 4.
+        constexpr uint32_t kTile16 = kBf16TileStride >> 4, kStage16 = kStageBytes >> 4;
+        const uint64_t ad0 = umma_desc(smem_u32(S.A[0])), bd0 = umma_desc(smem_u32(S.B[0]));
+        const uint64_t ax0 = umma_desc_plain(smem_u32(S.A[0]) + 2 * kKb, 0, 256);
+        const uint64_t bx0 = umma_desc_plain(smem_u32(S.B[0]) + kStageExt + 128, 0, 256);
+        uint32_t st = 0, sph = 0, tb = 0, tph = 0, loads = 0, cur = 0xffffffffu;
+        bool ok = true;
+        TopItem next = it0 < it1 ? g.titems[it0] : TopItem{};
+        for (uint32_t it = it0; it < it1 && ok; ++it) {
+            const TopItem item = next;
+            if (it + 1 < it1) next = g.titems[it + 1];
+            if (top_item_off(g, item)) continue;
+            if (item.a_tile != cur) {
+                if (loads && lane == 0) mma_commit(&S.a_empty);
+                if (!(ok = sl_wait(&S.a_full, loads & 1, abort_flag, err))) break;
+                cur = item.a_tile;
+                ++loads;
+            }
+            for (uint32_t t = 0; t < item.nt && ok; t += 2) {
+                if (!(ok = sl_wait(&S.b_full[st], sph, abort_flag, err))) break;
+                const uint32_t n = item.nt - t > 1 ? 256 : 128;
+                const uint32_t idesc = top_idesc(n, false), idesc_neg = top_idesc(n, true);
+#pragma unroll
+                for (uint32_t a = 0; a < 2; ++a) {
+                    if (a >= item.nat) break;
+                    if (!(ok = sl_wait(&S.t_empty[tb], tph ^ 1, abort_flag, err))) break;
+                    tc_fence_after();
+                    if (lane == 0) {
+                        const uint32_t d = tmem + tb * 256;
+                        const uint64_t ad = ad0 + (uint64_t)(a * kTile16), bd = bd0 + (uint64_t)(st * kStage16);
+#pragma unroll
+                        for (int k = 0; k < 8; ++k)  // K = 16 bf16 = 32 bytes per step; -a.b
+                            mma_f16(d, ad + (k >> 2) * (kKb >> 4) + (k & 3) * 2,
+                                    bd + (k >> 2) * (2 * kKb >> 4) + (k & 3) * 2, idesc_neg, k > 0);
+                        // + (|a|^2 + |b|^2) / 2
+                        mma_f16(d, ax0 + (uint64_t)(a * kTile16), bx0 + (uint64_t)(st * kStage16), idesc, true);
+                        mma_commit(&S.t_full[tb]);
+                    }
+                    __syncwarp();
+                    tb ^= 1;
+                    if (tb == 0) tph ^= 1;
+                }
+                if (lane == 0) mma_commit(&S.b_empty[st]);
+                __syncwarp();
+                if (++st == kTopStages) st = 0, sph ^= 1;
+            }
+        }
+    } else {
+        // ---------------------------------------------------------- epilogue
+        const int q = warp & 3, cg = (warp - 2) >> 2;
+        const uint32_t lane_addr = (uint32_t)(q * 32) << 16;
+        const int row = q * 32 + lane;
+        uint32_t tb = 0, tph = 0;
+        bool ok = true;
+        for (uint32_t it = it0; it < it1 && ok; ++it) {
+            const TopItem item = g.titems[it];
+            if (top_item_off(g, item)) continue;
+            RowTop s[2];
+            s[0].reset();
+            s[1].reset();
+            for (uint32_t t = 0; t < item.nt && ok; t += 2) {
+                // chunks of this stage holding columns of the pair (the rest are padding)
+                const uint32_t left = item.ncols - t * kTile;
+                const uint32_t nch = (min(left, 256u) + 15) / 16, c0 = t * (kTile / 16);
+#pragma unroll
+                for (int a = 0; a < 2; ++a) {
+                    if (a >= (int)item.nat) break;
+                    if (!(ok = sl_wait(&S.t_full[tb], tph, abort_flag, err))) break;
+                    tc_fence_after();
+                    const uint32_t tcol = tmem + lane_addr + tb * 256;
+                    if constexpr (DUMP) {
+                        if (item.pair == 0 && !item.dir) {
+                            const PairMeta pm = g.pairs[0];
+                            const uint32_t i = (item.a_tile + a) * kTile - pm.a_row0 + row;
+                            for (uint32_t c = cg; c < nch; c += 4) {
+                                uint32_t v[16];
+                                tmem_ld16(tcol + c * 16, v);
+                                tmem_wait_ld16(v);
+                                for (int k = 0; k < 16; ++k) {
+                                    const uint32_t j = item.j0 + (c0 + c) * 16 + k;
+                                    if (i < pm.na && j < pm.nb)
+                                        g.dump[(size_t)i * pm.nb + j] = 2.f * __uint_as_float(v[k]);
+                                }
+                            }
+                        }
+                    }
+                    uint32_t c = cg;
+#pragma unroll 1
+                    for (; c + 4 < nch; c += 8) {
+                        uint32_t v0[16], v1[16], n0, n1;
+                        tmem_ld16_min(tcol + c * 16, v0, n0);
+                        tmem_ld16_min(tcol + c * 16 + 64, v1, n1);
+                        asm volatile("tcgen05.wait::ld.sync.aligned;" : "+r"(n0), "+r"(n1)::"memory");
+                        tmem_tie16(v0);
+                        tmem_tie16(v1);
+#pragma unroll
+                        for (int k = 0; k < 16; ++k)
+                            s[a].cls[k] = min3f(s[a].cls[k], __uint_as_float(v0[k]), __uint_as_float(v1[k]));
+                        s[a].add_min(__uint_as_float(n0), c0 + c);
+                        s[a].add_min(__uint_as_float(n1), c0 + c + 4);
+                    }
+                    if (c < nch) {
+                        uint32_t v0[16], n0;
+                        tmem_ld16_min(tcol + c * 16, v0, n0);
+                        asm volatile("tcgen05.wait::ld.sync.aligned;" : "+r"(n0)::"memory");
+                        tmem_tie16(v0);
+#pragma unroll
+                        for (int k = 0; k < 16; ++k) s[a].cls[k] = fminf(s[a].cls[k], __uint_as_float(v0[k]));
+                        s[a].add_min(__uint_as_float(n0), c0 + c);
+                    }
+                    tc_fence_before();
+                    __syncwarp();
+                    if (lane == 0) mbar_arrive(&S.t_empty[tb]);
+                    tb ^= 1;
+                    if (tb == 0) tph ^= 1;
+                }
+            }
+            // the four column groups of a lane quarter merge: group a keeps a
+            // tile a's rows, the others hand theirs over (a barrier of the
+            // quarter's 128 threads before the buffer is written, one after).
+            // The first barrier also makes a timed-out wait the whole quarter's,
+            // so that no warp waits at a later item for one that has left.
+            float m1[2], m2[2];
+            uint32_t j[2];
+#pragma unroll
+            for (int a = 0; a < 2; ++a) {
+                s[a].close(j[a], m2[a]);
+                m1[a] = s[a].m1;
+            }
+            ok = bar_and(q + 1, 128, ok);
+#pragma unroll
+            for (int a = 0; a < 2; ++a)
+                if (cg != a) {
+                    const int slot = cg < a ? cg : cg - 1;
+                    S.mm[a][slot][row] = make_float2(m1[a], m2[a]);
+                    S.mj[a][slot][row] = j[a];
+                }
+            asm volatile("bar.sync %0, 128;" ::"r"(q + 1) : "memory");
+#pragma unroll
+            for (int a = 0; a < 2; ++a)
+                if (cg == a && a < (int)item.nat && ok) {
+                    float b1 = m1[a], b2 = m2[a];
+                    uint32_t bj = j[a];
+#pragma unroll
+                    for (int o = 0; o < 3; ++o) {
+                        const float2 v = S.mm[a][o][row];
+                        top2_merge(b1, b2, bj, v.x, v.y, S.mj[a][o][row]);
+                    }
+                    const size_t out = ((size_t)item.part << g.tshift) + a * kTile + row;
+                    g.topmm[out] = make_float2(2.f * b1, 2.f * b2);  // d~ from d~ / 2
+                    g.topj[out] = item.j0 + bj;
+                }
+        }
+    }
+    // Everyone done: no MMA in flight (the epilogue consumed every commit).
+    tc_fence_before();
+    __syncthreads();
+    if (warp == 1) {
+        tc_fence_after();
+        tmem_dealloc(tmem, 512);
+    }
+}
+
+// ------------------------------------------------------------- decisions
+
+// A row's two smallest estimates and nearest column: its segments' results
+// merged (one segment but where a CTA's share of the work ended inside its
+// columns). blk0: the side's first block.
+SLM_DEV void row_top2(const SlArgs &g, uint32_t blk0, uint32_t i, float &m1, float &m2, uint32_t &j) {
+    const uint2 b = g.tblk[blk0 + (i >> g.tshift)];  // {first part, parts}
+    const size_t r = ((size_t)b.x << g.tshift) + (i & ((1u << g.tshift) - 1));
+    const float2 v = g.topmm[r];
+    m1 = v.x;
+    m2 = v.y;
+    j = g.topj[r];
+    for (uint32_t s = 1; s < b.y; ++s) {
+        const size_t o = r + ((size_t)s << g.tshift);
+        const float2 w = g.topmm[o];
+        top2_merge(m1, m2, j, w.x, w.y, g.topj[o]);
+    }
+}
+
+// The cross-check of row i, whose exact distance to its nearest column j is at
+// least dlow: the column's nearest row is certain when every other row's
+// estimate is more than 2 eps above its best one; row i is certainly not it
+// when dlow lies above the largest distance the best row may have. Anything
+// else is queued for an exact column scan.
+SLM_DEV uint32_t mutual_from_top2(const SlArgs &g, uint32_t p, const SlPair &sp, uint32_t i, uint32_t j, float dlow) {
+    float c1, c2;
+    uint32_t i1;
+    row_top2(g, sp.tblk_b, j, c1, c2, i1);
+    if (__fsub_rd(c2, c1) > 2.f * sp.eps) return i1 == i ? j : kDecNone;
+    if (dlow > __fadd_ru(c1, sp.eps)) return kDecNone;
+    push_scan(g, p, 1, i, j);
+    return kDecPending;
+}
+
+// One thread per row of a (CTA per pair and 256 rows): the outcome the bounds
+// certify, or the row joins its pair's list of undecided rows. The last CTA
+// of a pair cuts that list into groups of 16 for sl_resolve_kernel.
+constexpr uint32_t kDecideRows = 256;
+__global__ void __launch_bounds__(kDecideRows) sl_decide_kernel(SlArgs g) {
+    const uint32_t p = blockIdx.x, row0 = blockIdx.y * kDecideRows;
+    const PairMeta pm = g.pairs[p];
+    if (row0 >= pm.na) return;  // block-uniform, as below
+    const SlPair sp = g.spairs[p];
+    if (!sl_pair_on(g, sp)) return;
+    __shared__ uint32_t last;
+    const uint32_t i = row0 + threadIdx.x, lane = threadIdx.x & 31;
+    uint32_t *pc = g.pairctl + 4 * (size_t)p;
+    bool open = false;
+    if (i < pm.na) {
+        uint32_t dec = kDecNone;
+        float m1, m2;
+        uint32_t j;
+        if (pm.nb) {
+            row_top2(g, sp.tblk_a, i, m1, m2, j);
+            // fewer than two columns: the exact second best is infinite (matching.rs:205)
+            if (m2 < __int_as_float(0x7f800000) && !certain_no_match(m1, m2, sp.eps, g.ratio2)) {
+                // the ratio test passes and every other column is certainly farther
+                if (certain_ratio_pass(m1, m2, sp.eps, g.ratio2) && __fsub_rd(m2, m1) > 2.f * sp.eps) {
+                    dec = g.mutual ? mutual_from_top2(g, p, sp, i, j, __fsub_rd(m1, sp.eps)) : j;
+                } else {
+                    dec = kDecPending;
+                    open = true;
+                }
+            }
+        }
+        g.rowdec[sp.rbase + i] = dec;
+    }
+    const uint32_t m = __ballot_sync(0xffffffffu, open);
+    if (m) {
+        uint32_t base = 0;
+        if (lane == 0) base = atomicAdd(&pc[kPcOpen], (uint32_t)__popc(m));
+        base = __shfl_sync(0xffffffffu, base, 0);
+        if (open) g.ulist[sp.rbase + base + __popc(m & ((1u << lane) - 1))] = i;
+    }
+    const uint32_t nblk = (pm.na + kDecideRows - 1) / kDecideRows;
+    if (nblk > 1) {
+        __threadfence();
+        __syncthreads();
+        if (threadIdx.x == 0) last = atomicAdd(&pc[kPcMidDone], 1u) == nblk - 1;
+        __syncthreads();
+        if (!last) return;
+        __threadfence();
+    } else {
+        __syncthreads();
+    }
+    __shared__ uint32_t first, n;
+    if (threadIdx.x == 0) {
+        n = (atomicAdd(&pc[kPcOpen], 0u) + kResolveRows - 1) / kResolveRows;
+        first = n ? atomicAdd(&g.ctl[kCtlGroups], n) : 0;
+    }
+    __syncthreads();
+    for (uint32_t k = threadIdx.x; k < n; k += kDecideRows) g.ugroups[first + k] = make_uint2(p, k * kResolveRows);
+}
+
+// --------------------------------------------------------------- resolve
+
+SLM_DEV void mma_16816(float (&c)[4], uint32_t a0, uint32_t a1, uint32_t a2, uint32_t a3, uint32_t b0, uint32_t b1) {
+    asm volatile(
+        "mma.sync.aligned.m16n8k16.row.col.f32.bf16.bf16.f32 {%0,%1,%2,%3}, {%4,%5,%6,%7}, {%8,%9}, {%0,%1,%2,%3};"
+        : "+f"(c[0]), "+f"(c[1]), "+f"(c[2]), "+f"(c[3])
+        : "r"(a0), "r"(a1), "r"(a2), "r"(a3), "r"(b0), "r"(b1));
+}
+
+// The 16-byte chunk c (0..15) of store row r of the BF16 operand image.
+SLM_DEV uint4 op_chunk(const SlArgs &g, uint32_t r, uint32_t c) {
+    const uint8_t *t = g.optiles + (size_t)(r / kTile) * kBf16TileStride + (c >> 3) * kKb + (r % kTile) * 128;
+    return *reinterpret_cast<const uint4 *>(t + (((c & 7) ^ (r & 7)) * 16));
+}
+
+// One CTA per group of 16 undecided rows of a pair (about 1 % of a zone's
+// rows): their estimates against every column once more, the columns within
+// the window m2 + 2 eps, the exact distances of those, and the reference's
+// row rule (matching.rs:182-187, 204-206). The group's rows lie scattered in
+// the view, which no shared-memory descriptor of tcgen05 can address without
+// staging, and 16 rows are a warp-level tile exactly: m16n8k16 with both
+// operands straight from the operand image. The sum over k may run in any
+// order, so lane t of four takes the 16-byte chunks 4 q + t of its row, on
+// both sides, and each chunk is the operand words of two steps.
+// A row with more columns in the window than g.cand_cap is scanned exactly
+// instead; a pair with more than 1/8 such rows goes to the exact kernel.
+__global__ void __launch_bounds__(256) sl_resolve_kernel(SlArgs g) {
+    __shared__ uint32_t cand[kResolveRows][4 * kSlHalfRecsMax / 2];
+    __shared__ float cval[kResolveRows][4 * kSlHalfRecsMax / 2];
+    __shared__ uint32_t cnt[kResolveRows], rows[kResolveRows];
+    __shared__ float win[kResolveRows], nrm[kResolveRows];
+    const uint32_t tid = threadIdx.x, warp = tid >> 5, lane = tid & 31;
+    const uint32_t gr = lane >> 2, t = lane & 3;
+    const float kInf = __int_as_float(0x7f800000);
+    const uint32_t ng = g.ctl[kCtlGroups];
+    uint32_t w_rows = 0;
+    float w_err = 0.f;
+    for (uint32_t e = blockIdx.x; e < ng; e += gridDim.x) {
+        const uint2 ug = g.ugroups[e];
+        const PairMeta pm = g.pairs[ug.x];
+        const SlPair sp = g.spairs[ug.x];
+        const uint32_t n = min(kResolveRows, g.pairctl[4 * (size_t)ug.x + kPcOpen] - ug.y);
+        if (tid < kResolveRows) {
+            // rows past the list's end repeat its first row and admit nothing
+            const uint32_t i = g.ulist[sp.rbase + ug.y + (tid < n ? tid : 0)];
+            float m1, m2;
+            uint32_t j;
+            row_top2(g, sp.tblk_a, i, m1, m2, j);
+            rows[tid] = i;
+            cnt[tid] = 0;
+            win[tid] = tid < n ? window_up(m2, sp.eps) : -kInf;
+            nrm[tid] = g.norms[pm.a_row0 + i];
+        }
+        __syncthreads();
+        uint32_t A[2][16];  // rows gr and gr + 8: word w of chunk q is A[.][4 q + w]
+#pragma unroll
+        for (int h = 0; h < 2; ++h)
+#pragma unroll
+            for (int q = 0; q < 4; ++q) {
+                const uint4 v = op_chunk(g, pm.a_row0 + rows[gr + 8 * h], 4 * q + t);
+                A[h][4 * q] = v.x, A[h][4 * q + 1] = v.y, A[h][4 * q + 2] = v.z, A[h][4 * q + 3] = v.w;
+            }
+        const float na0 = nrm[gr], na1 = nrm[gr + 8], w0 = win[gr], w1 = win[gr + 8];
+        const uint32_t n8 = (pm.nb + 7) / 8;  // columns past nb have a NaN norm: never admitted
+        for (uint32_t c8 = warp; c8 < n8; c8 += 16) {
+            uint4 B[2][4];
+            const bool two = c8 + 8 < n8;
+#pragma unroll
+            for (int u = 0; u < 2; ++u) {
+                const uint32_t r = pm.b_row0 + (c8 + (u && two ? 8 : 0)) * 8 + gr;
+#pragma unroll
+                for (int q = 0; q < 4; ++q) B[u][q] = op_chunk(g, r, 4 * q + t);
+            }
+#pragma unroll
+            for (int u = 0; u < 2; ++u) {
+                if (u && !two) break;
+                float acc[4] = {0.f, 0.f, 0.f, 0.f};
+#pragma unroll
+                for (int q = 0; q < 4; ++q) {
+                    mma_16816(acc, A[0][4 * q], A[1][4 * q], A[0][4 * q + 1], A[1][4 * q + 1], B[u][q].x, B[u][q].y);
+                    mma_16816(acc, A[0][4 * q + 2], A[1][4 * q + 2], A[0][4 * q + 3], A[1][4 * q + 3], B[u][q].z,
+                              B[u][q].w);
+                }
+                const uint32_t j = (c8 + 8 * u) * 8 + 2 * t;
+                const float2 nb = *reinterpret_cast<const float2 *>(g.norms + pm.b_row0 + j);
+                const float d[4] = {fmaf(-2.f, acc[0], na0 + nb.x), fmaf(-2.f, acc[1], na0 + nb.y),
+                                    fmaf(-2.f, acc[2], na1 + nb.x), fmaf(-2.f, acc[3], na1 + nb.y)};
+#pragma unroll
+                for (int k = 0; k < 4; ++k)
+                    if (d[k] <= (k < 2 ? w0 : w1)) {
+                        const uint32_t r = gr + (k < 2 ? 0 : 8);
+                        const uint32_t s = atomicAdd(&cnt[r], 1u);
+                        if (s < g.cand_cap) {
+                            cand[r][s] = j + (k & 1);
+                            cval[r][s] = d[k];
+                        }
+                    }
+            }
+        }
+        __syncthreads();
+        // exact distances: a warp per row, four columns at a time (8 lanes each)
+        for (uint32_t r = warp; r < n; r += 8) {
+            const uint32_t i = rows[r], m = cnt[r];
+            const float *a = g.raw + (size_t)(pm.a_row0 + i) * kDesc;
+            const float *B = g.raw + (size_t)pm.b_row0 * kDesc;
+            if (m > g.cand_cap) {
+                if (lane == 0) {
+                    push_scan(g, ug.x, 0, i, 0);
+                    const uint32_t over = atomicAdd(&g.pairctl[4 * (size_t)ug.x + kPcOver], 1u);
+                    if (over * 8 <= pm.na && (over + 1) * 8 > pm.na) {
+                        g.spairs[ug.x].routed = 1;
+                        atomicAdd(&g.ctl[kCtlRouteMarks], 1u);
+                    }
+                }
+                continue;
+            }
+            float e1 = kInf, e2 = kInf;
+            uint32_t ej = 0xffffffffu;
+            for (uint32_t s = 0; s < m; s += 4) {
+                const uint32_t mine = s + (lane >> 3);
+                const uint32_t j = cand[r][mine < m ? mine : s];
+                const float d = dist8(a, B + (size_t)j * kDesc);
+                if (mine < m) w_err = fmaxf(w_err, fabsf(d - cval[r][mine]));
+#pragma unroll
+                for (uint32_t q = 0; q < 4; ++q) {
+                    const float dq = __shfl_sync(0xffffffffu, d, q * 8);
+                    const uint32_t jq = __shfl_sync(0xffffffffu, j, q * 8);
+                    if (s + q < m) {
+                        if (dq < e1 || (dq == e1 && jq < ej)) {
+                            e2 = e1;
+                            e1 = dq;
+                            ej = jq;
+                        } else if (dq < e2) {
+                            e2 = dq;
+                        }
+                    }
+                }
+            }
+            if (lane == 0) {
+                ++w_rows;
+                uint32_t dec = kDecNone;
+                if (ej != 0xffffffffu && e2 < kInf && !(e1 >= __fmul_rn(g.ratio2, e2)))
+                    dec = g.mutual ? mutual_from_top2(g, ug.x, sp, i, ej, e1) : ej;
+                g.rowdec[sp.rbase + i] = dec;
+            }
+        }
+        __syncthreads();
+    }
+#pragma unroll
+    for (int o = 16; o; o >>= 1) w_err = fmaxf(w_err, __shfl_xor_sync(0xffffffffu, w_err, o));
+    if (lane == 0 && w_rows) {
+        atomicAdd(&g.ctl[kCtlRescored], w_rows);
+        atomicMax(&g.ctl[kCtlMaxErr], __float_as_uint(w_err));  // non-negative: bits order as values
+    }
+}
+
+}  // namespace
+
+cudaError_t init_top2_kernels() {
+    const cudaFuncAttribute at = cudaFuncAttributeMaxDynamicSharedMemorySize;
+    cudaError_t e = cudaFuncSetAttribute(sl_top2_kernel<false>, at, (int)kTopSmemBytes);
+    if (e == cudaSuccess) e = cudaFuncSetAttribute(sl_top2_kernel<true>, at, (int)kTopSmemBytes);
+    return e;
+}
+
+int launch_top2_pass(const SlArgs &a, cudaStream_t s) {
+    if (!a.tgrid) return 0;
+    if (a.dump)
+        sl_top2_kernel<true><<<a.tgrid, kTopThreads, kTopSmemBytes, s>>>(a);
+    else
+        sl_top2_kernel<false><<<a.tgrid, kTopThreads, kTopSmemBytes, s>>>(a);
+    return 1;
+}
+
+int launch_top2_decide(const SlArgs &a, cudaStream_t s) {
+    if (!a.npairs || !a.max_na) return 0;
+    sl_decide_kernel<<<dim3(a.npairs, (a.max_na + kDecideRows - 1) / kDecideRows), kDecideRows, 0, s>>>(a);
+    return 1;
+}
+
+int launch_top2_resolve(const SlArgs &a, int sms, cudaStream_t s) {
+    if (!a.npairs || !a.max_na) return 0;
+    sl_resolve_kernel<<<4 * sms, 256, 0, s>>>(a);
+    return 1;
+}
+
+}  // namespace slm

@@ -270,6 +270,14 @@ struct slm_plan {
     uint32_t row_blocks = 1;  // the most row blocks of any pair
     DevBuf d_sitems, d_spairs, d_rowpart, d_rownear, d_colmin, d_rowthr, d_colthr, d_rowcnt, d_rowrec, d_rowrecj, d_colcnt,
         d_rowdec, d_queue, d_rqueue, d_dump, d_xlist, d_xitems, d_xparts, d_blkcnt, d_pairctl;
+    // BF16 pass: segments in the order the CTAs run them, each CTA's first one,
+    // each block's parts; then its results and the undecided rows
+    std::vector<TopItem> titems;
+    std::vector<uint32_t> tstart;
+    std::vector<uint2> tblk;
+    uint32_t tshift = 8, max_na = 0;
+    uint64_t top_parts = 0;
+    DevBuf d_titems, d_tstart, d_tblk, d_topmm, d_topj, d_ulist, d_ugroups;
     bool dump = false;
     uint32_t min_matches = 0;        // pairs with fewer matches report none
     cudaGraphExec_t exec = nullptr;
@@ -292,12 +300,13 @@ struct slm_plan {
 
 // Every device buffer of a plan: all are used on the plan's stream only, and
 // allocated ordered on it (DevBuf::order_on).
-std::array<DevBuf *, 29> plan_buffers(slm_plan *p) {
+std::array<DevBuf *, 36> plan_buffers(slm_plan *p) {
     return {&p->d_meta, &p->d_items, &p->d_parts, &p->d_colbest, &p->d_slots, &p->d_counts, &p->d_ctl,
             &p->d_offsets, &p->d_dense, &p->d_sitems, &p->d_spairs, &p->d_rowpart, &p->d_rownear,
             &p->d_colmin, &p->d_rowthr, &p->d_colthr, &p->d_rowcnt, &p->d_rowrec, &p->d_rowrecj,
             &p->d_colcnt, &p->d_rowdec, &p->d_queue, &p->d_rqueue, &p->d_dump, &p->d_xlist, &p->d_xitems,
-            &p->d_xparts, &p->d_blkcnt, &p->d_pairctl};
+            &p->d_xparts, &p->d_blkcnt, &p->d_pairctl, &p->d_titems, &p->d_tstart, &p->d_tblk, &p->d_topmm,
+            &p->d_topj, &p->d_ulist, &p->d_ugroups};
 }
 // Frees a plan's buffers while its stream still exists (their frees are
 // ordered on it): owners call it before destroying that stream.
@@ -358,10 +367,89 @@ void plan_items(slm_plan *p) {
     });
 }
 
-// Shortlist plan: items of up to two 128-row a tiles against a range of
-// 128-column b tiles; per-row and per-column arrays padded to 128 entries per
-// pair so that every bulk copy starts on a 512-byte boundary.
-slm_status plan_build_shortlist(slm_plan *p, const slm_pair *pairs) {
+// The BF16 pass's work: every pair's row blocks (256 rows; 128 with row_tiles
+// 1) against the other view's tiles, and with the cross-check the other view's
+// row blocks against this one's, two column tiles a step. Blocks that share
+// their rows run one after the other, so that a CTA loads a block's tiles once
+// for all partners, and the sequence is cut into equal shares for the CTAs,
+// inside a block's columns where a share ends there: such a block's results
+// come in several parts.
+void plan_top2(slm_plan *p) {
+    struct Block {
+        uint32_t a_tile, nat, b_tile, nt, ncols, pair, dir, index;
+    };
+    const uint32_t sms = (uint32_t)std::max(1, p->ctx->sms);
+    auto tiles = [](uint32_t n) { return (n + kTile - 1) / kTile; };
+    uint64_t steps = 0;  // of two a tiles by two column tiles
+    for (const PairMeta &m : p->meta)
+        steps += (uint64_t)((tiles(m.na) + 1) / 2) * ((tiles(m.nb) + 1) / 2) * (p->mutual ? 2 : 1);
+    // too few such steps for every SM: one a tile per block doubles them
+    const uint32_t per = p->tune.row_tiles == 1 || steps <= sms ? 1u : 2u;
+    p->tshift = per == 1 ? 7 : 8;
+    std::vector<Block> found, blocks;
+    std::vector<uint32_t> first(p->st->rows_used / kTile + 2, 0);  // counting sort by a tile
+    uint32_t index = 0;
+    uint64_t total = 0, nsteps = 0;  // cost in 128 x 128 tiles; steps of up to two column tiles
+    for (uint32_t dir = 0; dir < (p->mutual ? 2u : 1u); ++dir)
+        for (uint32_t k = 0; k < p->np; ++k) {
+            const PairMeta &m = p->meta[k];
+            const uint32_t na = dir ? m.nb : m.na, nb = dir ? m.na : m.nb;
+            const uint32_t ra = (dir ? m.b_row0 : m.a_row0) / kTile, rb = (dir ? m.a_row0 : m.b_row0) / kTile;
+            (dir ? p->spairs[k].tblk_b : p->spairs[k].tblk_a) = index;
+            if (!na || !nb) continue;
+            for (uint32_t t = 0; t < tiles(na); t += per, ++index) {
+                const uint32_t nat = std::min(per, tiles(na) - t);
+                found.push_back(Block{ra + t, nat, rb, tiles(nb), nb, k, dir, index});
+                first[ra + t + 1]++;
+                total += (uint64_t)nat * tiles(nb);
+                nsteps += (tiles(nb) + 1) / 2;
+            }
+        }
+    p->tblk.assign(index, make_uint2(0, 0));
+    for (size_t t = 1; t < first.size(); ++t) first[t] += first[t - 1];
+    blocks.resize(found.size());
+    for (const Block &b : found) blocks[first[b.a_tile]++] = b;
+    const uint32_t grid = (uint32_t)std::min<uint64_t>(sms, nsteps);
+    p->titems.clear();
+    p->tstart.assign(1, 0);
+    uint64_t done = 0;
+    uint32_t part = 0;
+    for (const Block &b : blocks) {
+        p->tblk[b.index].x = part;
+        uint32_t t = 0;
+        while (t < b.nt) {
+            // this CTA's share ends after `share` tiles; at least one step goes to it
+            const uint64_t share = total * p->tstart.size() / grid;
+            uint32_t n = b.nt - t;
+            if (p->tstart.size() < grid && done + (uint64_t)n * b.nat > share) {
+                const uint64_t room = share > done ? (share - done) / b.nat : 0;
+                n = std::min(n, std::max<uint32_t>(2, (uint32_t)(room + 1) / 2 * 2));
+            }
+            TopItem it{};
+            it.a_tile = b.a_tile;
+            it.b_tile = b.b_tile + t;
+            it.nat = (uint16_t)b.nat;
+            it.dir = (uint16_t)b.dir;
+            it.nt = n;
+            it.j0 = t * kTile;
+            it.ncols = std::min(n * kTile, b.ncols - it.j0);
+            it.part = part++;
+            it.pair = b.pair;
+            p->titems.push_back(it);
+            p->tblk[b.index].y++;
+            done += (uint64_t)n * b.nat;
+            t += n;
+            if (p->tstart.size() < grid && done >= share) p->tstart.push_back((uint32_t)p->titems.size());
+        }
+    }
+    if (p->tstart.back() != p->titems.size()) p->tstart.push_back((uint32_t)p->titems.size());
+    p->top_parts = part;
+}
+
+// FP8 tier-0 items: up to two 128-row a tiles against a range of 128-column b
+// tiles; per-row and per-column arrays padded to 128 entries per pair so that
+// every bulk copy starts on a 512-byte boundary.
+slm_status plan_fp8_items(slm_plan *p, const slm_pair *pairs) {
     slm_ctx *c = p->ctx;
     uint64_t supers = 0;
     for (uint32_t k = 0; k < p->np; ++k)
@@ -370,21 +458,11 @@ slm_status plan_build_shortlist(slm_plan *p, const slm_pair *pairs) {
     uint32_t split = 1;
     if (supers && supers < want) split = (uint32_t)((want + supers - 1) / supers);
     p->sitems.clear();
-    p->spairs.assign(p->np, SlPair{});
-    uint64_t rb = 0, cb = 0, part = 0, row_tiles = 0, blk = 0, crb = 0;
-    p->row_blocks = 1;
+    uint64_t cb = 0, part = 0, crb = 0;
     for (uint32_t k = 0; k < p->np; ++k) {
         const PairMeta &m = p->meta[k];
         SlPair &sp = p->spairs[k];
-        row_tiles += (m.na + kTile - 1) / kTile;
-        // row blocks of the per-pair kernels after pass 1
-        sp.blk = (uint32_t)blk;
-        blk += (m.na + kSlRowBlock - 1) / kSlRowBlock;
-        p->row_blocks = std::max(p->row_blocks, (std::max(m.na, m.nb) + kSlRowBlock - 1) / kSlRowBlock);
-        sp.rbase = (uint32_t)rb;
         sp.cbase = (uint32_t)cb;
-        sp.view_a = pairs[k].i;
-        sp.view_b = pairs[k].j;
         const uint32_t rt_n = (m.na + kTile - 1) / kTile, ct_n = (m.nb + kTile - 1) / kTile;
         const uint32_t chunks = std::max(1u, std::min(std::min(split, ct_n), kSlMaxRanges));
         sp.nchunk = chunks;
@@ -412,11 +490,9 @@ slm_status plan_build_shortlist(slm_plan *p, const slm_pair *pairs) {
                 }
             part += (uint64_t)ns * chunks;
         }
-        rb += pad_rows(m.na);
         cb += pad_rows(m.nb);
     }
-    if (rb >= (1ull << 32) || cb >= (1ull << 32) || crb >= (1ull << 31))
-        return fail(SLM_CAPACITY, "batch too large for one plan");
+    if (cb >= (1ull << 32) || crb >= (1ull << 31)) return fail(SLM_CAPACITY, "batch too large for one plan");
     // The last row tile of a pair with an odd tile count makes a one-tile item,
     // which leaves half of the epilogue warps idle. Two such tiles of pairs
     // with the same b view and column range share one item.
@@ -449,36 +525,71 @@ slm_status plan_build_shortlist(slm_plan *p, const slm_pair *pairs) {
     std::stable_sort(p->sitems.begin(), p->sitems.end(), [](const SlItem &x, const SlItem &y) {
         return (uint64_t)(x.ct1 - x.ct0) * x.nat > (uint64_t)(y.ct1 - y.ct0) * y.nat;
     });
-    p->rows_pad = rb + 2 * kTile;
     p->cand_rows_pad = crb + 2 * kTile;
     p->cols_pad = cb + kTile;
     p->sl_parts = std::max<uint64_t>(part, 1);
+    p->half_recs = p->tune.shortlist_k ? p->tune.shortlist_k : kSlHalfRecs;
+    SLM_TRY(p->d_sitems.ensure(c, sizeof(SlItem) * std::max<size_t>(1, p->sitems.size())));
+    SLM_TRY(p->d_rowpart.ensure(c, sizeof(float2) * 256 * p->sl_parts));
+    SLM_TRY(p->d_rownear.ensure(c, sizeof(uint32_t) * 256 * p->sl_parts));
+    SLM_TRY(p->d_colmin.ensure(c, sizeof(uint32_t) * p->cols_pad));
+    SLM_TRY(p->d_rowthr.ensure(c, sizeof(float) * p->rows_pad));
+    SLM_TRY(p->d_colthr.ensure(c, sizeof(float) * p->cols_pad));
+    SLM_TRY(p->d_rowcnt.ensure(c, 2 * sizeof(uint32_t) * p->cand_rows_pad));
+    SLM_TRY(p->d_rowrec.ensure(c, sizeof(float4) * 2 * p->half_recs * p->cand_rows_pad));
+    SLM_TRY(p->d_rowrecj.ensure(c, sizeof(uint32_t) * 2 * p->half_recs * p->cand_rows_pad));
+    SLM_TRY(p->d_colcnt.ensure(c, sizeof(uint32_t) * p->cols_pad));
+    SLM_TRY(p->d_rqueue.ensure(c, sizeof(SlQueue) * p->queue_cap));
+    SLM_CU(cudaMemcpyAsync(p->d_sitems.p, p->sitems.data(), sizeof(SlItem) * p->sitems.size(), cudaMemcpyHostToDevice,
+                           p->stream));
+    return SLM_OK;
+}
+
+slm_status plan_build_shortlist(slm_plan *p, const slm_pair *pairs) {
+    slm_ctx *c = p->ctx;
+    p->spairs.assign(p->np, SlPair{});
+    uint64_t rb = 0, row_tiles = 0, blk = 0, groups = 0;
+    p->row_blocks = 1;
+    p->max_na = 0;
+    for (uint32_t k = 0; k < p->np; ++k) {
+        const PairMeta &m = p->meta[k];
+        SlPair &sp = p->spairs[k];
+        row_tiles += (m.na + kTile - 1) / kTile;
+        // row blocks of the per-pair kernels after the passes
+        sp.blk = (uint32_t)blk;
+        blk += (m.na + kSlRowBlock - 1) / kSlRowBlock;
+        p->row_blocks = std::max(p->row_blocks, (std::max(m.na, m.nb) + kSlRowBlock - 1) / kSlRowBlock);
+        p->max_na = std::max(p->max_na, m.na);
+        sp.rbase = (uint32_t)rb;
+        sp.view_a = pairs[k].i;
+        sp.view_b = pairs[k].j;
+        rb += pad_rows(m.na);
+        groups += (m.na + kResolveRows - 1) / kResolveRows;
+    }
+    p->rows_pad = rb + 2 * kTile;
     p->queue_cap = std::max<uint64_t>(p->n_slots, 1) + 64;
     // pairs routed to the exact kernel: at most (row tiles) + (4 x SMs) items
     p->xitem_cap = row_tiles + 4ull * (uint64_t)std::max(1, c->sms);
-    if (p->xitem_cap >= (1ull << 32)) return fail(SLM_CAPACITY, "batch too large for one plan");
-    SLM_TRY(p->d_sitems.ensure(c, sizeof(SlItem) * std::max<size_t>(1, p->sitems.size())));
-    SLM_TRY(p->d_spairs.ensure(c, sizeof(SlPair) * std::max<size_t>(1, p->np)));
-    SLM_TRY(p->d_rowpart.ensure(c, sizeof(float2) * 256 * p->sl_parts));
-    SLM_TRY(p->d_rownear.ensure(c, sizeof(uint32_t) * 256 * p->sl_parts));
+    if (rb >= (1ull << 32) || p->xitem_cap >= (1ull << 32)) return fail(SLM_CAPACITY, "batch too large for one plan");
+    if (p->prec == SLM_PREC_FP8) SLM_TRY(plan_fp8_items(p, pairs));
+    plan_top2(p);
     p->row_blocks_total = blk;
+    SLM_TRY(p->d_spairs.ensure(c, sizeof(SlPair) * std::max<size_t>(1, p->np)));
+    SLM_TRY(p->d_titems.ensure(c, sizeof(TopItem) * std::max<size_t>(1, p->titems.size())));
+    SLM_TRY(p->d_tstart.ensure(c, sizeof(uint32_t) * p->tstart.size()));
+    SLM_TRY(p->d_tblk.ensure(c, sizeof(uint2) * std::max<size_t>(1, p->tblk.size())));
+    SLM_TRY(p->d_topmm.ensure(c, sizeof(float2) * std::max<uint64_t>(1, p->top_parts << p->tshift)));
+    SLM_TRY(p->d_topj.ensure(c, sizeof(uint32_t) * std::max<uint64_t>(1, p->top_parts << p->tshift)));
+    SLM_TRY(p->d_ulist.ensure(c, sizeof(uint32_t) * p->rows_pad));
+    SLM_TRY(p->d_ugroups.ensure(c, sizeof(uint2) * std::max<uint64_t>(1, groups)));
     SLM_TRY(p->d_blkcnt.ensure(c, sizeof(uint32_t) * std::max<uint64_t>(1, blk)));
     SLM_TRY(p->d_pairctl.ensure(c, 4 * sizeof(uint32_t) * std::max<size_t>(1, p->np)));
     SLM_TRY(p->d_xlist.ensure(c, sizeof(uint32_t) * std::max<size_t>(1, p->np)));
     SLM_TRY(p->d_xitems.ensure(c, sizeof(Item) * p->xitem_cap));
     SLM_TRY(p->d_xparts.ensure(c, sizeof(RowPart) * kTile * p->xitem_cap));
     SLM_TRY(p->d_colbest.ensure(c, sizeof(unsigned long long) * std::max<uint64_t>(1, p->n_cols)));
-    SLM_TRY(p->d_colmin.ensure(c, sizeof(uint32_t) * p->cols_pad));
-    SLM_TRY(p->d_rowthr.ensure(c, sizeof(float) * p->rows_pad));
-    SLM_TRY(p->d_colthr.ensure(c, sizeof(float) * p->cols_pad));
-    SLM_TRY(p->d_rowcnt.ensure(c, 2 * sizeof(uint32_t) * p->cand_rows_pad));
-    p->half_recs = p->tune.shortlist_k ? p->tune.shortlist_k : kSlHalfRecs;
-    SLM_TRY(p->d_rowrec.ensure(c, sizeof(float4) * 2 * p->half_recs * p->cand_rows_pad));
-    SLM_TRY(p->d_rowrecj.ensure(c, sizeof(uint32_t) * 2 * p->half_recs * p->cand_rows_pad));
-    SLM_TRY(p->d_colcnt.ensure(c, sizeof(uint32_t) * p->cols_pad));
     SLM_TRY(p->d_rowdec.ensure(c, sizeof(uint32_t) * p->rows_pad));
     SLM_TRY(p->d_queue.ensure(c, sizeof(SlQueue) * p->queue_cap));
-    SLM_TRY(p->d_rqueue.ensure(c, sizeof(SlQueue) * p->queue_cap));
     if (p->dump && p->np) SLM_TRY(p->d_dump.ensure(c, sizeof(float) * std::max<uint64_t>(1, (uint64_t)p->meta[0].na * p->meta[0].nb)));
     SLM_TRY(p->d_meta.ensure(c, sizeof(PairMeta) * std::max<size_t>(1, p->np)));
     SLM_TRY(p->d_slots.ensure(c, sizeof(uint2) * std::max<uint64_t>(1, p->n_slots)));
@@ -491,8 +602,9 @@ slm_status plan_build_shortlist(slm_plan *p, const slm_pair *pairs) {
     SLM_CU(cudaMemcpyAsync(p->d_offsets.as<uint64_t>() + (p->np + 1), p->slot_off.data(),
                            sizeof(uint64_t) * (p->np + 1), cudaMemcpyHostToDevice, s));
     SLM_CU(cudaMemcpyAsync(p->d_spairs.p, p->spairs.data(), sizeof(SlPair) * p->np, cudaMemcpyHostToDevice, s));
-    SLM_CU(cudaMemcpyAsync(p->d_sitems.p, p->sitems.data(), sizeof(SlItem) * p->sitems.size(),
-                           cudaMemcpyHostToDevice, s));
+    SLM_CU(cudaMemcpyAsync(p->d_titems.p, p->titems.data(), sizeof(TopItem) * p->titems.size(), cudaMemcpyHostToDevice, s));
+    SLM_CU(cudaMemcpyAsync(p->d_tstart.p, p->tstart.data(), sizeof(uint32_t) * p->tstart.size(), cudaMemcpyHostToDevice, s));
+    SLM_CU(cudaMemcpyAsync(p->d_tblk.p, p->tblk.data(), sizeof(uint2) * p->tblk.size(), cudaMemcpyHostToDevice, s));
     return SLM_OK;
 }
 
@@ -548,9 +660,12 @@ slm_status plan_enqueue(slm_plan *p, cudaStream_t s) {
     SLM_CU(cudaMemsetAsync(ctl, 0, 64, s));
     if (p->prec != SLM_PREC_FP32) {
         slm_store *st = p->st;
-        launch_fill_u32(p->d_colmin.as<uint32_t>(), p->cols_pad, 0xff800000u, s);  // encodes +inf
-        SLM_CU(cudaMemsetAsync(p->d_rowcnt.p, 0, 2 * sizeof(uint32_t) * p->cand_rows_pad, s));
-        SLM_CU(cudaMemsetAsync(p->d_colcnt.p, 0, sizeof(uint32_t) * p->cols_pad, s));
+        const bool fp8 = p->prec == SLM_PREC_FP8;
+        if (fp8) {
+            launch_fill_u32(p->d_colmin.as<uint32_t>(), p->cols_pad, 0xff800000u, s);  // encodes +inf
+            SLM_CU(cudaMemsetAsync(p->d_rowcnt.p, 0, 2 * sizeof(uint32_t) * p->cand_rows_pad, s));
+            SLM_CU(cudaMemsetAsync(p->d_colcnt.p, 0, sizeof(uint32_t) * p->cols_pad, s));
+        }
         SLM_CU(cudaMemsetAsync(p->d_pairctl.p, 0, 4 * sizeof(uint32_t) * p->np, s));
         SLM_CU(cudaMemsetAsync(p->d_counts.p, 0, sizeof(uint32_t) * p->np, s));  // compact adds its blocks
         SlArgs a{};
@@ -596,20 +711,37 @@ slm_status plan_enqueue(slm_plan *p, cudaStream_t s) {
         a.xparts = p->d_xparts.as<RowPart>();
         a.colbest = p->d_colbest.as<unsigned long long>();
         a.want_items = 4u * (uint32_t)std::max(1, p->ctx->sms);
-        a.rescue = p->prec == SLM_PREC_FP8 ? 1u : 0u;
         a.tier = 0;
-        int nk = 1;  // the colmin fill
+        a.titems = p->d_titems.as<TopItem>();
+        a.tstart = p->d_tstart.as<uint32_t>();
+        a.tgrid = (uint32_t)p->tstart.size() - 1;
+        a.tshift = p->tshift;
+        a.tblk = p->d_tblk.as<uint2>();
+        a.topmm = p->d_topmm.as<float2>();
+        a.topj = p->d_topj.as<uint32_t>();
+        a.max_na = p->max_na;
+        a.cand_cap = 2 * (p->tune.shortlist_k ? p->tune.shortlist_k : (uint32_t)kSlHalfRecs);
+        a.ulist = p->d_ulist.as<uint32_t>();
+        a.ugroups = p->d_ugroups.as<uint2>();
+        int nk = fp8 ? 1 : 0;  // the colmin fill
         SLM_CU(record_event(p->ev0, s));
         nk += launch_shortlist_eps(a, s);
-        nk += launch_shortlist_pass(a, 1, p->ctx->sms, s);
-        SLM_CU(record_event(p->evp[0], s));
-        nk += launch_shortlist_mid(a, s);
-        SLM_CU(record_event(p->evp[1], s));
-        nk += launch_shortlist_pass(a, 2, p->ctx->sms, s);
-        SLM_CU(record_event(p->evp[2], s));
-        nk += launch_shortlist_finalize(a, s);
-        if (a.rescue) {
-            // tier 1: the BF16 passes over the pairs FP8 could not settle (their
+        if (!fp8) {
+            nk += launch_top2_pass(a, s);
+            SLM_CU(record_event(p->evp[0], s));
+            nk += launch_top2_decide(a, s);
+            SLM_CU(record_event(p->evp[1], s));
+            nk += launch_top2_resolve(a, p->ctx->sms, s);
+            SLM_CU(record_event(p->evp[2], s));
+        } else {
+            nk += launch_shortlist_pass(a, 1, p->ctx->sms, s);
+            SLM_CU(record_event(p->evp[0], s));
+            nk += launch_shortlist_mid(a, s);
+            SLM_CU(record_event(p->evp[1], s));
+            nk += launch_shortlist_pass(a, 2, p->ctx->sms, s);
+            SLM_CU(record_event(p->evp[2], s));
+            nk += launch_shortlist_finalize(a, s);
+            // tier 1: the BF16 pass over the pairs FP8 could not settle (its
             // kernels return at once when no pair was rescued)
             SlArgs b = a;
             const slm_store::LowpImage &bi = st->lowp[0];
@@ -619,13 +751,11 @@ slm_status plan_enqueue(slm_plan *p, cudaStream_t s) {
             b.vstats = bi.vstats.as<ViewStat>();
             b.fp8 = 0;
             b.dump = nullptr;
-            b.rescue = 0;
             b.tier = 1;
             nk += launch_shortlist_rescue_prep(b, s);
-            nk += launch_shortlist_pass(b, 1, p->ctx->sms, s);
-            nk += launch_shortlist_mid(b, s);
-            nk += launch_shortlist_pass(b, 2, p->ctx->sms, s);
-            nk += launch_shortlist_finalize(b, s);
+            nk += launch_top2_pass(b, s);
+            nk += launch_top2_decide(b, s);
+            nk += launch_top2_resolve(b, p->ctx->sms, s);
         }
         nk += launch_shortlist_tail(a, p->ctx->sms, s);
         SLM_CU(record_event(p->ev1, s));
@@ -899,6 +1029,7 @@ extern "C" slm_status slm_ctx_create(const slm_opts *opts, slm_ctx **out) {
     {
         cudaError_t ke = init_exact_kernels();
         if (ke == cudaSuccess) ke = init_shortlist_kernels();
+        if (ke == cudaSuccess) ke = init_top2_kernels();
         if (ke != cudaSuccess) {
             cudaGetLastError();
             return fail(SLM_NO_DEVICE, std::string("kernels do not load on this device: ") + cudaGetErrorString(ke));
@@ -1270,6 +1401,7 @@ extern "C" slm_status slm_autotune(slm_ctx *c, slm_store *st, const slm_pair *pa
     for (uint32_t a = 0; a < 2; ++a)
         for (uint32_t ki = 0; ki < (prec == SLM_PREC_FP32 ? 1u : 3u); ++ki)
             for (uint32_t ipsm : ips) {
+                if (prec == SLM_PREC_BF16 && ipsm != 4) continue;  // its pass is cut into equal shares
                 slm_tune t{};
                 t.use_graph = 2;
                 t.items_per_sm = ipsm;

@@ -4,12 +4,27 @@
 // a few distances per row: the two smallest, and, for the mutual check, the
 // smallest in the chosen column. The shortlist path finds them with tensor-core
 // distances d~ = |a|^2 + |b|^2 - 2 a.b whose error against the exact f32
-// distance d is bounded per image pair by eps (see shortlist_eps), then
-// settles every decision the bound cannot certify with exact spec-order FP32
+// distance d is bounded per image pair by eps (see pair_eps), then settles
+// every decision the bound cannot certify with exact spec-order FP32
 // arithmetic, so the match list is the reference's bit for bit.
 //
+// BF16 (k_top2.cu; also the rescue tier of FP8 plans):
+//   pass     (tcgen05)  for every row of a against b, and with the cross-check
+//                       for every row of b against a: m1 = min d~ with its
+//                       column, and m2 = the second smallest d~.
+//   decide              per row: certain no match when m1 - eps >= r^2 (m2 +
+//                       eps); certain match at its column when m1 + eps < r^2
+//                       (m2 - eps) and m2 - m1 > 2 eps; the cross-check from
+//                       the column's own two smallest. Other rows are listed
+//                       per pair, other columns queued for an exact scan.
+//   resolve             the listed rows, 16 of a pair at a time: every column
+//                       with d~ <= m2 + 2 eps, and their exact distances.
+//   scan                one CTA per queued row or column: exact full scans.
+//
+// FP8, tier 0 (k_shortlist.cu; the tile's per-descriptor scales keep the norms
+// out of the product):
 //   pass 1  (tcgen05)  per row: m1 = min d~ and m2' = second smallest of the
-//                      per-32-column minima (an upper bound of the second
+//                      16-column chunk minima (an upper bound of the second
 //                      smallest d~); per column: c1 = min d~.
 //   mid                per row: threshold T = m2' + 2 eps, or "certain no
 //                      match" when m1 - eps >= r^2 (m2' + eps); per column:
@@ -25,21 +40,22 @@
 //                      queued: rows to rescore exactly, rows to rescan, columns
 //                      to rescan.
 //   rescore            one warp per queued row: exact distances of S.
-//   scan               one CTA per queued row or column: exact full scans.
 //
 // Pair routing. When the bound is too loose for a pair's distances (FP8 on
 // unit-length descriptors: eps ~ 0.1 against distance gaps of the same size),
 // most rows would overflow S and be settled one row at a time. Such a pair is
 // routed instead to the tiled exact FP32 kernel, which settles every row and
 // column of it:
-//   - before pass 1: a pair with non-finite or huge inputs (unsafe);
-//   - after pass 1 (mid, FP8): more than 1/8 of its undecided rows are "wide":
+//   - before the passes: a pair with non-finite or huge inputs (unsafe);
+//   - FP8 after pass 1 (mid): more than 1/8 of its undecided rows are "wide":
 //     more than half of their 16-column chunks (and more than kSlRowSlots) had
-//     a minimum within 2 eps above the running row minimum; pass 2 skips
-//     routed pairs;
-//   - after pass 2 (finalize): more than 1/8 as many row halves as rows
+//     a minimum within 2 eps above the running row minimum; the BF16 passes
+//     take the pair over (rescue);
+//   - FP8 after pass 2 (finalize): more than 1/8 as many row halves as rows
 //     had a wide shortlist, more than half_recs / 2 hit groups of one
-//     column range (pass 2 counts them).
+//     column range (pass 2 counts them);
+//   - BF16 (resolve): more than 1/8 of its rows have more columns in their
+//     window than a shortlist holds (cand_cap).
 // The routed pairs' exact work items are planned on the device (route_plan,
 // route_apply), run by exact_kernel, and route_finalize writes their rows'
 // decisions; the results stay bit-exact whichever way a pair goes.
@@ -50,7 +66,7 @@
 
 namespace slm {
 
-// Pass 2 keeps, per row, column range and column half, up to half_recs
+// FP8 pass 2 keeps, per row, column range and column half, up to half_recs
 // (SlArgs; the autotuner's shortlist_k, default kSlHalfRecs) records of 4
 // consecutive columns (the group's first column and its 4 d~ values): one
 // vector store per hit group. A half with more hit groups overflows and the
@@ -63,23 +79,29 @@ constexpr int kSlRowSlots = 32;
 // rows); each range keeps its own records per row, so their memory is
 // (rows x ranges) x 2 half_recs records.
 constexpr uint32_t kSlMaxRanges = 4;
-constexpr int kSlStages = 4;       // b-tile ring depth (FP8; BF16 tiles are larger: 3)
+constexpr int kSlStages = 4;       // FP8 b-tile ring depth
 constexpr int kSlEpWarps = 16;     // epilogue warps
 constexpr int kSlThreads = 32 * (2 + kSlEpWarps);  // producer, MMA, epilogue
+constexpr int kTopEpWarps = 16;
+constexpr int kTopThreads = 32 * (2 + kTopEpWarps);
+constexpr uint32_t kResolveRows = 16;  // undecided rows per CTA of the resolve kernel
 
 // Operand tile sizes per 128 descriptors.
 //
 // BF16 tiles carry the squared norms into the tensor-core product: after the
-// 32 KiB K-major 128B-swizzled image of the components comes a 6 KiB
-// extension, K-major without swizzle, with three 16-byte core-matrix columns
-// per row: kc0 = [hi, lo, 1, 1, 0..], kc1 = [1, 1, hi, lo, 0..], kc2 = 0, where
-// hi + lo is |v|^2 / 2 split into two bf16. A tile read as operand A from kc0
-// and as operand B from kc1 contributes (|a|^2 + |b|^2) / 2 in one K = 16 step;
-// the 8 steps over the components run with B negated, so the accumulator holds
-// d~ / 2 = (|a|^2 + |b|^2) / 2 - a.b directly.
+// 32 KiB K-major 128B-swizzled image of the components comes a 4 KiB
+// extension, K-major without swizzle, per 8 rows one core matrix (8 x 16
+// bytes) for each operand role: kc0 = [hi, lo, 1, 1, 0..], kc1 = [1, 1, hi, lo,
+// 0..], where hi + lo is |v|^2 / 4 split into two bf16. One K = 16 step whose
+// descriptors' leading offset is 0 reads its core matrix twice along K: operand
+// A from kc0 and operand B from kc1 then contribute (|a|^2 + |b|^2) / 2; the 8
+// steps over the components run with B negated, so the accumulator holds
+// d~ / 2 = (|a|^2 + |b|^2) / 2 - a.b directly. (With a core matrix of zeros for
+// the second half, two a tiles and two stages of two b tiles would not fit
+// into a CTA's shared memory.)
 constexpr uint32_t kBf16TileBytes = 128 * 128 * 2;                    // 32 KiB components
-constexpr uint32_t kBf16ExtBytes = 16 * 3 * 128;                      // 6 KiB: 16 row groups x 3 core matrices
-constexpr uint32_t kBf16TileStride = kBf16TileBytes + kBf16ExtBytes;  // 38 KiB per tile (1024-byte multiple)
+constexpr uint32_t kBf16ExtBytes = 16 * 2 * 128;                      // 4 KiB: 16 row groups x 2 core matrices
+constexpr uint32_t kBf16TileStride = kBf16TileBytes + kBf16ExtBytes;  // 36 KiB per tile (1024-byte multiple)
 constexpr uint32_t kFp8TileBytes = 128 * 128;                         // 16 KiB
 
 // Per view, from the pack kernel: float bits of non-negative maxima
@@ -104,6 +126,17 @@ struct SlItem {
     uint32_t pad[3];
 };
 
+// One segment of the BF16 pass: nat (1 or 2) a tiles from store tile a_tile
+// against nt b tiles from store tile b_tile, of which ncols columns are the
+// pair's, the first of them column j0; the rows' results go to part `part`
+// (parts of 128 << (tshift - 7) rows, SlArgs). dir 0: a and b as the pair names
+// them, dir 1: exchanged.
+struct TopItem {
+    uint32_t a_tile, b_tile;
+    uint16_t nat, dir;
+    uint32_t nt, ncols, j0, part, pair;
+};
+
 // Per-pair extras of the shortlist path.
 struct SlPair {
     uint32_t rbase;    // first entry in per-row arrays (multiple of 128)
@@ -117,6 +150,7 @@ struct SlPair {
     uint32_t xpart;    // routed: first exact work item (= first RowPart block)
     uint32_t blk;      // first entry of the pair's row blocks in SlArgs::blkcnt
     uint32_t rescued;  // per launch (FP8 plans): settled by the BF16 passes instead
+    uint32_t tblk_a, tblk_b;  // BF16 pass: first block (SlArgs::tblk) of each direction
     uint32_t crbase;   // first candidate row: the records of row i and column range c at
                        // crbase + c * (na padded to 128) + i (sl_cand_row)
 };
@@ -147,8 +181,8 @@ struct SlQueue {
     uint32_t pair, kind, i, j;
 };
 
-// Counters in the plan's control block (u32 words after work/error).
-enum : int { kCtlRescored = 2, kCtlQueueRows = 3, kCtlQueueCols = 4, kCtlMaxErr = 5, kCtlScanLen = 6,
+// Counters in the plan's control block (word 1: the error word).
+enum : int { kCtlGroups = 0, kCtlRescored = 2, kCtlQueueRows = 3, kCtlQueueCols = 4, kCtlMaxErr = 5, kCtlScanLen = 6,
              kCtlRescoreLen = 7, kCtlXItems = 8, kCtlXWork = 9, kCtlRoutedPairs = 10, kCtlRoutedRows = 11,
              kCtlRoutedCols = 12, kCtlRouteMarks = 13, kCtlRescuedPairs = 14, kCtlRescuedRows = 15 };
 
@@ -202,8 +236,19 @@ struct SlArgs {
     // rescued by a second, BF16 run of eps / pass 1 / mid / pass 2 / finalize
     // over those pairs only (tier 1), instead of the exact kernel
     uint32_t half_recs;          // records per candidate row and column half (1..kSlHalfRecsMax)
-    uint32_t rescue;             // tier 0 of an FP8 plan: mid marks pairs rescued, not routed
     uint32_t tier;               // 0: the plan's precision; 1: the BF16 rescue of an FP8 plan
+    // BF16 pass
+    const TopItem *titems;       // in the order the CTAs run them
+    const uint32_t *tstart;      // CTA c runs titems[tstart[c] .. tstart[c + 1])
+    uint32_t tgrid;
+    uint32_t tshift;             // log2 of the rows per block and part: 7 or 8
+    const uint2 *tblk;           // per block of rows: {first part, parts}
+    float2 *topmm;               // per part row: (m1, m2)
+    uint32_t *topj;              // and the column of m1
+    uint32_t max_na;
+    uint32_t cand_cap;           // resolve: columns a row's shortlist holds
+    uint32_t *ulist;             // undecided rows by pair (from SlPair::rbase)
+    uint2 *ugroups;              // {pair, first entry of its list}, kResolveRows rows each
 };
 
 // Whether a pair takes part in this tier's per-pair kernels (pass 2, finalize,
@@ -220,15 +265,20 @@ void launch_pack_lowp(const uint4 *tab, uint32_t ntiles, const float *raw, int f
 
 // Kernel image / attribute set-up (outside stream capture).
 cudaError_t init_shortlist_kernels();
+cudaError_t init_top2_kernels();
 
-// The pipeline of one shortlist launch (after counters are cleared):
-// eps, pass 1, mid, pass 2, then finalize / routing / rescore / scan / compact.
-// Returns the number of kernels the call launched.
+// The pipeline of one shortlist launch (after counters are cleared). BF16:
+// eps, pass, decide, resolve; FP8: eps, pass 1, mid, pass 2, finalize, then the
+// BF16 steps over the rescued pairs; both: the tail. Each returns the number of
+// kernels it launched.
 int launch_shortlist_eps(const SlArgs &a, cudaStream_t s);
+int launch_top2_pass(const SlArgs &a, cudaStream_t s);
+int launch_top2_decide(const SlArgs &a, cudaStream_t s);
+int launch_top2_resolve(const SlArgs &a, int sms, cudaStream_t s);
 int launch_shortlist_pass(const SlArgs &a, int pass, int sms, cudaStream_t s);
 int launch_shortlist_mid(const SlArgs &a, cudaStream_t s);
 int launch_shortlist_finalize(const SlArgs &a, cudaStream_t s);
-// Tier 1 before its pass 1: the rescued pairs' BF16 eps, column minima and counters.
+// Before the rescue tier's pass: the rescued pairs' BF16 eps and counters.
 int launch_shortlist_rescue_prep(const SlArgs &a, cudaStream_t s);
 // After every tier's finalize: routing to the exact kernel, rescore, scans, compaction.
 int launch_shortlist_tail(const SlArgs &a, int sms, cudaStream_t s);

@@ -20,9 +20,9 @@ OUT = os.path.join(ROOT, "build")
 LIB = os.path.join(OUT, "libslm.so")
 
 ARCH = ["-gencode", "arch=compute_103a,code=sm_103a"]
-CU_SOURCES = ["k_exact.cu", "k_compact.cu", "k_shortlist.cu", "k_noalloc.cu", "k_sampson.cu", "k_features.cu", "k_tracks.cu"]
+CU_SOURCES = ["k_exact.cu", "k_compact.cu", "k_shortlist.cu", "k_top2.cu", "k_noalloc.cu", "k_sampson.cu", "k_features.cu", "k_tracks.cu"]
 CPP_SOURCES = ["slm.cpp"]
-HEADERS = ["pack.cuh", "ptx.cuh", "slm_internal.h", "slm_shortlist.h", "fmath_cr.h", "fmath_tables.h"]
+HEADERS = ["pack.cuh", "ptx.cuh", "slm_internal.h", "slm_shortlist.h", "shortlist.cuh", "fmath_cr.h", "fmath_tables.h"]
 
 
 def _nvcc() -> str:
