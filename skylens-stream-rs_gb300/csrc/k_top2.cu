@@ -40,6 +40,7 @@
 // before (N = 128; row and column minima, then the candidates of each row
 // recomputed against a threshold) took 1.33 and 1.64 ms, and the zone's batch
 // with its lists read back 3.50 ms; now 2.29.
+#include <cooperative_groups.h>
 #include <cuda_runtime.h>
 
 #include <cstdint>
@@ -238,7 +239,9 @@ __global__ void __maxnreg__(96) sl_top2_kernel(SlArgs g) {
             }
             for (uint32_t t = 0; t < item.nt && ok; t += 2) {
                 if (!(ok = sl_wait(&S.b_full[st], sph, abort_flag, err))) break;
-                const uint32_t n = item.nt - t > 1 ? 256 : 128;
+                // the pair's columns only, to the next 16 (1.73 -> 1.72 ms on the zone:
+                // tiles of zeros cost time, but little power, and power sets the clock)
+                const uint32_t n = (min(item.ncols - t * kTile, 256u) + 15) & ~15u;
                 const uint32_t idesc = top_idesc(n, false), idesc_neg = top_idesc(n, true);
 #pragma unroll
                 for (uint32_t a = 0; a < 2; ++a) {
@@ -401,78 +404,157 @@ SLM_DEV void row_top2(const SlArgs &g, uint32_t blk0, uint32_t i, float &m1, flo
 }
 
 // The cross-check of row i, whose exact distance to its nearest column j is at
-// least dlow: the column's nearest row is certain when every other row's
-// estimate is more than 2 eps above its best one; row i is certainly not it
-// when dlow lies above the largest distance the best row may have. Anything
-// else is queued for an exact column scan.
+// least dlow, from the column's two smallest estimates c1 (at row i1) and c2:
+// the column's nearest row is certain when every other row's estimate is more
+// than 2 eps above its best one; row i is certainly not it when dlow lies above
+// the largest distance the best row may have. Anything else is queued for an
+// exact column scan.
+SLM_DEV uint32_t mutual_decision(const SlArgs &g, uint32_t p, float eps, uint32_t i, uint32_t j, float dlow, float c1,
+                                 float c2, uint32_t i1) {
+    if (__fsub_rd(c2, c1) > 2.f * eps) return i1 == i ? j : kDecNone;
+    if (dlow > __fadd_ru(c1, eps)) return kDecNone;
+    push_scan(g, p, 1, i, j);
+    return kDecPending;
+}
 SLM_DEV uint32_t mutual_from_top2(const SlArgs &g, uint32_t p, const SlPair &sp, uint32_t i, uint32_t j, float dlow) {
     float c1, c2;
     uint32_t i1;
     row_top2(g, sp.tblk_b, j, c1, c2, i1);
-    if (__fsub_rd(c2, c1) > 2.f * sp.eps) return i1 == i ? j : kDecNone;
-    if (dlow > __fadd_ru(c1, sp.eps)) return kDecNone;
-    push_scan(g, p, 1, i, j);
-    return kDecPending;
+    return mutual_decision(g, p, sp.eps, i, j, dlow, c1, c2, i1);
 }
 
-// One thread per row of a (CTA per pair and 256 rows): the outcome the bounds
-// certify, or the row joins its pair's list of undecided rows. The last CTA
-// of a pair cuts that list into groups of 16 for sl_resolve_kernel.
-constexpr uint32_t kDecideRows = 256;
-__global__ void __launch_bounds__(kDecideRows) sl_decide_kernel(SlArgs g) {
-    const uint32_t p = blockIdx.x, row0 = blockIdx.y * kDecideRows;
+// Row i of pair p joins the undecided rows of its b view; whoever starts a new
+// run of 16 there registers that run as a group for sl_resolve_kernel.
+SLM_DEV void list_undecided(const SlArgs &g, const SlPair &sp, uint32_t p, uint32_t i) {
+    const uint32_t k = atomicAdd(&g.ucnt[sp.ubucket], 1u);
+    g.ulist[sp.ubase + k] = make_uint2(p, i);
+    if (k % kResolveRows == 0)
+        g.ugroups[atomicAdd(&g.ctl[kCtlGroups], 1u)] = make_uint4(sp.ubase + k, sp.ubucket, k, 0u);
+}
+
+// A row whose ratio test the estimates leave open, its nearest column j certain
+// and e1 its exact distance: only the second best's error remains. Returns
+// false when that still leaves it open.
+SLM_DEV bool settle_with_d1(const SlArgs &g, const SlPair &sp, uint32_t p, uint32_t i, uint32_t j, float e1, float m2) {
+    const bool fails = e1 >= __fmul_ru(__fmul_ru(g.ratio2, __fadd_ru(m2, sp.eps)), kUp);
+    const bool passes = e1 < __fmul_rd(__fmul_rd(g.ratio2, __fsub_rd(m2, sp.eps)), kDown);
+    if (!fails && !passes) return false;
+    g.rowdec[sp.rbase + i] = fails ? kDecNone : g.mutual ? mutual_from_top2(g, p, sp, i, j, e1) : j;
+    return true;
+}
+
+// CTA per pair and kDecideThreads x R rows of a, R rows a thread: the outcome
+// the bounds certify. A row whose nearest column is certain but whose ratio
+// test is not gets its exact d1 (settle_with_d1): 3 of 5 such rows, for 1 KB
+// read each, of those that sl_resolve_kernel would read a whole view for.
+// A row is a chain of dependent loads (block, result, the column's block and
+// result). R = 4 keeps four of them going in a thread (71 -> 54 us for the
+// 4.2 M rows of a zone) and lists the open rows for sl_nearest_kernel, 20 us
+// there. Batches too small to fill the GPU that way run R = 1 and take the
+// exact d1 in the CTA that finds the row (one 8192 pair: 13 us against 10 and
+// 13 in a kernel of its own).
+constexpr uint32_t kDecideThreads = 256;
+template <int R>
+__global__ void __launch_bounds__(kDecideThreads) sl_decide_kernel(SlArgs g) {
+    const uint32_t p = blockIdx.x, row0 = blockIdx.y * (kDecideThreads * R);
     const PairMeta pm = g.pairs[p];
     if (row0 >= pm.na) return;  // block-uniform, as below
     const SlPair sp = g.spairs[p];
     if (!sl_pair_on(g, sp)) return;
-    __shared__ uint32_t last;
-    const uint32_t i = row0 + threadIdx.x, lane = threadIdx.x & 31;
-    uint32_t *pc = g.pairctl + 4 * (size_t)p;
-    bool open = false;
-    if (i < pm.na) {
-        uint32_t dec = kDecNone;
-        float m1, m2;
-        uint32_t j;
-        if (pm.nb) {
-            row_top2(g, sp.tblk_a, i, m1, m2, j);
-            // fewer than two columns: the exact second best is infinite (matching.rs:205)
-            if (m2 < __int_as_float(0x7f800000) && !certain_no_match(m1, m2, sp.eps, g.ratio2)) {
-                // the ratio test passes and every other column is certainly farther
-                if (certain_ratio_pass(m1, m2, sp.eps, g.ratio2) && __fsub_rd(m2, m1) > 2.f * sp.eps) {
-                    dec = g.mutual ? mutual_from_top2(g, p, sp, i, j, __fsub_rd(m1, sp.eps)) : j;
-                } else {
-                    dec = kDecPending;
-                    open = true;
-                }
+    __shared__ uint4 found[R == 1 ? kDecideThreads : 1];  // R = 1: this CTA's open rows
+    __shared__ uint32_t n_found, n_settled;
+    if (R == 1 && threadIdx.x == 0) n_found = n_settled = 0;
+    if (R == 1) __syncthreads();
+    const uint32_t lane = threadIdx.x & 31;
+    const float eps = sp.eps;
+    uint32_t j[R], dec[R];
+    float m1[R], m2[R];
+    bool match[R];
+#pragma unroll
+    for (int r = 0; r < R; ++r) {
+        const uint32_t i = row0 + r * kDecideThreads + threadIdx.x;
+        m1[r] = m2[r] = __int_as_float(0x7f800000);
+        j[r] = 0;
+        if (i < pm.na && pm.nb) row_top2(g, sp.tblk_a, i, m1[r], m2[r], j[r]);
+    }
+#pragma unroll
+    for (int r = 0; r < R; ++r) {
+        // fewer than two columns: the exact second best is infinite (matching.rs:205)
+        const bool some = m2[r] < __int_as_float(0x7f800000) && !certain_no_match(m1[r], m2[r], eps, g.ratio2);
+        const bool unique = __fsub_rd(m2[r], m1[r]) > 2.f * eps;  // every other column is farther
+        match[r] = some && unique && certain_ratio_pass(m1[r], m2[r], eps, g.ratio2);
+        dec[r] = match[r] ? j[r] : some ? kDecPending : kDecNone;
+        const bool open = some && !match[r];
+        const uint32_t m = __ballot_sync(0xffffffffu, open);
+        if (m) {
+            uint32_t base = 0;
+            if (lane == 0) base = atomicAdd(R == 1 ? &n_found : &g.ctl[kCtlOpen], (uint32_t)__popc(m));
+            base = __shfl_sync(0xffffffffu, base, 0);
+            if (open)
+                (R == 1 ? found : g.olist)[base + __popc(m & ((1u << lane) - 1))] =
+                    make_uint4(p, row0 + r * kDecideThreads + threadIdx.x, unique ? j[r] : kDecNone,
+                               __float_as_uint(m2[r]));
+        }
+    }
+    if (g.mutual) {
+        float c1[R], c2[R];
+        uint32_t i1[R];
+#pragma unroll
+        for (int r = 0; r < R; ++r)
+            if (match[r]) row_top2(g, sp.tblk_b, j[r], c1[r], c2[r], i1[r]);
+#pragma unroll
+        for (int r = 0; r < R; ++r)
+            if (match[r])
+                dec[r] = mutual_decision(g, p, eps, row0 + r * kDecideThreads + threadIdx.x, j[r],
+                                         __fsub_rd(m1[r], eps), c1[r], c2[r], i1[r]);
+    }
+#pragma unroll
+    for (int r = 0; r < R; ++r) {
+        const uint32_t i = row0 + r * kDecideThreads + threadIdx.x;
+        if (i < pm.na) g.rowdec[sp.rbase + i] = dec[r];
+    }
+    if constexpr (R == 1) {
+        __syncthreads();  // the open rows are listed, and their decisions written as pending
+        for (uint32_t s0 = (threadIdx.x / 32) * 4; s0 < n_found; s0 += kDecideThreads / 8) {  // warp-uniform
+            const uint32_t s = s0 + (lane >> 3);
+            const uint4 o = found[min(s, n_found - 1)];
+            const bool exact = o.z != kDecNone;
+            const float e1 = dist8(g.raw + (size_t)(pm.a_row0 + o.y) * kDesc,
+                                   g.raw + (size_t)(pm.b_row0 + (exact ? o.z : 0)) * kDesc);
+            if (s < n_found && (lane & 7) == 0) {
+                if (exact && settle_with_d1(g, sp, p, o.y, o.z, e1, __uint_as_float(o.w)))
+                    atomicAdd(&n_settled, 1u);
+                else
+                    list_undecided(g, sp, p, o.y);
             }
         }
-        g.rowdec[sp.rbase + i] = dec;
-    }
-    const uint32_t m = __ballot_sync(0xffffffffu, open);
-    if (m) {
-        uint32_t base = 0;
-        if (lane == 0) base = atomicAdd(&pc[kPcOpen], (uint32_t)__popc(m));
-        base = __shfl_sync(0xffffffffu, base, 0);
-        if (open) g.ulist[sp.rbase + base + __popc(m & ((1u << lane) - 1))] = i;
-    }
-    const uint32_t nblk = (pm.na + kDecideRows - 1) / kDecideRows;
-    if (nblk > 1) {
-        __threadfence();
         __syncthreads();
-        if (threadIdx.x == 0) last = atomicAdd(&pc[kPcMidDone], 1u) == nblk - 1;
-        __syncthreads();
-        if (!last) return;
-        __threadfence();
-    } else {
-        __syncthreads();
+        if (threadIdx.x == 0 && n_settled) atomicAdd(&g.ctl[kCtlRescored], n_settled);
     }
-    __shared__ uint32_t first, n;
-    if (threadIdx.x == 0) {
-        n = (atomicAdd(&pc[kPcOpen], 0u) + kResolveRows - 1) / kResolveRows;
-        first = n ? atomicAdd(&g.ctl[kCtlGroups], n) : 0;
+}
+
+// The open rows of a large batch, two lanes each.
+__global__ void __launch_bounds__(256) sl_nearest_kernel(SlArgs g) {
+    const uint32_t lane = threadIdx.x & 31, n = g.ctl[kCtlOpen];
+    const uint32_t gw = (blockIdx.x * blockDim.x + threadIdx.x) >> 5, nw = (gridDim.x * blockDim.x) >> 5;
+    uint32_t settled = 0;
+    for (uint32_t s0 = gw * 16; s0 < n; s0 += nw * 16) {  // warp-uniform
+        const uint32_t s = s0 + (lane >> 1);
+        const uint4 o = g.olist[min(s, n - 1)];
+        const PairMeta pm = g.pairs[o.x];
+        const SlPair sp = g.spairs[o.x];
+        const bool exact = o.z != kDecNone;
+        const float e1 = dist2(g.raw + (size_t)(pm.a_row0 + o.y) * kDesc,
+                               g.raw + (size_t)(pm.b_row0 + (exact ? o.z : 0)) * kDesc);
+        if (s < n && (lane & 1) == 0) {
+            if (exact && settle_with_d1(g, sp, o.x, o.y, o.z, e1, __uint_as_float(o.w)))
+                ++settled;
+            else
+                list_undecided(g, sp, o.x, o.y);
+        }
     }
-    __syncthreads();
-    for (uint32_t k = threadIdx.x; k < n; k += kDecideRows) g.ugroups[first + k] = make_uint2(p, k * kResolveRows);
+    settled = __reduce_add_sync(0xffffffffu, settled);
+    if (lane == 0 && settled) atomicAdd(&g.ctl[kCtlRescored], settled);
 }
 
 // --------------------------------------------------------------- resolve
@@ -490,61 +572,75 @@ SLM_DEV uint4 op_chunk(const SlArgs &g, uint32_t r, uint32_t c) {
     return *reinterpret_cast<const uint4 *>(t + (((c & 7) ^ (r & 7)) * 16));
 }
 
-// One CTA per group of 16 undecided rows of a pair (about 1 % of a zone's
-// rows): their estimates against every column once more, the columns within
-// the window m2 + 2 eps, the exact distances of those, and the reference's
-// row rule (matching.rs:182-187, 204-206). The group's rows lie scattered in
-// the view, which no shared-memory descriptor of tcgen05 can address without
-// staging, and 16 rows are a warp-level tile exactly: m16n8k16 with both
-// operands straight from the operand image. The sum over k may run in any
-// order, so lane t of four takes the 16-byte chunks 4 q + t of its row, on
+// One cluster per group of 16 undecided rows (about 1 in 200 of a zone's) of
+// one b view: their estimates against every column once more, the columns
+// within the window m2 + 2 eps, the exact distances of those, and the
+// reference's row rule (matching.rs:182-187, 204-206). The group's rows lie
+// scattered over views, which no shared-memory descriptor of tcgen05 can
+// address without staging, and 16 rows are a warp-level tile exactly: m16n8k16
+// with both operands straight from the operand image. The sum over k may run in
+// any order, so lane t of four takes the 16-byte chunks 4 q + t of its row, on
 // both sides, and each chunk is the operand words of two steps.
+// Reading the b view (256 bytes a column) is the cost, so rows are grouped by b
+// view over all pairs, and the cluster's CTAs share a group's columns: a large
+// view is not one CTA's chain of loads. The candidates meet in CTA 0's shared
+// memory, and the exact distances are spread over the cluster's warps again.
 // A row with more columns in the window than g.cand_cap is scanned exactly
 // instead; a pair with more than 1/8 such rows goes to the exact kernel.
 __global__ void __launch_bounds__(256) sl_resolve_kernel(SlArgs g) {
-    __shared__ uint32_t cand[kResolveRows][4 * kSlHalfRecsMax / 2];
-    __shared__ float cval[kResolveRows][4 * kSlHalfRecsMax / 2];
-    __shared__ uint32_t cnt[kResolveRows], rows[kResolveRows];
+    constexpr uint32_t kCap = 2 * kSlHalfRecsMax;
+    __shared__ uint32_t cand_s[kResolveRows][kCap];
+    __shared__ float cval_s[kResolveRows][kCap];
+    __shared__ uint32_t cnt_s[kResolveRows];
+    __shared__ uint2 rows[kResolveRows];
+    __shared__ uint32_t arow[kResolveRows];
     __shared__ float win[kResolveRows], nrm[kResolveRows];
+    const cooperative_groups::cluster_group cl = cooperative_groups::this_cluster();
+    const uint32_t rank = cl.block_rank(), ncta = cl.num_blocks();
+    uint32_t (*cand)[kCap] = cl.map_shared_rank(cand_s, 0);
+    float (*cval)[kCap] = cl.map_shared_rank(cval_s, 0);
+    uint32_t *cnt = cl.map_shared_rank(cnt_s, 0);
     const uint32_t tid = threadIdx.x, warp = tid >> 5, lane = tid & 31;
     const uint32_t gr = lane >> 2, t = lane & 3;
+    const uint32_t gwarp = rank * (blockDim.x / 32) + warp, nwarp = ncta * (blockDim.x / 32);
     const float kInf = __int_as_float(0x7f800000);
     const uint32_t ng = g.ctl[kCtlGroups];
     uint32_t w_rows = 0;
     float w_err = 0.f;
-    for (uint32_t e = blockIdx.x; e < ng; e += gridDim.x) {
-        const uint2 ug = g.ugroups[e];
-        const PairMeta pm = g.pairs[ug.x];
-        const SlPair sp = g.spairs[ug.x];
-        const uint32_t n = min(kResolveRows, g.pairctl[4 * (size_t)ug.x + kPcOpen] - ug.y);
+    for (uint32_t e = blockIdx.x / ncta; e < ng; e += gridDim.x / ncta) {
+        const uint4 ug = g.ugroups[e];
+        const uint32_t n = min(kResolveRows, g.ucnt[ug.y] - ug.z);
+        const PairMeta pb = g.pairs[g.ulist[ug.x].x];  // every pair of the group has this b view
         if (tid < kResolveRows) {
             // rows past the list's end repeat its first row and admit nothing
-            const uint32_t i = g.ulist[sp.rbase + ug.y + (tid < n ? tid : 0)];
+            const uint2 r = g.ulist[ug.x + (tid < n ? tid : 0)];
+            const SlPair sp = g.spairs[r.x];
             float m1, m2;
             uint32_t j;
-            row_top2(g, sp.tblk_a, i, m1, m2, j);
-            rows[tid] = i;
-            cnt[tid] = 0;
+            row_top2(g, sp.tblk_a, r.y, m1, m2, j);
+            rows[tid] = r;
+            arow[tid] = g.pairs[r.x].a_row0 + r.y;
+            cnt_s[tid] = 0;
             win[tid] = tid < n ? window_up(m2, sp.eps) : -kInf;
-            nrm[tid] = g.norms[pm.a_row0 + i];
+            nrm[tid] = g.norms[arow[tid]];
         }
-        __syncthreads();
+        cl.sync();
         uint32_t A[2][16];  // rows gr and gr + 8: word w of chunk q is A[.][4 q + w]
 #pragma unroll
         for (int h = 0; h < 2; ++h)
 #pragma unroll
             for (int q = 0; q < 4; ++q) {
-                const uint4 v = op_chunk(g, pm.a_row0 + rows[gr + 8 * h], 4 * q + t);
+                const uint4 v = op_chunk(g, arow[gr + 8 * h], 4 * q + t);
                 A[h][4 * q] = v.x, A[h][4 * q + 1] = v.y, A[h][4 * q + 2] = v.z, A[h][4 * q + 3] = v.w;
             }
         const float na0 = nrm[gr], na1 = nrm[gr + 8], w0 = win[gr], w1 = win[gr + 8];
-        const uint32_t n8 = (pm.nb + 7) / 8;  // columns past nb have a NaN norm: never admitted
-        for (uint32_t c8 = warp; c8 < n8; c8 += 16) {
+        const uint32_t n8 = (pb.nb + 7) / 8;  // columns past nb have a NaN norm: never admitted
+        for (uint32_t c8 = gwarp; c8 < n8; c8 += 2 * nwarp) {
             uint4 B[2][4];
-            const bool two = c8 + 8 < n8;
+            const bool two = c8 + nwarp < n8;
 #pragma unroll
             for (int u = 0; u < 2; ++u) {
-                const uint32_t r = pm.b_row0 + (c8 + (u && two ? 8 : 0)) * 8 + gr;
+                const uint32_t r = pb.b_row0 + (c8 + (u && two ? nwarp : 0)) * 8 + gr;
 #pragma unroll
                 for (int q = 0; q < 4; ++q) B[u][q] = op_chunk(g, r, 4 * q + t);
             }
@@ -558,8 +654,8 @@ __global__ void __launch_bounds__(256) sl_resolve_kernel(SlArgs g) {
                     mma_16816(acc, A[0][4 * q + 2], A[1][4 * q + 2], A[0][4 * q + 3], A[1][4 * q + 3], B[u][q].z,
                               B[u][q].w);
                 }
-                const uint32_t j = (c8 + 8 * u) * 8 + 2 * t;
-                const float2 nb = *reinterpret_cast<const float2 *>(g.norms + pm.b_row0 + j);
+                const uint32_t j = (c8 + nwarp * u) * 8 + 2 * t;
+                const float2 nb = *reinterpret_cast<const float2 *>(g.norms + pb.b_row0 + j);
                 const float d[4] = {fmaf(-2.f, acc[0], na0 + nb.x), fmaf(-2.f, acc[1], na0 + nb.y),
                                     fmaf(-2.f, acc[2], na1 + nb.x), fmaf(-2.f, acc[3], na1 + nb.y)};
 #pragma unroll
@@ -574,57 +670,71 @@ __global__ void __launch_bounds__(256) sl_resolve_kernel(SlArgs g) {
                     }
             }
         }
-        __syncthreads();
-        // exact distances: a warp per row, four columns at a time (8 lanes each)
-        for (uint32_t r = warp; r < n; r += 8) {
-            const uint32_t i = rows[r], m = cnt[r];
+        cl.sync();
+        // exact distances, 2 lanes a column: a warp per row where the cluster has
+        // 16 warps, else 8 lanes per row, four rows of a warp side by side
+        const uint32_t width = nwarp >= kResolveRows ? 32 : 8, sub = lane & (width - 1);
+        const uint32_t per = 32 / width, cols = width / 2;
+        for (uint32_t r0 = gwarp * per; r0 < n; r0 += nwarp * per) {  // warp-uniform
+            const uint32_t r = min(r0 + lane / width, n - 1);
+            const bool have = r0 + lane / width < n;
+            const uint32_t p = rows[r].x, i = rows[r].y, m = cnt[r];
+            const PairMeta pm = g.pairs[p];
+            const SlPair sp = g.spairs[p];
             const float *a = g.raw + (size_t)(pm.a_row0 + i) * kDesc;
             const float *B = g.raw + (size_t)pm.b_row0 * kDesc;
-            if (m > g.cand_cap) {
-                if (lane == 0) {
-                    push_scan(g, ug.x, 0, i, 0);
-                    const uint32_t over = atomicAdd(&g.pairctl[4 * (size_t)ug.x + kPcOver], 1u);
-                    if (over * 8 <= pm.na && (over + 1) * 8 > pm.na) {
-                        g.spairs[ug.x].routed = 1;
-                        atomicAdd(&g.ctl[kCtlRouteMarks], 1u);
-                    }
-                }
-                continue;
-            }
+            const bool over = m > g.cand_cap;
+            const uint32_t mine_n = have && !over ? m : 0;
+            const uint32_t most = __reduce_max_sync(0xffffffffu, mine_n);
             float e1 = kInf, e2 = kInf;
             uint32_t ej = 0xffffffffu;
-            for (uint32_t s = 0; s < m; s += 4) {
-                const uint32_t mine = s + (lane >> 3);
-                const uint32_t j = cand[r][mine < m ? mine : s];
-                const float d = dist8(a, B + (size_t)j * kDesc);
-                if (mine < m) w_err = fmaxf(w_err, fabsf(d - cval[r][mine]));
-#pragma unroll
-                for (uint32_t q = 0; q < 4; ++q) {
-                    const float dq = __shfl_sync(0xffffffffu, d, q * 8);
-                    const uint32_t jq = __shfl_sync(0xffffffffu, j, q * 8);
-                    if (s + q < m) {
-                        if (dq < e1 || (dq == e1 && jq < ej)) {
-                            e2 = e1;
-                            e1 = dq;
-                            ej = jq;
-                        } else if (dq < e2) {
-                            e2 = dq;
-                        }
+            for (uint32_t s = 0; s < most; s += cols) {
+                const uint32_t mine = s + (sub >> 1);
+                const uint32_t j = mine < mine_n ? cand[r][mine] : 0;
+                const float d = dist2(a, B + (size_t)j * kDesc);
+                if (mine < mine_n) {
+                    w_err = fmaxf(w_err, fabsf(d - cval[r][mine]));
+                    if (d < e1 || (d == e1 && j < ej)) {
+                        e2 = e1;
+                        e1 = d;
+                        ej = j;
+                    } else if (d < e2) {
+                        e2 = d;
                     }
                 }
             }
-            if (lane == 0) {
-                ++w_rows;
-                uint32_t dec = kDecNone;
-                if (ej != 0xffffffffu && e2 < kInf && !(e1 >= __fmul_rn(g.ratio2, e2)))
-                    dec = g.mutual ? mutual_from_top2(g, ug.x, sp, i, ej, e1) : ej;
-                g.rowdec[sp.rbase + i] = dec;
+            // over the row's lane pairs (no column occurs twice)
+            for (uint32_t o = 2; o < width; o <<= 1) {
+                const float o1 = __shfl_xor_sync(0xffffffffu, e1, o), o2 = __shfl_xor_sync(0xffffffffu, e2, o);
+                const uint32_t oj = __shfl_xor_sync(0xffffffffu, ej, o);
+                e2 = fminf(fminf(e2, o2), fmaxf(e1, o1));
+                if (o1 < e1 || (o1 == e1 && oj < ej)) {
+                    e1 = o1;
+                    ej = oj;
+                }
+            }
+            if (have && sub == 0) {
+                if (over) {
+                    push_scan(g, p, 0, i, 0);
+                    const uint32_t was = atomicAdd(&g.pairctl[4 * (size_t)p + kPcOver], 1u);
+                    if (was * 8 <= pm.na && (was + 1) * 8 > pm.na) {
+                        g.spairs[p].routed = 1;
+                        atomicAdd(&g.ctl[kCtlRouteMarks], 1u);
+                    }
+                } else {
+                    ++w_rows;
+                    uint32_t dec = kDecNone;
+                    if (ej != 0xffffffffu && e2 < kInf && !(e1 >= __fmul_rn(g.ratio2, e2)))
+                        dec = g.mutual ? mutual_from_top2(g, p, sp, i, ej, e1) : ej;
+                    g.rowdec[sp.rbase + i] = dec;
+                }
             }
         }
-        __syncthreads();
+        cl.sync();  // CTA 0's lists are free, and no CTA leaves while they are read
     }
 #pragma unroll
     for (int o = 16; o; o >>= 1) w_err = fmaxf(w_err, __shfl_xor_sync(0xffffffffu, w_err, o));
+    w_rows = __reduce_add_sync(0xffffffffu, w_rows);
     if (lane == 0 && w_rows) {
         atomicAdd(&g.ctl[kCtlRescored], w_rows);
         atomicMax(&g.ctl[kCtlMaxErr], __float_as_uint(w_err));  // non-negative: bits order as values
@@ -649,15 +759,41 @@ int launch_top2_pass(const SlArgs &a, cudaStream_t s) {
     return 1;
 }
 
-int launch_top2_decide(const SlArgs &a, cudaStream_t s) {
+int launch_top2_decide(const SlArgs &a, int sms, cudaStream_t s) {
     if (!a.npairs || !a.max_na) return 0;
-    sl_decide_kernel<<<dim3(a.npairs, (a.max_na + kDecideRows - 1) / kDecideRows), kDecideRows, 0, s>>>(a);
-    return 1;
+    // four rows a thread once that still gives every SM its eight CTAs
+    if (a.n_rows < 8ull * sms * 4 * kDecideThreads) {
+        sl_decide_kernel<1><<<dim3(a.npairs, (a.max_na + kDecideThreads - 1) / kDecideThreads), kDecideThreads, 0,
+                              s>>>(a);
+        return 1;
+    }
+    sl_decide_kernel<4><<<dim3(a.npairs, (a.max_na + 4 * kDecideThreads - 1) / (4 * kDecideThreads)), kDecideThreads, 0,
+                          s>>>(a);
+    sl_nearest_kernel<<<2 * sms, 256, 0, s>>>(a);
+    return 2;
 }
 
 int launch_top2_resolve(const SlArgs &a, int sms, cudaStream_t s) {
     if (!a.npairs || !a.max_na) return 0;
-    sl_resolve_kernel<<<4 * sms, 256, 0, s>>>(a);
+    // A group is a chain of dependent loads. With many groups (1 undecided row
+    // in 100 assumed) they cover each other: four warps a group, four groups a
+    // SM. With few, eight warps a CTA and the largest portable cluster that does
+    // not exceed the GPU (zone: 136 us against 365 with clusters of 4; one 8192
+    // pair: 24 us against 93 with one CTA).
+    const uint64_t est = a.n_rows / (100 * kResolveRows) + 1;
+    const bool many = est >= (uint64_t)sms;
+    uint32_t c = 1;
+    while (!many && c < 8 && 2 * c * est <= 2ull * sms) c *= 2;
+    cudaLaunchConfig_t cfg{};
+    cudaLaunchAttribute at{};
+    at.id = cudaLaunchAttributeClusterDimension;
+    at.val.clusterDim = {c, 1, 1};
+    cfg.gridDim = dim3((unsigned)((many ? 4 : 2) * sms) / c * c);
+    cfg.blockDim = dim3(many ? 128 : 256);
+    cfg.stream = s;
+    cfg.attrs = &at;
+    cfg.numAttrs = 1;
+    cudaLaunchKernelEx(&cfg, sl_resolve_kernel, a);
     return 1;
 }
 

@@ -232,4 +232,31 @@ SLM_DEV float dist8(const float *__restrict__ p, const float *__restrict__ r) {
     return s;
 }
 
+// The same by 2 lanes, 16 distances a warp: lane h of a pair holds the sums of
+// components 8c + 4h .. 8c + 4h + 3; the even lane adds its four in order and
+// hands the sum to the odd lane, which adds its own. p and r (16-byte aligned)
+// may differ per pair of lanes; the result is valid in both.
+SLM_DEV float dist2(const float *__restrict__ p, const float *__restrict__ r) {
+    const uint32_t h = threadIdx.x & 1;
+    const float4 *p4 = reinterpret_cast<const float4 *>(p) + h, *r4 = reinterpret_cast<const float4 *>(r) + h;
+    float acc[4] = {0.f, 0.f, 0.f, 0.f};
+#pragma unroll
+    for (int c = 0; c < 16; ++c) {
+        const float4 x = p4[2 * c], y = r4[2 * c];
+        const float xs[4] = {x.x, x.y, x.z, x.w}, ys[4] = {y.x, y.y, y.z, y.w};
+#pragma unroll
+        for (int k = 0; k < 4; ++k) {
+            const float t = __fsub_rn(xs[k], ys[k]);
+            acc[k] = __fadd_rn(acc[k], __fmul_rn(t, t));
+        }
+    }
+    float s = 0.f;
+#pragma unroll
+    for (int k = 0; k < 4; ++k) s = __fadd_rn(s, acc[k]);
+    float u = __shfl_xor_sync(0xffffffffu, s, 1);  // the odd lane gets the even lane's sum
+#pragma unroll
+    for (int k = 0; k < 4; ++k) u = __fadd_rn(u, acc[k]);
+    return __shfl_sync(0xffffffffu, u, (threadIdx.x & 31) | 1);
+}
+
 }  // namespace slm

@@ -275,9 +275,9 @@ struct slm_plan {
     std::vector<TopItem> titems;
     std::vector<uint32_t> tstart;
     std::vector<uint2> tblk;
-    uint32_t tshift = 8, max_na = 0;
+    uint32_t tshift = 8, max_na = 0, buckets = 0;
     uint64_t top_parts = 0;
-    DevBuf d_titems, d_tstart, d_tblk, d_topmm, d_topj, d_ulist, d_ugroups;
+    DevBuf d_titems, d_tstart, d_tblk, d_topmm, d_topj, d_olist, d_ulist, d_ucnt, d_ugroups;
     bool dump = false;
     uint32_t min_matches = 0;        // pairs with fewer matches report none
     cudaGraphExec_t exec = nullptr;
@@ -300,13 +300,13 @@ struct slm_plan {
 
 // Every device buffer of a plan: all are used on the plan's stream only, and
 // allocated ordered on it (DevBuf::order_on).
-std::array<DevBuf *, 36> plan_buffers(slm_plan *p) {
+std::array<DevBuf *, 38> plan_buffers(slm_plan *p) {
     return {&p->d_meta, &p->d_items, &p->d_parts, &p->d_colbest, &p->d_slots, &p->d_counts, &p->d_ctl,
             &p->d_offsets, &p->d_dense, &p->d_sitems, &p->d_spairs, &p->d_rowpart, &p->d_rownear,
             &p->d_colmin, &p->d_rowthr, &p->d_colthr, &p->d_rowcnt, &p->d_rowrec, &p->d_rowrecj,
             &p->d_colcnt, &p->d_rowdec, &p->d_queue, &p->d_rqueue, &p->d_dump, &p->d_xlist, &p->d_xitems,
             &p->d_xparts, &p->d_blkcnt, &p->d_pairctl, &p->d_titems, &p->d_tstart, &p->d_tblk, &p->d_topmm,
-            &p->d_topj, &p->d_ulist, &p->d_ugroups};
+            &p->d_topj, &p->d_olist, &p->d_ulist, &p->d_ucnt, &p->d_ugroups};
 }
 // Frees a plan's buffers while its stream still exists (their frees are
 // ordered on it): owners call it before destroying that stream.
@@ -548,9 +548,13 @@ slm_status plan_fp8_items(slm_plan *p, const slm_pair *pairs) {
 slm_status plan_build_shortlist(slm_plan *p, const slm_pair *pairs) {
     slm_ctx *c = p->ctx;
     p->spairs.assign(p->np, SlPair{});
-    uint64_t rb = 0, row_tiles = 0, blk = 0, groups = 0;
+    uint64_t rb = 0, row_tiles = 0, blk = 0;
     p->row_blocks = 1;
-    p->max_na = 0;
+    p->max_na = p->buckets = 0;
+    // undecided rows are listed by b view: each view's share of the list holds
+    // every row that meets it
+    std::vector<uint32_t> bucket(p->st->n.size(), 0xffffffffu);
+    std::vector<uint64_t> bucket_rows;
     for (uint32_t k = 0; k < p->np; ++k) {
         const PairMeta &m = p->meta[k];
         SlPair &sp = p->spairs[k];
@@ -560,11 +564,28 @@ slm_status plan_build_shortlist(slm_plan *p, const slm_pair *pairs) {
         blk += (m.na + kSlRowBlock - 1) / kSlRowBlock;
         p->row_blocks = std::max(p->row_blocks, (std::max(m.na, m.nb) + kSlRowBlock - 1) / kSlRowBlock);
         p->max_na = std::max(p->max_na, m.na);
+        uint32_t &bk = bucket[pairs[k].j];
+        if (bk == 0xffffffffu) {
+            bk = p->buckets++;
+            bucket_rows.push_back(0);
+        }
+        sp.ubucket = bk;
+        bucket_rows[bk] += m.na;
         sp.rbase = (uint32_t)rb;
         sp.view_a = pairs[k].i;
         sp.view_b = pairs[k].j;
         rb += pad_rows(m.na);
-        groups += (m.na + kResolveRows - 1) / kResolveRows;
+    }
+    uint64_t groups = 0;
+    {
+        uint64_t at = 0;
+        for (uint64_t &r : bucket_rows) {
+            const uint64_t n = r;
+            r = at;
+            at += n;
+            groups += (n + kResolveRows - 1) / kResolveRows;
+        }
+        for (SlPair &sp : p->spairs) sp.ubase = (uint32_t)bucket_rows[sp.ubucket];
     }
     p->rows_pad = rb + 2 * kTile;
     p->queue_cap = std::max<uint64_t>(p->n_slots, 1) + 64;
@@ -580,8 +601,10 @@ slm_status plan_build_shortlist(slm_plan *p, const slm_pair *pairs) {
     SLM_TRY(p->d_tblk.ensure(c, sizeof(uint2) * std::max<size_t>(1, p->tblk.size())));
     SLM_TRY(p->d_topmm.ensure(c, sizeof(float2) * std::max<uint64_t>(1, p->top_parts << p->tshift)));
     SLM_TRY(p->d_topj.ensure(c, sizeof(uint32_t) * std::max<uint64_t>(1, p->top_parts << p->tshift)));
-    SLM_TRY(p->d_ulist.ensure(c, sizeof(uint32_t) * p->rows_pad));
-    SLM_TRY(p->d_ugroups.ensure(c, sizeof(uint2) * std::max<uint64_t>(1, groups)));
+    SLM_TRY(p->d_olist.ensure(c, sizeof(uint4) * std::max<uint64_t>(1, p->n_slots)));
+    SLM_TRY(p->d_ulist.ensure(c, sizeof(uint2) * std::max<uint64_t>(1, p->n_slots)));
+    SLM_TRY(p->d_ucnt.ensure(c, sizeof(uint32_t) * std::max<uint32_t>(1, p->buckets)));
+    SLM_TRY(p->d_ugroups.ensure(c, sizeof(uint4) * std::max<uint64_t>(1, groups)));
     SLM_TRY(p->d_blkcnt.ensure(c, sizeof(uint32_t) * std::max<uint64_t>(1, blk)));
     SLM_TRY(p->d_pairctl.ensure(c, 4 * sizeof(uint32_t) * std::max<size_t>(1, p->np)));
     SLM_TRY(p->d_xlist.ensure(c, sizeof(uint32_t) * std::max<size_t>(1, p->np)));
@@ -594,7 +617,7 @@ slm_status plan_build_shortlist(slm_plan *p, const slm_pair *pairs) {
     SLM_TRY(p->d_meta.ensure(c, sizeof(PairMeta) * std::max<size_t>(1, p->np)));
     SLM_TRY(p->d_slots.ensure(c, sizeof(uint2) * std::max<uint64_t>(1, p->n_slots)));
     SLM_TRY(p->d_counts.ensure(c, sizeof(uint32_t) * std::max<size_t>(1, p->np)));
-    SLM_TRY(p->d_ctl.ensure(c, 64));
+    SLM_TRY(p->d_ctl.ensure(c, kCtlBytes));
     SLM_TRY(p->d_offsets.ensure(c, sizeof(uint64_t) * (p->np + 1) * 2));
     SLM_TRY(p->d_dense.ensure(c, sizeof(uint2) * std::max<uint64_t>(1, p->n_slots)));
     cudaStream_t s = p->stream;
@@ -640,7 +663,7 @@ slm_status plan_build(slm_plan *p, const slm_pair *pairs) {
     SLM_TRY(p->d_colbest.ensure(c, sizeof(unsigned long long) * std::max<uint64_t>(1, col)));
     SLM_TRY(p->d_slots.ensure(c, sizeof(uint2) * std::max<uint64_t>(1, slot)));
     SLM_TRY(p->d_counts.ensure(c, sizeof(uint32_t) * std::max<size_t>(1, p->np)));
-    SLM_TRY(p->d_ctl.ensure(c, 64));
+    SLM_TRY(p->d_ctl.ensure(c, kCtlBytes));
     SLM_TRY(p->d_offsets.ensure(c, sizeof(uint64_t) * (p->np + 1) * 2));
     SLM_TRY(p->d_dense.ensure(c, sizeof(uint2) * std::max<uint64_t>(1, slot)));
     cudaStream_t s = p->stream;
@@ -657,7 +680,7 @@ slm_status plan_build(slm_plan *p, const slm_pair *pairs) {
 // Enqueue the whole batch on stream s (also used for graph capture).
 slm_status plan_enqueue(slm_plan *p, cudaStream_t s) {
     uint32_t *ctl = p->d_ctl.as<uint32_t>();  // [0] work counter, [1] error word, [2..] shortlist counters
-    SLM_CU(cudaMemsetAsync(ctl, 0, 64, s));
+    SLM_CU(cudaMemsetAsync(ctl, 0, kCtlBytes, s));
     if (p->prec != SLM_PREC_FP32) {
         slm_store *st = p->st;
         const bool fp8 = p->prec == SLM_PREC_FP8;
@@ -720,16 +743,20 @@ slm_status plan_enqueue(slm_plan *p, cudaStream_t s) {
         a.topmm = p->d_topmm.as<float2>();
         a.topj = p->d_topj.as<uint32_t>();
         a.max_na = p->max_na;
+        a.n_rows = p->n_slots;
+        a.olist = p->d_olist.as<uint4>();
         a.cand_cap = 2 * (p->tune.shortlist_k ? p->tune.shortlist_k : (uint32_t)kSlHalfRecs);
-        a.ulist = p->d_ulist.as<uint32_t>();
-        a.ugroups = p->d_ugroups.as<uint2>();
+        a.ulist = p->d_ulist.as<uint2>();
+        a.ucnt = p->d_ucnt.as<uint32_t>();
+        a.ugroups = p->d_ugroups.as<uint4>();
+        SLM_CU(cudaMemsetAsync(p->d_ucnt.p, 0, sizeof(uint32_t) * std::max<uint32_t>(1, p->buckets), s));
         int nk = fp8 ? 1 : 0;  // the colmin fill
         SLM_CU(record_event(p->ev0, s));
         nk += launch_shortlist_eps(a, s);
         if (!fp8) {
             nk += launch_top2_pass(a, s);
             SLM_CU(record_event(p->evp[0], s));
-            nk += launch_top2_decide(a, s);
+            nk += launch_top2_decide(a, p->ctx->sms, s);
             SLM_CU(record_event(p->evp[1], s));
             nk += launch_top2_resolve(a, p->ctx->sms, s);
             SLM_CU(record_event(p->evp[2], s));
@@ -754,7 +781,7 @@ slm_status plan_enqueue(slm_plan *p, cudaStream_t s) {
             b.tier = 1;
             nk += launch_shortlist_rescue_prep(b, s);
             nk += launch_top2_pass(b, s);
-            nk += launch_top2_decide(b, s);
+            nk += launch_top2_decide(b, p->ctx->sms, s);
             nk += launch_top2_resolve(b, p->ctx->sms, s);
         }
         nk += launch_shortlist_tail(a, p->ctx->sms, s);

@@ -15,9 +15,11 @@
 //   decide              per row: certain no match when m1 - eps >= r^2 (m2 +
 //                       eps); certain match at its column when m1 + eps < r^2
 //                       (m2 - eps) and m2 - m1 > 2 eps; the cross-check from
-//                       the column's own two smallest. Other rows are listed
-//                       per pair, other columns queued for an exact scan.
-//   resolve             the listed rows, 16 of a pair at a time: every column
+//                       the column's own two smallest. Rows short of that at
+//                       their ratio test get their exact d1; those still open
+//                       are listed by b view, other columns queued for an
+//                       exact scan.
+//   resolve             the listed rows, 16 of a b view at a time: every column
 //                       with d~ <= m2 + 2 eps, and their exact distances.
 //   scan                one CTA per queued row or column: exact full scans.
 //
@@ -150,6 +152,7 @@ struct SlPair {
     uint32_t xpart;    // routed: first exact work item (= first RowPart block)
     uint32_t blk;      // first entry of the pair's row blocks in SlArgs::blkcnt
     uint32_t rescued;  // per launch (FP8 plans): settled by the BF16 passes instead
+    uint32_t ubucket, ubase;  // undecided rows of the pair's b view: counter and first list entry
     uint32_t tblk_a, tblk_b;  // BF16 pass: first block (SlArgs::tblk) of each direction
     uint32_t crbase;   // first candidate row: the records of row i and column range c at
                        // crbase + c * (na padded to 128) + i (sl_cand_row)
@@ -184,7 +187,8 @@ struct SlQueue {
 // Counters in the plan's control block (word 1: the error word).
 enum : int { kCtlGroups = 0, kCtlRescored = 2, kCtlQueueRows = 3, kCtlQueueCols = 4, kCtlMaxErr = 5, kCtlScanLen = 6,
              kCtlRescoreLen = 7, kCtlXItems = 8, kCtlXWork = 9, kCtlRoutedPairs = 10, kCtlRoutedRows = 11,
-             kCtlRoutedCols = 12, kCtlRouteMarks = 13, kCtlRescuedPairs = 14, kCtlRescuedRows = 15 };
+             kCtlRoutedCols = 12, kCtlRouteMarks = 13, kCtlRescuedPairs = 14, kCtlRescuedRows = 15, kCtlOpen = 16 };
+constexpr size_t kCtlBytes = 128;
 
 // Routed pairs: at most this many column chunks per 128-row tile; the exact
 // items of a launch number at most (routed row tiles) + (4 x SMs).
@@ -246,9 +250,12 @@ struct SlArgs {
     float2 *topmm;               // per part row: (m1, m2)
     uint32_t *topj;              // and the column of m1
     uint32_t max_na;
+    uint64_t n_rows;             // of all pairs' a views
+    uint4 *olist;                // rows the bounds leave open: {pair, row, column where certain, m2}
     uint32_t cand_cap;           // resolve: columns a row's shortlist holds
-    uint32_t *ulist;             // undecided rows by pair (from SlPair::rbase)
-    uint2 *ugroups;              // {pair, first entry of its list}, kResolveRows rows each
+    uint2 *ulist;                // undecided rows {pair, row}, by b view (from SlPair::ubase)
+    uint32_t *ucnt;              // and their number per b view (SlPair::ubucket)
+    uint4 *ugroups;              // {first entry in ulist, bucket, entry within the bucket}, kResolveRows rows each
 };
 
 // Whether a pair takes part in this tier's per-pair kernels (pass 2, finalize,
@@ -273,7 +280,7 @@ cudaError_t init_top2_kernels();
 // kernels it launched.
 int launch_shortlist_eps(const SlArgs &a, cudaStream_t s);
 int launch_top2_pass(const SlArgs &a, cudaStream_t s);
-int launch_top2_decide(const SlArgs &a, cudaStream_t s);
+int launch_top2_decide(const SlArgs &a, int sms, cudaStream_t s);
 int launch_top2_resolve(const SlArgs &a, int sms, cudaStream_t s);
 int launch_shortlist_pass(const SlArgs &a, int pass, int sms, cudaStream_t s);
 int launch_shortlist_mid(const SlArgs &a, cudaStream_t s);
