@@ -263,7 +263,9 @@ struct slm_plan {
     uint64_t n_parts = 0, n_cols = 0, n_slots = 0, distances = 0;
     DevBuf d_meta, d_items, d_parts, d_colbest, d_slots, d_counts, d_ctl, d_offsets, d_dense;
     // shortlist path
-    std::vector<SlItem> sitems;
+    std::vector<SlItem> sitems;        // pass items, then the samples' items
+    std::vector<SlSample> samples;
+    uint32_t n_sitems = 0;             // pass items
     std::vector<SlPair> spairs;
     uint32_t half_recs = kSlHalfRecs;  // records per candidate row and column half
     uint64_t rows_pad = 0, cand_rows_pad = 0, cols_pad = 0, sl_parts = 0, queue_cap = 0, xitem_cap = 0, row_blocks_total = 0;
@@ -277,7 +279,7 @@ struct slm_plan {
     std::vector<uint2> tblk;
     uint32_t tshift = 8, max_na = 0, buckets = 0;
     uint64_t top_parts = 0;
-    DevBuf d_titems, d_tstart, d_tblk, d_topmm, d_topj, d_olist, d_ulist, d_ucnt, d_ugroups;
+    DevBuf d_samples, d_titems, d_tstart, d_tblk, d_topmm, d_topj, d_olist, d_ulist, d_ucnt, d_ugroups;
     bool dump = false;
     uint32_t min_matches = 0;        // pairs with fewer matches report none
     cudaGraphExec_t exec = nullptr;
@@ -300,12 +302,12 @@ struct slm_plan {
 
 // Every device buffer of a plan: all are used on the plan's stream only, and
 // allocated ordered on it (DevBuf::order_on).
-std::array<DevBuf *, 38> plan_buffers(slm_plan *p) {
+std::array<DevBuf *, 39> plan_buffers(slm_plan *p) {
     return {&p->d_meta, &p->d_items, &p->d_parts, &p->d_colbest, &p->d_slots, &p->d_counts, &p->d_ctl,
             &p->d_offsets, &p->d_dense, &p->d_sitems, &p->d_spairs, &p->d_rowpart, &p->d_rownear,
             &p->d_colmin, &p->d_rowthr, &p->d_colthr, &p->d_rowcnt, &p->d_rowrec, &p->d_rowrecj,
             &p->d_colcnt, &p->d_rowdec, &p->d_queue, &p->d_rqueue, &p->d_dump, &p->d_xlist, &p->d_xitems,
-            &p->d_xparts, &p->d_blkcnt, &p->d_pairctl, &p->d_titems, &p->d_tstart, &p->d_tblk, &p->d_topmm,
+            &p->d_xparts, &p->d_blkcnt, &p->d_pairctl, &p->d_samples, &p->d_titems, &p->d_tstart, &p->d_tblk, &p->d_topmm,
             &p->d_topj, &p->d_olist, &p->d_ulist, &p->d_ucnt, &p->d_ugroups};
 }
 // Frees a plan's buffers while its stream still exists (their frees are
@@ -525,6 +527,29 @@ slm_status plan_fp8_items(slm_plan *p, const slm_pair *pairs) {
     std::stable_sort(p->sitems.begin(), p->sitems.end(), [](const SlItem &x, const SlItem &y) {
         return (uint64_t)(x.ct1 - x.ct0) * x.nat > (uint64_t)(y.ct1 - y.ct0) * y.nat;
     });
+    p->n_sitems = (uint32_t)p->sitems.size();
+    p->samples.clear();
+    for (uint32_t k = 0; k < p->np && !p->dump; ++k) {  // a dump wants every estimate of its pair
+        const PairMeta &m = p->meta[k];
+        if ((uint64_t)m.na * m.nb < kSlSampleMin) continue;
+        const uint32_t ct_n = std::min<uint32_t>((m.nb + kTile - 1) / kTile, kSlSampleTiles);
+        SlSample sm{};
+        sm.pair = k;
+        sm.nat = std::min(2u, (m.na + kTile - 1) / kTile);
+        sm.ncols = std::min(m.nb, ct_n * kTile);
+        sm.part = (uint32_t)part;
+        for (uint32_t t = 0; t < ct_n; t += kSlSampleItemTiles, ++sm.parts, ++part) {
+            SlItem it{};
+            it.nat = sm.nat;
+            it.pair[0] = it.pair[1] = k;
+            it.rt[1] = 1;
+            it.part[0] = it.part[1] = (uint32_t)part;
+            it.ct0 = t;
+            it.ct1 = std::min(t + kSlSampleItemTiles, ct_n);
+            p->sitems.push_back(it);
+        }
+        p->samples.push_back(sm);
+    }
     p->cand_rows_pad = crb + 2 * kTile;
     p->cols_pad = cb + kTile;
     p->sl_parts = std::max<uint64_t>(part, 1);
@@ -542,6 +567,9 @@ slm_status plan_fp8_items(slm_plan *p, const slm_pair *pairs) {
     SLM_TRY(p->d_rqueue.ensure(c, sizeof(SlQueue) * p->queue_cap));
     SLM_CU(cudaMemcpyAsync(p->d_sitems.p, p->sitems.data(), sizeof(SlItem) * p->sitems.size(), cudaMemcpyHostToDevice,
                            p->stream));
+    SLM_TRY(p->d_samples.ensure(c, sizeof(SlSample) * std::max<size_t>(1, p->samples.size())));
+    SLM_CU(cudaMemcpyAsync(p->d_samples.p, p->samples.data(), sizeof(SlSample) * p->samples.size(),
+                           cudaMemcpyHostToDevice, p->stream));
     return SLM_OK;
 }
 
@@ -702,7 +730,10 @@ slm_status plan_enqueue(slm_plan *p, cudaStream_t s) {
         a.spairs = p->d_spairs.as<SlPair>();
         a.npairs = p->np;
         a.items = p->d_sitems.as<SlItem>();
-        a.n_items = (uint32_t)p->sitems.size();
+        a.n_items = p->n_sitems;
+        a.samples = p->d_samples.as<SlSample>();
+        a.n_samples = (uint32_t)p->samples.size();
+        a.n_sample_items = (uint32_t)p->sitems.size() - p->n_sitems;
         a.rowpart = p->d_rowpart.as<float2>();
         a.rownear = p->d_rownear.as<uint32_t>();
         a.colmin = p->d_colmin.as<uint32_t>();
@@ -761,6 +792,7 @@ slm_status plan_enqueue(slm_plan *p, cudaStream_t s) {
             nk += launch_top2_resolve(a, p->ctx->sms, s);
             SLM_CU(record_event(p->evp[2], s));
         } else {
+            nk += launch_shortlist_sample(a, p->ctx->sms, s);
             nk += launch_shortlist_pass(a, 1, p->ctx->sms, s);
             SLM_CU(record_event(p->evp[0], s));
             nk += launch_shortlist_mid(a, s);

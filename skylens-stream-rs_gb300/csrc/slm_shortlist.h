@@ -25,6 +25,8 @@
 //
 // FP8, tier 0 (k_shortlist.cu; the tile's per-descriptor scales keep the norms
 // out of the product):
+//   sample             large pairs: pass 1 and mid's rescue rule on their first
+//                      256 rows and 4096 columns.
 //   pass 1  (tcgen05)  per row: m1 = min d~ and m2' = second smallest of the
 //                      16-column chunk minima (an upper bound of the second
 //                      smallest d~); per column: c1 = min d~.
@@ -127,6 +129,17 @@ struct SlItem {
     uint32_t nat, ct0, ct1;
     uint32_t pad[3];
 };
+
+// FP8 plans: a large pair's sample, run before pass 1 decides whether that pass
+// is worth running: its first nat row tiles against its first ncols columns, in
+// `parts` items with row partials of their own from block `part` on.
+struct SlSample {
+    uint32_t pair, nat, ncols, part, parts;
+};
+// Pairs of at least this many distances are sampled (pass 1 takes about 15 us
+// then), up to this many column tiles, in items of this many.
+constexpr uint64_t kSlSampleMin = 1ull << 25;
+constexpr uint32_t kSlSampleTiles = 32, kSlSampleItemTiles = 4;
 
 // One segment of the BF16 pass: nat (1 or 2) a tiles from store tile a_tile
 // against nt b tiles from store tile b_tile, of which ncols columns are the
@@ -241,6 +254,8 @@ struct SlArgs {
     // over those pairs only (tier 1), instead of the exact kernel
     uint32_t half_recs;          // records per candidate row and column half (1..kSlHalfRecsMax)
     uint32_t tier;               // 0: the plan's precision; 1: the BF16 rescue of an FP8 plan
+    const SlSample *samples;     // FP8: the sampled pairs; their items follow the pass's own
+    uint32_t n_samples, n_sample_items;
     // BF16 pass
     const TopItem *titems;       // in the order the CTAs run them
     const uint32_t *tstart;      // CTA c runs titems[tstart[c] .. tstart[c + 1])
@@ -283,6 +298,7 @@ int launch_top2_pass(const SlArgs &a, cudaStream_t s);
 int launch_top2_decide(const SlArgs &a, int sms, cudaStream_t s);
 int launch_top2_resolve(const SlArgs &a, int sms, cudaStream_t s);
 int launch_shortlist_pass(const SlArgs &a, int pass, int sms, cudaStream_t s);
+int launch_shortlist_sample(const SlArgs &a, int sms, cudaStream_t s);
 int launch_shortlist_mid(const SlArgs &a, cudaStream_t s);
 int launch_shortlist_finalize(const SlArgs &a, cudaStream_t s);
 // Before the rescue tier's pass: the rescued pairs' BF16 eps and counters.

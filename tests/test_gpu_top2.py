@@ -66,3 +66,27 @@ def test_undecided_rows_of_shared_and_large_views(matcher, n):
     assert plan.stats["rows_rescored"] + plan.stats["rows_recomputed"] > 50
     plan.close()
     st.close()
+
+
+@pytest.mark.parametrize("na,nb", [(300, 112000), (100, 336000), (5800, 5800)])
+@pytest.mark.parametrize("kind", ["sift", "sparse"])
+def test_fp8_pairs_above_the_sample_threshold(matcher, kind, na, nb):
+    """Pairs just above 2^25 distances: their sample decides whether FP8 pass 1
+    runs. SIFT-like ones are rescued by it; sparse ones (one to three large
+    components, distances far apart) need not be. Either way the oracle's list."""
+    rng = np.random.Generator(np.random.PCG64(na))
+    if kind == "sift":
+        a, b = synth.sift_like(rng, na), synth.sift_like(rng, nb)
+    else:
+        def sparse(n):
+            x = np.zeros((n, 128), np.float32)
+            for _ in range(3):
+                x[np.arange(n), rng.integers(0, 128, n)] = rng.integers(1, 9, n)
+            return x
+        a, b = sparse(na), sparse(nb)
+    k = min(na, 64)
+    b[rng.permutation(nb)[:k]] = a[:k] + np.float32(0.01) * rng.standard_normal((k, 128), dtype=np.float32)
+    got = matcher.ratio_match_np(a, b, 0.8, True, "fp8")
+    assert np.array_equal(got, O.ratio_match_np(a, b, 0.8, True, threads=16))
+    if kind == "sift":
+        assert matcher.last_stats["pairs_rescued"] == 1
