@@ -32,9 +32,11 @@
 
 #ifdef __CUDACC__
 __device__ static const float slm_fm_exp2_dev[128] = {SLM_EXP2_TABLE};
+__device__ __align__(8) static const float slm_fm_expn_dev[2 * 641] = {SLM_EXPN_TABLE};
 __device__ static const float slm_fm_atan_dev[34] = {SLM_ATAN_TABLE};
 #endif
 static const float slm_fm_exp2_host[128] = {SLM_EXP2_TABLE};
+static const float slm_fm_expn_host[2 * 641] = {SLM_EXPN_TABLE};
 static const float slm_fm_atan_host[34] = {SLM_ATAN_TABLE};
 
 #ifdef __CUDA_ARCH__
@@ -129,6 +131,38 @@ SLM_FM float slm_expf_cr(float x) {
     float f = slm_round_checked(vh, ve + lo, 0x1p-41f, &ok);
     if (!ok) return (float)exp((double)x);
     return ldexpf(f, n >> 6);  // 2^(n >> 6) scaling: exact (results stay normal above e^-87)
+}
+
+// e^x for -10 < x <= 0, the window weights: the reduction by j/64 is exact, and
+// the rounding test adds and subtracts the error bound (Ziv's test as such).
+// Other arguments go to slm_expf_cr.
+SLM_FM float slm_expf_neg_cr(float x) {
+    if (!(x > -10.0f && x <= 0.0f)) return slm_expf_cr(x);
+    const float nf = rintf(x * -64.0f);  // 0 .. 640
+    const float r = fmaf(nf, 1.0f / 64.0f, x);  // exact, |r| <= 2^-7
+    const int j = (int)nf;
+#ifdef __CUDA_ARCH__
+    const float2 t = *reinterpret_cast<const float2 *>(slm_fm_expn_dev + 2 * j);
+    const float th = t.x, tl = t.y;
+#else
+    const float th = slm_fm_expn_host[2 * j], tl = slm_fm_expn_host[2 * j + 1];
+#endif
+    // e^r - 1 = r + r^2/2 + r^3 (1/6 + r/24 + r^2/120)
+    float sh, sl;
+    slm_two_prod(r, r, &sh, &sl);
+    const float c = sh * r * fmaf(r, fmaf(r, 1.0f / 120.0f, 1.0f / 24.0f), 1.0f / 6.0f);
+    const float a = 0.5f * sh;
+    const float qh = r + a;  // |r| >= a: the next line is the sum's exact error
+    const float ql = (a - (qh - r)) + fmaf(0.5f, sl, c);
+    // e^(-j/64) (1 + q), |q| < 2^-6
+    float ph, pl;
+    slm_two_prod(th, qh, &ph, &pl);
+    const float vh = th + ph;
+    const float lo = (ph - (vh - th)) + (tl + (pl + fmaf(th, ql, tl * qh)));
+    const float e = vh * 0x1p-41f;
+    const float f = vh + (lo + e);
+    if (f != vh + (lo - e)) return (float)exp((double)x);
+    return f;
 }
 
 // atan2(y, x)

@@ -1,5 +1,5 @@
 """Writes fmath_tables.h: the float-float constants of fmath_cr.h
-(2^(j/64) for j = 0..63, atan(j/16) for j = 0..16, pi / 2, pi, and the
+(2^(j/64) for j = 0..63, e^(-j/64) for j = 0..640, atan(j/16) for j = 0..16, pi / 2, pi, and the
 Cody-Waite split of ln2 / 64), each the exact value rounded to a float `hi`
 plus the rounded remainder `lo`, from 60-digit decimal arithmetic."""
 import math
@@ -48,6 +48,7 @@ def hx(v: float) -> str:
 
 def main():
     exp_tab = [split(Decimal(2) ** (Decimal(j) / 64)) for j in range(64)]
+    expn_tab = [split((-Decimal(j) / 64).exp()) for j in range(641)]
     atan_tab = [split(atan(Decimal(j) / 16)) for j in range(17)]
     pi = 4 * atan(Decimal(1))
     L = Decimal(2).ln() / 64
@@ -59,6 +60,8 @@ def main():
              "// 2^(j/64), j = 0..63: hi, lo",
              "#define SLM_EXP2_TABLE \\"]
     lines += [f"    {hx(h)}, {hx(l)}," + (" \\" if j < 63 else "") for j, (h, l) in enumerate(exp_tab)]
+    lines += ["", "// e^(-j/64), j = 0..640: hi, lo", "#define SLM_EXPN_TABLE \\"]
+    lines += [f"    {hx(h)}, {hx(l)}," + (" \\" if j < 640 else "") for j, (h, l) in enumerate(expn_tab)]
     lines += ["", "// atan(j/16), j = 0..16: hi, lo", "#define SLM_ATAN_TABLE \\"]
     lines += [f"    {hx(h)}, {hx(l)}," + (" \\" if j < 16 else "") for j, (h, l) in enumerate(atan_tab)]
     pio2, pi1 = split(pi / 2), split(pi)

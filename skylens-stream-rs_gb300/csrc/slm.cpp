@@ -3124,20 +3124,29 @@ slm_status feat_describe(slm_ctx *c, cudaStream_t st, DevBuf &buf, const FeatCor
     *d_desc = nullptr;
     if (list.empty()) return SLM_OK;
     if (list.size() >= (1ull << 31)) return fail(SLM_INVALID_ARG, "too many features in one call");
-    const uint64_t o_jobs = 0, o_desc = feat_align(sizeof(DescJob) * list.size()),
-                   bytes = o_desc + 4ull * kDesc * list.size();
+    const uint64_t o_jobs = 0, o_cs = feat_align(sizeof(DescJob) * list.size()),
+                   o_desc = feat_align(o_cs + sizeof(float2) * list.size()), bytes = o_desc + 4ull * kDesc * list.size();
     SLM_TRY(buf.ensure(c, bytes));
     std::vector<DescJob> jobs(list.size());
+    float top = 0.0f;
     for (size_t i = 0; i < list.size(); ++i) {
+        top = std::max(top, fc.cands[list[i].first].sig);
         jobs[i].cand = list[i].first;
         jobs[i].angle = fc.angles[(size_t)list[i].first * kMaxAngles + list[i].second];
         jobs[i].out_row = (uint32_t)i;
         jobs[i].pad = 0;
     }
+    // windows too large for one warp first
+    const auto small = std::stable_partition(jobs.begin(), jobs.end(), [&](const DescJob &j) {
+        return describe_side(fc.cands[j.cand].sig) > kDescWarpSide;
+    });
     unsigned char *d = buf.as<unsigned char>();
     SLM_CU(cudaMemcpyAsync(d + o_jobs, jobs.data(), sizeof(DescJob) * jobs.size(), cudaMemcpyHostToDevice, st));
     DescribeArgs da{};
     da.jobs = reinterpret_cast<const DescJob *>(d + o_jobs);
+    da.cs = reinterpret_cast<float2 *>(d + o_cs);
+    da.n_large = (uint32_t)(small - jobs.begin());
+    da.max_side = describe_side(top);
     da.cands = fc.d_cands;
     da.grads = fc.d_grads;
     da.geom = fc.d_geom;
@@ -3446,7 +3455,7 @@ extern "C" slm_status slm_describe(slm_ctx *c, const float *img, uint32_t w, uin
     // image, its gradient table, the geometry, keypoints, jobs, descriptors
     const uint64_t o_img = 0, o_grad = feat_align(4 * wh), o_geom = feat_align(o_grad + 8 * wh),
                    o_kps = feat_align(o_geom + sizeof(OctaveGeom)), o_jobs = feat_align(o_kps + sizeof(slm_keypoint) * n),
-                   o_desc = feat_align(o_jobs + sizeof(DescJob) * n), bytes = o_desc + 4ull * kDesc * n;
+                   o_cs = feat_align(o_jobs + sizeof(DescJob) * n), o_desc = feat_align(o_cs + sizeof(float2) * n), bytes = o_desc + 4ull * kDesc * n;
     slm_status st = ws->feat_pyr.ensure(c, bytes);
     if (st == SLM_OK) {
         unsigned char *d = ws->feat_pyr.as<unsigned char>();
@@ -3456,6 +3465,10 @@ extern "C" slm_status slm_describe(slm_ctx *c, const float *img, uint32_t w, uin
         g.layer_stride = wh;
         std::vector<DescJob> jobs(n);
         for (uint32_t i = 0; i < n; ++i) jobs[i] = DescJob{i, kps[i].angle, i, 0};
+        // largest windows first: a window is one CTA's chain, as long as sigma squared
+        std::sort(jobs.begin(), jobs.end(), [&](const DescJob &p, const DescJob &q) {
+            return kps[p.cand].sigma != kps[q.cand].sigma ? kps[p.cand].sigma > kps[q.cand].sigma : p.cand < q.cand;
+        });
         cudaError_t e = wh ? cudaMemcpyAsync(d + o_img, img, 4 * wh, cudaMemcpyDefault, st_) : cudaSuccess;
         if (e == cudaSuccess) e = cudaMemcpyAsync(d + o_geom, &g, sizeof g, cudaMemcpyHostToDevice, st_);
         if (e == cudaSuccess) e = cudaMemcpyAsync(d + o_kps, kps, sizeof(slm_keypoint) * n, cudaMemcpyDefault, st_);
@@ -3465,6 +3478,9 @@ extern "C" slm_status slm_describe(slm_ctx *c, const float *img, uint32_t w, uin
                         (int)h, 1, wh, 0, 1, st_);
             DescribeArgs da{};
             da.jobs = reinterpret_cast<const DescJob *>(d + o_jobs);
+            da.cs = reinterpret_cast<float2 *>(d + o_cs);
+            while (da.n_large < n && describe_side(kps[jobs[da.n_large].cand].sigma) > kDescWarpSide) ++da.n_large;
+            da.max_side = describe_side(kps[jobs[0].cand].sigma);
             da.kps = reinterpret_cast<const slm_keypoint *>(d + o_kps);
             da.grads = reinterpret_cast<const float2 *>(d + o_grad);
             da.geom = reinterpret_cast<const OctaveGeom *>(d + o_geom);

@@ -220,6 +220,9 @@ struct DescJob {
 
 struct DescribeArgs {
     const DescJob *jobs;
+    float2 *cs;             // scratch: cos and sin of each job's angle
+    uint32_t n_large;       // the first jobs, those of more than kDescWarpSide window rows: a CTA each
+    int max_side;           // the most window rows of any job (describe_side of the largest sigma)
     const FeatCand *cands;  // null: keypoints kps (image pixels) on one table, grads, geom[0]
     const slm_keypoint *kps;
     const float2 *grads;
@@ -242,6 +245,9 @@ void launch_grad(const float *gauss, float2 *grad, int w, int h, int s_, uint64_
                  cudaStream_t s);
 void launch_extrema(const ExtremaArgs &a, int nimg, cudaStream_t s);
 void launch_orient(const OrientArgs &a, uint32_t n, cudaStream_t s);
+constexpr int kDescWarpSide = 127;  // window rows one warp takes
+// Window rows of a feature of scale sigma (features.rs:526-528), at least.
+inline int describe_side(float sigma) { return 2 * ((int)(3.0f * sigma * 1.41421356f * 2.5f + 0.5f) + 1) + 1; }
 void launch_describe(const DescribeArgs &a, uint32_t njobs, cudaStream_t s);
 
 // ------------------------------------------------------ tracks (k_tracks.cu)
