@@ -1089,6 +1089,7 @@ extern "C" slm_status slm_ctx_create(const slm_opts *opts, slm_ctx **out) {
         cudaError_t ke = init_exact_kernels();
         if (ke == cudaSuccess) ke = init_shortlist_kernels();
         if (ke == cudaSuccess) ke = init_top2_kernels();
+        if (ke == cudaSuccess) ke = init_feature_kernels();
         if (ke != cudaSuccess) {
             cudaGetLastError();
             return fail(SLM_NO_DEVICE, std::string("kernels do not load on this device: ") + cudaGetErrorString(ke));

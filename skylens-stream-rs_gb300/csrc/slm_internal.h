@@ -231,6 +231,7 @@ struct DescribeArgs {
     float *desc;
 };
 
+cudaError_t init_feature_kernels();  // kernel attributes, once per device
 // Both passes of a blur of nimg images (src -> tmp -> dst); with dog, also
 // dog = dst - prev (prev strided as dst). Strides are per image, in floats.
 void launch_blur(const float *src, float *tmp, float *dst, const float *prev, float *dog, int w, int h, int nimg,
