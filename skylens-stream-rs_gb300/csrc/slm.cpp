@@ -3023,8 +3023,6 @@ slm_status feat_core(slm_ctx *c, Workspace *ws, const float *d_img, uint32_t n, 
             ea.octave = (int)o;
             ea.contrast = cfg.contrast;
             ea.edge_thr = edge_thr;
-            ea.sigma0 = cfg.sigma0;
-            ea.kstep = kstep;
             ea.cands = out.d_cands;
             ea.count = d_count;
             ea.cap = cap;
@@ -3048,6 +3046,7 @@ slm_status feat_core(slm_ctx *c, Workspace *ws, const float *d_img, uint32_t n, 
         oa.s = s;
         oa.angles = d_ang;
         oa.nang = d_nang;
+        launch_candidate_sigma(out.d_cands, count, cfg.sigma0, kstep, st);
         launch_orient(oa, count, st);
         SLM_CU(cudaGetLastError());
         // candidates, angle counts and angles into pinned host memory

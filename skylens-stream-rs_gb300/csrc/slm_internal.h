@@ -174,7 +174,7 @@ struct BlurTaps {
 // A refined DoG extremum that passed the contrast and edge tests.
 struct __align__(16) FeatCand {
     float x, y;        // refined position in octave pixels
-    float sig;         // sig_oct = sigma0 * kstep^s
+    float sig;         // sig_oct = sigma0 * kstep^s (s itself until launch_candidate_sigma)
     float value;       // refined DoG response
     uint16_t img;      // image of the batch
     uint8_t octave;
@@ -194,7 +194,7 @@ struct ExtremaArgs {
     const float *dog;       // [img][ng - 1][h][w]
     uint64_t layer_stride;
     int w, h, s, ng, octave;
-    float contrast, edge_thr, sigma0, kstep;
+    float contrast, edge_thr;
     FeatCand *cands;
     uint32_t *count;
     uint32_t cap;
@@ -245,6 +245,7 @@ void launch_gray_from_rgb8(const uint8_t *rgb, float *out, uint64_t n, cudaStrea
 void launch_grad(const float *gauss, float2 *grad, int w, int h, int s_, uint64_t img_stride, int l0, int nimg,
                  cudaStream_t s);
 void launch_extrema(const ExtremaArgs &a, int nimg, cudaStream_t s);
+void launch_candidate_sigma(FeatCand *cands, uint32_t n, float sigma0, float kstep, cudaStream_t s);
 void launch_orient(const OrientArgs &a, uint32_t n, cudaStream_t s);
 constexpr int kDescWarpSide = 127;  // window rows one warp takes
 // Window rows of a feature of scale sigma (features.rs:526-528), at least.
