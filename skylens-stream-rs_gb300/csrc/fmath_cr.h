@@ -26,14 +26,16 @@
 
 #ifdef __CUDACC__
 #define SLM_FM __host__ __device__ __forceinline__
+#define SLM_FM_RARE static __host__ __device__ __noinline__
 #else
 #define SLM_FM static inline
+#define SLM_FM_RARE static
 #endif
 
 #ifdef __CUDACC__
 __device__ static const float slm_fm_exp2_dev[128] = {SLM_EXP2_TABLE};
 __device__ __align__(8) static const float slm_fm_expn_dev[2 * 641] = {SLM_EXPN_TABLE};
-__device__ static const float slm_fm_atan_dev[34] = {SLM_ATAN_TABLE};
+__device__ __align__(8) static const float slm_fm_atan_dev[34] = {SLM_ATAN_TABLE};
 #endif
 static const float slm_fm_exp2_host[128] = {SLM_EXP2_TABLE};
 static const float slm_fm_expn_host[2 * 641] = {SLM_EXPN_TABLE};
@@ -41,10 +43,8 @@ static const float slm_fm_atan_host[34] = {SLM_ATAN_TABLE};
 
 #ifdef __CUDA_ARCH__
 #define SLM_FM_EXP2 slm_fm_exp2_dev
-#define SLM_FM_ATAN slm_fm_atan_dev
 #else
 #define SLM_FM_EXP2 slm_fm_exp2_host
-#define SLM_FM_ATAN slm_fm_atan_host
 #endif
 
 // s + e = a + b exactly
@@ -165,70 +165,84 @@ SLM_FM float slm_expf_neg_cr(float x) {
     return f;
 }
 
-// atan2(y, x)
+// About 1 / x (within an ulp), for quotients that a residual then corrects.
+SLM_FM float slm_rcp(float x) {
+#ifdef __CUDA_ARCH__
+    float r;
+    asm("rcp.approx.f32 %0, %1;" : "=f"(r) : "f"(x));
+    return r;
+#elif defined(SLM_FM_RCP_ULP)  // the host check moves it as the device's may lie
+    return slm_bitsf(slm_fbits(1.0f / x) + SLM_FM_RCP_ULP);
+#else
+    return 1.0f / x;
+#endif
+}
+
+// atan2 of arguments on an axis (a multiple of pi / 2, rounded), outside the
+// range of the float-float quotient (NaN, inf, ratios that could underflow), or
+// whose rounding that does not settle. Kept out of line: one branch in the
+// common path, whose code is a pixel's whole cost.
+SLM_FM_RARE float slm_atan2f_rare(float y, float x) {
+    const float ax = fabsf(x), ay = fabsf(y);
+    if ((ax == 0.0f || ay == 0.0f) && ax < 0x1p100f && ay < 0x1p100f) {
+        const float a = ay > ax ? SLM_PIO2_HI : (slm_fbits(x) >> 31) ? SLM_PI_HI : 0.0f;
+        return copysignf(a, y);
+    }
+    return (float)atan2((double)y, (double)x);
+}
+
+// atan2(y, x). Quotients are float-float (Dekker: an approximate quotient, its
+// exact remainder, a correction), and the octant is one sum K + s a.
 SLM_FM float slm_atan2f_cr(float y, float x) {
     const float ax = fabsf(x), ay = fabsf(y);
-    const bool swap = ay > ax;
+    const bool swap = ay > ax, neg = x < 0.0f;
     const float mn = swap ? ax : ay, mx = swap ? ay : ax;
-    // NaN, inf, zeros, and ratios whose float-float quotient could underflow
-    if (!(mx < 0x1p100f) || !(mn > 0x1p-60f * mx) || !(mn > 0x1p-60f))
-        return (float)atan2((double)y, (double)x);
-    // t = mn / mx in float-float (the division's remainder is exact with fmaf)
-    const float th = mn / mx;
-    const float tl = fmaf(-th, mx, mn) / mx;
+    const bool common = mx < 0x1p100f && mn > 0x1p-60f * mx && mn > 0x1p-60f;  // else what follows is not used
+    // t = mn / mx
+    const float rx = slm_rcp(mx);
+    const float th = mn * rx, tl = fmaf(-th, mx, mn) * rx;
     // t = c + delta (1 + t c) with c = j / 16: atan(t) = atan(c) + atan(delta)
-    const int j = (int)rintf(th * 16.0f);
-    const float c = (float)j * 0.0625f;
+    const float fj = rintf(th * 16.0f);
+    const int j = common ? (int)fj : 0;
+    const float c = fj * 0.0625f;
     float nh, nl;
     slm_two_sum(th - c, tl, &nh, &nl);  // th - c is exact (Sterbenz, or c = 0)
     float pc, pe;
     slm_two_prod(th, c, &pc, &pe);
-    float dh, de;
-    slm_two_sum(1.0f, pc, &dh, &de);
-    const float dl = de + fmaf(tl, c, pe);
-    const float q1 = nh / dh;
-    const float rem = fmaf(-q1, dh, nh) + (nl - q1 * dl);
-    float eh, el;
-    slm_two_sum(q1, rem / dh, &eh, &el);  // delta, |delta| <= 1/32
+    const float dh = 1.0f + pc;
+    const float dl = (pc - (dh - 1.0f)) + fmaf(tl, c, pe);
+    const float rd = slm_rcp(dh), q1 = nh * rd;
+    const float q2 = (fmaf(-q1, dh, nh) + (nl - q1 * dl)) * rd;
+    const float eh = q1 + q2, el = q2 - (eh - q1);  // delta, |delta| <= 1/32 (and a little)
     // atan(delta) = delta + delta P, P = -z/3 + z^2 (1/5 - z/7 + z^2/9), z = delta^2
     float zh, zl;
     slm_two_prod(eh, eh, &zh, &zl);
     zl = fmaf(2.0f * eh, el, zl);
-    const float z3 = zh / 3.0f;
-    const float z3l = (fmaf(-z3, 3.0f, zh) + zl) / 3.0f;
-    const float tail = zh * zh * fmaf(zh, fmaf(zh, 1.0f / 9.0f, -1.0f / 7.0f), 1.0f / 5.0f);
-    float Ph, Pl;
-    slm_two_sum(-z3, tail - z3l, &Ph, &Pl);
+    const float z3 = zh * SLM_THIRD_HI;
+    const float z3l = fmaf(zh, SLM_THIRD_HI, -z3) + fmaf(zh, SLM_THIRD_LO, zl * SLM_THIRD_HI);
+    const float tail = zh * zh * fmaf(zh, fmaf(zh, 1.0f / 9.0f, -1.0f / 7.0f), 1.0f / 5.0f) - z3l;
+    const float Ph = tail - z3, Pl = tail - (Ph + z3);  // |z3| >= |tail|
     float mh, ml;
     slm_two_prod(eh, Ph, &mh, &ml);
     ml = ml + fmaf(eh, Pl, el * Ph);
-    float ah, al;
-    slm_two_sum(eh, mh, &ah, &al);
-    al = al + (el + ml);
+    const float ah = eh + mh, al = (mh - (ah - eh)) + (el + ml);
     // + atan(c)
-    const float Ah = SLM_FM_ATAN[2 * j], Al = SLM_FM_ATAN[2 * j + 1];
+#ifdef __CUDA_ARCH__
+    const float2 A = *reinterpret_cast<const float2 *>(slm_fm_atan_dev + 2 * j);
+    const float Ah = A.x, Al = A.y;
+#else
+    const float Ah = slm_fm_atan_host[2 * j], Al = slm_fm_atan_host[2 * j + 1];
+#endif
     float sh, se;
     slm_two_sum(Ah, ah, &sh, &se);
     float sl = se + (Al + al);
-    // octants: pi/2 - a when |y| > |x|, pi - a when x < 0, the sign of y
-    if (swap) {
-        float u, ue;
-        slm_two_sum(SLM_PIO2_HI, -sh, &u, &ue);
-        sl = ue + (SLM_PIO2_LO - sl);
-        sh = u;
-    }
-    if (x < 0.0f) {
-        float u, ue;
-        slm_two_sum(SLM_PI_HI, -sh, &u, &ue);
-        sl = ue + (SLM_PI_LO - sl);
-        sh = u;
-    }
-    if (y < 0.0f) {
-        sh = -sh;
-        sl = -sl;
-    }
-    bool ok;
-    const float f = slm_round_checked(sh, sl, 0x1p-40f, &ok);
-    if (!ok) return (float)atan2((double)y, (double)x);
-    return f;
+    // a, pi/2 - a, pi/2 + a, pi - a; then the sign of y
+    const float Kh = swap ? SLM_PIO2_HI : neg ? SLM_PI_HI : 0.0f, Kl = swap ? SLM_PIO2_LO : neg ? SLM_PI_LO : 0.0f;
+    if (swap != neg) sh = -sh, sl = -sl;
+    float vh, ve;
+    slm_two_sum(Kh, sh, &vh, &ve);
+    const float lo = ve + (Kl + sl), e = vh * 0x1p-40f;  // vh > 0
+    const float f = vh + (lo + e);
+    if (!common || f != vh + (lo - e)) return slm_atan2f_rare(y, x);
+    return copysignf(f, y);
 }

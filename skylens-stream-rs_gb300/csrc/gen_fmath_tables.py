@@ -1,5 +1,5 @@
 """Writes fmath_tables.h: the float-float constants of fmath_cr.h
-(2^(j/64) for j = 0..63, e^(-j/64) for j = 0..640, atan(j/16) for j = 0..16, pi / 2, pi, and the
+(2^(j/64) for j = 0..63, e^(-j/64) for j = 0..640, atan(j/16) for j = 0..16, pi / 2, pi, 1 / 3, and the
 Cody-Waite split of ln2 / 64), each the exact value rounded to a float `hi`
 plus the rounded remainder `lo`, from 60-digit decimal arithmetic."""
 import math
@@ -67,6 +67,7 @@ def main():
     pio2, pi1 = split(pi / 2), split(pi)
     lines += ["", f"#define SLM_PIO2_HI {hx(pio2[0])}", f"#define SLM_PIO2_LO {hx(pio2[1])}",
               f"#define SLM_PI_HI {hx(pi1[0])}", f"#define SLM_PI_LO {hx(pi1[1])}",
+              f"#define SLM_THIRD_HI {hx(split(Decimal(1) / 3)[0])}", f"#define SLM_THIRD_LO {hx(split(Decimal(1) / 3)[1])}",
               "// ln2 / 64 = L1 + L2 + L3 (L1: 11 significant bits), 64 / ln2",
               f"#define SLM_LN2_64_1 {hx(L1)}", f"#define SLM_LN2_64_2 {hx(L2)}", f"#define SLM_LN2_64_3 {hx(L3)}",
               f"#define SLM_INV_LN2_64 {hx(f32(Decimal(64) / Decimal(2).ln()))}", ""]

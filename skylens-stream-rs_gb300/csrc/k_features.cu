@@ -225,21 +225,36 @@ __global__ void gray_from_rgb8_kernel(const uint8_t *__restrict__ rgb, float *__
 
 // GradTable (features.rs:335-359) of s consecutive layers from l0: |g| and
 // atan2(gy, gx) of central differences at interior pixels (pixel_grad,
-// :327-332); grad is [img][s][h][w].
-__global__ void grad_kernel(const float *__restrict__ gauss, float2 *__restrict__ grad, int w, int h, int s,
-                            uint64_t layer_stride, uint64_t img_stride, int l0) {
-    const int x = blockIdx.x * blockDim.x + threadIdx.x, y = blockIdx.y;
+// :327-332); grad is [img][s][h][w]. Bound by instruction issue (the atan2 and
+// the square root): a thread walks kGradRows rows of a column, so that address
+// arithmetic and two of a pixel's four loads are shared. 0.49 -> 0.30 ms for the
+// octaves of 24 views of 960 x 540, the atan2's part of it included.
+constexpr int kGradRows = 6;
+__global__ void __launch_bounds__(128) grad_kernel(const float *__restrict__ gauss, float2 *__restrict__ grad, int w,
+                                                   int h, int s, uint64_t layer_stride, uint64_t img_stride, int l0) {
+    const int x = blockIdx.x * blockDim.x + threadIdx.x, y0 = blockIdx.y * kGradRows;
     const int b = blockIdx.z / s, l = blockIdx.z % s;
     if (x >= w) return;
-    float2 g = make_float2(0.0f, 0.0f);
-    if (x >= 1 && y >= 1 && x + 1 < w && y + 1 < h) {
-        const float *im = gauss + (uint64_t)b * img_stride + (uint64_t)(l0 + l) * layer_stride;
-        const float gx = im[(uint64_t)y * w + x + 1] - im[(uint64_t)y * w + x - 1];
-        const float gy = im[(uint64_t)(y + 1) * w + x] - im[(uint64_t)(y - 1) * w + x];
-        g.x = sqrtf(gx * gx + gy * gy);
-        g.y = atan2_cr(gy, gx);
+    const bool inside = x >= 1 && x + 1 < w;
+    const float *im = gauss + (uint64_t)b * img_stride + (uint64_t)(l0 + l) * layer_stride + (uint64_t)y0 * w + x;
+    float2 *out = grad + ((uint64_t)b * s + l) * layer_stride + (uint64_t)y0 * w + x;
+    float above = inside && y0 >= 1 ? im[-w] : 0.0f, here = im[0];
+#pragma unroll
+    for (int k = 0; k < kGradRows; ++k, im += w, out += w) {
+        const int y = y0 + k;
+        if (y >= h) return;
+        const float below = y + 1 < h ? im[w] : 0.0f;
+        float2 g = make_float2(0.0f, 0.0f);
+        if (inside && y >= 1 && y + 1 < h) {
+            const float gx = im[1] - im[-1];
+            const float gy = below - above;
+            g.x = sqrtf(gx * gx + gy * gy);
+            g.y = atan2_cr(gy, gx);
+        }
+        *out = g;
+        above = here;
+        here = below;
     }
-    grad[((uint64_t)b * s + l) * layer_stride + (uint64_t)y * w + x] = g;
 }
 
 // ---------------------------------------------------------------- extrema
@@ -1006,8 +1021,8 @@ void launch_gray_from_rgb8(const uint8_t *rgb, float *out, uint64_t n, cudaStrea
 
 void launch_grad(const float *gauss, float2 *grad, int w, int h, int s_, uint64_t img_stride, int l0, int nimg,
                  cudaStream_t s) {
-    grad_kernel<<<dim3((w + 255) / 256, h, nimg * s_), 256, 0, s>>>(gauss, grad, w, h, s_, (uint64_t)w * h,
-                                                                    img_stride, l0);
+    grad_kernel<<<dim3((w + 127) / 128, (h + kGradRows - 1) / kGradRows, nimg * s_), 128, 0, s>>>(
+        gauss, grad, w, h, s_, (uint64_t)w * h, img_stride, l0);
 }
 
 void launch_extrema(const ExtremaArgs &a, int nimg, cudaStream_t s) {
