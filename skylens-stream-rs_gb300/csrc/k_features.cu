@@ -746,15 +746,18 @@ __device__ __forceinline__ float desc_norm(const float *sq) {
 // and a bin's owner then runs through its list.
 //   one warp a feature (windows of up to kDescWarpSide rows: everything the
 //   detector makes), four bins a lane. No barriers.
-//   one CTA a feature (larger windows, the first n_large jobs), one bin a
-//   thread: the warps sort 32 samples each, then a thread takes its own first
-//   group with samples, then its next, so that cells far apart in a row
-//   progress together, and busy bins are spread over the warps.
+//   one CTA of 8 warps a feature (larger windows, and all when there are few
+//   features: the first n_large jobs): the warps sort 32 samples each, then the
+//   threads of four of them, one a bin, take their own first group with
+//   samples, then the next, so that cells far apart in a row progress together;
+//   busy bins are spread over the four warps. (Four warps in all: the 1500
+//   keypoints below took 0.76 ms instead of 0.47, the largest window's chain.)
 // Bound by instruction issue. Before, with a CTA per feature, each bin walked
 // the bits of its samples and formed each product from a 48-byte record: 2.70 ->
-// 1.40 ms for the 28.8 K features of 24 views of 960 x 540, 2.4 -> 0.76 ms for
+// 1.31 ms for the 28.8 K features of 24 views of 960 x 540, 2.4 -> 0.47 ms for
 // 1500 keypoints of sigma 1.6 to 13.
 constexpr int kDescWarps = kDescThreads / 32;
+constexpr int kDescCtaWarps = 8, kDescCtaThreads = 32 * kDescCtaWarps;  // of a large window
 
 struct __align__(16) DescWarpSmem {  // one per warp, side by side: list is read as float4
     DescGroup g;
@@ -763,8 +766,8 @@ struct __align__(16) DescWarpSmem {  // one per warp, side by side: list is read
 };
 static_assert(sizeof(DescWarpSmem) % 16 == 0 && sizeof(DescGroup) % 16 == 0, "alignment of the vector accesses");
 struct __align__(16) DescCtaSmem {
-    DescGroup g[2][kDescWarps];
-    uint32_t wsum[kDescWarps];
+    DescGroup g[2][kDescCtaWarps];
+    uint32_t wsum[kDescCtaWarps];
     float norm;
 };
 
@@ -852,7 +855,7 @@ __device__ void describe_cta(const DescribeArgs &a, uint32_t k, DescCtaSmem &S, 
     const DescWindow W = desc_window(a, k, (a.max_side - 1) / 2);
     const int side = 2 * W.r + 1;
     uint32_t total = 0;
-    for (int base = 0; base < side; base += kDescThreads) {
+    for (int base = 0; base < side; base += kDescCtaThreads) {
         const int row = base + tid;
         int lo = 0;
         const uint32_t n = row < side ? desc_row(W, row, lo) : 0;
@@ -866,7 +869,7 @@ __device__ void describe_cta(const DescribeArgs &a, uint32_t k, DescCtaSmem &S, 
         __syncthreads();
         uint32_t all = 0, mine = total + s - n;
 #pragma unroll
-        for (int g = 0; g < kDescWarps; ++g) {
+        for (int g = 0; g < kDescCtaWarps; ++g) {
             if (g < warp) mine += S.wsum[g];
             all += S.wsum[g];
         }
@@ -879,13 +882,16 @@ __device__ void describe_cta(const DescribeArgs &a, uint32_t k, DescCtaSmem &S, 
     }
     if (tid == 0) first[side] = total;
     __syncthreads();
+    const bool owner = warp < 4;
     desc_group_init(S.g[0][warp], lane);
     desc_group_init(S.g[1][warp], lane);
-    const int iv = (lane >> 4) * 2 + (warp >> 1), iu = (lane >> 2) & 3, io = (lane & 3) * 2 + (warp & 1);
+    // bins: one a thread of warps 0-3, busy ones (neighbouring rows and
+    // orientations) in different warps
+    const int iv = (lane >> 4) * 2 + ((warp >> 1) & 1), iu = (lane >> 2) & 3, io = (lane & 3) * 2 + (warp & 1);
     const uint32_t place = ((iv + 1) * 6 + iu + 1) * 8 + io;
     float acc = 0.0f;  // bin (iv, iu, io)
     int row = 0, par = 0;
-    for (uint32_t base = 0; base < total; base += kDescThreads, par ^= 1) {
+    for (uint32_t base = 0; base < total; base += kDescCtaThreads, par ^= 1) {
         const uint32_t t = base + tid;
         uint32_t code = 0, n[4], at;
         float prod[8];
@@ -896,21 +902,20 @@ __device__ void describe_cta(const DescribeArgs &a, uint32_t k, DescCtaSmem &S, 
             valid = desc_sample(W, px, py, prod, code);
         }
         desc_group(prod, code, valid, lane, S.g[par][warp], n, at);
-        __syncthreads();  // one per 128 samples: the buffers take turns
-        uint32_t mine[kDescWarps], some = 0;
+        __syncthreads();  // one per 256 samples: the buffers take turns
+        if (!owner) continue;
+        uint32_t some = 0;
 #pragma unroll
-        for (int g = 0; g < kDescWarps; ++g) {
+        for (int g = 0; g < kDescCtaWarps; ++g) {
             const DescGroup &G = S.g[par][g];
-            mine[g] = __popc(G.any[1 + iv] & G.any[7 + iu] & G.any[12 + io]);
-            some |= mine[g] ? 1u << g : 0u;
+            some |= (G.any[1 + iv] & G.any[7 + iu] & G.any[12 + io]) ? 1u << g : 0u;
         }
         while (some) {
-            const int g = __ffs(some) - 1;
+            const DescGroup &G = S.g[par][__ffs(some) - 1];
             some &= some - 1;
-            const DescGroup &G = S.g[par][g];
             const float4 *l = reinterpret_cast<const float4 *>(G.list + G.off[place]);
-            const uint32_t m = g == 0 ? mine[0] : g == 1 ? mine[1] : g == 2 ? mine[2] : mine[3];
-            for (uint32_t i = 0; i < m; i += 4, ++l) {
+            const int m = __popc(G.any[1 + iv] & G.any[7 + iu] & G.any[12 + io]);
+            for (int i = 0; i < m; i += 4, ++l) {
                 const float4 f = *l;
                 acc += f.x;
                 acc += f.y;
@@ -924,7 +929,7 @@ __device__ void describe_cta(const DescribeArgs &a, uint32_t k, DescCtaSmem &S, 
     float *sq = S.g[0][0].list;
     float v = acc;
     for (int pass = 0; pass < 2; ++pass) {
-        sq[bin] = v * v;
+        if (owner) sq[bin] = v * v;
         __syncthreads();
         if (tid == 0) S.norm = desc_norm(sq);
         __syncthreads();
@@ -932,22 +937,27 @@ __device__ void describe_cta(const DescribeArgs &a, uint32_t k, DescCtaSmem &S, 
         if (nrm > 0.0f) v = v / nrm;
         if (pass == 0) v = fminf(v, 0.2f);
     }
-    a.desc[(uint64_t)a.jobs[k].out_row * kDesc + bin] = v;
+    if (owner) a.desc[(uint64_t)a.jobs[k].out_row * kDesc + bin] = v;
 }
 
-// Blocks 0 .. n_large - 1: a large window each; the rest: four jobs each. One
+union DescMixedSmem {  // followed by a large window's rows: 4 (max_side + 1) + 2 max_side bytes
+    DescWarpSmem warp[kDescCtaWarps];
+    DescCtaSmem cta;
+};
+// Rows of the largest window a detector configuration can ask for: its base
+// blur takes sigma0 up to 42.4, a candidate's scale is at most 2^1.5 of that.
+constexpr int kDescMaxSide = 2600;
+
+// Blocks 0 .. n_large - 1: a large window each; the rest: eight jobs each. One
 // launch for both, so that small windows fill the GPU beside the last large ones.
-__global__ void __launch_bounds__(kDescThreads) describe_mixed_kernel(DescribeArgs a, uint32_t njobs) {
-    extern __shared__ uint32_t rows_of_cta[];
-    __shared__ __align__(16) union {
-        DescWarpSmem warp[kDescWarps];
-        DescCtaSmem cta;
-    } S;
+__global__ void __launch_bounds__(kDescCtaThreads) describe_mixed_kernel(DescribeArgs a, uint32_t njobs) {
+    extern __shared__ __align__(16) unsigned char desc_smem[];
+    DescMixedSmem &S = *reinterpret_cast<DescMixedSmem *>(desc_smem);
     if (blockIdx.x < a.n_large) {
-        describe_cta(a, blockIdx.x, S.cta, rows_of_cta);
+        describe_cta(a, blockIdx.x, S.cta, reinterpret_cast<uint32_t *>(desc_smem + sizeof(DescMixedSmem)));
         return;
     }
-    const uint32_t k = a.n_large + (blockIdx.x - a.n_large) * kDescWarps + (threadIdx.x >> 5);
+    const uint32_t k = a.n_large + (blockIdx.x - a.n_large) * kDescCtaWarps + (threadIdx.x >> 5);
     if (k < njobs) describe_warp(a, k, S.warp[threadIdx.x >> 5], threadIdx.x & 31);
 }
 
@@ -984,7 +994,8 @@ cudaError_t init_feature_kernels() {
             const cudaError_t e = cudaFuncSetAttribute(f.kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)f.smem);
             if (e != cudaSuccess) return e;
         }
-    return cudaSuccess;
+    return cudaFuncSetAttribute(describe_mixed_kernel, cudaFuncAttributeMaxDynamicSharedMemorySize,
+                                (int)(sizeof(DescMixedSmem) + 6 * (kDescMaxSide + 1)));
 }
 
 void launch_blur(const float *src, float *tmp, float *dst, const float *prev, float *dog, int w, int h, int nimg,
@@ -1048,8 +1059,9 @@ void launch_describe(const DescribeArgs &a, uint32_t njobs, cudaStream_t s) {
         describe_kernel<<<(njobs + kDescWarps - 1) / kDescWarps, kDescThreads, 0, s>>>(a, njobs);
         return;
     }
-    const size_t rows = 4 * (size_t)(a.max_side + 1) + 2 * (size_t)a.max_side;
-    describe_mixed_kernel<<<a.n_large + (njobs - a.n_large + kDescWarps - 1) / kDescWarps, kDescThreads, rows, s>>>(a, njobs);
+    const size_t rows = sizeof(DescMixedSmem) + 4 * (size_t)(a.max_side + 1) + 2 * (size_t)a.max_side;
+    describe_mixed_kernel<<<a.n_large + (njobs - a.n_large + kDescCtaWarps - 1) / kDescCtaWarps, kDescCtaThreads, rows,
+                            s>>>(a, njobs);
 }
 
 }  // namespace slm

@@ -3138,7 +3138,7 @@ slm_status feat_describe(slm_ctx *c, cudaStream_t st, DevBuf &buf, const FeatCor
     }
     // windows too large for one warp first
     const auto small = std::stable_partition(jobs.begin(), jobs.end(), [&](const DescJob &j) {
-        return describe_side(fc.cands[j.cand].sig) > kDescWarpSide;
+        return describe_side(fc.cands[j.cand].sig) > describe_warp_side(list.size());
     });
     unsigned char *d = buf.as<unsigned char>();
     SLM_CU(cudaMemcpyAsync(d + o_jobs, jobs.data(), sizeof(DescJob) * jobs.size(), cudaMemcpyHostToDevice, st));
@@ -3479,7 +3479,7 @@ extern "C" slm_status slm_describe(slm_ctx *c, const float *img, uint32_t w, uin
             DescribeArgs da{};
             da.jobs = reinterpret_cast<const DescJob *>(d + o_jobs);
             da.cs = reinterpret_cast<float2 *>(d + o_cs);
-            while (da.n_large < n && describe_side(kps[jobs[da.n_large].cand].sigma) > kDescWarpSide) ++da.n_large;
+            while (da.n_large < n && describe_side(kps[jobs[da.n_large].cand].sigma) > describe_warp_side(n)) ++da.n_large;
             da.max_side = describe_side(kps[jobs[0].cand].sigma);
             da.kps = reinterpret_cast<const slm_keypoint *>(d + o_kps);
             da.grads = reinterpret_cast<const float2 *>(d + o_grad);

@@ -248,6 +248,11 @@ void launch_extrema(const ExtremaArgs &a, int nimg, cudaStream_t s);
 void launch_candidate_sigma(FeatCand *cands, uint32_t n, float sigma0, float kstep, cudaStream_t s);
 void launch_orient(const OrientArgs &a, uint32_t n, cudaStream_t s);
 constexpr int kDescWarpSide = 127;  // window rows one warp takes
+// The window rows from which a feature gets a CTA instead of a warp: those a
+// warp cannot take, or, with fewer features than four warps for each of the
+// GPU's 608 sub-partitions, all: the chain of one warp then decides (one 717 x
+// 531 photo's 1026 features 0.39 ms as warps, 0.13 as CTAs).
+inline int describe_warp_side(size_t features) { return features < 2432 ? 0 : kDescWarpSide; }
 // Window rows of a feature of scale sigma (features.rs:526-528), at least.
 inline int describe_side(float sigma) { return 2 * ((int)(3.0f * sigma * 1.41421356f * 2.5f + 0.5f) + 1) + 1; }
 void launch_describe(const DescribeArgs &a, uint32_t njobs, cudaStream_t s);

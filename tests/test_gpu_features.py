@@ -229,3 +229,19 @@ def test_candidate_overflow_reruns_with_room(matcher):
     got = F.detect_and_describe(matcher, img, cfg)[0]
     assert len(got[0]) == int(cfg.max_features)
     check_equal(got, img, cfg)
+
+
+@pytest.mark.parametrize("n", [1, 9, 2431, 2432, 2440])
+def test_describe_by_warps_and_by_ctas(matcher, n):
+    """Keypoint counts on both sides of the rule that gives a feature a CTA or a
+    warp, windows from a few rows to hundreds (one warp's limit, 127 rows, among
+    them), mixed in one call, some of them over the image's borders or off it."""
+    img = synth.scene_canvas(150, 131, seed=3)
+    rng = np.random.default_rng(n)
+    sig = np.where(rng.random(n) < 0.9, rng.uniform(0.2, 2.0, n), rng.uniform(5.5, 20.0, n))
+    sig[: min(n, 6)] = np.asarray([5.88, 5.93, 5.98, 6.03, 64.0, 0.05])[: min(n, 6)]
+    kp = np.stack([rng.uniform(-20, 170, n), rng.uniform(-20, 150, n), sig, np.zeros(n), rng.uniform(-1, 7, n)], 1).astype(np.float32)
+    kp[:: 50, 4] = (0.0, np.pi / 2)[n % 2]  # rows along a cell edge
+    got = F.describe(matcher, img, kp)
+    want = np.stack([O.describe(img, *(float(v) for v in (k[0], k[1], k[2], k[4])), cr=True) for k in kp])
+    assert np.array_equal(got, want)
