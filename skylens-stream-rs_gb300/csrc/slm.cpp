@@ -2502,11 +2502,23 @@ extern "C" slm_status slm_sampson_score(slm_ctx *c, const double *pts, const uin
     SLM_TRY(ctx_check_device(c));
     Workspace *w = nullptr;
     SLM_TRY(ws_acquire(c, &w));
+    // The hypotheses are most of a call's bytes and each is read once, by one
+    // warp: the kernel reads them (and their pairs and mask offsets) where they
+    // lie if the device can read host memory, else they are copied first.
+    auto in_place = [&](const void *p, size_t align) {
+        if (!c->host_direct || !p || (reinterpret_cast<uintptr_t>(p) & (align - 1))) return false;
+        cudaPointerAttributes at{};
+        const bool ok = cudaPointerGetAttributes(&at, p) == cudaSuccess &&
+                        (at.type == cudaMemoryTypeUnregistered || at.type == cudaMemoryTypeHost);
+        cudaGetLastError();
+        return ok;
+    };
+    const bool e_there = in_place(E, 8), hp_there = in_place(hyp_pair, 4), mo_there = in_place(mask_off, 8);
     auto al = [](size_t x) { return (x + 255) & ~size_t(255); };
     const size_t o_pts = 0, o_off = al(o_pts + 32 * m), o_th = al(o_off + 8 * (uint64_t)(np + 1)),
-                 o_e = al(o_th + 8 * (uint64_t)np), o_hp = al(o_e + 72 * (uint64_t)nh),
-                 o_cnt = al(o_hp + 4 * (uint64_t)nh), o_moff = al(o_cnt + 4 * (uint64_t)nh),
-                 o_mask = al(o_moff + (mask_off ? 8 * (uint64_t)nh : 0)),
+                 o_e = al(o_th + 8 * (uint64_t)np), o_hp = al(o_e + (e_there ? 0 : 72 * (uint64_t)nh)),
+                 o_cnt = al(o_hp + (hp_there ? 0 : 4 * (uint64_t)nh)), o_moff = al(o_cnt + 4 * (uint64_t)nh),
+                 o_mask = al(o_moff + (mask_off && !mo_there ? 8 * (uint64_t)nh : 0)),
                  o_p32 = al(o_mask + (mask_off ? 4 * mask_words : 0)), bytes = al(o_p32 + 16 * m);
     slm_status st = w->score.ensure(c, bytes);
     if (st == SLM_OK) {
@@ -2518,9 +2530,9 @@ extern "C" slm_status slm_sampson_score(slm_ctx *c, const double *pts, const uin
         cudaError_t e = up(o_pts, pts, 32 * m);
         if (e == cudaSuccess) e = up(o_off, pair_off, 8 * (uint64_t)(np + 1));
         if (e == cudaSuccess) e = up(o_th, thresh, 8 * (uint64_t)np);
-        if (e == cudaSuccess) e = up(o_e, E, 72 * (uint64_t)nh);
-        if (e == cudaSuccess) e = up(o_hp, hyp_pair, 4 * (uint64_t)nh);
-        if (e == cudaSuccess && mask_off) e = up(o_moff, mask_off, 8 * (uint64_t)nh);
+        if (e == cudaSuccess && !e_there) e = up(o_e, E, 72 * (uint64_t)nh);
+        if (e == cudaSuccess && !hp_there) e = up(o_hp, hyp_pair, 4 * (uint64_t)nh);
+        if (e == cudaSuccess && mask_off && !mo_there) e = up(o_moff, mask_off, 8 * (uint64_t)nh);
         if (e == cudaSuccess && mask_off && mask_words) e = cudaMemsetAsync(d + o_mask, 0, 4 * mask_words, s);
         if (e == cudaSuccess) {
             SampsonArgs a{};
@@ -2529,11 +2541,11 @@ extern "C" slm_status slm_sampson_score(slm_ctx *c, const double *pts, const uin
             a.pts32 = reinterpret_cast<float4 *>(d + o_p32);
             a.pair_off = reinterpret_cast<const uint64_t *>(d + o_off);
             a.thresh = reinterpret_cast<const double *>(d + o_th);
-            a.E = reinterpret_cast<const double *>(d + o_e);
-            a.hyp_pair = reinterpret_cast<const uint32_t *>(d + o_hp);
+            a.E = e_there ? E : reinterpret_cast<const double *>(d + o_e);
+            a.hyp_pair = hp_there ? hyp_pair : reinterpret_cast<const uint32_t *>(d + o_hp);
             a.nh = nh;
             a.counts = reinterpret_cast<uint32_t *>(d + o_cnt);
-            a.mask_off = mask_off ? reinterpret_cast<const uint64_t *>(d + o_moff) : nullptr;
+            a.mask_off = !mask_off ? nullptr : mo_there ? mask_off : reinterpret_cast<const uint64_t *>(d + o_moff);
             a.masks = mask_off ? reinterpret_cast<uint32_t *>(d + o_mask) : nullptr;
             launch_sampson(a, s);
             e = cudaGetLastError();
