@@ -264,25 +264,38 @@ struct TrackPair {  // slm_pair_matches
     uint64_t first, count;
 };
 
+// Counters of one call (TrackArgs::ctl).
+enum : int { kTrEdges, kTrInvalid, kTrMembers, kTrComps, kTrLarge, kTrConflicts, kTrShort, kTrTracks, kTrObs, kTrCount };
+constexpr uint32_t kTrWarpMax = 256;  // members of a component one warp sorts
+
 struct TrackArgs {
     const TrackPair *pairs;
     const uint2 *matches;     // (feature of image_a, feature of image_b)
     const uint32_t *nf;       // features per image
-    const uint64_t *off;      // first node of each image
+    const uint64_t *off;      // first node of each image, and the number of nodes
     uint32_t n_images;
+    uint64_t n;               // nodes
+    uint32_t min_length;
     unsigned long long *table;  // open-addressing edge set, all ones = empty
     uint64_t table_mask;      // slots - 1 (a power of two)
-    unsigned long long *edges;  // the distinct edges, in insertion order
-    unsigned long long *n_edges;
-    unsigned long long *n_invalid;
+    unsigned long long *ctl;  // kTr* counters, zeroed
+    // per node
+    uint32_t *parent;
+    uint8_t *used;            // has an edge
+    uint32_t *cnt;            // of a root: members; after track_sort_kernel the track's length, or 0
+    uint32_t *start;          // of a root: first of its members
+    // per node with an edge, in component order
+    uint32_t *members, *spare;  // spare may be parent's memory
+    uint2 *sorted;            // members in order as (image, feature); may be the table's memory
+    uint2 *comps;             // components {root, members}: small ones from the front, large from the back
+    uint64_t max_comps;
+    uint64_t share;           // nodes per CTA of the last two kernels, at most 1024 CTAs
+    uint2 *sums;
+    uint64_t *track_off;
+    uint2 *obs;
 };
 
-void launch_track_edges(const TrackArgs &a, uint32_t n_pairs, cudaStream_t s);
-void launch_track_init(uint32_t *parent, uint8_t *used, uint64_t n, int grid, cudaStream_t s);
-void launch_track_mark(const unsigned long long *edges, const unsigned long long *n_edges, uint8_t *used, int grid,
-                       cudaStream_t s);
-void launch_track_hook(const unsigned long long *edges, const unsigned long long *n_edges, uint32_t *parent,
-                       uint32_t *changed, int grid, cudaStream_t s);
-void launch_track_jump(uint32_t *parent, uint64_t n, int grid, cudaStream_t s);
+// The whole of a call on the device: track_off, obs and the counters.
+void launch_tracks(const TrackArgs &a, uint32_t n_pairs, int sms, cudaStream_t s);
 
 }  // namespace slm

@@ -135,3 +135,31 @@ def test_matches_read_in_place_or_copied(matcher):
                                                 ctypes.byref(no), ctypes.byref(st)) == 0
         got = [[(int(i), int(f)) for i, f in obs[int(toff[t]):int(toff[t + 1])]] for t in range(nt.value)]
         assert got == want[0] and st.as_dict() == want[1]
+
+
+@pytest.mark.parametrize("length", [31, 32, 33, 255, 256, 257, 511, 700])
+@pytest.mark.parametrize("twist", ["none", "conflict", "gaps"])
+def test_long_components(matcher, length, twist):
+    # tracks through `length` images, joined in random order: a warp's and a
+    # CTA's sort, a conflict between two far members, and images without features
+    # (which share their first node with the next image)
+    rng = np.random.default_rng(length)
+    n_images = 2 * length if twist == "gaps" else length
+    imgs = np.sort(rng.choice(n_images, length, replace=False))
+    nf = np.zeros(n_images, np.int64)
+    nf[imgs] = rng.integers(4, 9, length)
+    pairs = []
+    for t in range(3):
+        feat = [int(rng.integers(0, nf[i] - 3)) + t for i in imgs]
+        pairs += [(int(imgs[k]), int(imgs[k + 1]), [(feat[k], feat[k + 1])]) for k in range(length - 1)]
+    if twist == "conflict":
+        # the first image's last feature, seen again by the last image's
+        pairs.append((int(imgs[0]), int(imgs[-1]), [(int(nf[imgs[0]]) - 1, int(nf[imgs[-1]]) - 1)]))
+    pairs = [pairs[k] for k in rng.permutation(len(pairs))]
+    both(matcher, nf.tolist(), pairs)
+    both(matcher, nf.tolist(), pairs, max_tracks=1)
+
+
+def test_every_match_invalid(matcher):
+    assert both(matcher, [0, 0], [(0, 1, [(0, 0), (1, 0)])])[1]["invalid_matches"] == 2
+    assert both(matcher, [], [(0, 1, [(0, 0)])])[1]["invalid_matches"] == 1
