@@ -261,7 +261,37 @@ struct slm_plan {
     std::vector<Item> items;
     std::vector<uint64_t> slot_off;  // np + 1
     uint64_t n_parts = 0, n_cols = 0, n_slots = 0, distances = 0;
-    DevBuf d_meta, d_items, d_parts, d_colbest, d_slots, d_counts, d_ctl, d_offsets, d_dense;
+    DevBuf d_parts, d_colbest, d_slots, d_dense;
+    // What the host makes of a plan, in one block and one upload: the pairs, then
+    // the work items and tables at their offsets.
+    DevBuf d_up;
+    std::vector<unsigned char> up;
+    uint64_t o_slot = 0, o_items = 0, o_spairs = 0, o_sitems = 0, o_samples = 0, o_titems = 0, o_tstart = 0, o_tblk = 0;
+    template <class T>
+    uint64_t add_up(const std::vector<T> &v) {
+        const uint64_t at = (up.size() + 255) / 256 * 256;
+        up.resize(at + sizeof(T) * v.size());
+        if (!v.empty()) std::memcpy(up.data() + at, v.data(), sizeof(T) * v.size());
+        return at;
+    }
+    template <class T>
+    T *up_at(uint64_t o) const {
+        return reinterpret_cast<T *>(d_up.as<unsigned char>() + o);
+    }
+    // The control words, the matches' offsets (the two come back in one copy), and
+    // the counters that start at zero, in one block that one memset clears.
+    DevBuf d_ctl;
+    uint64_t o_counts = 0, o_pairctl = 0, o_ucnt = 0, ctl_bytes = 0;
+    uint64_t *offsets() const { return reinterpret_cast<uint64_t *>(d_ctl.as<unsigned char>() + kCtlBytes); }
+    uint32_t *counts() const { return reinterpret_cast<uint32_t *>(d_ctl.as<unsigned char>() + o_counts); }
+    slm_status ensure_ctl(bool shortlist) {
+        const uint64_t n = std::max<uint64_t>(1, np);
+        o_pairctl = kCtlBytes + (8 * (n + 1) + 15) / 16 * 16;
+        o_counts = o_pairctl + (shortlist ? 16 * n : 0);
+        o_ucnt = o_counts + 4 * n;
+        ctl_bytes = o_ucnt + (shortlist ? 4 * std::max<uint64_t>(1, buckets) : 0);
+        return d_ctl.ensure(ctx, ctl_bytes);
+    }
     // shortlist path
     std::vector<SlItem> sitems;        // pass items, then the samples' items
     std::vector<SlSample> samples;
@@ -270,8 +300,8 @@ struct slm_plan {
     uint32_t half_recs = kSlHalfRecs;  // records per candidate row and column half
     uint64_t rows_pad = 0, cand_rows_pad = 0, cols_pad = 0, sl_parts = 0, queue_cap = 0, xitem_cap = 0, row_blocks_total = 0;
     uint32_t row_blocks = 1;  // the most row blocks of any pair
-    DevBuf d_sitems, d_spairs, d_rowpart, d_rownear, d_colmin, d_rowthr, d_colthr, d_rowcnt, d_rowrec, d_rowrecj, d_colcnt,
-        d_rowdec, d_queue, d_rqueue, d_dump, d_xlist, d_xitems, d_xparts, d_blkcnt, d_pairctl;
+    DevBuf d_rowpart, d_rownear, d_colmin, d_rowthr, d_colthr, d_rowcnt, d_rowrec, d_rowrecj, d_colcnt,
+        d_rowdec, d_queue, d_rqueue, d_dump, d_xlist, d_xitems, d_xparts, d_blkcnt;
     // BF16 pass: segments in the order the CTAs run them, each CTA's first one,
     // each block's parts; then its results and the undecided rows
     std::vector<TopItem> titems;
@@ -279,7 +309,7 @@ struct slm_plan {
     std::vector<uint2> tblk;
     uint32_t tshift = 8, max_na = 0, buckets = 0;
     uint64_t top_parts = 0;
-    DevBuf d_samples, d_titems, d_tstart, d_tblk, d_topmm, d_topj, d_olist, d_ulist, d_ucnt, d_ugroups;
+    DevBuf d_topmm, d_topj, d_olist, d_ulist, d_ugroups;
     bool dump = false;
     uint32_t min_matches = 0;        // pairs with fewer matches report none
     cudaGraphExec_t exec = nullptr;
@@ -290,6 +320,7 @@ struct slm_plan {
     void *graph_optiles[2] = {nullptr, nullptr};  // store buffers the captured graph reads
     void *graph_tiled = nullptr;
     bool launched = false;
+    bool timed = true;  // record the events: off where no caller reads the times
     ~slm_plan() {
         if (exec) cudaGraphExecDestroy(exec);
         if (graph) cudaGraphDestroy(graph);
@@ -302,13 +333,11 @@ struct slm_plan {
 
 // Every device buffer of a plan: all are used on the plan's stream only, and
 // allocated ordered on it (DevBuf::order_on).
-std::array<DevBuf *, 39> plan_buffers(slm_plan *p) {
-    return {&p->d_meta, &p->d_items, &p->d_parts, &p->d_colbest, &p->d_slots, &p->d_counts, &p->d_ctl,
-            &p->d_offsets, &p->d_dense, &p->d_sitems, &p->d_spairs, &p->d_rowpart, &p->d_rownear,
-            &p->d_colmin, &p->d_rowthr, &p->d_colthr, &p->d_rowcnt, &p->d_rowrec, &p->d_rowrecj,
-            &p->d_colcnt, &p->d_rowdec, &p->d_queue, &p->d_rqueue, &p->d_dump, &p->d_xlist, &p->d_xitems,
-            &p->d_xparts, &p->d_blkcnt, &p->d_pairctl, &p->d_samples, &p->d_titems, &p->d_tstart, &p->d_tblk, &p->d_topmm,
-            &p->d_topj, &p->d_olist, &p->d_ulist, &p->d_ucnt, &p->d_ugroups};
+std::array<DevBuf *, 28> plan_buffers(slm_plan *p) {
+    return {&p->d_up, &p->d_parts, &p->d_colbest, &p->d_slots, &p->d_ctl, &p->d_dense, &p->d_rowpart, &p->d_rownear,
+            &p->d_colmin, &p->d_rowthr, &p->d_colthr, &p->d_rowcnt, &p->d_rowrec, &p->d_rowrecj, &p->d_colcnt,
+            &p->d_rowdec, &p->d_queue, &p->d_rqueue, &p->d_dump, &p->d_xlist, &p->d_xitems, &p->d_xparts, &p->d_blkcnt,
+            &p->d_topmm, &p->d_topj, &p->d_olist, &p->d_ulist, &p->d_ugroups};
 }
 // Frees a plan's buffers while its stream still exists (their frees are
 // ordered on it): owners call it before destroying that stream.
@@ -554,7 +583,6 @@ slm_status plan_fp8_items(slm_plan *p, const slm_pair *pairs) {
     p->cols_pad = cb + kTile;
     p->sl_parts = std::max<uint64_t>(part, 1);
     p->half_recs = p->tune.shortlist_k ? p->tune.shortlist_k : kSlHalfRecs;
-    SLM_TRY(p->d_sitems.ensure(c, sizeof(SlItem) * std::max<size_t>(1, p->sitems.size())));
     SLM_TRY(p->d_rowpart.ensure(c, sizeof(float2) * 256 * p->sl_parts));
     SLM_TRY(p->d_rownear.ensure(c, sizeof(uint32_t) * 256 * p->sl_parts));
     SLM_TRY(p->d_colmin.ensure(c, sizeof(uint32_t) * p->cols_pad));
@@ -565,11 +593,13 @@ slm_status plan_fp8_items(slm_plan *p, const slm_pair *pairs) {
     SLM_TRY(p->d_rowrecj.ensure(c, sizeof(uint32_t) * 2 * p->half_recs * p->cand_rows_pad));
     SLM_TRY(p->d_colcnt.ensure(c, sizeof(uint32_t) * p->cols_pad));
     SLM_TRY(p->d_rqueue.ensure(c, sizeof(SlQueue) * p->queue_cap));
-    SLM_CU(cudaMemcpyAsync(p->d_sitems.p, p->sitems.data(), sizeof(SlItem) * p->sitems.size(), cudaMemcpyHostToDevice,
-                           p->stream));
-    SLM_TRY(p->d_samples.ensure(c, sizeof(SlSample) * std::max<size_t>(1, p->samples.size())));
-    SLM_CU(cudaMemcpyAsync(p->d_samples.p, p->samples.data(), sizeof(SlSample) * p->samples.size(),
-                           cudaMemcpyHostToDevice, p->stream));
+    return SLM_OK;
+}
+
+slm_status plan_upload(slm_plan *p) {
+    SLM_TRY(p->d_up.ensure(p->ctx, std::max<size_t>(1, p->up.size())));
+    if (!p->up.empty())
+        SLM_CU(cudaMemcpyAsync(p->d_up.p, p->up.data(), p->up.size(), cudaMemcpyHostToDevice, p->stream));
     return SLM_OK;
 }
 
@@ -623,18 +653,12 @@ slm_status plan_build_shortlist(slm_plan *p, const slm_pair *pairs) {
     if (p->prec == SLM_PREC_FP8) SLM_TRY(plan_fp8_items(p, pairs));
     plan_top2(p);
     p->row_blocks_total = blk;
-    SLM_TRY(p->d_spairs.ensure(c, sizeof(SlPair) * std::max<size_t>(1, p->np)));
-    SLM_TRY(p->d_titems.ensure(c, sizeof(TopItem) * std::max<size_t>(1, p->titems.size())));
-    SLM_TRY(p->d_tstart.ensure(c, sizeof(uint32_t) * p->tstart.size()));
-    SLM_TRY(p->d_tblk.ensure(c, sizeof(uint2) * std::max<size_t>(1, p->tblk.size())));
     SLM_TRY(p->d_topmm.ensure(c, sizeof(float2) * std::max<uint64_t>(1, p->top_parts << p->tshift)));
     SLM_TRY(p->d_topj.ensure(c, sizeof(uint32_t) * std::max<uint64_t>(1, p->top_parts << p->tshift)));
     SLM_TRY(p->d_olist.ensure(c, sizeof(uint4) * std::max<uint64_t>(1, p->n_slots)));
     SLM_TRY(p->d_ulist.ensure(c, sizeof(uint2) * std::max<uint64_t>(1, p->n_slots)));
-    SLM_TRY(p->d_ucnt.ensure(c, sizeof(uint32_t) * std::max<uint32_t>(1, p->buckets)));
     SLM_TRY(p->d_ugroups.ensure(c, sizeof(uint4) * std::max<uint64_t>(1, groups)));
     SLM_TRY(p->d_blkcnt.ensure(c, sizeof(uint32_t) * std::max<uint64_t>(1, blk)));
-    SLM_TRY(p->d_pairctl.ensure(c, 4 * sizeof(uint32_t) * std::max<size_t>(1, p->np)));
     SLM_TRY(p->d_xlist.ensure(c, sizeof(uint32_t) * std::max<size_t>(1, p->np)));
     SLM_TRY(p->d_xitems.ensure(c, sizeof(Item) * p->xitem_cap));
     SLM_TRY(p->d_xparts.ensure(c, sizeof(RowPart) * kTile * p->xitem_cap));
@@ -642,21 +666,18 @@ slm_status plan_build_shortlist(slm_plan *p, const slm_pair *pairs) {
     SLM_TRY(p->d_rowdec.ensure(c, sizeof(uint32_t) * p->rows_pad));
     SLM_TRY(p->d_queue.ensure(c, sizeof(SlQueue) * p->queue_cap));
     if (p->dump && p->np) SLM_TRY(p->d_dump.ensure(c, sizeof(float) * std::max<uint64_t>(1, (uint64_t)p->meta[0].na * p->meta[0].nb)));
-    SLM_TRY(p->d_meta.ensure(c, sizeof(PairMeta) * std::max<size_t>(1, p->np)));
     SLM_TRY(p->d_slots.ensure(c, sizeof(uint2) * std::max<uint64_t>(1, p->n_slots)));
-    SLM_TRY(p->d_counts.ensure(c, sizeof(uint32_t) * std::max<size_t>(1, p->np)));
-    SLM_TRY(p->d_ctl.ensure(c, kCtlBytes));
-    SLM_TRY(p->d_offsets.ensure(c, sizeof(uint64_t) * (p->np + 1) * 2));
     SLM_TRY(p->d_dense.ensure(c, sizeof(uint2) * std::max<uint64_t>(1, p->n_slots)));
-    cudaStream_t s = p->stream;
-    SLM_CU(cudaMemcpyAsync(p->d_meta.p, p->meta.data(), sizeof(PairMeta) * p->np, cudaMemcpyHostToDevice, s));
-    SLM_CU(cudaMemcpyAsync(p->d_offsets.as<uint64_t>() + (p->np + 1), p->slot_off.data(),
-                           sizeof(uint64_t) * (p->np + 1), cudaMemcpyHostToDevice, s));
-    SLM_CU(cudaMemcpyAsync(p->d_spairs.p, p->spairs.data(), sizeof(SlPair) * p->np, cudaMemcpyHostToDevice, s));
-    SLM_CU(cudaMemcpyAsync(p->d_titems.p, p->titems.data(), sizeof(TopItem) * p->titems.size(), cudaMemcpyHostToDevice, s));
-    SLM_CU(cudaMemcpyAsync(p->d_tstart.p, p->tstart.data(), sizeof(uint32_t) * p->tstart.size(), cudaMemcpyHostToDevice, s));
-    SLM_CU(cudaMemcpyAsync(p->d_tblk.p, p->tblk.data(), sizeof(uint2) * p->tblk.size(), cudaMemcpyHostToDevice, s));
-    return SLM_OK;
+    p->o_spairs = p->add_up(p->spairs);
+    p->o_titems = p->add_up(p->titems);
+    p->o_tstart = p->add_up(p->tstart);
+    p->o_tblk = p->add_up(p->tblk);
+    if (p->prec == SLM_PREC_FP8) {
+        p->o_sitems = p->add_up(p->sitems);
+        p->o_samples = p->add_up(p->samples);
+    }
+    SLM_TRY(p->ensure_ctl(true));
+    return plan_upload(p);
 }
 
 slm_status plan_build(slm_plan *p, const slm_pair *pairs) {
@@ -684,31 +705,26 @@ slm_status plan_build(slm_plan *p, const slm_pair *pairs) {
     p->n_cols = col;
     p->n_slots = slot;
     p->distances = dist;
+    if (p->prec == SLM_PREC_FP32) plan_items(p);  // fills the pairs' parts
+    p->up.clear();
+    p->add_up(p->meta);  // at 0
+    p->o_slot = p->add_up(p->slot_off);
     if (p->prec != SLM_PREC_FP32) return plan_build_shortlist(p, pairs);
-    plan_items(p);
     slm_ctx *c = p->ctx;
-    SLM_TRY(p->d_meta.ensure(c, sizeof(PairMeta) * std::max<size_t>(1, p->np)));
     SLM_TRY(p->d_colbest.ensure(c, sizeof(unsigned long long) * std::max<uint64_t>(1, col)));
     SLM_TRY(p->d_slots.ensure(c, sizeof(uint2) * std::max<uint64_t>(1, slot)));
-    SLM_TRY(p->d_counts.ensure(c, sizeof(uint32_t) * std::max<size_t>(1, p->np)));
-    SLM_TRY(p->d_ctl.ensure(c, kCtlBytes));
-    SLM_TRY(p->d_offsets.ensure(c, sizeof(uint64_t) * (p->np + 1) * 2));
     SLM_TRY(p->d_dense.ensure(c, sizeof(uint2) * std::max<uint64_t>(1, slot)));
-    cudaStream_t s = p->stream;
-    SLM_CU(cudaMemcpyAsync(p->d_meta.p, p->meta.data(), sizeof(PairMeta) * p->np, cudaMemcpyHostToDevice, s));
-    // slot offsets live in the second half of d_offsets
-    SLM_CU(cudaMemcpyAsync(p->d_offsets.as<uint64_t>() + (p->np + 1), p->slot_off.data(),
-                           sizeof(uint64_t) * (p->np + 1), cudaMemcpyHostToDevice, s));
-    SLM_TRY(p->d_items.ensure(c, sizeof(Item) * std::max<size_t>(1, p->items.size())));
     SLM_TRY(p->d_parts.ensure(c, sizeof(RowPart) * kTile * std::max<uint64_t>(1, p->n_parts)));
-    SLM_CU(cudaMemcpyAsync(p->d_items.p, p->items.data(), sizeof(Item) * p->items.size(), cudaMemcpyHostToDevice, s));
-    return SLM_OK;
+    p->o_items = p->add_up(p->items);
+    SLM_TRY(p->ensure_ctl(false));
+    return plan_upload(p);
 }
 
 // Enqueue the whole batch on stream s (also used for graph capture).
 slm_status plan_enqueue(slm_plan *p, cudaStream_t s) {
     uint32_t *ctl = p->d_ctl.as<uint32_t>();  // [0] work counter, [1] error word, [2..] shortlist counters
-    SLM_CU(cudaMemsetAsync(ctl, 0, kCtlBytes, s));
+    // the shortlist's counters follow the control words; the exact path writes its counts
+    SLM_CU(cudaMemsetAsync(ctl, 0, p->prec != SLM_PREC_FP32 ? p->ctl_bytes : kCtlBytes, s));
     if (p->prec != SLM_PREC_FP32) {
         slm_store *st = p->st;
         const bool fp8 = p->prec == SLM_PREC_FP8;
@@ -717,8 +733,6 @@ slm_status plan_enqueue(slm_plan *p, cudaStream_t s) {
             SLM_CU(cudaMemsetAsync(p->d_rowcnt.p, 0, 2 * sizeof(uint32_t) * p->cand_rows_pad, s));
             SLM_CU(cudaMemsetAsync(p->d_colcnt.p, 0, sizeof(uint32_t) * p->cols_pad, s));
         }
-        SLM_CU(cudaMemsetAsync(p->d_pairctl.p, 0, 4 * sizeof(uint32_t) * p->np, s));
-        SLM_CU(cudaMemsetAsync(p->d_counts.p, 0, sizeof(uint32_t) * p->np, s));  // compact adds its blocks
         SlArgs a{};
         const slm_store::LowpImage &im = st->lowp[p->prec == SLM_PREC_FP8 ? 1 : 0];
         a.optiles = im.optiles.as<uint8_t>();
@@ -726,12 +740,12 @@ slm_status plan_enqueue(slm_plan *p, cudaStream_t s) {
         a.raw = st->raw.as<float>();
         a.qscale = p->prec == SLM_PREC_FP8 ? im.qscale.as<float>() : nullptr;
         a.vstats = im.vstats.as<ViewStat>();
-        a.pairs = p->d_meta.as<PairMeta>();
-        a.spairs = p->d_spairs.as<SlPair>();
+        a.pairs = p->up_at<PairMeta>(0);
+        a.spairs = p->up_at<SlPair>(p->o_spairs);
         a.npairs = p->np;
-        a.items = p->d_sitems.as<SlItem>();
+        a.items = p->up_at<SlItem>(p->o_sitems);
         a.n_items = p->n_sitems;
-        a.samples = p->d_samples.as<SlSample>();
+        a.samples = p->up_at<SlSample>(p->o_samples);
         a.n_samples = (uint32_t)p->samples.size();
         a.n_sample_items = (uint32_t)p->sitems.size() - p->n_sitems;
         a.rowpart = p->d_rowpart.as<float2>();
@@ -754,9 +768,9 @@ slm_status plan_enqueue(slm_plan *p, cudaStream_t s) {
         a.fp8 = p->prec == SLM_PREC_FP8;
         a.dump = p->dump ? p->d_dump.as<float>() : nullptr;
         a.slots = p->d_slots.as<uint2>();
-        a.counts = p->d_counts.as<uint32_t>();
+        a.counts = p->counts();
         a.blkcnt = p->d_blkcnt.as<uint32_t>();
-        a.pairctl = p->d_pairctl.as<uint32_t>();
+        a.pairctl = reinterpret_cast<uint32_t *>(p->d_ctl.as<unsigned char>() + p->o_pairctl);
         a.row_blocks = p->row_blocks;
         a.tiled = st->tiled.as<float>();
         a.xlist = p->d_xlist.as<uint32_t>();
@@ -766,11 +780,11 @@ slm_status plan_enqueue(slm_plan *p, cudaStream_t s) {
         a.colbest = p->d_colbest.as<unsigned long long>();
         a.want_items = 4u * (uint32_t)std::max(1, p->ctx->sms);
         a.tier = 0;
-        a.titems = p->d_titems.as<TopItem>();
-        a.tstart = p->d_tstart.as<uint32_t>();
+        a.titems = p->up_at<TopItem>(p->o_titems);
+        a.tstart = p->up_at<uint32_t>(p->o_tstart);
         a.tgrid = (uint32_t)p->tstart.size() - 1;
         a.tshift = p->tshift;
-        a.tblk = p->d_tblk.as<uint2>();
+        a.tblk = p->up_at<uint2>(p->o_tblk);
         a.topmm = p->d_topmm.as<float2>();
         a.topj = p->d_topj.as<uint32_t>();
         a.max_na = p->max_na;
@@ -778,27 +792,26 @@ slm_status plan_enqueue(slm_plan *p, cudaStream_t s) {
         a.olist = p->d_olist.as<uint4>();
         a.cand_cap = 2 * (p->tune.shortlist_k ? p->tune.shortlist_k : (uint32_t)kSlHalfRecs);
         a.ulist = p->d_ulist.as<uint2>();
-        a.ucnt = p->d_ucnt.as<uint32_t>();
+        a.ucnt = reinterpret_cast<uint32_t *>(p->d_ctl.as<unsigned char>() + p->o_ucnt);
         a.ugroups = p->d_ugroups.as<uint4>();
-        SLM_CU(cudaMemsetAsync(p->d_ucnt.p, 0, sizeof(uint32_t) * std::max<uint32_t>(1, p->buckets), s));
         int nk = fp8 ? 1 : 0;  // the colmin fill
-        SLM_CU(record_event(p->ev0, s));
+        if (p->timed) SLM_CU(record_event(p->ev0, s));
         nk += launch_shortlist_eps(a, s);
         if (!fp8) {
             nk += launch_top2_pass(a, s);
-            SLM_CU(record_event(p->evp[0], s));
+            if (p->timed) SLM_CU(record_event(p->evp[0], s));
             nk += launch_top2_decide(a, p->ctx->sms, s);
-            SLM_CU(record_event(p->evp[1], s));
+            if (p->timed) SLM_CU(record_event(p->evp[1], s));
             nk += launch_top2_resolve(a, p->ctx->sms, s);
-            SLM_CU(record_event(p->evp[2], s));
+            if (p->timed) SLM_CU(record_event(p->evp[2], s));
         } else {
             nk += launch_shortlist_sample(a, p->ctx->sms, s);
             nk += launch_shortlist_pass(a, 1, p->ctx->sms, s);
-            SLM_CU(record_event(p->evp[0], s));
+            if (p->timed) SLM_CU(record_event(p->evp[0], s));
             nk += launch_shortlist_mid(a, s);
-            SLM_CU(record_event(p->evp[1], s));
+            if (p->timed) SLM_CU(record_event(p->evp[1], s));
             nk += launch_shortlist_pass(a, 2, p->ctx->sms, s);
-            SLM_CU(record_event(p->evp[2], s));
+            if (p->timed) SLM_CU(record_event(p->evp[2], s));
             nk += launch_shortlist_finalize(a, s);
             // tier 1: the BF16 pass over the pairs FP8 could not settle (its
             // kernels return at once when no pair was rescued)
@@ -817,15 +830,15 @@ slm_status plan_enqueue(slm_plan *p, cudaStream_t s) {
             nk += launch_top2_resolve(b, p->ctx->sms, s);
         }
         nk += launch_shortlist_tail(a, p->ctx->sms, s);
-        SLM_CU(record_event(p->ev1, s));
+        if (p->timed) SLM_CU(record_event(p->ev1, s));
         p->kernels = (uint64_t)nk + 2;  // + scan_counts, gather
         if (p->min_matches > 1) {
-            launch_filter_counts(p->d_counts.as<uint32_t>(), p->np, p->min_matches, s);
+            launch_filter_counts(p->counts(), p->np, p->min_matches, s);
             p->kernels++;
         }
-        uint64_t *offsets = p->d_offsets.as<uint64_t>();
-        launch_scan_counts(p->d_counts.as<uint32_t>(), p->np, offsets, s);
-        launch_gather_blocks(a, offsets + (p->np + 1), offsets, p->d_dense.as<uint2>(), p->n_slots, s);
+        uint64_t *offsets = p->offsets();
+        launch_scan_counts(p->counts(), p->np, offsets, s);
+        launch_gather_blocks(a, p->up_at<uint64_t>(p->o_slot), offsets, p->d_dense.as<uint2>(), p->n_slots, s);
         SLM_CU(cudaGetLastError());
         return SLM_OK;
     }
@@ -834,9 +847,9 @@ slm_status plan_enqueue(slm_plan *p, cudaStream_t s) {
     {
         ExactArgs a{};
         a.tiled = p->st->tiled.as<float>();
-        a.items = p->d_items.as<Item>();
+        a.items = p->up_at<Item>(p->o_items);
         a.n_items = (uint32_t)p->items.size();
-        a.pairs = p->d_meta.as<PairMeta>();
+        a.pairs = p->up_at<PairMeta>(0);
         a.parts = p->d_parts.as<RowPart>();
         a.colbest = p->d_colbest.as<unsigned long long>();
         a.work = ctl;
@@ -844,28 +857,28 @@ slm_status plan_enqueue(slm_plan *p, cudaStream_t s) {
         a.mutual = p->mutual;
         a.x2 = p->tune.variant == 1 ? 0 : 1;  // packed f32x2 arithmetic; 1: all scalar
         // External records so that the events become timing nodes under graph capture.
-        SLM_CU(record_event(p->ev0, s));
+        if (p->timed) SLM_CU(record_event(p->ev0, s));
         if (a.n_items) launch_exact(a, std::min<int>(p->ctx->sms, (int)a.n_items), s);
-        SLM_CU(record_event(p->ev1, s));
+        if (p->timed) SLM_CU(record_event(p->ev1, s));
         p->kernels = (p->mutual ? 1 : 0) + (a.n_items ? 1 : 0) + (p->np ? 1 : 0) + 1 + (p->np ? 1 : 0);
         FinalizeArgs f{};
-        f.pairs = p->d_meta.as<PairMeta>();
+        f.pairs = p->up_at<PairMeta>(0);
         f.npairs = p->np;
         f.parts = p->d_parts.as<RowPart>();
         f.colbest = p->d_colbest.as<unsigned long long>();
         f.ratio2 = ratio2;
         f.mutual = p->mutual;
         f.slots = p->d_slots.as<uint2>();
-        f.counts = p->d_counts.as<uint32_t>();
+        f.counts = p->counts();
         launch_finalize(f, s);
     }
     if (p->min_matches > 1) {
-        launch_filter_counts(p->d_counts.as<uint32_t>(), p->np, p->min_matches, s);
+        launch_filter_counts(p->counts(), p->np, p->min_matches, s);
         p->kernels++;
     }
-    uint64_t *offsets = p->d_offsets.as<uint64_t>();
-    launch_scan_counts(p->d_counts.as<uint32_t>(), p->np, offsets, s);
-    launch_gather(p->d_slots.as<uint2>(), offsets + (p->np + 1), p->d_counts.as<uint32_t>(), offsets, p->np,
+    uint64_t *offsets = p->offsets();
+    launch_scan_counts(p->counts(), p->np, offsets, s);
+    launch_gather(p->d_slots.as<uint2>(), p->up_at<uint64_t>(p->o_slot), p->counts(), offsets, p->np,
                   p->d_dense.as<uint2>(), p->n_slots, s);
     SLM_CU(cudaGetLastError());
     return SLM_OK;
@@ -1030,7 +1043,7 @@ slm_status fill_stats(slm_plan *p, slm_stats *st, uint64_t matches, const uint32
         std::memcpy(&e, &w[kCtlMaxErr], sizeof(e));
         st->max_abs_err = e;
     }
-    if (p->launched && p->ev0 && p->ev1) {
+    if (p->launched && p->timed && p->ev0 && p->ev1) {
         float ms = 0;
         if (cudaEventElapsedTime(&ms, p->ev0, p->ev1) == cudaSuccess) st->kernel_ms = ms;
         if (p->prec != SLM_PREC_FP32) {
@@ -1401,10 +1414,12 @@ slm_status plan_launch_on(slm_plan *p, cudaStream_t s, bool use_graph) {
     p->graph_tiled = p->st->tiled.p;
     p->graph_optiles[0] = p->st->lowp[0].optiles.p;
     p->graph_optiles[1] = p->st->lowp[1].optiles.p;
-    if (!p->ev0) SLM_CU(cudaEventCreate(&p->ev0));
-    if (!p->ev1) SLM_CU(cudaEventCreate(&p->ev1));
-    for (cudaEvent_t &e : p->evp)
-        if (!e) SLM_CU(cudaEventCreate(&e));
+    if (p->timed) {
+        if (!p->ev0) SLM_CU(cudaEventCreate(&p->ev0));
+        if (!p->ev1) SLM_CU(cudaEventCreate(&p->ev1));
+        for (cudaEvent_t &e : p->evp)
+            if (!e) SLM_CU(cudaEventCreate(&e));
+    }
     if (use_graph) {
         if (!p->exec) {
             SLM_CU(cudaStreamBeginCapture(s, cudaStreamCaptureModeThreadLocal));
@@ -1569,10 +1584,15 @@ extern "C" slm_status slm_plan_results(slm_plan *p, slm_pair *out, uint64_t cap,
     if (!p->launched) return fail(SLM_INVALID_ARG, "plan was not launched");
     SLM_TRY(ctx_check_device(p->ctx));
     SLM_CU(cudaStreamSynchronize(p->stream));
-    SLM_TRY(check_status_word(p));
-    SLM_CU(cudaMemcpy(offsets, p->d_offsets.p, sizeof(uint64_t) * (p->np + 1), cudaMemcpyDeviceToHost));
+    // the control words and the offsets in one copy
+    std::vector<unsigned char> head(kCtlBytes + sizeof(uint64_t) * (p->np + 1));
+    SLM_CU(cudaMemcpy(head.data(), p->d_ctl.p, head.size(), cudaMemcpyDeviceToHost));
+    uint32_t ctl[16];
+    std::memcpy(ctl, head.data(), sizeof(ctl));
+    SLM_TRY(status_of_word(ctl[1]));
+    std::memcpy(offsets, head.data() + kCtlBytes, sizeof(uint64_t) * (p->np + 1));
     const uint64_t total = offsets[p->np];
-    SLM_TRY(fill_stats(p, st, total));
+    SLM_TRY(fill_stats(p, st, total, ctl));
     if (total > cap) return fail(SLM_CAPACITY, "need " + std::to_string(total) + " pairs, have " + std::to_string(cap));
     if (total) SLM_CU(cudaMemcpy(out, p->d_dense.p, sizeof(slm_pair) * total, cudaMemcpyDeviceToHost));
     return SLM_OK;
@@ -1581,7 +1601,7 @@ extern "C" slm_status slm_plan_results(slm_plan *p, slm_pair *out, uint64_t cap,
 extern "C" slm_status slm_plan_device_results(slm_plan *p, const uint32_t **d_counts, const slm_pair **d_slots,
                                               const uint64_t **h_slot_offsets) {
     if (!p) return fail(SLM_INVALID_ARG, "NULL plan");
-    if (d_counts) *d_counts = p->d_counts.as<uint32_t>();
+    if (d_counts) *d_counts = p->counts();
     if (d_slots) *d_slots = p->d_slots.as<slm_pair>();
     if (h_slot_offsets) *h_slot_offsets = p->slot_off.data();
     return SLM_OK;
@@ -1589,15 +1609,23 @@ extern "C" slm_status slm_plan_device_results(slm_plan *p, const uint32_t **d_co
 
 extern "C" uint64_t slm_plan_bytes(slm_plan *p) {
     if (!p) return 0;
-    return p->d_meta.bytes + p->d_items.bytes + p->d_parts.bytes + p->d_colbest.bytes + p->d_slots.bytes +
-           p->d_counts.bytes + p->d_ctl.bytes + p->d_offsets.bytes + p->d_dense.bytes;
+    return p->d_up.bytes + p->d_parts.bytes + p->d_colbest.bytes + p->d_slots.bytes + p->d_ctl.bytes + p->d_dense.bytes;
 }
+
+// A plan that is launched once: plain launches. Capturing, instantiating and
+// destroying a graph for it cost 50 us of a call, event records, separate
+// uploads, memsets and result copies of a few hundred bytes another 35: 30 pairs
+// of 500 to 4000 descriptors 242 us before, 196 without the graph, 161 with one
+// upload, one memset, one copy back before the matches and no events unless the
+// caller asked for times.
+static constexpr slm_tune kOneLaunch{0, 0, 2, 0, 0, 0};
 
 extern "C" slm_status slm_match_batch(slm_ctx *c, slm_store *st, const slm_pair *pairs, uint32_t np, float ratio,
                                       int mutual, slm_precision prec, slm_pair *out, uint64_t cap, uint64_t *offsets,
                                       slm_stats *stats) {
     slm_plan *p = nullptr;
-    SLM_TRY(slm_plan_create(c, st, pairs, np, ratio, mutual, prec, nullptr, &p));
+    SLM_TRY(slm_plan_create(c, st, pairs, np, ratio, mutual, prec, &kOneLaunch, &p));
+    p->timed = stats != nullptr;
     slm_status s = slm_plan_launch(p);
     if (s == SLM_OK) s = slm_plan_results(p, out, cap, offsets, stats);
     std::string keep = g_last_error;
@@ -1637,8 +1665,9 @@ extern "C" slm_status slm_match_pairs(slm_ctx *c, slm_store *st, const uint64_t 
     SLM_TRY(slm_scheduled_pairs(views, nv, sch ? sch : &def, pairs.data(), total, &total));
     const uint32_t np = (uint32_t)total;
     slm_plan *p = nullptr;
-    SLM_TRY(slm_plan_create(c, st, pairs.data(), np, ratio, mutual, prec, nullptr, &p));
+    SLM_TRY(slm_plan_create(c, st, pairs.data(), np, ratio, mutual, prec, &kOneLaunch, &p));
     p->min_matches = min_matches;
+    p->timed = stats != nullptr;
     std::vector<uint64_t> off(np + 1, 0);
     s = slm_plan_launch(p);
     if (s == SLM_OK) s = slm_plan_results(p, out, cap, off.data(), stats);
@@ -1673,7 +1702,7 @@ namespace {
 // Run one pair through a workspace: load a and b into its two-view store,
 // plan and enqueue on its stream. The caller synchronises.
 slm_status single_pair_enqueue(slm_ctx *c, Workspace *w, const float *a, uint32_t na, const float *b, uint32_t nb,
-                               float ratio, int mutual, slm_precision prec, bool device_src) {
+                               float ratio, int mutual, slm_precision prec, bool device_src, bool timed) {
     slm_store *st = &w->store;
     const uint64_t rows = pad_rows(na) + pad_rows(nb);
     SLM_TRY(store_reserve(st, std::max<uint64_t>(rows, kTile)));
@@ -1691,6 +1720,7 @@ slm_status single_pair_enqueue(slm_ctx *c, Workspace *w, const float *a, uint32_
     slm_tune t{};
     t.use_graph = 2;  // one-off shapes: plain launches, no graph
     SLM_TRY(plan_init(&w->plan, c, st, &pr, 1, ratio, mutual, prec, &t, w->stream));
+    w->plan.timed = timed;
     return plan_launch_on(&w->plan, w->stream, false);
 }
 
@@ -1796,27 +1826,27 @@ extern "C" slm_status slm_ratio_match(slm_ctx *c, const float *a, uint32_t na, c
     SLM_TRY(ws_acquire(c, &w));
     WsGuard guard{c, w};
     if (prec == SLM_PREC_FP32) return single_pair_fp32(c, w, a, na, b, nb, ratio, mutual, out, cap, n_out, st);
-    SLM_TRY(single_pair_enqueue(c, w, a, na, b, nb, ratio, mutual, prec, false));
+    SLM_TRY(single_pair_enqueue(c, w, a, na, b, nb, ratio, mutual, prec, false, st != nullptr));
     slm_plan *p = &w->plan;
     // the control words, the offsets and every slot the pairs may fill come
     // back with the launch into pinned memory: one synchronisation per call
     const size_t pair_bytes = sizeof(slm_pair) * p->n_slots;
-    SLM_TRY(ws_host_block(w, 80 + pair_bytes));
+    constexpr size_t head = kCtlBytes + 16;
+    SLM_TRY(ws_host_block(w, head + pair_bytes));
     unsigned char *h = w->single_host;
-    SLM_CU(cudaMemcpyAsync(h, p->d_ctl.p, 64, cudaMemcpyDeviceToHost, w->stream));
-    SLM_CU(cudaMemcpyAsync(h + 64, p->d_offsets.p, 16, cudaMemcpyDeviceToHost, w->stream));
-    if (pair_bytes) SLM_CU(cudaMemcpyAsync(h + 80, p->d_dense.p, pair_bytes, cudaMemcpyDeviceToHost, w->stream));
+    SLM_CU(cudaMemcpyAsync(h, p->d_ctl.p, head, cudaMemcpyDeviceToHost, w->stream));
+    if (pair_bytes) SLM_CU(cudaMemcpyAsync(h + head, p->d_dense.p, pair_bytes, cudaMemcpyDeviceToHost, w->stream));
     SLM_CU(cudaStreamSynchronize(w->stream));
     uint32_t ctl[16];
     std::memcpy(ctl, h, sizeof(ctl));
     SLM_TRY(status_of_word(ctl[1]));
     uint64_t off[2];
-    std::memcpy(off, h + 64, sizeof(off));
+    std::memcpy(off, h + kCtlBytes, sizeof(off));
     const uint64_t total = off[1];
     *n_out = (uint32_t)total;
     SLM_TRY(fill_stats(p, st, total, ctl));
     if (total > cap) return fail(SLM_CAPACITY, "need " + std::to_string(total) + " pairs, have " + std::to_string(cap));
-    if (total) std::memcpy(out, h + 80, sizeof(slm_pair) * total);
+    if (total) std::memcpy(out, h + head, sizeof(slm_pair) * total);
     return SLM_OK;
 }
 
@@ -1848,10 +1878,10 @@ extern "C" slm_status slm_ratio_match_device(slm_ctx *c, const float *d_a, uint3
     SLM_CU(cudaEventCreateWithFlags(&e1, cudaEventDisableTiming));
     SLM_CU(cudaEventRecord(e0, c->stream));
     SLM_CU(cudaStreamWaitEvent(w->stream, e0, 0));
-    slm_status s = single_pair_enqueue(c, w, d_a, na, d_b, nb, ratio, mutual, prec, true);
+    slm_status s = single_pair_enqueue(c, w, d_a, na, d_b, nb, ratio, mutual, prec, true, false);
     if (s == SLM_OK) {
         slm_plan *p = &w->plan;
-        launch_copy_pairs(p->d_dense.as<uint2>(), p->d_offsets.as<uint64_t>() + 1, d_out, cap, d_count, w->stream);
+        launch_copy_pairs(p->d_dense.as<uint2>(), p->offsets() + 1, d_out, cap, d_count, w->stream);
         cudaError_t le = cudaGetLastError();
         if (le != cudaSuccess) s = fail(SLM_CUDA_ERROR, std::string("copy kernel: ") + cudaGetErrorString(le));
     }
@@ -2029,7 +2059,7 @@ slm_status serve_read_results(ServeSlot *s, std::vector<uint64_t> &off) {
     SLM_CU(cudaStreamSynchronize(p->stream));
     SLM_TRY(check_status_word(p));
     SLM_TRY(s->grow(s->pin_off, s->pin_off_cap, p->np + 1));
-    SLM_CU(cudaMemcpyAsync(s->pin_off, p->d_offsets.p, sizeof(uint64_t) * (p->np + 1), cudaMemcpyDeviceToHost,
+    SLM_CU(cudaMemcpyAsync(s->pin_off, p->offsets(), sizeof(uint64_t) * (p->np + 1), cudaMemcpyDeviceToHost,
                            p->stream));
     SLM_CU(cudaStreamSynchronize(p->stream));
     off.assign(s->pin_off, s->pin_off + p->np + 1);
@@ -2242,6 +2272,7 @@ void serve_loop(slm_server *srv) {
                 t.use_graph = 2;
                 ps = plan_init(&s->plan, srv->ctx, srv->store, pairs.data(), (uint32_t)pairs.size(), srv->opts.ratio,
                                srv->opts.mutual, srv->opts.prec, &t, s->stream);
+                s->plan.timed = false;
                 if (ps == SLM_OK) ps = plan_launch_on(&s->plan, s->stream, false);
             }
             if (ps == SLM_OK && cudaEventRecord(s->done, s->stream) != cudaSuccess)
@@ -2627,16 +2658,16 @@ void coal_finish(Coalescer *co, CoalReq *r, slm_status s, const std::string &err
 void coal_collect(Coalescer *co, CoalSlot *s) {
     slm_plan *p = &s->w.plan;
     const uint32_t *hw = static_cast<const uint32_t *>(s->host);
-    const uint64_t *off = reinterpret_cast<const uint64_t *>(hw + 2);
+    const uint64_t *off = reinterpret_cast<const uint64_t *>(static_cast<const unsigned char *>(s->host) + kCtlBytes);
     const slm_pair *dense = reinterpret_cast<const slm_pair *>(off + p->np + 1);
     slm_status rs = SLM_OK;
     if (cudaEventQuery(s->done) != cudaSuccess) {
         cudaGetLastError();
         rs = fail(SLM_CUDA_ERROR, "batch failed on the device");
-    } else if (hw[0] == DERR_TIMEOUT_BAR || hw[0] == DERR_TIMEOUT_MMA) {
-        rs = fail(SLM_TIMEOUT, "device wait gave up (code " + std::to_string(hw[0]) + ")");
-    } else if (hw[0]) {
-        rs = fail(SLM_INTERNAL, "device invariant failed (code " + std::to_string(hw[0]) + ")");
+    } else if (hw[1] == DERR_TIMEOUT_BAR || hw[1] == DERR_TIMEOUT_MMA) {
+        rs = fail(SLM_TIMEOUT, "device wait gave up (code " + std::to_string(hw[1]) + ")");
+    } else if (hw[1]) {
+        rs = fail(SLM_INTERNAL, "device invariant failed (code " + std::to_string(hw[1]) + ")");
     }
     const std::string err = rs == SLM_OK ? std::string() : g_last_error;
     for (size_t k = 0; k < s->reqs.size(); ++k) {
@@ -2697,6 +2728,7 @@ slm_status coal_issue(Coalescer *co, CoalSlot *s, std::vector<CoalReq *> &take) 
     }
     slm_tune t{};
     t.use_graph = 2;  // a new shape every batch: plain launches
+    w->plan.timed = false;
     SLM_TRY(plan_init(&w->plan, c, st, pr.data(), (uint32_t)pr.size(), take[0]->ratio, take[0]->mutual,
                       resolve_prec(SLM_PREC_AUTO, dist), &t, w->stream));
     SLM_TRY(plan_launch_on(&w->plan, w->stream, false));
@@ -2704,7 +2736,7 @@ slm_status coal_issue(Coalescer *co, CoalSlot *s, std::vector<CoalReq *> &take) 
     // the offsets and every slot the pairs may fill
     slm_plan *p = &w->plan;
     const size_t off_bytes = sizeof(uint64_t) * (p->np + 1), pair_bytes = sizeof(slm_pair) * p->n_slots;
-    const size_t need = 8 + off_bytes + pair_bytes;
+    const size_t head = kCtlBytes + off_bytes, need = head + pair_bytes;
     if (need > s->host_bytes) {
         if (s->host) {
             cudaStreamSynchronize(w->stream);  // a failed earlier batch may have left copies pending
@@ -2716,9 +2748,8 @@ slm_status coal_issue(Coalescer *co, CoalSlot *s, std::vector<CoalReq *> &take) 
         s->host_bytes = need + need / 4;
     }
     unsigned char *h = static_cast<unsigned char *>(s->host);
-    SLM_CU(cudaMemcpyAsync(h, p->d_ctl.as<uint32_t>() + 1, sizeof(uint32_t), cudaMemcpyDeviceToHost, w->stream));
-    SLM_CU(cudaMemcpyAsync(h + 8, p->d_offsets.p, off_bytes, cudaMemcpyDeviceToHost, w->stream));
-    if (pair_bytes) SLM_CU(cudaMemcpyAsync(h + 8 + off_bytes, p->d_dense.p, pair_bytes, cudaMemcpyDeviceToHost, w->stream));
+    SLM_CU(cudaMemcpyAsync(h, p->d_ctl.p, head, cudaMemcpyDeviceToHost, w->stream));
+    if (pair_bytes) SLM_CU(cudaMemcpyAsync(h + head, p->d_dense.p, pair_bytes, cudaMemcpyDeviceToHost, w->stream));
     SLM_CU(cudaEventRecord(s->done, w->stream));
     return SLM_OK;
 }
