@@ -8,13 +8,16 @@
 
 #include <cstdint>
 
+#include "ptx.cuh"
 #include "slm.h"
 
 namespace slm {
 
 // Single CTA: offsets[k] = sum of counts[0..k), offsets[np] = total.
-__global__ void __launch_bounds__(1024) scan_counts_kernel(const uint32_t *__restrict__ counts, uint32_t np,
-                                                           uint64_t *__restrict__ offsets) {
+__global__ void __launch_bounds__(1024) scan_counts_kernel(const uint32_t *counts, uint32_t np,
+                                                           uint64_t *offsets) {
+    grid_wait();
+    grid_go();
     __shared__ uint64_t warp_sum[32];
     __shared__ uint64_t carry_sh;
     const int tid = threadIdx.x, lane = tid & 31, wid = tid >> 5;
@@ -52,11 +55,12 @@ __global__ void __launch_bounds__(1024) scan_counts_kernel(const uint32_t *__res
 }
 
 // One CTA per pair: dense[offsets[k] + t] = slots[slot_off[k] + t].
-__global__ void __launch_bounds__(256) gather_kernel(const uint2 *__restrict__ slots,
-                                                     const uint64_t *__restrict__ slot_off,
-                                                     const uint32_t *__restrict__ counts,
-                                                     const uint64_t *__restrict__ offsets, uint2 *__restrict__ dense,
+__global__ void __launch_bounds__(256) gather_kernel(const uint2 *slots,
+                                                     const uint64_t *slot_off,
+                                                     const uint32_t *counts,
+                                                     const uint64_t *offsets, uint2 *dense,
                                                      uint64_t cap) {
+    grid_wait();
     const uint32_t k = blockIdx.x;
     const uint32_t n = counts[k];
     const uint64_t src = slot_off[k], dst = offsets[k];
@@ -66,8 +70,9 @@ __global__ void __launch_bounds__(256) gather_kernel(const uint2 *__restrict__ s
 
 // Single pair into a caller buffer: copies min(total, cap) pairs and writes
 // the full count.
-__global__ void copy_pairs_kernel(const uint2 *__restrict__ src, const uint64_t *__restrict__ total,
-                                  slm_pair *__restrict__ dst, uint32_t cap, uint32_t *__restrict__ d_count) {
+__global__ void copy_pairs_kernel(const uint2 *src, const uint64_t *total,
+                                  slm_pair *dst, uint32_t cap, uint32_t *d_count) {
+    grid_wait();
     const uint64_t n = *total;
     for (uint64_t t = blockIdx.x * (uint64_t)blockDim.x + threadIdx.x; t < n && t < cap;
          t += (uint64_t)gridDim.x * blockDim.x) {
@@ -81,7 +86,9 @@ __global__ void copy_pairs_kernel(const uint2 *__restrict__ src, const uint64_t 
 // match_pairs' filter (pipeline.rs:494-496: pairs with fewer than min_matches
 // matches are dropped before RANSAC): such pairs report no matches, so their
 // lists are neither gathered nor copied to the host.
-__global__ void filter_counts_kernel(uint32_t *__restrict__ counts, uint32_t np, uint32_t min_matches) {
+__global__ void filter_counts_kernel(uint32_t *counts, uint32_t np, uint32_t min_matches) {
+    grid_wait();
+    grid_go();
     for (uint32_t k = blockIdx.x * blockDim.x + threadIdx.x; k < np; k += gridDim.x * blockDim.x)
         if (counts[k] < min_matches) counts[k] = 0;
 }
@@ -170,21 +177,21 @@ void launch_fill_u32(uint32_t *p, uint64_t n, uint32_t v, cudaStream_t s) {
 }
 
 void launch_filter_counts(uint32_t *counts, uint32_t np, uint32_t min_matches, cudaStream_t s) {
-    if (np) filter_counts_kernel<<<(np + 255) / 256 < 1024 ? (np + 255) / 256 : 1024, 256, 0, s>>>(counts, np, min_matches);
+    if (np) launch_next(filter_counts_kernel, (np + 255) / 256 < 1024 ? (np + 255) / 256 : 1024, 256, 0, s, counts, np, min_matches);
 }
 
 void launch_scan_counts(const uint32_t *counts, uint32_t np, uint64_t *offsets, cudaStream_t s) {
-    scan_counts_kernel<<<1, 1024, 0, s>>>(counts, np, offsets);
+    launch_next(scan_counts_kernel, 1, 1024, 0, s, counts, np, offsets);
 }
 
 void launch_gather(const uint2 *slots, const uint64_t *slot_off, const uint32_t *counts, const uint64_t *offsets,
                    uint32_t np, uint2 *dense, uint64_t cap, cudaStream_t s) {
-    if (np) gather_kernel<<<np, 256, 0, s>>>(slots, slot_off, counts, offsets, dense, cap);
+    if (np) launch_next(gather_kernel, np, 256, 0, s, slots, slot_off, counts, offsets, dense, cap);
 }
 
 void launch_copy_pairs(const uint2 *src, const uint64_t *total, slm_pair *dst, uint32_t cap, uint32_t *d_count,
                        cudaStream_t s) {
-    copy_pairs_kernel<<<64, 256, 0, s>>>(src, total, dst, cap, d_count);
+    launch_next(copy_pairs_kernel, 64, 256, 0, s, src, total, dst, cap, d_count);
 }
 
 }  // namespace slm

@@ -59,10 +59,12 @@ __global__ void __launch_bounds__(256) pack_fp32_tiles_kernel(const uint4 *__res
 // (the only readers of FP32 tiles on that path), packed on the device once the
 // routed pairs are known; with nothing routed every CTA returns at once. A
 // view shared by several routed pairs is packed once per pair (same values).
-__global__ void __launch_bounds__(256) pack_routed_kernel(const PairMeta *__restrict__ pairs,
-                                                          const uint32_t *__restrict__ xlist,
-                                                          const uint32_t *__restrict__ count,
-                                                          const float *__restrict__ raw, float *__restrict__ tiled) {
+__global__ void __launch_bounds__(256) pack_routed_kernel(const PairMeta *pairs,
+                                                          const uint32_t *xlist,
+                                                          const uint32_t *count,
+                                                          const float *raw, float *tiled) {
+    grid_wait();
+    grid_go();
     __shared__ float sm[32][kDesc + 1];
     const uint32_t n = *count;
     for (uint32_t k = 0; k < n; ++k) {
@@ -77,7 +79,7 @@ __global__ void __launch_bounds__(256) pack_routed_kernel(const PairMeta *__rest
 
 void launch_pack_routed(const PairMeta *pairs, const uint32_t *xlist, const uint32_t *count, const float *raw,
                         float *tiled, int grid, cudaStream_t s) {
-    pack_routed_kernel<<<grid, 256, 0, s>>>(pairs, xlist, count, raw, tiled);
+    launch_next(pack_routed_kernel, grid, 256, 0, s, pairs, xlist, count, raw, tiled);
 }
 
 void launch_pack_fp32_tiles(const uint4 *tab, uint32_t ntiles, const float *raw, float *tiled, cudaStream_t s) {
@@ -238,6 +240,7 @@ SLM_DEV int col_of(int tx, int c) { return c < 4 ? tx * 4 + c : 64 + tx * 4 + (c
 
 template <bool X2>
 __global__ void __launch_bounds__(kThreads, 1) exact_kernel(ExactArgs g) {
+    grid_wait();
     extern __shared__ __align__(1024) unsigned char smem_raw[];
     ExactSmem &S = *reinterpret_cast<ExactSmem *>(smem_raw);
     const int tid = threadIdx.x;
@@ -403,10 +406,7 @@ cudaError_t init_exact_kernels() {
 
 void launch_exact(const ExactArgs &a, int grid, cudaStream_t s) {
     const size_t smem = sizeof(ExactSmem);
-    if (a.x2)
-        exact_kernel<true><<<grid, kThreads, smem, s>>>(a);
-    else
-        exact_kernel<false><<<grid, kThreads, smem, s>>>(a);
+    launch_next(a.x2 ? exact_kernel<true> : exact_kernel<false>, grid, kThreads, smem, s, a);
 }
 
 // -------------------------------------------------------------- finalize
@@ -420,6 +420,7 @@ constexpr int kFinThreadsMax = 1024;
 
 template <int kThreads>
 __global__ void __launch_bounds__(kThreads) finalize_kernel(FinalizeArgs g) {
+    grid_wait();
     __shared__ uint32_t warp_tot[kThreads / 32];
     constexpr uint32_t nthr = kThreads;
     constexpr int nwarps = kThreads / 32;
@@ -478,9 +479,9 @@ __global__ void __launch_bounds__(kThreads) finalize_kernel(FinalizeArgs g) {
 void launch_finalize(const FinalizeArgs &a, cudaStream_t s) {
     if (!a.npairs) return;
     if (a.npairs <= kFewPairs)
-        finalize_kernel<kFinThreadsMax><<<a.npairs, kFinThreadsMax, 0, s>>>(a);
+        launch_next(finalize_kernel<kFinThreadsMax>, a.npairs, kFinThreadsMax, 0, s, a);
     else
-        finalize_kernel<256><<<a.npairs, 256, 0, s>>>(a);
+        launch_next(finalize_kernel<256>, a.npairs, 256, 0, s, a);
 }
 
 // Self-test of the bounded waits: thread 0 waits on an mbarrier that expects

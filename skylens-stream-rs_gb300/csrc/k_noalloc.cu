@@ -31,6 +31,7 @@
 
 #include "pack.cuh"
 #include "slm.h"
+#include "ptx.cuh"
 #include "slm_internal.h"
 
 namespace slm {
@@ -123,6 +124,7 @@ __global__ void __launch_bounds__(256) single_prep_kernel(unsigned char *scratch
 // the full count, or 0xffffffff if a bounded device wait gave up.
 __global__ void single_copy_kernel(const unsigned char *scratch, SingleLayout L, slm_pair *out, uint32_t cap,
                                    uint32_t *d_count) {
+    grid_wait();
     const uint2 *slots = reinterpret_cast<const uint2 *>(scratch + L.slots);
     const uint32_t n = *reinterpret_cast<const uint32_t *>(scratch + L.counts);
     const uint32_t err = reinterpret_cast<const uint32_t *>(scratch + L.ctl)[1];
@@ -239,7 +241,7 @@ cudaError_t single_exact_enqueue(unsigned char *sc, const SingleLayout &L, const
         f.slots = reinterpret_cast<uint2 *>(sc + L.slots);
         f.counts = reinterpret_cast<uint32_t *>(sc + L.counts);
         launch_finalize(f, s);
-        single_copy_kernel<<<16, 256, 0, s>>>(sc, L, d_out, cap, d_count);
+        launch_next(single_copy_kernel, 16, 256, 0, s, sc, L, d_out, cap, d_count);
     }
     return cudaGetLastError();
 }

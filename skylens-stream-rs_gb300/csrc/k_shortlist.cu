@@ -261,6 +261,7 @@ static_assert(kSlMaxRegs == 96, "register budget of the 18-warp pass kernel");
 
 template <int PASS, bool DUMP>
 __global__ void __maxnreg__(kSlMaxRegs) sl_pass_kernel(SlArgs g) {
+    grid_wait();
     extern __shared__ uint8_t sl_smem_raw[];
     const uint32_t pad = (1024u - (smem_u32(sl_smem_raw) & 1023u)) & 1023u;
     SlSmem &S = *reinterpret_cast<SlSmem *>(sl_smem_raw + pad);
@@ -642,6 +643,8 @@ __global__ void __maxnreg__(kSlMaxRegs) sl_pass_kernel(SlArgs g) {
 // statistics. A pair with non-finite or huge inputs cannot be certified and is
 // routed to the exact kernel.
 __global__ void __launch_bounds__(256) sl_eps_kernel(SlArgs g) {
+    grid_wait();
+    grid_go();
     const uint32_t p = blockIdx.x * blockDim.x + threadIdx.x;
     if (p >= g.npairs) return;
     const PairMeta pm = g.pairs[p];
@@ -659,6 +662,8 @@ __global__ void __launch_bounds__(256) sl_eps_kernel(SlArgs g) {
 // rescued pair, the BF16 bound and its counters back to 0 (tier 0's mid wrote
 // them).
 __global__ void __launch_bounds__(256) sl_rescue_prep_kernel(SlArgs g) {
+    grid_wait();
+    grid_go();
     const uint32_t p = blockIdx.x * blockDim.x + threadIdx.x;
     if (p >= g.npairs) return;
     const SlPair sp = g.spairs[p];
@@ -684,6 +689,8 @@ __global__ void __launch_bounds__(256) sl_rescue_prep_kernel(SlArgs g) {
 // the bound sets the register budget the compiler schedules for.
 template <int kThreads>
 __global__ void __launch_bounds__(kThreads) sl_mid_kernel(SlArgs g) {
+    grid_wait();
+    grid_go();
     __shared__ uint32_t wide_sh, open_sh, last_sh;
     const uint32_t p = blockIdx.x, blk = blockIdx.y;
     const PairMeta pm = g.pairs[p];
@@ -787,6 +794,8 @@ __global__ void __launch_bounds__(kThreads) sl_mid_kernel(SlArgs g) {
 // that could certify nothing: 0.45 ms of a 32768 x 32768 pair's 0.94 (the
 // sample takes 0.015).
 __global__ void __launch_bounds__(256) sl_sample_kernel(SlArgs g) {
+    grid_wait();
+    grid_go();
     const SlSample sm = g.samples[blockIdx.x];
     const PairMeta pm = g.pairs[sm.pair];
     const SlPair sp = g.spairs[sm.pair];
@@ -830,6 +839,8 @@ SLM_DEV uint32_t mutual_from_counts(const SlArgs &g, uint32_t p, const SlPair &s
 // rescoring of long shortlists or scans per row would cost more).
 template <int kThreads>
 __global__ void __launch_bounds__(kThreads, 1) sl_finalize_kernel(SlArgs g) {
+    grid_wait();
+    grid_go();
     const uint32_t p = blockIdx.x, blk = blockIdx.y;
     const PairMeta pm = g.pairs[p];
     const SlPair sp = g.spairs[p];
@@ -917,6 +928,8 @@ __global__ void __launch_bounds__(kThreads, 1) sl_finalize_kernel(SlArgs g) {
 // the reference's row rule (matching.rs:182-187, 204-206), then the mutual
 // check from the column window counts.
 __global__ void __launch_bounds__(256) sl_rescore_kernel(SlArgs g) {
+    grid_wait();
+    grid_go();
     const uint32_t lane = threadIdx.x & 31, grp = lane >> 3;
     const uint32_t gw = (blockIdx.x * blockDim.x + threadIdx.x) >> 5;
     const uint32_t nw = (gridDim.x * blockDim.x) >> 5;
@@ -1028,6 +1041,8 @@ SLM_DEV void block_argmin(float &d, uint32_t &idx, float *sd, uint32_t *si) {
 // One CTA per entry of the scan queue: exact full scans, 32 distances at a
 // time (8 lanes each).
 __global__ void __launch_bounds__(256) sl_scan_kernel(SlArgs g) {
+    grid_wait();
+    grid_go();
     __shared__ float sd[8], s2[8];
     __shared__ uint32_t si[8];
     const uint32_t lane = threadIdx.x & 31, grp = threadIdx.x >> 3;  // 32 groups of 8 lanes
@@ -1157,6 +1172,8 @@ SLM_DEV uint32_t block_scan_1024(uint32_t v, uint32_t *sh, uint32_t &total) {
 // Writes each routed pair's first item and chunk count, the list of routed
 // pairs and the counters.
 __global__ void __launch_bounds__(1024) sl_route_plan_kernel(SlArgs g) {
+    grid_wait();
+    grid_go();
     __shared__ uint32_t sh[32];
     __shared__ uint32_t carry_items, carry_list;
     if (g.ctl[kCtlRouteMarks] == 0) return;  // nothing routed: the counters stay 0
@@ -1221,6 +1238,8 @@ __global__ void __launch_bounds__(1024) sl_route_plan_kernel(SlArgs g) {
 // Writes the exact work items of the routed pairs and resets their column
 // minima keys (one CTA per routed pair at a time).
 __global__ void __launch_bounds__(256) sl_route_apply_kernel(SlArgs g) {
+    grid_wait();
+    grid_go();
     const uint32_t n = g.ctl[kCtlRoutedPairs];
     for (uint32_t k = blockIdx.x; k < n; k += gridDim.x) {
         const uint32_t p = g.xlist[k];
@@ -1247,6 +1266,8 @@ __global__ void __launch_bounds__(256) sl_route_apply_kernel(SlArgs g) {
 // After exact_kernel: the routed pairs' row decisions, as finalize_kernel
 // makes them (matching.rs:204-214), into rowdec.
 __global__ void __launch_bounds__(256) sl_route_finalize_kernel(SlArgs g) {
+    grid_wait();
+    grid_go();
     const uint32_t n = g.ctl[kCtlRoutedPairs];
     const float kInf = __int_as_float(0x7f800000);
     for (uint32_t k = blockIdx.x; k < n; k += gridDim.x) {
@@ -1274,65 +1295,84 @@ __global__ void __launch_bounds__(256) sl_route_finalize_kernel(SlArgs g) {
 
 // Matches of a pair's row block in ascending i, at the block's slot range
 // (CTA per pair and row block); the block's count goes to blkcnt and the
-// pair's total to counts.
+// pair's total to counts. The block's rows are read before any of them is
+// placed: 256 at a time, placed before the next are read, took 9.2 us for one
+// 8192-row pair, now 4.8.
 __global__ void __launch_bounds__(256) sl_compact_kernel(SlArgs g) {
-    __shared__ uint32_t warp_tot[8];
+    constexpr uint32_t kRuns = kSlRowBlock / 256;
+    __shared__ uint32_t run_tot[kRuns * 8];  // by run, then warp: ascending rows
+    grid_wait();
+    grid_go();
     const uint32_t p = blockIdx.x, blk = blockIdx.y;
     const PairMeta pm = g.pairs[p];
     const SlPair sp = g.spairs[p];
     const uint32_t r0 = blk * kSlRowBlock;
     if (r0 >= pm.na) return;  // block-uniform
     const uint32_t r1 = min(r0 + kSlRowBlock, pm.na);
-    const int tid = threadIdx.x, lane = tid & 31, wid = tid >> 5;
-    uint32_t base = 0;
-    for (uint32_t row0 = r0; row0 < r1; row0 += 256) {
-        const uint32_t i = row0 + tid;
-        uint32_t dec = kDecNone;
-        if (i < r1) dec = g.rowdec[sp.rbase + i];
-        if (dec == kDecPending) {
+    const uint32_t tid = threadIdx.x, lane = tid & 31, wid = tid >> 5;
+    uint32_t dec[kRuns], pre[kRuns];
+#pragma unroll
+    for (uint32_t k = 0; k < kRuns; ++k) {
+        const uint32_t i = r0 + 256 * k + tid;
+        dec[k] = i < r1 ? g.rowdec[sp.rbase + i] : kDecNone;
+    }
+#pragma unroll
+    for (uint32_t k = 0; k < kRuns; ++k) {
+        if (dec[k] == kDecPending) {
             atomicCAS(g.ctl + 1, 0u, (uint32_t)DERR_BAD_ITEM);
-            dec = kDecNone;
+            dec[k] = kDecNone;
         }
-        const uint32_t flag = dec != kDecNone;
-        const uint32_t ballot = __ballot_sync(0xffffffffu, flag);
-        const uint32_t wpre = __popc(ballot & ((1u << lane) - 1u));
-        if (lane == 0) warp_tot[wid] = __popc(ballot);
-        __syncthreads();
-        uint32_t off = 0, tot = 0;
-        for (int w = 0; w < 8; ++w) {
-            off += (w < wid) ? warp_tot[w] : 0;
-            tot += warp_tot[w];
+        const uint32_t ballot = __ballot_sync(0xffffffffu, dec[k] != kDecNone);
+        pre[k] = __popc(ballot & ((1u << lane) - 1u));
+        if (lane == 0) run_tot[8 * k + wid] = __popc(ballot);
+    }
+    __syncthreads();
+    static_assert(kRuns * 8 == 64, "two entries a lane");
+    if (wid == 0) {  // exclusive scan of the 64 runs
+        const uint32_t t0 = run_tot[2 * lane], t1 = run_tot[2 * lane + 1];
+        uint32_t x = t0 + t1;
+#pragma unroll
+        for (int o = 1; o < 32; o <<= 1) {
+            const uint32_t y = __shfl_up_sync(0xffffffffu, x, o);
+            if (lane >= o) x += y;
         }
-        if (flag) g.slots[pm.slot_off + r0 + base + off + wpre] = make_uint2(i, dec);
-        base += tot;
-        __syncthreads();
+        run_tot[2 * lane] = x - t0 - t1;
+        run_tot[2 * lane + 1] = x - t1;
+        if (lane == 31) {
+            g.blkcnt[sp.blk + blk] = x;
+            if (x) atomicAdd(&g.counts[p], x);
+        }
     }
-    if (tid == 0) {
-        g.blkcnt[sp.blk + blk] = base;
-        if (base) atomicAdd(&g.counts[p], base);
-    }
+    __syncthreads();
+#pragma unroll
+    for (uint32_t k = 0; k < kRuns; ++k)
+        if (dec[k] != kDecNone)
+            g.slots[pm.slot_off + r0 + run_tot[8 * k + wid] + pre[k]] = make_uint2(r0 + 256 * k + tid, dec[k]);
 }
 
-// One CTA per pair: its row blocks' matches, in order, to the dense list.
-__global__ void __launch_bounds__(256) sl_gather_kernel(SlArgs g, const uint64_t *__restrict__ slot_off,
-                                                        const uint64_t *__restrict__ offsets, uint2 *__restrict__ dense,
+// A pair's row block's matches, behind those of the blocks before it, to the
+// dense list (CTA per pair and row block: one CTA per pair took 12 us for one
+// 8192-row pair, now 7).
+__global__ void __launch_bounds__(256) sl_gather_kernel(SlArgs g, const uint64_t *slot_off,
+                                                        const uint64_t *offsets, uint2 *dense,
                                                         uint64_t cap) {
-    const uint32_t p = blockIdx.x;
+    grid_wait();
+    const uint32_t p = blockIdx.x, b = blockIdx.y;
     if (g.counts[p] == 0) return;  // no matches, or filtered out
-    const uint32_t na = g.pairs[p].na, blk = g.spairs[p].blk;
+    if (b * kSlRowBlock >= g.pairs[p].na) return;
+    const uint32_t blk = g.spairs[p].blk;
     uint64_t dst = offsets[p];
-    for (uint32_t b = 0; b * kSlRowBlock < na; ++b) {
-        const uint32_t n = g.blkcnt[blk + b];
-        const uint64_t src = slot_off[p] + (uint64_t)b * kSlRowBlock;
-        for (uint32_t t = threadIdx.x; t < n; t += blockDim.x)
-            if (dst + t < cap) dense[dst + t] = g.slots[src + t];
-        dst += n;
-    }
+    for (uint32_t q = 0; q < b; ++q) dst += g.blkcnt[blk + q];
+    const uint32_t n = g.blkcnt[blk + b];
+    const uint64_t src = slot_off[p] + (uint64_t)b * kSlRowBlock;
+#pragma unroll 4
+    for (uint32_t t = threadIdx.x; t < n; t += 256)
+        if (dst + t < cap) dense[dst + t] = g.slots[src + t];
 }
 
 void launch_gather_blocks(const SlArgs &a, const uint64_t *slot_off, const uint64_t *offsets, uint2 *dense,
                           uint64_t cap, cudaStream_t s) {
-    if (a.npairs) sl_gather_kernel<<<a.npairs, 256, 0, s>>>(a, slot_off, offsets, dense, cap);
+    if (a.npairs) launch_next(sl_gather_kernel, dim3(a.npairs, a.row_blocks), 256, 0, s, a, slot_off, offsets, dense, cap);
 }
 
 // ---------------------------------------------------------------- launch
@@ -1347,7 +1387,7 @@ cudaError_t init_shortlist_kernels() {
 
 int launch_shortlist_eps(const SlArgs &a, cudaStream_t s) {
     if (!a.npairs) return 0;
-    sl_eps_kernel<<<(a.npairs + 255) / 256, 256, 0, s>>>(a);
+    launch_next(sl_eps_kernel, (a.npairs + 255) / 256, 256, 0, s, a);
     return 1;
 }
 
@@ -1355,10 +1395,9 @@ int launch_shortlist_pass(const SlArgs &a, int pass, int sms, cudaStream_t s) {
     const int grid = (int)(a.n_items < (uint32_t)sms ? a.n_items : (uint32_t)sms);
     if (!grid) return 0;
     if (pass == 1)
-        a.dump ? sl_pass_kernel<1, true><<<grid, kSlThreads, kSlSmemBytes, s>>>(a)
-               : sl_pass_kernel<1, false><<<grid, kSlThreads, kSlSmemBytes, s>>>(a);
+        launch_next(a.dump ? sl_pass_kernel<1, true> : sl_pass_kernel<1, false>, grid, kSlThreads, kSlSmemBytes, s, a);
     else
-        sl_pass_kernel<2, false><<<grid, kSlThreads, kSlSmemBytes, s>>>(a);
+        launch_next(sl_pass_kernel<2, false>, grid, kSlThreads, kSlSmemBytes, s, a);
     return 1;
 }
 
@@ -1368,16 +1407,16 @@ int launch_shortlist_sample(const SlArgs &a, int sms, cudaStream_t s) {
     b.items = a.items + a.n_items;  // the sample's items follow the pass's
     b.n_items = a.n_sample_items;
     const int n = launch_shortlist_pass(b, 1, sms, s);
-    sl_sample_kernel<<<a.n_samples, 256, 0, s>>>(a);
+    launch_next(sl_sample_kernel, a.n_samples, 256, 0, s, a);
     return n + 1;
 }
 
 int launch_shortlist_mid(const SlArgs &a, cudaStream_t s) {
     if (!a.npairs) return 0;
     if (a.npairs <= kFewPairs)
-        sl_mid_kernel<1024><<<dim3(a.npairs, a.row_blocks), 1024, 0, s>>>(a);
+        launch_next(sl_mid_kernel<1024>, dim3(a.npairs, a.row_blocks), 1024, 0, s, a);
     else
-        sl_mid_kernel<256><<<dim3(a.npairs, a.row_blocks), 256, 0, s>>>(a);
+        launch_next(sl_mid_kernel<256>, dim3(a.npairs, a.row_blocks), 256, 0, s, a);
     return 1;
 }
 
@@ -1385,15 +1424,15 @@ int launch_shortlist_finalize(const SlArgs &a, cudaStream_t s) {
     if (!a.npairs) return 0;
     const dim3 per_block(a.npairs, a.row_blocks);  // CTA per pair and row block
     if (a.npairs <= kFewPairs)
-        sl_finalize_kernel<1024><<<per_block, 1024, 0, s>>>(a);
+        launch_next(sl_finalize_kernel<1024>, per_block, 1024, 0, s, a);
     else
-        sl_finalize_kernel<256><<<per_block, 256, 0, s>>>(a);
+        launch_next(sl_finalize_kernel<256>, per_block, 256, 0, s, a);
     return 1;
 }
 
 int launch_shortlist_rescue_prep(const SlArgs &a, cudaStream_t s) {
     if (!a.npairs) return 0;
-    sl_rescue_prep_kernel<<<(a.npairs + 255) / 256, 256, 0, s>>>(a);
+    launch_next(sl_rescue_prep_kernel, (a.npairs + 255) / 256, 256, 0, s, a);
     return 1;
 }
 
@@ -1402,8 +1441,8 @@ int launch_shortlist_tail(const SlArgs &a, int sms, cudaStream_t s) {
     const unsigned rgrid = (unsigned)(a.npairs < (uint32_t)(4 * sms) ? a.npairs : (uint32_t)(4 * sms));
     const dim3 per_block(a.npairs, a.row_blocks);  // CTA per pair and row block
     // routed pairs: plan, exact kernel over all their rows and columns, decisions
-    sl_route_plan_kernel<<<1, 1024, 0, s>>>(a);
-    sl_route_apply_kernel<<<rgrid, 256, 0, s>>>(a);
+    launch_next(sl_route_plan_kernel, 1, 1024, 0, s, a);
+    launch_next(sl_route_apply_kernel, rgrid, 256, 0, s, a);
     ExactArgs x{};
     x.tiled = a.tiled;
     x.items = a.xitems;
@@ -1422,10 +1461,10 @@ int launch_shortlist_tail(const SlArgs &a, int sms, cudaStream_t s) {
     if (!a.fp8)
         launch_pack_routed(a.pairs, a.xlist, a.ctl + kCtlRoutedPairs, a.raw, const_cast<float *>(a.tiled), 2 * sms, s);
     launch_exact(x, sms, s);
-    sl_route_finalize_kernel<<<dim3(rgrid, a.row_blocks), 256, 0, s>>>(a);
-    if (a.fp8) sl_rescore_kernel<<<5 * sms, 256, 0, s>>>(a);  // 40 warps per SM: latency-bound gathers
-    sl_scan_kernel<<<2 * sms, 256, 0, s>>>(a);
-    sl_compact_kernel<<<per_block, 256, 0, s>>>(a);
+    launch_next(sl_route_finalize_kernel, dim3(rgrid, a.row_blocks), 256, 0, s, a);
+    if (a.fp8) launch_next(sl_rescore_kernel, 5 * sms, 256, 0, s, a);  // 40 warps per SM: latency-bound gathers
+    launch_next(sl_scan_kernel, 2 * sms, 256, 0, s, a);
+    launch_next(sl_compact_kernel, per_block, 256, 0, s, a);
     return 7;
 }
 

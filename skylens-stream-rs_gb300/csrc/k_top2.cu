@@ -152,6 +152,7 @@ SLM_DEV bool top_item_off(const SlArgs &g, const TopItem &it) {
 
 template <bool DUMP>
 __global__ void __maxnreg__(96) sl_top2_kernel(SlArgs g) {
+    grid_wait();
     extern __shared__ uint8_t top_smem_raw[];
     const uint32_t pad = (1024u - (smem_u32(top_smem_raw) & 1023u)) & 1023u;
     TopSmem &S = *reinterpret_cast<TopSmem *>(top_smem_raw + pad);
@@ -456,6 +457,8 @@ SLM_DEV bool settle_with_d1(const SlArgs &g, const SlPair &sp, uint32_t p, uint3
 constexpr uint32_t kDecideThreads = 256;
 template <int R>
 __global__ void __launch_bounds__(kDecideThreads) sl_decide_kernel(SlArgs g) {
+    grid_wait();
+    grid_go();
     const uint32_t p = blockIdx.x, row0 = blockIdx.y * (kDecideThreads * R);
     const PairMeta pm = g.pairs[p];
     if (row0 >= pm.na) return;  // block-uniform, as below
@@ -535,6 +538,8 @@ __global__ void __launch_bounds__(kDecideThreads) sl_decide_kernel(SlArgs g) {
 
 // The open rows of a large batch, two lanes each.
 __global__ void __launch_bounds__(256) sl_nearest_kernel(SlArgs g) {
+    grid_wait();
+    grid_go();
     const uint32_t lane = threadIdx.x & 31, n = g.ctl[kCtlOpen];
     const uint32_t gw = (blockIdx.x * blockDim.x + threadIdx.x) >> 5, nw = (gridDim.x * blockDim.x) >> 5;
     uint32_t settled = 0;
@@ -588,6 +593,8 @@ SLM_DEV uint4 op_chunk(const SlArgs &g, uint32_t r, uint32_t c) {
 // A row with more columns in the window than g.cand_cap is scanned exactly
 // instead; a pair with more than 1/8 such rows goes to the exact kernel.
 __global__ void __launch_bounds__(256) sl_resolve_kernel(SlArgs g) {
+    grid_wait();
+    grid_go();
     constexpr uint32_t kCap = 2 * kSlHalfRecsMax;
     __shared__ uint32_t cand_s[kResolveRows][kCap];
     __shared__ float cval_s[kResolveRows][kCap];
@@ -752,10 +759,7 @@ cudaError_t init_top2_kernels() {
 
 int launch_top2_pass(const SlArgs &a, cudaStream_t s) {
     if (!a.tgrid) return 0;
-    if (a.dump)
-        sl_top2_kernel<true><<<a.tgrid, kTopThreads, kTopSmemBytes, s>>>(a);
-    else
-        sl_top2_kernel<false><<<a.tgrid, kTopThreads, kTopSmemBytes, s>>>(a);
+    launch_next(a.dump ? sl_top2_kernel<true> : sl_top2_kernel<false>, a.tgrid, kTopThreads, kTopSmemBytes, s, a);
     return 1;
 }
 
@@ -763,13 +767,13 @@ int launch_top2_decide(const SlArgs &a, int sms, cudaStream_t s) {
     if (!a.npairs || !a.max_na) return 0;
     // four rows a thread once that still gives every SM its eight CTAs
     if (a.n_rows < 8ull * sms * 4 * kDecideThreads) {
-        sl_decide_kernel<1><<<dim3(a.npairs, (a.max_na + kDecideThreads - 1) / kDecideThreads), kDecideThreads, 0,
-                              s>>>(a);
+        launch_next(sl_decide_kernel<1>, dim3(a.npairs, (a.max_na + kDecideThreads - 1) / kDecideThreads), kDecideThreads,
+                    0, s, a);
         return 1;
     }
-    sl_decide_kernel<4><<<dim3(a.npairs, (a.max_na + 4 * kDecideThreads - 1) / (4 * kDecideThreads)), kDecideThreads, 0,
-                          s>>>(a);
-    sl_nearest_kernel<<<2 * sms, 256, 0, s>>>(a);
+    launch_next(sl_decide_kernel<4>, dim3(a.npairs, (a.max_na + 4 * kDecideThreads - 1) / (4 * kDecideThreads)),
+                kDecideThreads, 0, s, a);
+    launch_next(sl_nearest_kernel, 2 * sms, 256, 0, s, a);
     return 2;
 }
 
@@ -785,14 +789,16 @@ int launch_top2_resolve(const SlArgs &a, int sms, cudaStream_t s) {
     uint32_t c = 1;
     while (!many && c < 8 && 2 * c * est <= 2ull * sms) c *= 2;
     cudaLaunchConfig_t cfg{};
-    cudaLaunchAttribute at{};
-    at.id = cudaLaunchAttributeClusterDimension;
-    at.val.clusterDim = {c, 1, 1};
+    cudaLaunchAttribute at[2]{};
+    at[0].id = cudaLaunchAttributeClusterDimension;
+    at[0].val.clusterDim = {c, 1, 1};
+    at[1].id = cudaLaunchAttributeProgrammaticStreamSerialization;
+    at[1].val.programmaticStreamSerializationAllowed = 1;
     cfg.gridDim = dim3((unsigned)((many ? 4 : 2) * sms) / c * c);
     cfg.blockDim = dim3(many ? 128 : 256);
     cfg.stream = s;
-    cfg.attrs = &at;
-    cfg.numAttrs = 1;
+    cfg.attrs = at;
+    cfg.numAttrs = 2;
     cudaLaunchKernelEx(&cfg, sl_resolve_kernel, a);
     return 1;
 }
