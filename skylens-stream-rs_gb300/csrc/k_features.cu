@@ -24,6 +24,7 @@
 #include <cstdint>
 
 #include "fmath_cr.h"
+#include "ptx.cuh"
 #include "slm_internal.h"
 
 namespace slm {
@@ -68,7 +69,7 @@ __global__ void __launch_bounds__(kBlurX) blur_rows_kernel(const float *__restri
                                                            int w, int h, uint64_t img_stride_src,
                                                            uint64_t img_stride_dst, BlurTaps t) {
     __shared__ float row[kBlurX + 2 * kMaxBlurR];
-    const int y = blockIdx.y, b = blockIdx.z;
+    const int y = grid_wait(blockIdx.y), b = blockIdx.z;
     const int x0 = blockIdx.x * kBlurX;
     const float *s = src + b * img_stride_src + (uint64_t)y * w;
     const int n = kBlurX + 2 * t.r;
@@ -89,7 +90,7 @@ __global__ void __launch_bounds__(kBlurX) blur_cols_kernel(const float *__restri
                                                            int w, int h, uint64_t img_stride_tmp,
                                                            uint64_t img_stride_out, uint64_t img_stride_dog,
                                                            BlurTaps t) {
-    const int x = blockIdx.x * kBlurX + threadIdx.x, y = blockIdx.y, b = blockIdx.z;
+    const int x = blockIdx.x * kBlurX + threadIdx.x, y = grid_wait(blockIdx.y), b = blockIdx.z;
     if (x >= w) return;
     const float *c = tmp + b * img_stride_tmp + x;
     float acc = 0.0f;
@@ -137,7 +138,8 @@ __global__ void __launch_bounds__(256) blur_fused_kernel(const float *__restrict
     constexpr int V = kFY / 4;  // a column's run: 64 columns x 4 runs = 256 threads
     float *in = blur_tile, *hs = blur_tile + rows * kFInPitch;
     const int b = blockIdx.z, warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
-    const int x0 = blockIdx.x * kFX, y0 = blockIdx.y * kFY;
+    const int x0 = blockIdx.x * kFX, y0 = grid_wait(blockIdx.y) * kFY;
+    grid_go();
     const float *S = src + b * img_stride_src;
 #pragma unroll 4
     for (int ry = warp; ry < rows; ry += 8) {
@@ -191,7 +193,8 @@ __global__ void __launch_bounds__(256) blur_fused_kernel(const float *__restrict
 // base of the next octave: the even pixels of gauss[s] (GrayImage::downsample)
 __global__ void downsample_kernel(const float *__restrict__ src, float *__restrict__ dst, int w, int h, int nw, int nh,
                                   uint64_t img_stride_src, uint64_t img_stride_dst) {
-    const int x = blockIdx.x * blockDim.x + threadIdx.x, y = blockIdx.y, b = blockIdx.z;
+    const int x = blockIdx.x * blockDim.x + threadIdx.x, y = grid_wait(blockIdx.y), b = blockIdx.z;
+    grid_go();
     if (x >= nw) return;
     dst[b * img_stride_dst + (uint64_t)y * nw + x] = src[b * img_stride_src + (uint64_t)(2 * y) * w + 2 * x];
 }
@@ -199,7 +202,8 @@ __global__ void downsample_kernel(const float *__restrict__ src, float *__restri
 // GrayImage::upsample2 (features.rs:62-85): bilinear at pixel centres.
 __global__ void upsample2_kernel(const float *__restrict__ src, float *__restrict__ dst, int w, int h) {
     const int W = 2 * w;
-    const int x = blockIdx.x * blockDim.x + threadIdx.x, y = blockIdx.y, b = blockIdx.z;
+    const int x = blockIdx.x * blockDim.x + threadIdx.x, y = grid_wait(blockIdx.y), b = blockIdx.z;
+    grid_go();
     if (x >= W) return;
     const float *s = src + (uint64_t)b * w * h;
     const float sy = ((float)y + 0.5f) / 2.0f - 0.5f;
@@ -213,15 +217,33 @@ __global__ void upsample2_kernel(const float *__restrict__ src, float *__restric
     dst[(uint64_t)b * W * (2 * h) + (uint64_t)y * W + x] = top * (1.0f - fy) + bot * fy;
 }
 
-// GrayImage::from_rgb (features.rs:165-189)
-__global__ void gray_from_rgb8_kernel(const uint8_t *__restrict__ rgb, float *__restrict__ out, uint64_t n) {
-    const uint64_t i = (uint64_t)blockIdx.x * blockDim.x + threadIdx.x;
-    if (i >= n) return;
-    const uint8_t *c = rgb + 3 * i;
-    out[i] = (0.299f * (float)c[0] + 0.587f * (float)c[1] + 0.114f * (float)c[2]) / 255.0f;
+// GrayImage::from_rgb (features.rs:165-189). Four pixels a thread where the
+// bytes lie on a 4-byte boundary: three word loads, one 16-byte store.
+__device__ __forceinline__ float gray_of(uint32_t r, uint32_t g, uint32_t b) {
+    return (0.299f * (float)r + 0.587f * (float)g + 0.114f * (float)b) / 255.0f;
+}
+__global__ void __launch_bounds__(256) gray_from_rgb8_kernel(const uint8_t *rgb, float *out, uint64_t n, bool wide) {
+    grid_wait();
+    grid_go();
+    const uint64_t i = ((uint64_t)blockIdx.x * 256 + threadIdx.x) * 4;
+    if (wide && i + 4 <= n) {
+        const uint32_t *c = reinterpret_cast<const uint32_t *>(rgb + 3 * i);
+        const uint32_t u = c[0], v = c[1], t = c[2];
+        *reinterpret_cast<float4 *>(out + i) =
+            make_float4(gray_of(u & 255, u >> 8 & 255, u >> 16 & 255), gray_of(u >> 24, v & 255, v >> 8 & 255),
+                        gray_of(v >> 16 & 255, v >> 24, t & 255), gray_of(t >> 8 & 255, t >> 16 & 255, t >> 24));
+        return;
+    }
+    for (uint64_t k = i; k < n && k < i + 4; ++k) out[k] = gray_of(rgb[3 * k], rgb[3 * k + 1], rgb[3 * k + 2]);
 }
 
-// ------------------------------------------------------------- gradients
+// Images that lie in host memory the device reads where it is: one read over
+// the link, 16 bytes a thread.
+__global__ void __launch_bounds__(256) read_images_kernel(const float4 *src, float4 *dst, uint64_t n4) {
+    grid_wait();
+    grid_go();
+    for (uint64_t i = (uint64_t)blockIdx.x * 256 + threadIdx.x; i < n4; i += (uint64_t)gridDim.x * 256) dst[i] = src[i];
+}
 
 // GradTable (features.rs:335-359) of s consecutive layers from l0: |g| and
 // atan2(gy, gx) of central differences at interior pixels (pixel_grad,
@@ -232,7 +254,8 @@ __global__ void gray_from_rgb8_kernel(const uint8_t *__restrict__ rgb, float *__
 constexpr int kGradRows = 6;
 __global__ void __launch_bounds__(128) grad_kernel(const float *__restrict__ gauss, float2 *__restrict__ grad, int w,
                                                    int h, int s, uint64_t layer_stride, uint64_t img_stride, int l0) {
-    const int x = blockIdx.x * blockDim.x + threadIdx.x, y0 = blockIdx.y * kGradRows;
+    const int x = blockIdx.x * blockDim.x + threadIdx.x, y0 = grid_wait(blockIdx.y) * kGradRows;
+    grid_go();
     const int b = blockIdx.z / s, l = blockIdx.z % s;
     if (x >= w) return;
     const bool inside = x >= 1 && x + 1 < w;
@@ -312,6 +335,8 @@ __global__ void __launch_bounds__(32 * kExtremaWarps) extrema_kernel(ExtremaArgs
     __shared__ uint32_t found[30 * kExtremaRows * kExtremaWarps / 2];
     __shared__ uint32_t n_found;
     if (threadIdx.x == 0) n_found = 0;
+    grid_wait();
+    grid_go();
     __syncthreads();
     const int lane = threadIdx.x & 31, strip = blockIdx.y * kExtremaWarps + (threadIdx.x >> 5);
     const int b = blockIdx.z / a.s, l0 = 1 + blockIdx.z % a.s;
@@ -421,9 +446,13 @@ __device__ void refine_candidate(const ExtremaArgs &a, const float *dog, int b, 
 // sig_oct = sigma0 * kstep^s (features.rs:747) of every candidate, one a thread:
 // pow in double is some 300 operations at 2 per clock and SM, which a lone
 // lane of the scan paid for by itself.
-__global__ void __launch_bounds__(256) candidate_sigma_kernel(FeatCand *cands, uint32_t n, float sigma0, float kstep) {
-    const uint32_t i = blockIdx.x * blockDim.x + threadIdx.x;
-    if (i < n) cands[i].sig = sigma0 * (float)pow((double)kstep, (double)cands[i].sig);
+__global__ void __launch_bounds__(256) candidate_sigma_kernel(FeatCand *cands, const uint32_t *count, uint32_t cap,
+                                                              float sigma0, float kstep) {
+    grid_wait();
+    grid_go();
+    const uint32_t n = min(*count, cap);
+    for (uint32_t i = blockIdx.x * 256 + threadIdx.x; i < n; i += gridDim.x * 256)
+        cands[i].sig = sigma0 * (float)pow((double)kstep, (double)cands[i].sig);
 }
 
 // --------------------------------------------------------------- orientations
@@ -437,96 +466,98 @@ __global__ void __launch_bounds__(256) orient_kernel(OrientArgs a) {
     __shared__ float hs[8][kOriBins];
     __shared__ float vals[8][32];
     const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
-    const uint32_t ci = blockIdx.x * 8 + warp;
+    grid_wait();
+    grid_go();
     const uint32_t n = min(*a.count, a.cap);
-    if (ci >= n) return;
-    const FeatCand c = a.cands[ci];
-    const OctaveGeom &G = a.geom[c.octave];
-    const float2 *grad = a.grads + G.grad_off + ((uint64_t)c.img * a.s + (c.layer - 1)) * G.layer_stride;
-    const int w = G.w, h = G.h;
-    const float sw = 1.5f * c.sig;
-    const int r = f2i(roundf(3.0f * sw));
-    const int xi = f2i(roundf(c.x)), yi = f2i(roundf(c.y));
-    const int side = 2 * r + 1;
-    const int total = side * side;
-    float h0 = 0.0f, h1 = 0.0f;
-    // the bits that make a bin number this lane's, and (lanes 0-3) this lane's + 32
-    uint32_t inv[5];
+    for (uint32_t ci = blockIdx.x * 8 + warp; ci < n; ci += gridDim.x * 8) {  // warp-uniform
+        const FeatCand c = a.cands[ci];
+        const OctaveGeom &G = a.geom[c.octave];
+        const float2 *grad = a.grads + G.grad_off + ((uint64_t)c.img * a.s + (c.layer - 1)) * G.layer_stride;
+        const int w = G.w, h = G.h;
+        const float sw = 1.5f * c.sig;
+        const int r = f2i(roundf(3.0f * sw));
+        const int xi = f2i(roundf(c.x)), yi = f2i(roundf(c.y));
+        const int side = 2 * r + 1;
+        const int total = side * side;
+        float h0 = 0.0f, h1 = 0.0f;
+        // the bits that make a bin number this lane's, and (lanes 0-3) this lane's + 32
+        uint32_t inv[5];
 #pragma unroll
-    for (int k = 0; k < 5; ++k) inv[k] = (lane >> k) & 1 ? 0u : ~0u;
-    for (int base = 0; base < total; base += 32) {
-        const int t = base + lane;
-        int bin = 63;  // none: no lane's bin
-        float val = 0.0f;
-        if (t < total) {
-            const int px = xi + (t % side) - r, py = yi + (t / side) - r;
-            if (!(px < 1 || py < 1 || px >= w - 1 || py >= h - 1)) {
-                const float2 gm = grad[(uint64_t)py * w + px];
-                const float fx = (float)px - c.x, fy = (float)py - c.y;
-                const float wgt = exp_cr(-(fx * fx + fy * fy) / (2.0f * sw * sw));
-                const float ang = rem_euclid(gm.y, kTwoPi);
-                const float bf = roundf(ang / kTwoPi * (float)kOriBins);
-                bin = (int)((unsigned)(bf < 0.0f ? 0 : f2i(bf)) % kOriBins);
-                val = wgt * gm.x;
+        for (int k = 0; k < 5; ++k) inv[k] = (lane >> k) & 1 ? 0u : ~0u;
+        for (int base = 0; base < total; base += 32) {
+            const int t = base + lane;
+            int bin = 63;  // none: no lane's bin
+            float val = 0.0f;
+            if (t < total) {
+                const int px = xi + (t % side) - r, py = yi + (t / side) - r;
+                if (!(px < 1 || py < 1 || px >= w - 1 || py >= h - 1)) {
+                    const float2 gm = grad[(uint64_t)py * w + px];
+                    const float fx = (float)px - c.x, fy = (float)py - c.y;
+                    const float wgt = exp_cr(-(fx * fx + fy * fy) / (2.0f * sw * sw));
+                    const float ang = rem_euclid(gm.y, kTwoPi);
+                    const float bf = roundf(ang / kTwoPi * (float)kOriBins);
+                    bin = (int)((unsigned)(bf < 0.0f ? 0 : f2i(bf)) % kOriBins);
+                    val = wgt * gm.x;
+                }
             }
-        }
-        uint32_t low = ~0u;
+            uint32_t low = ~0u;
 #pragma unroll
-        for (int k = 0; k < 5; ++k) low &= __ballot_sync(0xffffffffu, (bin >> k) & 1) ^ inv[k];
-        const uint32_t high = __ballot_sync(0xffffffffu, bin >> 5);
-        vals[warp][lane] = val;
-        __syncwarp();
-        for (uint32_t m = low & ~high; m; m &= m - 1) h0 += vals[warp][__ffs(m) - 1];
-        if (lane < kOriBins - 32)
-            for (uint32_t m = low & high; m; m &= m - 1) h1 += vals[warp][__ffs(m) - 1];
-        __syncwarp();
-    }
-    // six [1,1,1]/3 smoothings, lane b computing bins b and b + 32 (each bin
-    // from the previous pass's three, ((l + c) + r) / 3 as the reference)
-    float *hist = hs[warp];
-    const int b1 = lane + 32;
-    const bool has1 = b1 < kOriBins;
-    for (int it = 0; it < 6; ++it) {
+            for (int k = 0; k < 5; ++k) low &= __ballot_sync(0xffffffffu, (bin >> k) & 1) ^ inv[k];
+            const uint32_t high = __ballot_sync(0xffffffffu, bin >> 5);
+            vals[warp][lane] = val;
+            __syncwarp();
+            for (uint32_t m = low & ~high; m; m &= m - 1) h0 += vals[warp][__ffs(m) - 1];
+            if (lane < kOriBins - 32)
+                for (uint32_t m = low & high; m; m &= m - 1) h1 += vals[warp][__ffs(m) - 1];
+            __syncwarp();
+        }
+        // six [1,1,1]/3 smoothings, lane b computing bins b and b + 32 (each bin
+        // from the previous pass's three, ((l + c) + r) / 3 as the reference)
+        float *hist = hs[warp];
+        const int b1 = lane + 32;
+        const bool has1 = b1 < kOriBins;
+        for (int it = 0; it < 6; ++it) {
+            hist[lane] = h0;
+            if (has1) hist[b1] = h1;
+            __syncwarp();
+            const float n0 = (hist[(lane + kOriBins - 1) % kOriBins] + h0 + hist[(lane + 1) % kOriBins]) / 3.0f;
+            const float n1 = has1 ? (hist[(b1 + kOriBins - 1) % kOriBins] + h1 + hist[(b1 + 1) % kOriBins]) / 3.0f : 0.0f;
+            __syncwarp();
+            h0 = n0;
+            h1 = n1;
+        }
         hist[lane] = h0;
         if (has1) hist[b1] = h1;
         __syncwarp();
-        const float n0 = (hist[(lane + kOriBins - 1) % kOriBins] + h0 + hist[(lane + 1) % kOriBins]) / 3.0f;
-        const float n1 = has1 ? (hist[(b1 + kOriBins - 1) % kOriBins] + h1 + hist[(b1 + 1) % kOriBins]) / 3.0f : 0.0f;
-        __syncwarp();
-        h0 = n0;
-        h1 = n1;
-    }
-    hist[lane] = h0;
-    if (has1) hist[b1] = h1;
-    __syncwarp();
-    // fold(0.0, f32::max): fmaxf is order-free (NaN ignored either way)
-    float mx = fmaxf(h0, has1 ? h1 : 0.0f);
+        // fold(0.0, f32::max): fmaxf is order-free (NaN ignored either way)
+        float mx = fmaxf(h0, has1 ? h1 : 0.0f);
 #pragma unroll
-    for (int o = 16; o; o >>= 1) mx = fmaxf(mx, __shfl_xor_sync(0xffffffffu, mx, o));
-    mx = fmaxf(0.0f, mx);
-    // peaks in bin order: bins 0..31 by lane, then 32..35
-    float *out = a.angles + (uint64_t)ci * kMaxAngles;
-    int na = 0;
-    if (mx > 0.0f) {
+        for (int o = 16; o; o >>= 1) mx = fmaxf(mx, __shfl_xor_sync(0xffffffffu, mx, o));
+        mx = fmaxf(0.0f, mx);
+        // peaks in bin order: bins 0..31 by lane, then 32..35
+        float *out = a.angles + (uint64_t)ci * kMaxAngles;
+        int na = 0;
+        if (mx > 0.0f) {
 #pragma unroll
-        for (int half = 0; half < 2; ++half) {
-            const int i = half ? b1 : lane;
-            bool peak = false;
-            float ang = 0.0f;
-            if (i < kOriBins) {
-                const float l = hist[(i + kOriBins - 1) % kOriBins], cc = hist[i], rr = hist[(i + 1) % kOriBins];
-                if (cc >= 0.8f * mx && cc > l && cc > rr) {
-                    const float off = 0.5f * (l - rr) / (l - 2.0f * cc + rr);
-                    ang = rem_euclid(((float)i + off) / (float)kOriBins * kTwoPi, kTwoPi);
-                    peak = true;
+            for (int half = 0; half < 2; ++half) {
+                const int i = half ? b1 : lane;
+                bool peak = false;
+                float ang = 0.0f;
+                if (i < kOriBins) {
+                    const float l = hist[(i + kOriBins - 1) % kOriBins], cc = hist[i], rr = hist[(i + 1) % kOriBins];
+                    if (cc >= 0.8f * mx && cc > l && cc > rr) {
+                        const float off = 0.5f * (l - rr) / (l - 2.0f * cc + rr);
+                        ang = rem_euclid(((float)i + off) / (float)kOriBins * kTwoPi, kTwoPi);
+                        peak = true;
+                    }
                 }
+                const unsigned m = __ballot_sync(0xffffffffu, peak);
+                if (peak) out[na + __popc(m & ((1u << lane) - 1u))] = ang;
+                na += __popc(m);
             }
-            const unsigned m = __ballot_sync(0xffffffffu, peak);
-            if (peak) out[na + __popc(m & ((1u << lane) - 1u))] = ang;
-            na += __popc(m);
         }
+        if (lane == 0) a.nang[ci] = (uint8_t)na;
     }
-    if (lane == 0) a.nang[ci] = (uint8_t)na;
 }
 
 // ----------------------------------------------------------------- describe
@@ -537,6 +568,8 @@ constexpr int kDescThreads = 128;
 // thread, since FP64 runs at 2 operations per clock and SM (in the describing
 // CTAs four warps each repeated them).
 __global__ void __launch_bounds__(128) describe_angle_kernel(const DescJob *jobs, float2 *cs, uint32_t n) {
+    grid_wait();
+    grid_go();
     const uint32_t i = blockIdx.x * blockDim.x + threadIdx.x;
     if (i >= n) return;
     const double a = (double)jobs[i].angle;
@@ -953,6 +986,7 @@ constexpr int kDescMaxSide = 2600;
 __global__ void __launch_bounds__(kDescCtaThreads) describe_mixed_kernel(DescribeArgs a, uint32_t njobs) {
     extern __shared__ __align__(16) unsigned char desc_smem[];
     DescMixedSmem &S = *reinterpret_cast<DescMixedSmem *>(desc_smem);
+    grid_wait();
     if (blockIdx.x < a.n_large) {
         describe_cta(a, blockIdx.x, S.cta, reinterpret_cast<uint32_t *>(desc_smem + sizeof(DescMixedSmem)));
         return;
@@ -965,6 +999,7 @@ __global__ void __launch_bounds__(kDescCtaThreads) describe_mixed_kernel(Describ
 // fewer registers a CTA.
 __global__ void __launch_bounds__(kDescThreads, 8) describe_kernel(DescribeArgs a, uint32_t njobs) {
     __shared__ DescWarpSmem S[kDescWarps];
+    grid_wait();
     const uint32_t k = blockIdx.x * kDescWarps + (threadIdx.x >> 5);
     if (k < njobs) describe_warp(a, k, S[threadIdx.x >> 5], threadIdx.x & 31);
 }
@@ -1006,34 +1041,43 @@ void launch_blur(const float *src, float *tmp, float *dst, const float *prev, fl
         const uint64_t tiles = (uint64_t)((w + kFX - 1) / kFX) * ((h + 63) / 64) * nimg;
         const BlurFused f = blur_of_radius<1>(t.r, tiles >= 608);
         const dim3 g((w + kFX - 1) / kFX, (h + f.rows - 1) / f.rows, nimg);
-        f.kernel<<<g, 256, f.smem, s>>>(src, dst, dog, w, h, stride_src, stride_dst, stride_dog, t);
+        launch_next(f.kernel, g, 256, f.smem, s, src, dst, dog, w, h, stride_src, stride_dst, stride_dog, t);
         return;
     }
     const dim3 grid((w + kBlurX - 1) / kBlurX, h, nimg);
-    blur_rows_kernel<<<grid, kBlurX, 0, s>>>(src, tmp, w, h, stride_src, (uint64_t)w * h, t);
-    blur_cols_kernel<<<grid, kBlurX, 0, s>>>(tmp, dst, prev, dog, w, h, (uint64_t)w * h, stride_dst, stride_dog, t);
+    launch_next(blur_rows_kernel, grid, kBlurX, 0, s, src, tmp, w, h, stride_src, (uint64_t)w * h, t);
+    launch_next(blur_cols_kernel, grid, kBlurX, 0, s, tmp, dst, prev, dog, w, h, (uint64_t)w * h, stride_dst, stride_dog, t);
 }
 
 void launch_downsample(const float *src, float *dst, int w, int h, int nimg, uint64_t stride_src,
                        uint64_t stride_dst, cudaStream_t s) {
     const int nw = w / 2, nh = h / 2;
     if (!nw || !nh) return;
-    downsample_kernel<<<dim3((nw + 255) / 256, nh, nimg), 256, 0, s>>>(src, dst, w, h, nw, nh, stride_src,
-                                                                       stride_dst);
+    launch_next(downsample_kernel, dim3((nw + 255) / 256, nh, nimg), 256, 0, s, src, dst, w, h, nw, nh, stride_src,
+                stride_dst);
 }
 
 void launch_upsample2(const float *src, float *dst, int w, int h, int nimg, cudaStream_t s) {
-    upsample2_kernel<<<dim3((2 * w + 255) / 256, 2 * h, nimg), 256, 0, s>>>(src, dst, w, h);
+    launch_next(upsample2_kernel, dim3((2 * w + 255) / 256, 2 * h, nimg), 256, 0, s, src, dst, w, h);
 }
 
 void launch_gray_from_rgb8(const uint8_t *rgb, float *out, uint64_t n, cudaStream_t s) {
-    if (n) gray_from_rgb8_kernel<<<(unsigned)((n + 255) / 256), 256, 0, s>>>(rgb, out, n);
+    if (n)
+        launch_next(gray_from_rgb8_kernel, (unsigned)((n + 1023) / 1024), 256, 0, s, rgb, out, n,
+                    (reinterpret_cast<uintptr_t>(rgb) & 3) == 0);
+}
+
+void launch_read_images(const float *src, float *dst, uint64_t n, int sms, cudaStream_t s) {
+    const uint64_t n4 = n / 4;
+    if (n4)
+        launch_next(read_images_kernel, (unsigned)((n4 + 255) / 256 < 8ull * sms ? (n4 + 255) / 256 : 8ull * sms), 256, 0, s,
+                    reinterpret_cast<const float4 *>(src), reinterpret_cast<float4 *>(dst), n4);
 }
 
 void launch_grad(const float *gauss, float2 *grad, int w, int h, int s_, uint64_t img_stride, int l0, int nimg,
                  cudaStream_t s) {
-    grad_kernel<<<dim3((w + 127) / 128, (h + kGradRows - 1) / kGradRows, nimg * s_), 128, 0, s>>>(
-        gauss, grad, w, h, s_, (uint64_t)w * h, img_stride, l0);
+    launch_next(grad_kernel, dim3((w + 127) / 128, (h + kGradRows - 1) / kGradRows, nimg * s_), 128, 0, s, gauss, grad, w, h,
+                s_, (uint64_t)w * h, img_stride, l0);
 }
 
 void launch_extrema(const ExtremaArgs &a, int nimg, cudaStream_t s) {
@@ -1041,27 +1085,33 @@ void launch_extrema(const ExtremaArgs &a, int nimg, cudaStream_t s) {
     // strips of 16 rows where that leaves every SM its 16 warps, else of 4
     const uint64_t warps = (uint64_t)((a.w + 27) / 30) * ((a.h + 13) / 16) * nimg * a.s;
     const int rows = warps >= 16 * 152 ? kExtremaRows : 4, strip = kExtremaWarps * rows;
-    extrema_kernel<<<dim3((a.w + 27) / 30, (a.h - 2 + strip - 1) / strip, nimg * a.s), 32 * kExtremaWarps, 0, s>>>(a, rows);
+    launch_next(extrema_kernel, dim3((a.w + 27) / 30, (a.h - 2 + strip - 1) / strip, nimg * a.s), 32 * kExtremaWarps, 0, s,
+                a, rows);
 }
 
-void launch_candidate_sigma(FeatCand *cands, uint32_t n, float sigma0, float kstep, cudaStream_t s) {
-    if (n) candidate_sigma_kernel<<<(n + 255) / 256, 256, 0, s>>>(cands, n, sigma0, kstep);
+// The number of candidates is the device's: grids for as many as there may be,
+// up to what the SMs hold a few times over.
+void launch_candidate_sigma(FeatCand *cands, const uint32_t *count, uint32_t cap, float sigma0, float kstep, int sms,
+                            cudaStream_t s) {
+    const uint32_t grid = (cap + 255) / 256 < 2u * sms ? (cap + 255) / 256 : 2u * sms;
+    launch_next(candidate_sigma_kernel, grid, 256, 0, s, cands, count, cap, sigma0, kstep);
 }
 
-void launch_orient(const OrientArgs &a, uint32_t n, cudaStream_t s) {
-    if (n) orient_kernel<<<(n + 7) / 8, 256, 0, s>>>(a);
+void launch_orient(const OrientArgs &a, int sms, cudaStream_t s) {
+    const uint32_t grid = (a.cap + 7) / 8 < 16u * sms ? (a.cap + 7) / 8 : 16u * sms;
+    launch_next(orient_kernel, grid, 256, 0, s, a);
 }
 
 void launch_describe(const DescribeArgs &a, uint32_t njobs, cudaStream_t s) {
     if (!njobs) return;
-    describe_angle_kernel<<<(njobs + 127) / 128, 128, 0, s>>>(a.jobs, a.cs, njobs);
+    launch_next(describe_angle_kernel, (njobs + 127) / 128, 128, 0, s, a.jobs, a.cs, njobs);
     if (!a.n_large) {
-        describe_kernel<<<(njobs + kDescWarps - 1) / kDescWarps, kDescThreads, 0, s>>>(a, njobs);
+        launch_next(describe_kernel, (njobs + kDescWarps - 1) / kDescWarps, kDescThreads, 0, s, a, njobs);
         return;
     }
     const size_t rows = sizeof(DescMixedSmem) + 4 * (size_t)(a.max_side + 1) + 2 * (size_t)a.max_side;
-    describe_mixed_kernel<<<a.n_large + (njobs - a.n_large + kDescCtaWarps - 1) / kDescCtaWarps, kDescCtaThreads, rows,
-                            s>>>(a, njobs);
+    launch_next(describe_mixed_kernel, a.n_large + (njobs - a.n_large + kDescCtaWarps - 1) / kDescCtaWarps, kDescCtaThreads,
+                rows, s, a, njobs);
 }
 
 }  // namespace slm

@@ -17,13 +17,20 @@ constexpr uint32_t kWaitLimit = 1u << 24;
 // Programmatic dependent launch. A kernel started by launch_next is set up while
 // the one before it still runs; its grid_wait() returns once all work before it
 // is done and visible, so it comes before any access to memory (and such kernels
-// take no __restrict__ inputs, whose loads the compiler may move up). grid_go() lets
+// take no __restrict__ inputs, whose loads the compiler may move up, or make
+// every address from grid_wait's value). grid_go() lets
 // the next kernel be set up from here on; kernels whose CTAs fill the SMs leave
 // it out (the end of the grid does it then). A batch's dozen kernels after the
 // pass find little or nothing to do: with ordinary launches 30 pairs of 500 to
 // 4000 descriptors took 161 us and one pair of 8192 rows 198, now 126 and 161
 // (with the faster compact and gather kernels).
 SLM_DEV void grid_wait() { asm volatile("griddepcontrol.wait;" ::: "memory"); }
+// The value back, after the wait: loads at addresses made from it stay behind
+// the wait whatever their pointers are declared.
+SLM_DEV uint32_t grid_wait(uint32_t v) {
+    asm volatile("griddepcontrol.wait;" : "+r"(v)::"memory");
+    return v;
+}
 SLM_DEV void grid_go() { asm volatile("griddepcontrol.launch_dependents;" ::: "memory"); }
 
 template <class... P, class... A>

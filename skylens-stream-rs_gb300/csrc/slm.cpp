@@ -3022,17 +3022,16 @@ slm_status feat_core(slm_ctx *c, Workspace *ws, const float *d_img, uint32_t n, 
     }
     for (int attempt = 0; attempt < 2; ++attempt) {
         const uint64_t o_geom = 0, o_gauss = feat_align(o_geom + sizeof(OctaveGeom) * out.geom.size()),
-                       o_dog = feat_align(o_gauss + 4 * (uint64_t)n * ng * wh0),
+                       o_odd = feat_align(o_gauss + 4 * (uint64_t)n * ng * wh0),  // odd octaves' layers
+                       o_dog = feat_align(o_odd + 4 * (uint64_t)n * ng * wh1),
                        o_tmp = feat_align(o_dog + 4 * (uint64_t)n * (ng - 1) * wh0),
-                       o_base = feat_align(o_tmp + 4 * (uint64_t)n * wh0),
-                       o_grad = feat_align(o_base + 4 * (uint64_t)n * wh1),
+                       o_grad = feat_align(o_tmp + 4 * (uint64_t)n * wh0),
                        o_cand = feat_align(o_grad + 8 * ngrad), o_cnt = feat_align(o_cand + sizeof(FeatCand) * cap),
                        o_ang = feat_align(o_cnt + 16), o_nang = feat_align(o_ang + 4ull * kMaxAngles * cap),
                        bytes = feat_align(o_nang + cap);
         SLM_TRY(pyr.ensure(c, bytes));
         unsigned char *d = pyr.as<unsigned char>();
-        float *gauss = reinterpret_cast<float *>(d + o_gauss), *dog = reinterpret_cast<float *>(d + o_dog),
-              *tmp = reinterpret_cast<float *>(d + o_tmp), *base = reinterpret_cast<float *>(d + o_base);
+        float *dog = reinterpret_cast<float *>(d + o_dog), *tmp = reinterpret_cast<float *>(d + o_tmp);
         out.d_geom = reinterpret_cast<OctaveGeom *>(d + o_geom);
         out.d_grads = reinterpret_cast<float2 *>(d + o_grad);
         out.d_cands = reinterpret_cast<FeatCand *>(d + o_cand);
@@ -3045,12 +3044,14 @@ slm_status feat_core(slm_ctx *c, Workspace *ws, const float *d_img, uint32_t n, 
         for (size_t o = 0; o < out.geom.size(); ++o) {
             const OctaveGeom &G = out.geom[o];
             const uint64_t wh = G.layer_stride;
+            // an octave's first layer comes from the one before it, so they alternate
+            float *gauss = reinterpret_cast<float *>(d + (o & 1 ? o_odd : o_gauss));
             if (o == 0) {
                 launch_blur(d_img, tmp, gauss, nullptr, nullptr, G.w, G.h, (int)n, wh, ng * wh, 0, taps[0], st);
             } else {
                 const OctaveGeom &P = out.geom[o - 1];
-                launch_downsample(gauss + s * P.layer_stride, base, P.w, P.h, (int)n, ng * P.layer_stride, wh, st);
-                SLM_CU(cudaMemcpy2DAsync(gauss, 4 * ng * wh, base, 4 * wh, 4 * wh, n, cudaMemcpyDeviceToDevice, st));
+                const float *before = reinterpret_cast<const float *>(d + (o & 1 ? o_gauss : o_odd));
+                launch_downsample(before + s * P.layer_stride, gauss, P.w, P.h, (int)n, ng * P.layer_stride, ng * wh, st);
             }
             for (int i = 1; i < ng; ++i)
                 launch_blur(gauss + (i - 1) * wh, tmp, gauss + i * wh, gauss + (i - 1) * wh, dog + (i - 1) * wh, G.w,
@@ -3071,15 +3072,6 @@ slm_status feat_core(slm_ctx *c, Workspace *ws, const float *d_img, uint32_t n, 
             ea.cap = cap;
             launch_extrema(ea, (int)n, st);
         }
-        SLM_CU(cudaGetLastError());
-        uint32_t count = 0;
-        SLM_CU(cudaMemcpyAsync(&count, d_count, 4, cudaMemcpyDeviceToHost, st));
-        SLM_CU(cudaStreamSynchronize(st));
-        if (count > cap) {  // the list overflowed: run again with room for every candidate
-            if (attempt) return fail(SLM_INTERNAL, "feature candidates overflowed twice");
-            cap = count;
-            continue;
-        }
         OrientArgs oa{};
         oa.cands = out.d_cands;
         oa.count = d_count;
@@ -3089,23 +3081,37 @@ slm_status feat_core(slm_ctx *c, Workspace *ws, const float *d_img, uint32_t n, 
         oa.s = s;
         oa.angles = d_ang;
         oa.nang = d_nang;
-        launch_candidate_sigma(out.d_cands, count, cfg.sigma0, kstep, st);
-        launch_orient(oa, count, st);
+        launch_candidate_sigma(out.d_cands, d_count, cap, cfg.sigma0, kstep, c->sms, st);
+        launch_orient(oa, c->sms, st);
         SLM_CU(cudaGetLastError());
-        // candidates, angle counts and angles into pinned host memory
-        const uint64_t h_ang = feat_align(sizeof(FeatCand) * (uint64_t)count),
-                       h_nang = feat_align(h_ang + 4ull * kMaxAngles * count), h_bytes = h_nang + count + 16;
-        SLM_TRY(ws_host_block(ws, h_bytes));
-        unsigned char *hb = ws->single_host;
-        out.cands = reinterpret_cast<const FeatCand *>(hb);
-        out.angles = reinterpret_cast<const float *>(hb + h_ang);
-        const uint8_t *nang = hb + h_nang;
-        if (count) {
-            SLM_CU(cudaMemcpyAsync(hb, out.d_cands, sizeof(FeatCand) * count, cudaMemcpyDeviceToHost, st));
-            SLM_CU(cudaMemcpyAsync(hb + h_ang, d_ang, 4ull * kMaxAngles * count, cudaMemcpyDeviceToHost, st));
-            SLM_CU(cudaMemcpyAsync(hb + h_nang, d_nang, count, cudaMemcpyDeviceToHost, st));
+        // candidates, angle counts and angles into pinned host memory, with their
+        // number: as many as images usually have come back before it is known
+        // (1300 for a 960 x 540 view), the rest in a second copy
+        uint32_t room = std::min<uint64_t>(cap, std::max<uint64_t>(2048, 1536ull * n)), count = 0;
+        uint64_t h_ang = 0, h_nang = 0;
+        for (bool again = false;; again = true) {
+            const uint64_t h_cand = 16;
+            h_ang = feat_align(h_cand + sizeof(FeatCand) * (uint64_t)room);
+            h_nang = feat_align(h_ang + 4ull * kMaxAngles * room);
+            SLM_TRY(ws_host_block(ws, h_nang + room + 16));
+            unsigned char *hb = ws->single_host;
+            out.cands = reinterpret_cast<const FeatCand *>(hb + h_cand);
+            SLM_CU(cudaMemcpyAsync(hb, d_count, 4, cudaMemcpyDeviceToHost, st));
+            SLM_CU(cudaMemcpyAsync(hb + h_cand, out.d_cands, sizeof(FeatCand) * room, cudaMemcpyDeviceToHost, st));
+            SLM_CU(cudaMemcpyAsync(hb + h_ang, d_ang, 4ull * kMaxAngles * room, cudaMemcpyDeviceToHost, st));
+            SLM_CU(cudaMemcpyAsync(hb + h_nang, d_nang, room, cudaMemcpyDeviceToHost, st));
+            SLM_CU(cudaStreamSynchronize(st));
+            std::memcpy(&count, hb, 4);
+            if (again || count <= room || count > cap) break;
+            room = count;
         }
-        SLM_CU(cudaStreamSynchronize(st));
+        if (count > cap) {  // the list overflowed: run again with room for every candidate
+            if (attempt) return fail(SLM_INTERNAL, "feature candidates overflowed twice");
+            cap = count;
+            continue;
+        }
+        out.angles = reinterpret_cast<const float *>(ws->single_host + h_ang);
+        const uint8_t *nang = ws->single_host + h_nang;
         // the reference's emission order (octave, layer, row, column of the
         // scanned extremum; angles in bin order), then its stable sort by
         // |response| descending (f32::total_cmp of abs(): the bits of |v|) and
@@ -3375,7 +3381,22 @@ slm_status feat_call(slm_ctx *c, const void *imgs, bool rgb, uint32_t n, uint32_
             unsigned char *d = W->feat_in.as<unsigned char>();
             if (r == SLM_OK) {
                 const unsigned char *src = static_cast<const unsigned char *>(imgs) + (rgb ? 3 : 4) * bnd[p] * wh;
-                if (cudaMemcpyAsync(rgb ? d + o_rgb : d, src, (rgb ? 3 : 4) * np * wh, cudaMemcpyDefault,
+                // gray images in pageable memory the device reads where they lie (1.5 MB:
+                // 11 us; 26 with a copy call, which stages them)
+                cudaPointerAttributes pa{};
+                const bool pageable = cudaPointerGetAttributes(&pa, src) == cudaSuccess &&
+                                      pa.type == cudaMemoryTypeUnregistered;
+                cudaGetLastError();
+                if (pageable && !rgb && c->host_direct && np * wh >= 4 && (reinterpret_cast<uintptr_t>(src) & 15) == 0) {
+                    const uint64_t whole = np * wh / 4 * 4;
+                    launch_read_images(reinterpret_cast<const float *>(src), reinterpret_cast<float *>(d), whole, c->sms,
+                                       W->stream);
+                    if (cudaGetLastError() != cudaSuccess) r = fail(SLM_CUDA_ERROR, "image read launch failed");
+                    if (r == SLM_OK && whole < np * wh &&
+                        cudaMemcpyAsync(d + 4 * whole, src + 4 * whole, 4 * (np * wh - whole), cudaMemcpyDefault,
+                                        W->stream) != cudaSuccess)
+                        r = fail(SLM_CUDA_ERROR, std::string("image upload: ") + cudaGetErrorString(cudaGetLastError()));
+                } else if (cudaMemcpyAsync(rgb ? d + o_rgb : d, src, (rgb ? 3 : 4) * np * wh, cudaMemcpyDefault,
                                     W->stream) != cudaSuccess)
                     r = fail(SLM_CUDA_ERROR, std::string("image upload: ") + cudaGetErrorString(cudaGetLastError()));
             }

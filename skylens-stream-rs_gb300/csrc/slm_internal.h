@@ -240,13 +240,16 @@ void launch_downsample(const float *src, float *dst, int w, int h, int nimg, uin
                        uint64_t stride_dst, cudaStream_t s);
 void launch_upsample2(const float *src, float *dst, int w, int h, int nimg, cudaStream_t s);
 void launch_gray_from_rgb8(const uint8_t *rgb, float *out, uint64_t n, cudaStream_t s);
+// n floats (whole groups of four) the device reads where they lie, 16-byte aligned
+void launch_read_images(const float *src, float *dst, uint64_t n, int sms, cudaStream_t s);
 // gradient tables of layers l0 .. l0 + s_ - 1 of each image (image k's layer l
 // at gauss + k * img_stride + l * w * h); grad: [img][s_][h][w]
 void launch_grad(const float *gauss, float2 *grad, int w, int h, int s_, uint64_t img_stride, int l0, int nimg,
                  cudaStream_t s);
 void launch_extrema(const ExtremaArgs &a, int nimg, cudaStream_t s);
-void launch_candidate_sigma(FeatCand *cands, uint32_t n, float sigma0, float kstep, cudaStream_t s);
-void launch_orient(const OrientArgs &a, uint32_t n, cudaStream_t s);
+void launch_candidate_sigma(FeatCand *cands, const uint32_t *count, uint32_t cap, float sigma0, float kstep, int sms,
+                            cudaStream_t s);
+void launch_orient(const OrientArgs &a, int sms, cudaStream_t s);
 constexpr int kDescWarpSide = 127;  // window rows one warp takes
 // The window rows from which a feature gets a CTA instead of a warp: those a
 // warp cannot take, or, with fewer features than four warps for each of the
