@@ -9,22 +9,24 @@
 // to the distance in lane order. Every operation is an explicit _rn IEEE op
 // (no FMA contraction), so each d(i, j) equals the reference's f32 value.
 //
-// Kernel. A persistent CTA (256 threads, one per SM) takes work items (a
-// 128-row tile of a against a range of 128-column tiles of b) from a global
-// counter. The a tile is bulk-copied (TMA) into shared memory once per item;
-// b tiles stream through a two-slot TMA/mbarrier ring. Each thread owns an
-// 8 x 8 register block of distances (rows ty*4+{0..3}, 64+ty*4+{0..3};
-// columns tx*4+{0..3}, 64+tx*4+{0..3}).
+// Kernel. A persistent CTA (eight computing warps and one that loads, one CTA per
+// SM) takes work items (a 128-row tile of a against a range of 128-column tiles
+// of b) from a global counter. The a tile is bulk-copied (TMA) into shared memory
+// once per item; b tiles stream in halves through a four-slot TMA/mbarrier ring.
+// Each thread owns an 8 x 8 register block of distances: two neighbouring rows
+// and columns in each group of 32 (row_of, col_of).
 //   rows:    best / second-best / argmin are carried in registers across the
 //            b tiles and merged across the 16 column threads at the end of
 //            the item with warp shuffles (order-independent: min, lowest j on
 //            ties, second smallest of the multiset).
-//   columns: (bits(d) << 32 | i) keys are min-reduced in the warp, then in
-//            shared memory, then with one global atomicMin per column and
-//            tile; unsigned order of the key is (d, lowest i) because d >= +0.
+//   columns: (bits(d) << 32 | i) keys are min-reduced in the warp, then with one
+//            global atomicMin per column, warp and tile; unsigned order of the
+//            key is (d, lowest i) because d >= +0.
 // The finalize kernel merges row partials, applies the ratio test
 // (d1 < (r*r)*d2 in f32) and the mutual check, and compacts in ascending i.
 #include <cuda_runtime.h>
+
+#include <type_traits>
 
 #include "pack.cuh"
 #include "ptx.cuh"
@@ -100,15 +102,24 @@ void launch_fill_u64(unsigned long long *p, uint64_t n, unsigned long long v, cu
 
 // ----------------------------------------------------------- exact match
 
-constexpr int kThreads = 256;
-constexpr uint32_t kTileBytes = kTileFloats * 4;
+constexpr int kWarps = 8;                        // each 16 of a tile's rows against its 128 columns
+constexpr int kThreads = 32 * (kWarps + 4);      // and a group of four, of which one loads
+// Registers a thread: 168 at launch (504 a lane for the three warps of a
+// scheduler), the loading group's given to the two computing warps: 40 + 2 x 232.
+constexpr int kLoadRegs = 40, kComputeRegs = 232;
+static_assert(kLoadRegs + 2 * kComputeRegs <= 3 * 168 && 3 * 168 * 32 <= 16384, "registers of a scheduler");
+constexpr int kRing = 4;                         // halves of b tiles in flight
+constexpr uint32_t kHalfFloats = kTileFloats / 2;  // 64 of the 128 dimensions
+constexpr uint32_t kHalfBytes = kHalfFloats * 4;
+constexpr int kUnroll = 5;
+constexpr uint32_t kNoItem = 0xffffffffu;
 
 struct ExactSmem {
-    float A[kTileFloats];
-    float B[2][kTileFloats];
-    unsigned long long colred[2][kTile];
-    uint64_t barA, barB[2];
-    uint32_t item;
+    float A[2][kHalfFloats];
+    float B[kRing][kHalfFloats];
+    uint64_t fullA[2], emptyA[2], fullB[kRing], emptyB[kRing];
+    Item item[2];
+    PairMeta pm[2];
 };
 
 typedef unsigned long long u64;
@@ -141,259 +152,332 @@ SLM_DEV u64 f2_pack(float lo, float hi) {
 SLM_DEV float f2_lo(u64 v) { return __uint_as_float(static_cast<uint32_t>(v)); }
 SLM_DEV float f2_hi(u64 v) { return __uint_as_float(static_cast<uint32_t>(v >> 32)); }
 
-// 8 x 8 block of spec-order distances between the thread's rows of A and
-// columns of B (both tiles in [slot][row] layout).
-template <bool X2>
-SLM_DEV void tile_distances(const float *__restrict__ sa, const float *__restrict__ sb, int ty, int tx,
-                            u64 zero2, float (&d)[8][8]) {
-    if constexpr (!X2) {
-        float s[8][8];
-#pragma unroll
-        for (int r = 0; r < 8; ++r)
-#pragma unroll
-            for (int c = 0; c < 8; ++c) s[r][c] = 0.0f;
+// A thread's rows and columns of a tile: two neighbours in each 32 (group q).
+SLM_DEV int row_of(int ty, int r) { return 32 * (r >> 1) + 2 * ty + (r & 1); }
+SLM_DEV int col_of(int tx, int c) { return 32 * (c >> 1) + 2 * tx + (c & 1); }
+
+// Half of the spec-order distances' sums between the thread's rows and columns
+// (tile halves in [slot][row] layout), in the first NR row and NC column groups:
+// lanes 0..3 or 4..7 of the reference's eight partial sums, added to s in order.
+template <bool X2, int NR, int NC>
+SLM_DEV void half_distances(const float *sa, const float *sb, int ty, int tx, u64 zero2, u64 (&s)[8][4]) {
 #pragma unroll 1
-        for (int lane = 0; lane < 8; ++lane) {
-            float acc[8][8];
-            const float *pa = sa + lane * 16 * kTile;
-            const float *pb = sb + lane * 16 * kTile;
+    for (int lane = 0; lane < 4; ++lane) {
+        u64 acc[8][4];
+        const float *pa = sa + lane * 16 * kTile + 2 * ty;
+        const float *pb = sb + lane * 16 * kTile + 2 * tx;
+        const auto step = [&](auto first) {
+            float av[2 * NR];
+            u64 bv[NC];
 #pragma unroll
-            for (int c16 = 0; c16 < 16; ++c16) {
-                const float4 a0 = *reinterpret_cast<const float4 *>(pa + c16 * kTile + ty * 4);
-                const float4 a1 = *reinterpret_cast<const float4 *>(pa + c16 * kTile + 64 + ty * 4);
-                const float4 b0 = *reinterpret_cast<const float4 *>(pb + c16 * kTile + tx * 4);
-                const float4 b1 = *reinterpret_cast<const float4 *>(pb + c16 * kTile + 64 + tx * 4);
-                const float av[8] = {a0.x, a0.y, a0.z, a0.w, a1.x, a1.y, a1.z, a1.w};
-                const float bv[8] = {b0.x, b0.y, b0.z, b0.w, b1.x, b1.y, b1.z, b1.w};
-#pragma unroll
-                for (int r = 0; r < 8; ++r)
-#pragma unroll
-                    for (int c = 0; c < 8; ++c) {
-                        const float t = __fsub_rn(av[r], bv[c]);
-                        const float tt = __fmul_rn(t, t);
-                        acc[r][c] = (c16 == 0) ? tt : __fadd_rn(acc[r][c], tt);
-                    }
+            for (int q = 0; q < NR; ++q) {
+                const float2 v = *reinterpret_cast<const float2 *>(pa + 32 * q);
+                av[2 * q] = v.x;
+                av[2 * q + 1] = v.y;
             }
 #pragma unroll
-            for (int r = 0; r < 8; ++r)
+            for (int q = 0; q < NC; ++q) bv[q] = *reinterpret_cast<const u64 *>(pb + 32 * q);
+            pa += kTile;
+            pb += kTile;
 #pragma unroll
-                for (int c = 0; c < 8; ++c) s[r][c] = __fadd_rn(s[r][c], acc[r][c]);
-        }
-#pragma unroll
-        for (int r = 0; r < 8; ++r)
-#pragma unroll
-            for (int c = 0; c < 8; ++c) d[r][c] = s[r][c];
-    } else {
-        // Packed pairs of columns (c, c+1): {a_r, a_r} - {b_c, b_c+1}. A packed
-        // multiply followed by a packed add is contracted to a packed FMA by the
-        // code generator (measured: 25 % of distances off by an ulp). The square
-        // is therefore a packed FMA t * t + z with z a run-time zero (a kernel
-        // argument the compiler cannot fold): rounded once, it is exactly
-        // RN(t * t) (t * t >= 0, + 0 changes nothing), and no contraction with
-        // the following add is possible.
-        u64 s[8][4];
-#pragma unroll
-        for (int r = 0; r < 8; ++r)
-#pragma unroll
-            for (int c = 0; c < 4; ++c) s[r][c] = 0ull;
-#pragma unroll 1
-        for (int lane = 0; lane < 8; ++lane) {
-            u64 acc[8][4];
-            const float *pa = sa + lane * 16 * kTile;
-            const float *pb = sb + lane * 16 * kTile;
-#pragma unroll
-            for (int c16 = 0; c16 < 16; ++c16) {
-                const float4 a0 = *reinterpret_cast<const float4 *>(pa + c16 * kTile + ty * 4);
-                const float4 a1 = *reinterpret_cast<const float4 *>(pa + c16 * kTile + 64 + ty * 4);
-                const ulonglong2 b0 = *reinterpret_cast<const ulonglong2 *>(pb + c16 * kTile + tx * 4);
-                const ulonglong2 b1 = *reinterpret_cast<const ulonglong2 *>(pb + c16 * kTile + 64 + tx * 4);
-                const float av[8] = {a0.x, a0.y, a0.z, a0.w, a1.x, a1.y, a1.z, a1.w};
-                const u64 bv[4] = {b0.x, b0.y, b1.x, b1.y};
-#pragma unroll
-                for (int r = 0; r < 8; ++r) {
+            for (int r = 0; r < 2 * NR; ++r) {
+                if constexpr (X2) {
+                    // Packed pairs of columns: {a_r, a_r} - {b_c, b_c+1}. A packed
+                    // multiply followed by a packed add is contracted to a packed FMA by
+                    // the code generator (measured: 25 % of distances off by an ulp). The
+                    // square is therefore a packed FMA t * t + z with z a run-time zero (a
+                    // kernel argument the compiler cannot fold): rounded once, it is
+                    // exactly RN(t * t) (t * t >= 0, + 0 changes nothing), and no
+                    // contraction with the following add is possible.
                     const u64 ar = f2_pack(av[r], av[r]);
 #pragma unroll
-                    for (int c = 0; c < 4; ++c) {
+                    for (int c = 0; c < NC; ++c) {
                         const u64 t = f2_sub(ar, bv[c]);
                         const u64 tt = f2_fma(t, t, zero2);
-                        acc[r][c] = (c16 == 0) ? tt : f2_add(acc[r][c], tt);
+                        acc[r][c] = decltype(first)::value ? tt : f2_add(acc[r][c], tt);
+                    }
+                } else {
+#pragma unroll
+                    for (int c = 0; c < NC; ++c) {
+                        const float t0 = __fsub_rn(av[r], f2_lo(bv[c])), t1 = __fsub_rn(av[r], f2_hi(bv[c]));
+                        const float q0 = __fmul_rn(t0, t0), q1 = __fmul_rn(t1, t1);
+                        acc[r][c] = decltype(first)::value
+                                        ? f2_pack(q0, q1)
+                                        : f2_pack(__fadd_rn(f2_lo(acc[r][c]), q0), __fadd_rn(f2_hi(acc[r][c]), q1));
                     }
                 }
             }
+        };
+        step(std::true_type{});
+        // (all 15 unrolled, the code of warps out of step outgrows the instruction
+        // caches: 13.2 ms for the 60 views below; 3 at a time 11.1, 5 at a time 11.0)
+#pragma unroll kUnroll
+        for (int c16 = 1; c16 < 16; ++c16) step(std::false_type{});
 #pragma unroll
-            for (int r = 0; r < 8; ++r)
+        for (int r = 0; r < 2 * NR; ++r)
 #pragma unroll
-                for (int c = 0; c < 4; ++c) s[r][c] = f2_add(s[r][c], acc[r][c]);
-        }
-#pragma unroll
-        for (int r = 0; r < 8; ++r)
-#pragma unroll
-            for (int c = 0; c < 4; ++c) {
-                d[r][2 * c] = f2_lo(s[r][c]);
-                d[r][2 * c + 1] = f2_hi(s[r][c]);
-            }
+            for (int c = 0; c < NC; ++c)
+                s[r][c] = X2 ? f2_add(s[r][c], acc[r][c])
+                             : f2_pack(__fadd_rn(f2_lo(s[r][c]), f2_lo(acc[r][c])),
+                                       __fadd_rn(f2_hi(s[r][c]), f2_hi(acc[r][c])));
     }
 }
 
-SLM_DEV int row_of(int ty, int r) { return r < 4 ? ty * 4 + r : 64 + ty * 4 + (r - 4); }
-SLM_DEV int col_of(int tx, int c) { return c < 4 ? tx * 4 + c : 64 + tx * 4 + (c - 4); }
+// What a consumer warp carries through an item.
+struct ExactWarp {
+    const ExactArgs &g;
+    ExactSmem &S;
+    int tx, ty, lane;
+    u64 zero2;
+    uint32_t seq;  // halves of b tiles consumed: ring slot and parity
+    uint32_t a1;   // second halves of a tiles consumed
+    float d1[8], d2[8];
+    uint32_t j1[8];
+};
 
+// One b tile: its distances in two halves, then ratio_match's row update and the
+// column minima. CHECK: the tile's last row and column groups are not whole.
+// False when a bounded wait gave up.
+template <bool X2, int NR, int NC, bool CHECK>
+SLM_DEV bool exact_tile(ExactWarp &w, const PairMeta &pm, uint32_t row0, uint32_t col0, bool first, bool last) {
+    ExactSmem &S = w.S;
+    u64 s[8][4];
+#pragma unroll
+    for (int r = 0; r < 2 * NR; ++r)
+#pragma unroll
+        for (int c = 0; c < NC; ++c) s[r][c] = 0ull;
+#pragma unroll 1
+    for (int h = 0; h < 2; ++h, ++w.seq) {
+        const uint32_t slot = w.seq % kRing;
+        // (the item's first half was waited for before the item was read)
+        bool ok = !first || h == 0 || mbar_wait(&S.fullA[1], w.a1 & 1, w.g.err);
+        ok = ok && mbar_wait(&S.fullB[slot], (w.seq / kRing) & 1, w.g.err);
+        if (!__all_sync(0xffffffffu, ok)) return false;
+        half_distances<X2, NR, NC>(S.A[h], S.B[slot], w.ty, w.tx, w.zero2, s);
+        __syncwarp();
+        if (w.lane == 0) {
+            mbar_arrive(&S.emptyB[slot]);
+            if (last) mbar_arrive(&S.emptyA[h]);
+        }
+    }
+    float d[2 * NR][2 * NC];
+#pragma unroll
+    for (int r = 0; r < 2 * NR; ++r)
+#pragma unroll
+        for (int c = 0; c < NC; ++c) {
+            d[r][2 * c] = f2_lo(s[r][c]);
+            d[r][2 * c + 1] = f2_hi(s[r][c]);
+        }
+    // rows: ratio_match's update (matching.rs:182-187), columns in increasing j;
+    // a NaN changes nothing (fminf takes the other operand)
+#pragma unroll
+    for (int c = 0; c < 2 * NC; ++c) {
+        const uint32_t j = col0 + col_of(w.tx, c);
+        if (CHECK && c >= 2 * NC - 2 && j >= pm.nb) break;
+#pragma unroll
+        for (int r = 0; r < 2 * NR; ++r) {
+            const float v = d[r][c];
+            const bool less = v < w.d1[r];
+            const float other = fminf(w.d2[r], v);
+            w.d2[r] = less ? w.d1[r] : other;
+            w.d1[r] = fminf(w.d1[r], v);
+            w.j1[r] = less ? j : w.j1[r];
+        }
+    }
+    // columns: (d, lowest i) (matching.rs:188-190, 196-203). Only finite minima
+    // matter: a row's best column always holds one.
+    if (w.g.mutual) {
+        u64 key[2 * NC];
+#pragma unroll
+        for (int c = 0; c < 2 * NC; ++c) {
+            float best = __int_as_float(0x7f800000);
+            uint32_t at = 0xffffffffu;
+#pragma unroll
+            for (int r = 0; r < 2 * NR; ++r) {
+                const uint32_t i = row0 + row_of(w.ty, r);
+                if (d[r][c] < best && !(CHECK && r >= 2 * NR - 2 && i >= pm.na)) {
+                    best = d[r][c];
+                    at = i;
+                }
+            }
+            key[c] = (u64)__float_as_uint(best) << 32 | at;
+            const u64 o = __shfl_xor_sync(0xffffffffu, key[c], 16);
+            key[c] = o < key[c] ? o : key[c];
+        }
+        // the even columns by one half warp, the odd ones by the other
+#pragma unroll
+        for (int c = 0; c < 2 * NC; c += 2) {
+            const u64 k = w.lane < 16 ? key[c] : key[c + 1];
+            const uint32_t j = col0 + col_of(w.tx, c) + (w.lane >> 4);
+            if ((uint32_t)k != 0xffffffffu && (!CHECK || j < pm.nb)) atomicMin(&w.g.colbest[pm.col_base + j], k);
+        }
+    }
+    return true;
+}
+
+template <bool X2, int NR>
+SLM_DEV bool exact_edge(uint32_t nc, ExactWarp &w, const PairMeta &pm, uint32_t row0, uint32_t col0, bool first,
+                        bool last) {
+    switch (nc) {
+        case 1: return exact_tile<X2, NR, 1, true>(w, pm, row0, col0, first, last);
+        case 2: return exact_tile<X2, NR, 2, true>(w, pm, row0, col0, first, last);
+        case 3: return exact_tile<X2, NR, 3, true>(w, pm, row0, col0, first, last);
+        default: return exact_tile<X2, NR, 4, true>(w, pm, row0, col0, first, last);
+    }
+}
+
+// Persistent: a warp that loads and eight that compute, which meet only at the
+// tiles' mbarriers. Bound by the FP32 pipe (three operations per dimension and
+// distance, a packed one every other clock): the row and column updates are ALU
+// work, and a warp's run behind the others' distances as long as no barrier ties
+// the warps together, so the halves of the tiles are released one by one, a ring
+// of four holds the next, and column minima go straight to the pair's (a shared
+// reduction needed a barrier a tile). Views are rarely whole tiles: the last row
+// and column tile of a pair compute only the groups of 32 that hold any.
+// 60 views' pairs of about 1150 x 1150 rows: 12.6 ms with a barrier a tile and
+// whole tiles (77 % of the pipe counting real distances), now 11.0 (90 %); one pair
+// of 317 x 300 rows 57.5 us before, now 54.5.
 template <bool X2>
 __global__ void __launch_bounds__(kThreads, 1) exact_kernel(ExactArgs g) {
-    grid_wait();
     extern __shared__ __align__(1024) unsigned char smem_raw[];
     ExactSmem &S = *reinterpret_cast<ExactSmem *>(smem_raw);
-    const int tid = threadIdx.x;
-    const int tx = tid & 15, ty = tid >> 4;
-    const int lane = tid & 31;
-
+    const int tid = threadIdx.x, lane = tid & 31, warp = tid >> 5;
     if (tid == 0) {
-        mbar_init(&S.barA, 1);
-        mbar_init(&S.barB[0], 1);
-        mbar_init(&S.barB[1], 1);
+        for (int h = 0; h < 2; ++h) {
+            mbar_init(&S.fullA[h], 1);
+            mbar_init(&S.emptyA[h], kWarps);
+        }
+        for (int q = 0; q < kRing; ++q) {
+            mbar_init(&S.fullB[q], 1);
+            mbar_init(&S.emptyB[q], kWarps);
+        }
         fence_mbar_init();
     }
-    for (int c = tid; c < 2 * kTile; c += kThreads) (&S.colred[0][0])[c] = ~0ull;
     __syncthreads();
+    grid_wait();
     // Items planned on the device (pairs routed from the shortlist path) come
     // with their count in device memory, written by an earlier kernel.
     const uint32_t n_items = g.n_items_dev ? min(*g.n_items_dev, g.n_items) : g.n_items;
-    const u64 zero2 = f2_pack(g.zero, g.zero);
-
-    uint32_t a_phase = 0;
-    uint32_t seq = 0;  // b tiles consumed by this CTA (selects ring slot and parity)
-    bool ok = true;    // CTA-uniform: every barrier below reduces it with AND
-    for (;;) {
-        if (tid == 0) S.item = atomicAdd(g.work, 1u);
-        ok = __syncthreads_and(ok);
-        const uint32_t it = S.item;
-        if (it >= n_items || !ok) break;
-        const Item item = g.items[it];
-        const PairMeta pm = g.pairs[item.pair];
-        const float *atile = g.tiled + (size_t)(pm.a_row0 / kTile + item.rt) * kTileFloats;
-        const float *bbase = g.tiled + (size_t)(pm.b_row0 / kTile) * kTileFloats;
-        const int ntiles = (int)item.ct1 - (int)item.ct0;
-        if (tid == 0) {
-            mbar_arrive_expect_tx(&S.barA, kTileBytes);
-            bulk_g2s(S.A, atile, kTileBytes, &S.barA);
-            if (ntiles > 0) {
-                const uint32_t slot = seq & 1;
-                mbar_arrive_expect_tx(&S.barB[slot], kTileBytes);
-                bulk_g2s(S.B[slot], bbase + (size_t)item.ct0 * kTileFloats, kTileBytes, &S.barB[slot]);
-            }
-        }
-        uint32_t irow[8];
-        bool rvalid[8];
-#pragma unroll
-        for (int r = 0; r < 8; ++r) {
-            irow[r] = item.rt * kTile + row_of(ty, r);
-            rvalid[r] = irow[r] < pm.na;
-        }
-        float d1[8], d2[8];
-        uint32_t j1[8];
-#pragma unroll
-        for (int r = 0; r < 8; ++r) {
-            d1[r] = __int_as_float(0x7f800000);
-            d2[r] = __int_as_float(0x7f800000);
-            j1[r] = 0xffffffffu;
-        }
-        bool mine = mbar_wait(&S.barA, a_phase, g.err);
-        a_phase ^= 1;
-
-        for (int t = 0; t < ntiles; ++t) {
-            const uint32_t slot = seq & 1, parity = (seq >> 1) & 1;
-            const uint32_t ct = item.ct0 + t;
-            if (tid == 0 && t + 1 < ntiles) {
-                mbar_arrive_expect_tx(&S.barB[slot ^ 1], kTileBytes);
-                bulk_g2s(S.B[slot ^ 1], bbase + (size_t)(ct + 1) * kTileFloats, kTileBytes, &S.barB[slot ^ 1]);
-            }
-            mine = mine && mbar_wait(&S.barB[slot], parity, g.err);
-            const uint32_t cb = seq & 1;
-            if (mine) {
-                float d[8][8];
-                tile_distances<X2>(S.A, S.B[slot], ty, tx, zero2, d);
-
-                uint32_t jc[8];
-                bool cvalid[8];
-#pragma unroll
-                for (int c = 0; c < 8; ++c) {
-                    jc[c] = ct * kTile + col_of(tx, c);
-                    cvalid[c] = jc[c] < pm.nb;
+    if (warp >= kWarps) {
+        asm volatile("setmaxnreg.dec.sync.aligned.u32 %0;" ::"n"(kLoadRegs));
+        if (tid == 32 * kWarps) {
+            uint32_t k = 0, seq = 0, a0 = 0, a1 = 0;  // items; halves of b and of a tiles loaded so far
+            bool ok = true;
+            for (;; ++k) {
+                const uint32_t it = atomicAdd(g.work, 1u);
+                // every warp is done with the a tile's first half, so with the item before its own
+                ok = k == 0 || mbar_wait(&S.emptyA[0], (k - 1) & 1, g.err);
+                if (!ok) break;
+                if (it >= n_items) {
+                    S.item[k & 1].pair = kNoItem;
+                    mbar_arrive(&S.fullA[0]);
+                    break;
                 }
-                // rows: ratio_match's update (matching.rs:182-187), columns in increasing j.
-#pragma unroll
-                for (int r = 0; r < 8; ++r)
-#pragma unroll
-                    for (int c = 0; c < 8; ++c) {
-                        const float v = d[r][c];
-                        if (cvalid[c]) {
-                            if (v < d1[r]) {
-                                d2[r] = d1[r];
-                                d1[r] = v;
-                                j1[r] = jc[c];
-                            } else if (v < d2[r]) {
-                                d2[r] = v;
-                            }
+                const Item item = g.items[it];
+                const PairMeta pm = g.pairs[item.pair];
+                S.item[k & 1] = item;
+                S.pm[k & 1] = pm;
+                const float *at = g.tiled + (size_t)(pm.a_row0 / kTile + item.rt) * kTileFloats;
+                const float *bt = g.tiled + (size_t)(pm.b_row0 / kTile + item.ct0) * kTileFloats;
+                const uint32_t nh = 2 * (item.ct1 - item.ct0);
+                mbar_arrive_expect_tx(&S.fullA[0], kHalfBytes);
+                bulk_g2s(S.A[0], at, kHalfBytes, &S.fullA[0]);
+                ++a0;
+                for (uint32_t q = 0; q < nh && ok; ++q, ++seq) {
+                    const uint32_t slot = seq % kRing, use = seq / kRing;
+                    ok = use == 0 || mbar_wait(&S.emptyB[slot], (use - 1) & 1, g.err);
+                    if (!ok) break;
+                    mbar_arrive_expect_tx(&S.fullB[slot], kHalfBytes);
+                    bulk_g2s(S.B[slot], bt + (size_t)q * kHalfFloats, kHalfBytes, &S.fullB[slot]);
+                    if (q == 0) {
+                        ok = a1 == 0 || mbar_wait(&S.emptyA[1], (a1 - 1) & 1, g.err);
+                        if (!ok) {
+                            ++seq;
+                            break;
                         }
-                    }
-                // columns: (d, lowest i) (matching.rs:188-190, 196-203).
-                if (g.mutual) {
-#pragma unroll
-                    for (int c = 0; c < 8; ++c) {
-                        u64 key = ~0ull;
-#pragma unroll
-                        for (int r = 0; r < 8; ++r) {
-                            const u64 k = ((u64)__float_as_uint(d[r][c]) << 32) | irow[r];
-                            if (rvalid[r] && k < key) key = k;
-                        }
-                        const u64 o = __shfl_xor_sync(0xffffffffu, key, 16);
-                        key = o < key ? o : key;
-                        if (lane < 16 && key != ~0ull) atomicMin(&S.colred[cb][col_of(tx, c)], key);
+                        mbar_arrive_expect_tx(&S.fullA[1], kHalfBytes);
+                        bulk_g2s(S.A[1], at + kHalfFloats, kHalfBytes, &S.fullA[1]);
+                        ++a1;
                     }
                 }
+                if (!ok) break;
             }
-            ok = __syncthreads_and(mine);
-            if (!ok) break;
-            if (g.mutual && tid < kTile) {
-                const u64 v = S.colred[cb][tid];
-                const uint32_t j = ct * kTile + tid;
-                if (v != ~0ull && j < pm.nb) atomicMin(&g.colbest[pm.col_base + j], v);
-                S.colred[cb][tid] = ~0ull;
+            if (!ok) {  // a wait gave up: no copy may be in flight when the CTA ends
+                if (a0) mbar_wait(&S.fullA[0], (a0 - 1) & 1, g.err);
+                if (a1) mbar_wait(&S.fullA[1], (a1 - 1) & 1, g.err);
+                for (uint32_t q = 0; q < kRing; ++q)
+                    if (seq > q) mbar_wait(&S.fullB[q], ((seq - 1 - q) / kRing) & 1, g.err);
             }
-            ++seq;
         }
-        // End of item: every thread is done with S.item and the a tile before
-        // thread 0 fetches the next item (also when the item had no b tiles).
-        ok = __syncthreads_and(ok && mine);
+        __syncwarp();
+        __syncthreads();
+        return;
+    }
+    asm volatile("setmaxnreg.inc.sync.aligned.u32 %0;" ::"n"(kComputeRegs));
+    ExactWarp w{g, S, lane & 15, tid >> 4, lane, f2_pack(g.zero, g.zero), 0u, 0u, {}, {}, {}};
+    for (uint32_t k = 0;; ++k) {
+        if (!__all_sync(0xffffffffu, mbar_wait(&S.fullA[0], k & 1, g.err))) break;
+        const Item item = S.item[k & 1];
+        if (item.pair == kNoItem) break;
+        const PairMeta pm = S.pm[k & 1];
+#pragma unroll
+        for (int r = 0; r < 8; ++r) {
+            w.d1[r] = __int_as_float(0x7f800000);
+            w.d2[r] = __int_as_float(0x7f800000);
+            w.j1[r] = 0xffffffffu;
+        }
+        const uint32_t row0 = item.rt * kTile, nr = min((pm.na - row0 + 31) / 32, 4u);
+        bool ok = true;
+        for (uint32_t ct = item.ct0; ct < item.ct1 && ok; ++ct) {
+            const uint32_t col0 = ct * kTile, nc = min((pm.nb - col0 + 31) / 32, 4u);
+            const bool first = ct == item.ct0, last = ct + 1 == item.ct1;
+            if (row0 + kTile <= pm.na && col0 + kTile <= pm.nb)
+                ok = exact_tile<X2, 4, 4, false>(w, pm, row0, col0, first, last);
+            else if (nr == 1)
+                ok = exact_edge<X2, 1>(nc, w, pm, row0, col0, first, last);
+            else if (nr == 2)
+                ok = exact_edge<X2, 2>(nc, w, pm, row0, col0, first, last);
+            else if (nr == 3)
+                ok = exact_edge<X2, 3>(nc, w, pm, row0, col0, first, last);
+            else
+                ok = exact_edge<X2, 4>(nc, w, pm, row0, col0, first, last);
+        }
         if (!ok) break;
+        if (item.ct0 < item.ct1) {
+            ++w.a1;
+        } else {  // no b tiles, and no second half of the a tile was loaded
+            __syncwarp();
+            if (lane == 0) mbar_arrive(&S.emptyA[0]);
+        }
         // Merge row states across the 16 column threads (lanes xor 1..8).
 #pragma unroll
         for (int r = 0; r < 8; ++r) {
 #pragma unroll
             for (int off = 1; off < 16; off <<= 1) {
-                const float o1 = __shfl_xor_sync(0xffffffffu, d1[r], off);
-                const float o2 = __shfl_xor_sync(0xffffffffu, d2[r], off);
-                const uint32_t oj = __shfl_xor_sync(0xffffffffu, j1[r], off);
-                const float nd2 = fminf(fmaxf(d1[r], o1), fminf(d2[r], o2));
-                if (o1 < d1[r] || (o1 == d1[r] && oj < j1[r])) {
-                    d1[r] = o1;
-                    j1[r] = oj;
+                const float o1 = __shfl_xor_sync(0xffffffffu, w.d1[r], off);
+                const float o2 = __shfl_xor_sync(0xffffffffu, w.d2[r], off);
+                const uint32_t oj = __shfl_xor_sync(0xffffffffu, w.j1[r], off);
+                const float nd2 = fminf(fmaxf(w.d1[r], o1), fminf(w.d2[r], o2));
+                if (o1 < w.d1[r] || (o1 == w.d1[r] && oj < w.j1[r])) {
+                    w.d1[r] = o1;
+                    w.j1[r] = oj;
                 }
-                d2[r] = nd2;
+                w.d2[r] = nd2;
             }
         }
-        if (tx == 0) {
+        if (w.tx == 0) {
 #pragma unroll
             for (int r = 0; r < 8; ++r) {
                 RowPart p;
-                p.d1 = d1[r];
-                p.d2 = d2[r];
-                p.j1 = j1[r];
+                p.d1 = w.d1[r];
+                p.d2 = w.d2[r];
+                p.j1 = w.j1[r];
                 p.pad = 0;
-                g.parts[(size_t)item.part * kTile + row_of(ty, r)] = p;
+                g.parts[(size_t)item.part * kTile + row_of(w.ty, r)] = p;
             }
         }
     }
+    __syncthreads();
 }
 
 cudaError_t init_exact_kernels() {
