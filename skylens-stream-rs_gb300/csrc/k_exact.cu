@@ -10,8 +10,8 @@
 // (no FMA contraction), so each d(i, j) equals the reference's f32 value.
 //
 // Kernel. A persistent CTA (eight computing warps and one that loads, one CTA per
-// SM) takes work items (a 128-row tile of a against a range of 128-column tiles
-// of b) from a global counter. The a tile is bulk-copied (TMA) into shared memory
+// SM) takes work items (a 128-row tile of a, or some of its groups of 32 rows,
+// against a range of b's groups of 32 columns) from a global counter. The a tile is bulk-copied (TMA) into shared memory
 // once per item; b tiles stream in halves through a four-slot TMA/mbarrier ring.
 // Each thread owns an 8 x 8 register block of distances: two neighbouring rows
 // and columns in each group of 32 (row_of, col_of).
@@ -253,7 +253,7 @@ SLM_DEV bool exact_tile(ExactWarp &w, const PairMeta &pm, uint32_t row0, uint32_
         bool ok = !first || h == 0 || mbar_wait(&S.fullA[1], w.a1 & 1, w.g.err);
         ok = ok && mbar_wait(&S.fullB[slot], (w.seq / kRing) & 1, w.g.err);
         if (!__all_sync(0xffffffffu, ok)) return false;
-        half_distances<X2, NR, NC>(S.A[h], S.B[slot], w.ty, w.tx, w.zero2, s);
+        half_distances<X2, NR, NC>(S.A[h] + row0 % kTile, S.B[slot] + col0 % kTile, w.ty, w.tx, w.zero2, s);
         __syncwarp();
         if (w.lane == 0) {
             mbar_arrive(&S.emptyB[slot]);
@@ -378,8 +378,8 @@ __global__ void __launch_bounds__(kThreads, 1) exact_kernel(ExactArgs g) {
                 S.item[k & 1] = item;
                 S.pm[k & 1] = pm;
                 const float *at = g.tiled + (size_t)(pm.a_row0 / kTile + item.rt) * kTileFloats;
-                const float *bt = g.tiled + (size_t)(pm.b_row0 / kTile + item.ct0) * kTileFloats;
-                const uint32_t nh = 2 * (item.ct1 - item.ct0);
+                const float *bt = g.tiled + (size_t)(pm.b_row0 / kTile + item.q0 / 4) * kTileFloats;
+                const uint32_t nh = item.q0 < item.q1 ? 2 * ((item.q1 + 3) / 4 - item.q0 / 4) : 0;
                 mbar_arrive_expect_tx(&S.fullA[0], kHalfBytes);
                 bulk_g2s(S.A[0], at, kHalfBytes, &S.fullA[0]);
                 ++a0;
@@ -426,12 +426,13 @@ __global__ void __launch_bounds__(kThreads, 1) exact_kernel(ExactArgs g) {
             w.d2[r] = __int_as_float(0x7f800000);
             w.j1[r] = 0xffffffffu;
         }
-        const uint32_t row0 = item.rt * kTile, nr = min((pm.na - row0 + 31) / 32, 4u);
+        const uint32_t row0 = item.rt * kTile + 32 * item.g0, nr = min((pm.na - row0 + 31) / 32, item.g1 - item.g0);
         bool ok = true;
-        for (uint32_t ct = item.ct0; ct < item.ct1 && ok; ++ct) {
-            const uint32_t col0 = ct * kTile, nc = min((pm.nb - col0 + 31) / 32, 4u);
-            const bool first = ct == item.ct0, last = ct + 1 == item.ct1;
-            if (row0 + kTile <= pm.na && col0 + kTile <= pm.nb)
+        for (uint32_t q = item.q0, end; q < item.q1 && ok; q = end) {
+            end = min(q / 4 * 4 + 4, item.q1);  // of this tile's groups
+            const uint32_t col0 = 32 * q, nc = end - q;
+            const bool first = q == item.q0, last = end == item.q1;
+            if (nr == 4 && nc == 4 && row0 + kTile <= pm.na && col0 + kTile <= pm.nb)
                 ok = exact_tile<X2, 4, 4, false>(w, pm, row0, col0, first, last);
             else if (nr == 1)
                 ok = exact_edge<X2, 1>(nc, w, pm, row0, col0, first, last);
@@ -443,7 +444,7 @@ __global__ void __launch_bounds__(kThreads, 1) exact_kernel(ExactArgs g) {
                 ok = exact_edge<X2, 4>(nc, w, pm, row0, col0, first, last);
         }
         if (!ok) break;
-        if (item.ct0 < item.ct1) {
+        if (item.q0 < item.q1) {
             ++w.a1;
         } else {  // no b tiles, and no second half of the a tile was loaded
             __syncwarp();
@@ -468,12 +469,13 @@ __global__ void __launch_bounds__(kThreads, 1) exact_kernel(ExactArgs g) {
         if (w.tx == 0) {
 #pragma unroll
             for (int r = 0; r < 8; ++r) {
+                if ((uint32_t)r / 2 >= nr) break;  // other items' rows, or none
                 RowPart p;
                 p.d1 = w.d1[r];
                 p.d2 = w.d2[r];
                 p.j1 = w.j1[r];
                 p.pad = 0;
-                g.parts[(size_t)item.part * kTile + row_of(w.ty, r)] = p;
+                g.parts[(size_t)item.part * kTile + 32 * item.g0 + row_of(w.ty, r)] = p;
             }
         }
     }

@@ -46,7 +46,7 @@ constexpr size_t align256(size_t x) { return (x + 255) / 256 * 256; }
 // Largest layout (na = nb = kNaMax): the size of the static array.
 constexpr size_t max_layout_bytes() {
     const size_t tiles = kNaMax / kTile;
-    const size_t items = tiles * kChunksMax;
+    const size_t items = tiles * kChunksMax;  // small pairs have more items, of part of a tile, but few tiles
     return align256(sizeof(float) * (size_t)kTileFloats * 2 * tiles) + align256(sizeof(Item) * items) +
            align256(sizeof(RowPart) * kTile * items) + align256(sizeof(PairMeta)) +
            align256(sizeof(unsigned long long) * kNaMax) + align256(sizeof(uint2) * kNaMax) +
@@ -79,16 +79,19 @@ __global__ void __launch_bounds__(256) single_prep_kernel(unsigned char *scratch
         PairMeta *meta = reinterpret_cast<PairMeta *>(scratch + L.meta);
         uint32_t *ctl = reinterpret_cast<uint32_t *>(scratch + L.ctl);
         uint32_t *counts = reinterpret_cast<uint32_t *>(scratch + L.counts);
-        const uint32_t chunks = L.chunks, n_items = L.rt_n * chunks;
-        for (uint32_t k = threadIdx.x; k < n_items; k += blockDim.x) {
-            const uint32_t rt = k / chunks, c = k % chunks;
+        const uint32_t chunks = L.chunks, cols = (nb + 31) / 32;
+        for (uint32_t k = threadIdx.x; k < L.n_items; k += blockDim.x) {
+            const uint32_t r = k / chunks, c = k % chunks, g = r * L.rows;  // row groups from g on
             Item it;
             it.pair = 0;
-            it.rt = rt;
-            it.ct0 = (uint32_t)((uint64_t)L.ct_n * c / chunks);
-            it.ct1 = (uint32_t)((uint64_t)L.ct_n * (c + 1) / chunks);
-            it.part = k;  // = rt * chunks + c, the layout finalize_kernel reads
-            it.pad[0] = it.pad[1] = it.pad[2] = 0;
+            it.rt = g / 4;
+            it.g0 = g % 4;
+            it.g1 = it.g0 + L.rows;
+            it.q0 = L.few ? (uint32_t)((uint64_t)cols * c / chunks) : 4 * (uint32_t)((uint64_t)L.ct_n * c / chunks);
+            it.q1 = L.few ? (uint32_t)((uint64_t)cols * (c + 1) / chunks)
+                          : min(cols, 4 * (uint32_t)((uint64_t)L.ct_n * (c + 1) / chunks));
+            it.part = it.rt * chunks + c;  // the layout finalize_kernel reads
+            it.pad = 0;
             items[k] = it;
         }
         if (threadIdx.x == 0) {
@@ -184,12 +187,19 @@ SingleLayout single_layout(uint32_t na, uint32_t nb, int sms, bool inputs) {
     uint32_t chunks = L.rt_n ? (want + L.rt_n - 1) / L.rt_n : 1;
     chunks = chunks > L.ct_n ? L.ct_n : chunks;
     chunks = chunks > kChunksMax ? kChunksMax : chunks;
+    ExactShapes shapes;
+    shapes.add(na, nb);
+    L.few = shapes.few(sms > 0 ? sms : 1);
+    const ExactShape shape = L.few ? shapes.best(sms > 0 ? sms : 1) : ExactShape{};
+    if (L.few) chunks = ExactShapes::chunks_of(nb, shape.cols);
+    L.rows = shape.rows;
     L.chunks = chunks < 1 ? 1 : chunks;
-    const size_t items = (size_t)L.rt_n * L.chunks;
+    L.n_items = (groups32(na) + L.rows - 1) / L.rows * L.chunks;
+    const size_t parts = (size_t)L.rt_n * L.chunks;
     size_t o = 0;
     L.tiled = o, o += align256(sizeof(float) * (size_t)kTileFloats * (L.rt_n + L.ct_n));
-    L.items = o, o += align256(sizeof(Item) * items);
-    L.parts = o, o += align256(sizeof(RowPart) * kTile * items);
+    L.items = o, o += align256(sizeof(Item) * L.n_items);
+    L.parts = o, o += align256(sizeof(RowPart) * kTile * parts);
     L.meta = o, o += align256(sizeof(PairMeta));
     L.colbest = o, o += align256(sizeof(unsigned long long) * (nb ? nb : 1));
     L.slots = o, o += align256(sizeof(uint2) * (na ? na : 1));
@@ -208,7 +218,7 @@ SingleLayout single_layout(uint32_t na, uint32_t nb, int sms, bool inputs) {
 cudaError_t single_exact_enqueue(unsigned char *sc, const SingleLayout &L, const float *d_a, uint32_t na,
                                  const float *d_b, uint32_t nb, float ratio, int mutual, slm_pair *d_out,
                                  uint32_t cap, uint32_t *d_count, int sms, cudaStream_t s) {
-    const uint32_t n_items = L.rt_n * L.chunks;
+    const uint32_t n_items = L.n_items;
     float *tiled = reinterpret_cast<float *>(sc + L.tiled);
     single_prep_kernel<<<4 * (L.rt_n + L.ct_n), 256, 0, s>>>(sc, L, d_a, na, d_b, nb, mutual);
     ExactArgs a{};

@@ -1252,10 +1252,12 @@ __global__ void __launch_bounds__(256) sl_route_apply_kernel(SlArgs g) {
             Item it;
             it.pair = p;
             it.rt = rt;
-            it.ct0 = (uint32_t)((uint64_t)ct_n * c / chunks);
-            it.ct1 = (uint32_t)((uint64_t)ct_n * (c + 1) / chunks);
+            it.q0 = 4 * (uint32_t)((uint64_t)ct_n * c / chunks);
+            it.q1 = min((pm.nb + 31) / 32, 4 * (uint32_t)((uint64_t)ct_n * (c + 1) / chunks));
             it.part = sp.xpart + t;  // = xpart + rt * chunks + c
-            it.pad[0] = it.pad[1] = it.pad[2] = 0;
+            it.g0 = 0;
+            it.g1 = 4;
+            it.pad = 0;
             if (sp.xpart + t < g.xitem_cap) g.xitems[sp.xpart + t] = it;
         }
         if (g.mutual)

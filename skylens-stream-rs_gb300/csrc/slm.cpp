@@ -368,32 +368,41 @@ void plan_items(slm_plan *p) {
     const uint64_t want = (uint64_t)std::max(1, p->ctx->sms) * (p->tune.items_per_sm ? p->tune.items_per_sm : 4);
     uint32_t split = 1;
     if (row_tiles && row_tiles < want) split = (uint32_t)((want + row_tiles - 1) / row_tiles);
+    ExactShapes shapes;
+    for (uint32_t k = 0; k < p->np; ++k) shapes.add(p->meta[k].na, p->meta[k].nb);
+    const bool few = !p->tune.items_per_sm && shapes.few(std::max(1, p->ctx->sms));
+    const ExactShape shape = few ? shapes.best(std::max(1, p->ctx->sms)) : ExactShape{};
     p->items.clear();
     uint32_t part = 0;
     for (uint32_t k = 0; k < p->np; ++k) {
         PairMeta &m = p->meta[k];
         const uint32_t rt_n = (m.na + kTile - 1) / kTile;
-        const uint32_t ct_n = (m.nb + kTile - 1) / kTile;
-        uint32_t chunks = std::max(1u, std::min(split, ct_n));
+        const uint32_t ct_n = (m.nb + kTile - 1) / kTile, cols = groups32(m.nb);
+        const uint32_t chunks = few ? ExactShapes::chunks_of(m.nb, shape.cols) : std::max(1u, std::min(split, ct_n));
         m.nchunk = chunks;
         m.part_base = part;
         for (uint32_t rt = 0; rt < rt_n; ++rt)
-            for (uint32_t c = 0; c < chunks; ++c) {
-                Item it{};
-                it.pair = k;
-                it.rt = rt;
-                it.ct0 = (uint32_t)((uint64_t)ct_n * c / chunks);
-                it.ct1 = (uint32_t)((uint64_t)ct_n * (c + 1) / chunks);
-                it.part = part + rt * chunks + c;
-                p->items.push_back(it);
-            }
+            for (uint32_t c = 0; c < chunks; ++c)
+                for (uint32_t g = 0; g < 4 && rt * kTile + 32 * g < m.na; g += shape.rows) {
+                    Item it{};
+                    it.pair = k;
+                    it.rt = rt;
+                    // whole tiles but in a batch of few
+                    it.q0 = few ? (uint32_t)((uint64_t)cols * c / chunks) : 4 * (uint32_t)((uint64_t)ct_n * c / chunks);
+                    it.q1 = few ? (uint32_t)((uint64_t)cols * (c + 1) / chunks)
+                                : std::min(cols, 4 * (uint32_t)((uint64_t)ct_n * (c + 1) / chunks));
+                    it.g0 = g;
+                    it.g1 = g + shape.rows;
+                    it.part = part + rt * chunks + c;
+                    p->items.push_back(it);
+                }
         part += rt_n * chunks;
         (void)st;
     }
     p->n_parts = part;
     // Longest items first (cost ~ rows x columns) for the dynamic queue.
     std::stable_sort(p->items.begin(), p->items.end(), [&](const Item &x, const Item &y) {
-        const uint64_t cx = (uint64_t)(x.ct1 - x.ct0), cy = (uint64_t)(y.ct1 - y.ct0);
+        const uint64_t cx = (uint64_t)(x.q1 - x.q0), cy = (uint64_t)(y.q1 - y.q0);
         return cx > cy;
     });
 }

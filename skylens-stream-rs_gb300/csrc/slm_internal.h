@@ -60,12 +60,12 @@ struct PairMeta {
     uint64_t slot_off;        // first output slot (capacity na)
 };
 
-// One unit of the exact kernel: rows [rt*128, rt*128+128) of pair `pair`
-// against store column tiles [ct0, ct1) of b.
+// One unit of the exact kernel: row groups [g0, g1) (of 32 rows, up to four) of
+// the 128-row tile rt of pair `pair` against columns [32 q0, 32 q1) of b.
 struct Item {
-    uint32_t pair, rt, ct0, ct1;
-    uint32_t part;  // RowPart block receiving the result
-    uint32_t pad[3];
+    uint32_t pair, rt, q0, q1;
+    uint32_t part;  // RowPart block receiving the result (items of one tile and other rows share it)
+    uint32_t g0, g1, pad;
 };
 
 struct ExactArgs {
@@ -118,9 +118,52 @@ void set_last_error(const char *msg);
 
 // Scratch layout of one exact FP32 pair match with its metadata made on the
 // device (byte offsets; `inputs` adds room for copies of the row-major inputs).
+constexpr uint32_t kSplitChunksMax = 16;  // finalize merges a row's chunks one after the other
+inline uint32_t groups32(uint32_t n) { return (n + 31) / 32; }
+// The shape of the items of a batch of few tiles (below two a SM): time counts
+// rounds of the SMs, an item about 2.5 us and 1.55 us for each 32 x 32 block it
+// holds, so a small batch gets small items and one of a tile a SM whole tiles.
+// add() every pair, then the shape with the least time. One 317 x 300 pair's call
+// took 54 us with whole tiles, 31 with single blocks; 1000 x 1000 rows 67 (before
+// the kernels were launched early) and 48 (tiles' halves by rows), 1500 x 1500
+// (144 tiles) 73 and 70.
+struct ExactShape {
+    uint32_t rows = 4, cols = 4;
+};
+struct ExactShapes {
+    static constexpr ExactShape kShapes[6] = {{4, 4}, {2, 4}, {1, 4}, {2, 2}, {1, 2}, {1, 1}};
+    uint64_t items[6] = {};
+    uint32_t widest[6] = {};  // groups in the longest run of columns
+    uint64_t tiles = 0;
+    static uint32_t chunks_of(uint32_t nb, uint32_t cols) {
+        const uint32_t n = (groups32(nb) + cols - 1) / cols;
+        return n < 1 ? 1 : n > kSplitChunksMax ? kSplitChunksMax : n;
+    }
+    void add(uint32_t na, uint32_t nb) {
+        tiles += (uint64_t)((na + kTile - 1) / kTile) * ((nb + kTile - 1) / kTile);
+        for (int k = 0; k < 6; ++k) {
+            const uint32_t chunks = chunks_of(nb, kShapes[k].cols), run = (groups32(nb) + chunks - 1) / chunks;
+            items[k] += (uint64_t)((groups32(na) + kShapes[k].rows - 1) / kShapes[k].rows) * chunks;
+            if (run > widest[k]) widest[k] = run;
+        }
+    }
+    bool few(int sms) const { return tiles < 2ull * (uint64_t)sms; }
+    ExactShape best(int sms) const {
+        int at = 0;
+        double least = 0;
+        for (int k = 0; k < 6; ++k) {
+            const double t = (double)((items[k] + sms - 1) / sms) * (2.5 + 1.55 * kShapes[k].rows * widest[k]);
+            if (k == 0 || t < least) least = t, at = k;
+        }
+        return kShapes[at];
+    }
+};
+
 struct SingleLayout {
     size_t tiled, items, parts, meta, colbest, slots, counts, ctl, raw_a, raw_b, bytes;
     uint32_t rt_n, ct_n, chunks;
+    uint32_t rows, n_items;  // row groups of an item
+    bool few;                // items of part of a tile (ExactShapes)
 };
 SingleLayout single_layout(uint32_t na, uint32_t nb, int sms, bool inputs);
 // Whether finalize may write the match list straight into d_out: there must be

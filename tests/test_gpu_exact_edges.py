@@ -59,3 +59,25 @@ def test_rows_that_are_not_finite(matcher, views, n, bad, mutual):
             v[r, rng.integers(0, 128)] = bad
     want = O.ratio_match_np(a, b, 0.8, mutual, threads=16)
     assert np.array_equal(matcher.ratio_match_np(a, b, 0.8, mutual, "fp32"), want)
+
+
+@pytest.mark.parametrize("na,nb", [(31, 33), (64, 96), (129, 255), (257, 700), (700, 257), (1, 1500), (1500, 2),
+                                   (1000, 1000), (1700, 1300)])
+def test_items_of_part_of_a_tile(matcher, na, nb):
+    # few tiles: items of one 32 x 32 block up to a tile, by the call's size; the
+    # pair alone and with others in a plan
+    rng = np.random.Generator(np.random.PCG64(na * 4099 + nb))
+    b = synth.sift_like(rng, nb)
+    k = min(na, nb) // 2
+    a = np.concatenate([synth.noisy_copy(rng, b[rng.permutation(nb)[:k]], 0.05), synth.sift_like(rng, na - k)])
+    want = {m: O.ratio_match_np(a, b, 0.8, m, threads=16) for m in (True, False)}
+    for mutual in (True, False):
+        assert np.array_equal(matcher.ratio_match_np(a, b, 0.8, mutual, "fp32"), want[mutual])
+    st = matcher.store(na + nb + 200, 3)
+    ids = [st.add_view(v) for v in (a, b, synth.sift_like(rng, 70))]
+    plan = st.plan([(ids[0], ids[1]), (ids[2], ids[0]), (ids[0], ids[1])], 0.8, True, "fp32")
+    plan.launch()
+    got = plan.per_pair()
+    assert np.array_equal(got[0], want[True]) and np.array_equal(got[2], want[True])
+    plan.close()
+    st.close()
