@@ -98,9 +98,9 @@ __global__ void fill_u32_kernel(uint32_t *p, uint64_t n, uint32_t v) {
         p[i] = v;
 }
 
-// Rows of many views from one staging buffer into their padded store rows.
+// Rows of many views from one staging buffer into their rows of the store.
 // The table travels as the kernel parameter (no upload):
-// e[v] = {first staging row, first store row, rows, 0}; blockIdx.x = view,
+// e[v] = {first staging row, first row of the store, rows, 0}; blockIdx.x = view,
 // blockIdx.y strides over its rows.
 constexpr uint32_t kScatterMax = 1024;
 struct ScatterTab {
@@ -129,8 +129,8 @@ void launch_scatter_rows(const uint4 *tab, uint32_t n, const float *src, float *
 }
 
 // Rows of many views, each from its own source address (host memory the
-// device can read directly, or device memory), into their padded store rows:
-// e[v] = {source address low, high 32 bits, first store row, rows}.
+// device can read directly, or device memory), into their rows of the store:
+// e[v] = {source address low, high 32 bits, first row of the store, rows}.
 // Each thread issues four 16-byte loads before it stores any of them, so that
 // many loads are in flight: reads of host memory over the chip-to-chip link are
 // bound by their latency.

@@ -36,25 +36,23 @@ namespace slm {
 
 // ------------------------------------------------------------------ pack
 
-// Tile `tile` of the view whose rows start at store row `row0` (n rows): raw
-// rows -> tile[slot][row]. Called by all 256 threads of a CTA alike.
-SLM_DEV void pack_view_tile(const float *__restrict__ raw, float *__restrict__ tiled, uint32_t row0, uint32_t n,
-                            uint32_t tile, float (&sm)[32][kDesc + 1]) {
-    const float *src = raw + (size_t)row0 * kDesc;
+// Tile `tile` of the view whose tiles start at store row `row0` and whose n rows
+// start at raw0: raw rows -> tile[slot][row]. Called by all 256 threads of a CTA alike.
+SLM_DEV void pack_view_tile(const float *__restrict__ raw, float *__restrict__ tiled, uint32_t raw0, uint32_t row0,
+                            uint32_t n, uint32_t tile, float (&sm)[32][kDesc + 1]) {
+    const float *src = raw + (size_t)raw0 * kDesc;
     float *dst = tiled + (size_t)(row0 / kTile + tile) * kTileFloats;
     for (int g = 0; g < 4; ++g) pack_group(src, n, dst, tile, g, sm);
 }
 
 // Many views at once: one CTA per 32-row group (blockIdx.y) of each entry of
-// a tile table {first store row of the view, rows of the view, tile within the
-// view, view}.
+// a tile table {first row-major row, rows from it on, store tile, view}.
 __global__ void __launch_bounds__(256) pack_fp32_tiles_kernel(const uint4 *__restrict__ tab,
                                                               const float *__restrict__ raw,
                                                               float *__restrict__ tiled) {
     __shared__ float sm[32][kDesc + 1];
     const uint4 e = tab[blockIdx.x];
-    pack_group(raw + (size_t)e.x * kDesc, e.y, tiled + (size_t)(e.x / kTile + e.z) * kTileFloats, e.z, blockIdx.y,
-               sm);
+    pack_group(raw + (size_t)e.x * kDesc, e.y, tiled + (size_t)e.z * kTileFloats, 0u, blockIdx.y, sm);
 }
 
 // The FP32 tiles of both views of every routed pair of a low-precision batch
@@ -74,7 +72,8 @@ __global__ void __launch_bounds__(256) pack_routed_kernel(const PairMeta *pairs,
         const uint32_t ta = (pm.na + kTile - 1) / kTile, tb = (pm.nb + kTile - 1) / kTile;
         for (uint32_t t = blockIdx.x; t < ta + tb; t += gridDim.x) {
             const bool is_a = t < ta;
-            pack_view_tile(raw, tiled, is_a ? pm.a_row0 : pm.b_row0, is_a ? pm.na : pm.nb, is_a ? t : t - ta, sm);
+            pack_view_tile(raw, tiled, is_a ? pm.a_raw0 : pm.b_raw0, is_a ? pm.a_row0 : pm.b_row0,
+                           is_a ? pm.na : pm.nb, is_a ? t : t - ta, sm);
         }
     }
 }

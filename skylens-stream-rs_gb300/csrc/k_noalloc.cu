@@ -98,6 +98,7 @@ __global__ void __launch_bounds__(256) single_prep_kernel(unsigned char *scratch
             PairMeta m;
             m.a_row0 = 0;
             m.b_row0 = L.rt_n * kTile;
+            m.a_raw0 = m.b_raw0 = 0;  // no row-major array
             m.na = na;
             m.nb = nb;
             m.nchunk = chunks;

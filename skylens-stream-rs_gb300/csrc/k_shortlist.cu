@@ -94,15 +94,13 @@ template <bool FP8>
 __global__ void __launch_bounds__(128) pack_lowp_kernel(const uint4 *__restrict__ tab, const float *__restrict__ raw,
                                                         uint8_t *__restrict__ optiles, float *__restrict__ norms,
                                                         float *__restrict__ qscale, ViewStat *__restrict__ vstats) {
-    const uint4 te = tab[blockIdx.x];  // {first store row of the view, rows, tile within the view, view}
-    const uint32_t row0 = te.x, n = te.y, view = te.w;
-    const uint32_t r = threadIdx.x;
-    const uint32_t tile = te.z;
-    const uint32_t row = tile * kTile + r;  // row within the view
-    const bool valid = row < n;
-    const float *src = raw + (size_t)(row0 + row) * kDesc;
+    const uint4 te = tab[blockIdx.x];  // {first row-major row, rows from it on, store tile, view}
+    const uint32_t view = te.w, r = threadIdx.x;
+    const uint32_t row = te.z * kTile + r;  // store row
+    const bool valid = r < te.y;
+    const float *src = raw + (size_t)(te.x + r) * kDesc;
     constexpr uint32_t kTileBytes = FP8 ? kFp8TileBytes : kBf16TileStride;
-    uint8_t *dst = optiles + (size_t)(row0 / kTile + tile) * kTileBytes;
+    uint8_t *dst = optiles + (size_t)te.z * kTileBytes;
     float x[kDesc];
 #pragma unroll
     for (int q = 0; q < 32; ++q) {
@@ -187,8 +185,8 @@ __global__ void __launch_bounds__(128) pack_lowp_kernel(const uint4 *__restrict_
         *reinterpret_cast<uint4 *>(ext) = make_uint4(hl, ones, 0u, 0u);        // kc0: hi lo 1 1
         *reinterpret_cast<uint4 *>(ext + 128) = make_uint4(ones, hl, 0u, 0u);  // kc1: 1 1 hi lo
     }
-    norms[row0 + row] = valid ? nrm : __int_as_float(0x7fc00000);  // FP8: NaN distances to padding rows too
-    if constexpr (FP8) qscale[row0 + row] = inv;
+    norms[row] = valid ? nrm : __int_as_float(0x7fc00000);  // FP8: NaN distances to padding rows too
+    if constexpr (FP8) qscale[row] = inv;
     // statistics (non-negative floats compare as their bit patterns)
     float s_n = valid ? sqrtf(nrm) : 0.f, s_r = valid ? sqrtf(res) : 0.f, s_q = valid ? sqrtf(nq) : 0.f;
     if (!isfinite(s_n) || !isfinite(s_r) || !isfinite(s_q)) bad = bad || valid;
@@ -942,8 +940,8 @@ __global__ void __launch_bounds__(256) sl_rescore_kernel(SlArgs g) {
         const PairMeta pm = g.pairs[qe.pair];
         const SlPair sp = g.spairs[qe.pair];
         const uint32_t ridx = sp.rbase + qe.i;
-        const float *a = g.raw + (size_t)(pm.a_row0 + qe.i) * kDesc;
-        const float *B = g.raw + (size_t)pm.b_row0 * kDesc;
+        const float *a = g.raw + (size_t)(pm.a_raw0 + qe.i) * kDesc;
+        const float *B = g.raw + (size_t)pm.b_raw0 * kDesc;
         float e1 = kInf, e2 = kInf, ad = kInf, maxerr = 0.f;
         uint32_t ej = 0xffffffffu;
         // S = the records' columns with d~ <= T, four entries at a time: lane group
@@ -1054,8 +1052,8 @@ __global__ void __launch_bounds__(256) sl_scan_kernel(SlArgs g) {
         const SlPair sp = g.spairs[qe.pair];
         if (sp.routed) continue;  // block-uniform: the exact kernel settled the whole pair
         if (threadIdx.x == 0) atomicAdd(&g.ctl[qe.kind == 0 ? kCtlQueueRows : kCtlQueueCols], 1u);
-        const float *A = g.raw + (size_t)pm.a_row0 * kDesc;
-        const float *B = g.raw + (size_t)pm.b_row0 * kDesc;
+        const float *A = g.raw + (size_t)pm.a_raw0 * kDesc;
+        const float *B = g.raw + (size_t)pm.b_raw0 * kDesc;
         uint32_t dec = kDecNone, col = qe.j;
         bool check_col = qe.kind == 1;
         if (qe.kind == 0) {

@@ -522,8 +522,8 @@ __global__ void __launch_bounds__(kDecideThreads) sl_decide_kernel(SlArgs g) {
             const uint32_t s = s0 + (lane >> 3);
             const uint4 o = found[min(s, n_found - 1)];
             const bool exact = o.z != kDecNone;
-            const float e1 = dist8(g.raw + (size_t)(pm.a_row0 + o.y) * kDesc,
-                                   g.raw + (size_t)(pm.b_row0 + (exact ? o.z : 0)) * kDesc);
+            const float e1 = dist8(g.raw + (size_t)(pm.a_raw0 + o.y) * kDesc,
+                                   g.raw + (size_t)(pm.b_raw0 + (exact ? o.z : 0)) * kDesc);
             if (s < n_found && (lane & 7) == 0) {
                 if (exact && settle_with_d1(g, sp, p, o.y, o.z, e1, __uint_as_float(o.w)))
                     atomicAdd(&n_settled, 1u);
@@ -549,8 +549,8 @@ __global__ void __launch_bounds__(256) sl_nearest_kernel(SlArgs g) {
         const PairMeta pm = g.pairs[o.x];
         const SlPair sp = g.spairs[o.x];
         const bool exact = o.z != kDecNone;
-        const float e1 = dist2(g.raw + (size_t)(pm.a_row0 + o.y) * kDesc,
-                               g.raw + (size_t)(pm.b_row0 + (exact ? o.z : 0)) * kDesc);
+        const float e1 = dist2(g.raw + (size_t)(pm.a_raw0 + o.y) * kDesc,
+                               g.raw + (size_t)(pm.b_raw0 + (exact ? o.z : 0)) * kDesc);
         if (s < n && (lane & 1) == 0) {
             if (exact && settle_with_d1(g, sp, o.x, o.y, o.z, e1, __uint_as_float(o.w)))
                 ++settled;
@@ -688,8 +688,8 @@ __global__ void __launch_bounds__(256) sl_resolve_kernel(SlArgs g) {
             const uint32_t p = rows[r].x, i = rows[r].y, m = cnt[r];
             const PairMeta pm = g.pairs[p];
             const SlPair sp = g.spairs[p];
-            const float *a = g.raw + (size_t)(pm.a_row0 + i) * kDesc;
-            const float *B = g.raw + (size_t)pm.b_row0 * kDesc;
+            const float *a = g.raw + (size_t)(pm.a_raw0 + i) * kDesc;
+            const float *B = g.raw + (size_t)pm.b_raw0 * kDesc;
             const bool over = m > g.cand_cap;
             const uint32_t mine_n = have && !over ? m : 0;
             const uint32_t most = __reduce_max_sync(0xffffffffu, mine_n);

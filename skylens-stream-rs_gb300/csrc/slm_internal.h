@@ -53,6 +53,7 @@ __device__ __forceinline__ void merge_rowpart(const RowPart &p, float &d1, float
 // Per image pair, as planned on the host.
 struct PairMeta {
     uint32_t a_row0, b_row0;  // first store row of the two views (multiples of 128)
+    uint32_t a_raw0, b_raw0;  // their first rows in the store's row-major array
     uint32_t na, nb;          // descriptor counts
     uint32_t nchunk;          // column chunks per row tile (exact path)
     uint32_t part_base;       // first RowPart block (128 rows per block)

@@ -210,7 +210,7 @@ constexpr uint32_t kXChunkMax = 16;
 struct SlArgs {
     const uint8_t *optiles;      // operand tiles by store row / 128
     const float *norms;          // squared f32 norms by store row
-    const float *raw;            // row-major f32 descriptors by store row
+    const float *raw;            // row-major f32 descriptors the views one after the other (a_raw0)
     const float *qscale;         // FP8: per-row inverse scale (nullptr for BF16)
     const ViewStat *vstats;
     const PairMeta *pairs;
@@ -280,8 +280,8 @@ __host__ __device__ inline bool sl_pair_on(const SlArgs &g, const SlPair &sp) {
     return g.tier ? (sp.rescued && !sp.routed) : !(sp.routed || sp.rescued);
 }
 
-// Store-side builder: one CTA per entry {first store row of the view, rows,
-// tile within the view, view} of the tile table.
+// Store-side builder: one CTA per entry {first row-major row, rows from it on,
+// store tile, view} of the tile table.
 void launch_pack_lowp(const uint4 *tab, uint32_t ntiles, const float *raw, int fp8, uint8_t *optiles, float *norms,
                       float *qscale, ViewStat *vstats, cudaStream_t s);
 
