@@ -252,11 +252,11 @@ __global__ void __launch_bounds__(256) read_images_kernel(const float4 *src, flo
 // arithmetic and two of a pixel's four loads are shared. 0.49 -> 0.30 ms for the
 // octaves of 24 views of 960 x 540, the atan2's part of it included.
 constexpr int kGradRows = 6;
-__global__ void __launch_bounds__(128) grad_kernel(const float *__restrict__ gauss, float2 *__restrict__ grad, int w,
-                                                   int h, int s, uint64_t layer_stride, uint64_t img_stride, int l0) {
-    const int x = blockIdx.x * blockDim.x + threadIdx.x, y0 = grid_wait(blockIdx.y) * kGradRows;
-    grid_go();
-    const int b = blockIdx.z / s, l = blockIdx.z % s;
+constexpr int kGradThreads = 128;
+__device__ __forceinline__ void grad_tile(const float *__restrict__ gauss, float2 *__restrict__ grad, int w, int h, int s,
+                                          uint64_t layer_stride, uint64_t img_stride, int l0, uint3 block) {
+    const int x = block.x * kGradThreads + threadIdx.x, y0 = block.y * kGradRows;
+    const int b = block.z / s, l = block.z % s;
     if (x >= w) return;
     const bool inside = x >= 1 && x + 1 < w;
     const float *im = gauss + (uint64_t)b * img_stride + (uint64_t)(l0 + l) * layer_stride + (uint64_t)y0 * w + x;
@@ -278,6 +278,14 @@ __global__ void __launch_bounds__(128) grad_kernel(const float *__restrict__ gau
         above = here;
         here = below;
     }
+}
+
+__global__ void __launch_bounds__(kGradThreads) grad_kernel(const float *__restrict__ gauss, float2 *__restrict__ grad,
+                                                            int w, int h, int s, uint64_t layer_stride,
+                                                            uint64_t img_stride, int l0) {
+    const uint32_t y = grid_wait(blockIdx.y);
+    grid_go();
+    grad_tile(gauss, grad, w, h, s, layer_stride, img_stride, l0, make_uint3(blockIdx.x, y, blockIdx.z));
 }
 
 // ---------------------------------------------------------------- extrema
@@ -330,18 +338,16 @@ __device__ void refine_candidate(const ExtremaArgs &a, const float *dog, int b, 
 // the CTA's strips are through and are then refined side by side instead of one
 // lane at a time. 0.49 -> 0.23 ms for the octaves of 24 views of 960 x 540.
 constexpr int kExtremaWarps = 4, kExtremaRows = 16;
-__global__ void __launch_bounds__(32 * kExtremaWarps) extrema_kernel(ExtremaArgs a, int rows) {
+__device__ __forceinline__ void extrema_strips(const ExtremaArgs &a, int rows, uint3 block) {
     // no two maxima, and no two minima, are neighbours: at most one of each in 2 x 2 pixels
     __shared__ uint32_t found[30 * kExtremaRows * kExtremaWarps / 2];
     __shared__ uint32_t n_found;
     if (threadIdx.x == 0) n_found = 0;
-    grid_wait();
-    grid_go();
     __syncthreads();
-    const int lane = threadIdx.x & 31, strip = blockIdx.y * kExtremaWarps + (threadIdx.x >> 5);
-    const int b = blockIdx.z / a.s, l0 = 1 + blockIdx.z % a.s;
+    const int lane = threadIdx.x & 31, strip = block.y * kExtremaWarps + (threadIdx.x >> 5);
+    const int b = block.z / a.s, l0 = 1 + block.z % a.s;
     const int w = a.w, h = a.h;
-    const int x = (int)blockIdx.x * 30 + lane, y0 = 1 + strip * rows;  // lanes 1 .. 30 test pixel x
+    const int x = (int)block.x * 30 + lane, y0 = 1 + strip * rows;  // lanes 1 .. 30 test pixel x
     const float *dog = a.dog + (uint64_t)b * (a.ng - 1) * a.layer_stride;
     if (y0 < h - 1) {  // warp-uniform
         const float *lo = dog + (uint64_t)(l0 - 1) * a.layer_stride + min(x, w - 1);
@@ -441,6 +447,23 @@ __device__ void refine_candidate(const ExtremaArgs &a, const float *dog, int b, 
     fc.layer = (uint8_t)cl;
     fc.key = ((uint64_t)a.octave << 48) | ((uint64_t)l0 << 32) | ((uint64_t)y << 16) | (uint64_t)x;
     a.cands[slot] = fc;
+}
+
+// An octave's gradient tables and its extrema in one launch, the extrema's blocks
+// first: neither needs the other, and in small octaves each is a few microseconds
+// of latency (one 717 x 531 image with its upsampled detection 1.12 -> 1.05 ms).
+static_assert(kGradThreads == 32 * kExtremaWarps, "one block size");
+__global__ void __launch_bounds__(kGradThreads) layers_kernel(ExtremaArgs a, int rows, uint3 eg, const float *gauss,
+                                                              float2 *grad, uint64_t img_stride, uint3 gg) {
+    uint32_t k = grid_wait(blockIdx.x);
+    grid_go();
+    const uint32_t ne = eg.x * eg.y * eg.z;
+    if (k < ne) {  // block-uniform
+        extrema_strips(a, rows, make_uint3(k % eg.x, k / eg.x % eg.y, k / (eg.x * eg.y)));
+    } else {
+        k -= ne;
+        grad_tile(gauss, grad, a.w, a.h, a.s, a.layer_stride, img_stride, 1, make_uint3(k % gg.x, k / gg.x % gg.y, k / (gg.x * gg.y)));
+    }
 }
 
 // sig_oct = sigma0 * kstep^s (features.rs:747) of every candidate, one a thread:
@@ -1076,17 +1099,21 @@ void launch_read_images(const float *src, float *dst, uint64_t n, int sms, cudaS
 
 void launch_grad(const float *gauss, float2 *grad, int w, int h, int s_, uint64_t img_stride, int l0, int nimg,
                  cudaStream_t s) {
-    launch_next(grad_kernel, dim3((w + 127) / 128, (h + kGradRows - 1) / kGradRows, nimg * s_), 128, 0, s, gauss, grad, w, h,
-                s_, (uint64_t)w * h, img_stride, l0);
+    launch_next(grad_kernel, dim3((w + kGradThreads - 1) / kGradThreads, (h + kGradRows - 1) / kGradRows, nimg * s_),
+                kGradThreads, 0, s, gauss, grad, w, h, s_, (uint64_t)w * h, img_stride, l0);
 }
 
-void launch_extrema(const ExtremaArgs &a, int nimg, cudaStream_t s) {
-    if (a.w < 3 || a.h < 3) return;
+void launch_layers(const ExtremaArgs &a, const float *gauss, float2 *grad, uint64_t img_stride, int nimg,
+                   cudaStream_t s) {
     // strips of 16 rows where that leaves every SM its 16 warps, else of 4
     const uint64_t warps = (uint64_t)((a.w + 27) / 30) * ((a.h + 13) / 16) * nimg * a.s;
     const int rows = warps >= 16 * 152 ? kExtremaRows : 4, strip = kExtremaWarps * rows;
-    launch_next(extrema_kernel, dim3((a.w + 27) / 30, (a.h - 2 + strip - 1) / strip, nimg * a.s), 32 * kExtremaWarps, 0, s,
-                a, rows);
+    const uint32_t layers = (uint32_t)nimg * a.s;
+    const uint3 gg = make_uint3((a.w + kGradThreads - 1) / kGradThreads, (a.h + kGradRows - 1) / kGradRows, layers);
+    const uint3 eg = a.w < 3 || a.h < 3 ? make_uint3(1, 1, 0)
+                                        : make_uint3((a.w + 27) / 30, (a.h - 2 + strip - 1) / strip, layers);
+    launch_next(layers_kernel, eg.x * eg.y * eg.z + gg.x * gg.y * gg.z, kGradThreads, 0, s, a, rows, eg, gauss, grad,
+                img_stride, gg);
 }
 
 // The number of candidates is the device's: grids for as many as there may be,

@@ -3090,7 +3090,6 @@ slm_status feat_core(slm_ctx *c, Workspace *ws, const float *d_img, uint32_t n, 
             for (int i = 1; i < ng; ++i)
                 launch_blur(gauss + (i - 1) * wh, tmp, gauss + i * wh, gauss + (i - 1) * wh, dog + (i - 1) * wh, G.w,
                             G.h, (int)n, ng * wh, ng * wh, (ng - 1) * wh, taps[i], st);
-            launch_grad(gauss, out.d_grads + G.grad_off, G.w, G.h, s, ng * wh, 1, (int)n, st);
             ExtremaArgs ea{};
             ea.dog = dog;
             ea.layer_stride = wh;
@@ -3104,7 +3103,7 @@ slm_status feat_core(slm_ctx *c, Workspace *ws, const float *d_img, uint32_t n, 
             ea.cands = out.d_cands;
             ea.count = d_count;
             ea.cap = cap;
-            launch_extrema(ea, (int)n, st);
+            launch_layers(ea, gauss, out.d_grads + G.grad_off, ng * wh, (int)n, st);
         }
         OrientArgs oa{};
         oa.cands = out.d_cands;

@@ -290,7 +290,10 @@ void launch_read_images(const float *src, float *dst, uint64_t n, int sms, cudaS
 // at gauss + k * img_stride + l * w * h); grad: [img][s_][h][w]
 void launch_grad(const float *gauss, float2 *grad, int w, int h, int s_, uint64_t img_stride, int l0, int nimg,
                  cudaStream_t s);
-void launch_extrema(const ExtremaArgs &a, int nimg, cudaStream_t s);
+// an octave's extrema, and the gradient tables of its layers 1 .. s (image k's layer
+// l at gauss + k * img_stride + l * layer_stride)
+void launch_layers(const ExtremaArgs &a, const float *gauss, float2 *grad, uint64_t img_stride, int nimg,
+                   cudaStream_t s);
 void launch_candidate_sigma(FeatCand *cands, const uint32_t *count, uint32_t cap, float sigma0, float kstep, int sms,
                             cudaStream_t s);
 void launch_orient(const OrientArgs &a, int sms, cudaStream_t s);
