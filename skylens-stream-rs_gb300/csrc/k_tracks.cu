@@ -19,12 +19,13 @@
 // applied, and the tracks laid out in root order, which is first-observation
 // order: 0.05 ms, and the host sees finished lists. The call for the 1.7 M matches
 // and 276 K nodes of a 240-view zone: 2.28 ms with a host synchronisation a round
-// and the grouping on the host, now 0.36 ms, bound by latency of the matches' reads
+// and the grouping on the host, now 0.34 ms, bound by latency of the matches' reads
 // and of the hash set's atomics.
 #include <cuda_runtime.h>
 
 #include <cstdint>
 
+#include "ptx.cuh"
 #include "slm_internal.h"
 
 namespace slm {
@@ -87,6 +88,8 @@ __device__ __forceinline__ void join(uint32_t *parent, uint32_t u, uint32_t v) {
 constexpr int kEdgeThreads = 256, kEdgeLoads = 4;
 
 __global__ void __launch_bounds__(kEdgeThreads) track_edges_kernel(TrackArgs a) {
+    grid_wait();
+    grid_go();
     const TrackPair tp = a.pairs[blockIdx.x];
     const uint32_t ia = tp.image_a, ib = tp.image_b;
     const bool pair_ok = ia != ib && ia < a.n_images && ib < a.n_images;
@@ -133,6 +136,8 @@ __global__ void __launch_bounds__(kEdgeThreads) track_edges_kernel(TrackArgs a) 
 // Every edge again; LAST: until it is joined.
 template <bool LAST>
 __global__ void __launch_bounds__(256) track_join_kernel(TrackArgs a) {
+    grid_wait();
+    grid_go();
     for (uint64_t x = blockIdx.x * 256ull + threadIdx.x; x <= a.table_mask; x += gridDim.x * 256ull) {
         const unsigned long long key = a.table[x];
         if (key == kEmpty) continue;
@@ -146,11 +151,15 @@ __global__ void __launch_bounds__(256) track_join_kernel(TrackArgs a) {
 
 // Every node's parent becomes its root.
 __global__ void __launch_bounds__(256) track_jump_kernel(TrackArgs a) {
+    grid_wait();
+    grid_go();
     for (uint64_t x = blockIdx.x * 256ull + threadIdx.x; x < a.n; x += gridDim.x * 256ull)
         a.parent[x] = old_root(a.parent, (uint32_t)x);
 }
 
 __global__ void __launch_bounds__(256) track_init_kernel(TrackArgs a) {
+    grid_wait();
+    grid_go();
     for (uint64_t x = blockIdx.x * 256ull + threadIdx.x; x < a.n; x += gridDim.x * 256ull) {
         a.parent[x] = (uint32_t)x;
         a.used[x] = 0;
@@ -163,6 +172,8 @@ __global__ void __launch_bounds__(256) track_init_kernel(TrackArgs a) {
 // on its way: only x's own thread writes parent[x] here, so that it is the root
 // when the kernel ends.
 __global__ void __launch_bounds__(256) track_count_kernel(TrackArgs a) {
+    grid_wait();
+    grid_go();
     const volatile uint32_t *parent = a.parent;
     const uint32_t lane = threadIdx.x & 31;
     for (uint64_t x0 = blockIdx.x * 256ull + (threadIdx.x & ~31u); x0 < a.n; x0 += gridDim.x * 256ull) {  // warp-uniform
@@ -182,6 +193,8 @@ __global__ void __launch_bounds__(256) track_count_kernel(TrackArgs a) {
 // Room for each component's members, and the components' list: those that a
 // warp sorts, and from the other end those that take a CTA.
 __global__ void __launch_bounds__(256) track_list_kernel(TrackArgs a) {
+    grid_wait();
+    grid_go();
     const uint32_t lane = threadIdx.x & 31;
     for (uint64_t x0 = blockIdx.x * 256ull + (threadIdx.x & ~31u); x0 < a.n; x0 += gridDim.x * 256ull) {  // warp-uniform
         const uint64_t x = x0 + lane;
@@ -212,6 +225,8 @@ __global__ void __launch_bounds__(256) track_list_kernel(TrackArgs a) {
 }
 
 __global__ void __launch_bounds__(256) track_fill_kernel(TrackArgs a) {
+    grid_wait();
+    grid_go();
     const uint32_t lane = threadIdx.x & 31;
     for (uint64_t x0 = blockIdx.x * 256ull + (threadIdx.x & ~31u); x0 < a.n; x0 += gridDim.x * 256ull) {  // warp-uniform
         const uint64_t x = x0 + lane;
@@ -316,6 +331,8 @@ __device__ __forceinline__ void sort_large(const TrackArgs &a, uint32_t root, ui
 }
 
 __global__ void __launch_bounds__(256) track_sort_kernel(TrackArgs a) {
+    grid_wait();
+    grid_go();
     const uint32_t lane = threadIdx.x & 31;
     const uint64_t n = a.ctl[kTrComps], large = a.ctl[kTrLarge];
     for (uint64_t k = blockIdx.x * 8ull + (threadIdx.x >> 5); k < n; k += gridDim.x * 8ull) {  // warp-uniform
@@ -330,6 +347,8 @@ __global__ void __launch_bounds__(256) track_sort_kernel(TrackArgs a) {
 
 // Tracks and observations of each CTA's share of the nodes.
 __global__ void __launch_bounds__(256) track_sums_kernel(TrackArgs a) {
+    grid_wait();
+    grid_go();
     __shared__ uint32_t ws[2][8];
     const uint64_t x0 = blockIdx.x * a.share, x1 = min(x0 + a.share, a.n);
     uint32_t t = 0, o = 0;
@@ -350,6 +369,8 @@ __global__ void __launch_bounds__(256) track_sums_kernel(TrackArgs a) {
 
 // Their lists, in root order: track k is obs[track_off[k] .. track_off[k + 1]).
 __global__ void __launch_bounds__(256) track_emit_kernel(TrackArgs a) {
+    grid_wait();
+    grid_go();
     __shared__ uint32_t ws[2][8];
     const uint32_t lane = threadIdx.x & 31, warp = threadIdx.x >> 5;
     auto total = [&](uint32_t t, uint32_t o, uint32_t &pt, uint32_t &po, uint32_t &at, uint32_t &ao) {  // scan of (t, o)
@@ -399,21 +420,21 @@ __global__ void __launch_bounds__(256) track_emit_kernel(TrackArgs a) {
 
 void launch_tracks(const TrackArgs &a, uint32_t n_pairs, int sms, cudaStream_t s) {
     const int grid = 8 * sms;
-    track_init_kernel<<<grid, 256, 0, s>>>(a);
-    if (n_pairs) track_edges_kernel<<<n_pairs, kEdgeThreads, 0, s>>>(a);
+    launch_next(track_init_kernel, grid, 256, 0, s, a);
+    if (n_pairs) launch_next(track_edges_kernel, n_pairs, kEdgeThreads, 0, s, a);
     for (int round = 0; round < 2; ++round) {
-        track_jump_kernel<<<grid, 256, 0, s>>>(a);
-        track_join_kernel<false><<<grid, 256, 0, s>>>(a);
+        launch_next(track_jump_kernel, grid, 256, 0, s, a);
+        launch_next(track_join_kernel<false>, grid, 256, 0, s, a);
     }
-    track_jump_kernel<<<grid, 256, 0, s>>>(a);
-    track_join_kernel<true><<<grid, 256, 0, s>>>(a);
-    track_count_kernel<<<grid, 256, 0, s>>>(a);
-    track_list_kernel<<<grid, 256, 0, s>>>(a);
-    track_fill_kernel<<<grid, 256, 0, s>>>(a);
-    track_sort_kernel<<<grid, 256, 0, s>>>(a);
+    launch_next(track_jump_kernel, grid, 256, 0, s, a);
+    launch_next(track_join_kernel<true>, grid, 256, 0, s, a);
+    launch_next(track_count_kernel, grid, 256, 0, s, a);
+    launch_next(track_list_kernel, grid, 256, 0, s, a);
+    launch_next(track_fill_kernel, grid, 256, 0, s, a);
+    launch_next(track_sort_kernel, grid, 256, 0, s, a);
     const unsigned blocks = a.n ? (unsigned)((a.n + a.share - 1) / a.share) : 1u;
-    track_sums_kernel<<<blocks, 256, 0, s>>>(a);
-    track_emit_kernel<<<blocks, 256, 0, s>>>(a);
+    launch_next(track_sums_kernel, blocks, 256, 0, s, a);
+    launch_next(track_emit_kernel, blocks, 256, 0, s, a);
 }
 
 }  // namespace slm
