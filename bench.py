@@ -846,15 +846,20 @@ def main():
     p2ms = float(np.mean([k[2] for k in kern_ms]))
     dist_n = z.distances
     if prec in ("bf16", "fp8"):
-        # Each tensor-core pass contracts every (row, column) once: 2*128 flops per
-        # distance. The dominant kernel is the slower pass, timed alone by events.
-        flops = 2.0 * 128 * dist_n
-        dom_ms, dom = (p2ms, "sl_pass_kernel<2> (pass 2)") if p2ms >= p1ms else (p1ms, "sl_pass_kernel<1> (pass 1)")
+        # 2*128 flops per distance and contraction. A BF16 batch's one pass launch
+        # (pass_ms[0]) contracts every (row, column) once per direction; each FP8 pass
+        # contracts them once, and the dominant kernel is the slower one.
+        flops = 2.0 * 128 * dist_n * (2 if prec == "bf16" else 1)
+        if prec == "bf16":
+            dom_ms, dom = p1ms, "sl_top2_kernel (both directions)"
+        else:
+            dom_ms, dom = max((p1ms, "sl_pass_kernel<1> (pass 1)"), (p2ms, "sl_pass_kernel<2> (pass 2)"))
         achieved = flops / (dom_ms / 1e3) / 1e12
         peak = pk["bf16_tflops"] * (2 if prec == "fp8" else 1)
         roof = {"bound": "tensor", "achieved": achieved, "peak": peak, "unit": "TFLOP/s", "frac": achieved / peak,
                 "traffic": None, "kernel": dom, "kernel_ms": dom_ms, "pass1_ms": p1ms, "pass2_ms": p2ms,
-                "pipeline_ms": kms, "algorithmic": "256 flops per distance x %d distances" % dist_n,
+                "pipeline_ms": kms, "algorithmic": "256 flops per distance%s x %d distances" % (
+                    " and direction" if prec == "bf16" else "", dist_n),
                 "peak_source": f"{pk_kind} bf16_tflops (burst) of MEASURED_PEAKS.json"}
     else:
         # 384 FP32 instructions per distance (sub, mul, add per component, matching.rs:146-155)
@@ -866,7 +871,7 @@ def main():
                 "frac": achieved / peak, "traffic": None, "kernel": "exact_kernel",
                 "peak_source": f"{sm_count} SMs x 128 lanes x {mhz:.0f} MHz (sampled)"}
     # DRAM bytes per launch of the dominant kernel from an ncu capture of this workload
-    prof = os.path.join(REPO, "profiles", "sl_pass_kernel_zone240_dram.json")
+    prof = os.path.join(REPO, "profiles", "sl_top2_kernel_zone240_dram.json")
     if os.path.exists(prof) and WORKLOAD == "zone240" and args.positions == 80:
         try:
             roof["traffic"] = json.load(open(prof)).get(roof["kernel"])

@@ -57,9 +57,10 @@ typedef enum {
                           batch), FP32 below, where the shortlist's fixed cost dominates */
 } slm_precision;
 
-/* SLM_PREC_AUTO's switch point, measured on GB300 through slm_ratio_match from
- * host arrays: 2500 x 2500 descriptors FP32 0.18 ms / BF16 0.19 ms,
- * 3072 x 3072 0.21 / 0.20 ms, 4096 x 4096 0.31 / 0.22 ms. */
+/* SLM_PREC_AUTO's switch point. Measured on GB300 through slm_ratio_match from
+ * host arrays, FP32 / BF16: 2048 x 2048 descriptors 0.10 / 0.11 ms, 2500 x 2500
+ * 0.16 / 0.12, 3072 x 3072 0.19 / 0.12, 4096 x 4096 0.28 / 0.13: the two meet
+ * near 5 M distances. Part of the interface, so it stays where it was set. */
 #define SLM_AUTO_BF16_DISTANCES 8000000ull
 
 typedef struct {
@@ -202,8 +203,10 @@ slm_status slm_store_destroy(slm_store *st);
 slm_status slm_store_add_view(slm_store *st, const float *desc, uint32_t n, uint32_t *view_id);
 /* Append many views from one buffer: view v has counts[v] rows starting at
  * row offsets[v] of desc. ids[v] receives its id. desc may be pageable host
- * memory (one copy and a scatter kernel), pinned host memory or device memory
- * (one copy per view, copy engines only; up to 4096 views per call).
+ * memory (one copy if the views follow one another, else one copy into a staging
+ * buffer and a scatter kernel), pinned host memory or device memory
+ * (one copy per run of views that follow one another, copy engines only; up to
+ * 4096 runs per call).
  * Asynchronous on the context stream like slm_store_add_view. */
 slm_status slm_store_add_views(slm_store *st, const float *desc, const uint64_t *offsets, const uint32_t *counts,
                                uint32_t nviews, uint32_t *ids);
