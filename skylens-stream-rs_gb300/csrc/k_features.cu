@@ -669,10 +669,13 @@ __device__ __forceinline__ uint32_t desc_row(const DescWindow &W, int row, int &
 }
 
 // One sample (features.rs:534-573): false when it lies outside the cells; else
-// its 8 products m wv wu wo, in the reference's order of factors, out[k] with k's
-// bits the upper row, column and orientation, and its lower cell row + 1, cell
+// its weighted magnitude, its place between cells, and its lower cell row + 1, cell
 // column + 1 and orientation, 3 bits each.
-__device__ __forceinline__ bool desc_sample(const DescWindow &W, int px, int py, float (&out)[8], uint32_t &code) {
+struct DescSample {
+    float m, du, dv, dob;
+    uint32_t code;
+};
+__device__ __forceinline__ bool desc_sample(const DescWindow &W, int px, int py, DescSample &s) {
     const int NC = 4, NO = 8;
     const float fx = (float)px - W.x, fy = (float)py - W.y;
     const float pu = W.c * fx + W.sn * fy, pv_ = -W.sn * fx + W.c * fy;
@@ -685,98 +688,124 @@ __device__ __forceinline__ bool desc_sample(const DescWindow &W, int px, int py,
     const float ori = rem_euclid(gm.y - W.angle, kTwoPi);
     const float bo = ori / kTwoPi * (float)NO;
     const float wgt = exp_cr(-(u * u + v * v) / (2.0f * 4.0f));
-    const float m = gm.x * wgt;
+    s.m = gm.x * wgt;
     const float u0 = floorf(bu), v0 = floorf(bv), o0 = floorf(bo);
-    const float du = bu - u0, dv = bv - v0, dob = bo - o0;
-    const float pv[2] = {m * (1.0f - dv), m * dv}, wu[2] = {1.0f - du, du}, wo[2] = {1.0f - dob, dob};
-#pragma unroll
-    for (int k = 0; k < 8; ++k) out[k] = pv[k >> 2] * wu[(k >> 1) & 1] * wo[k & 1];
+    s.du = bu - u0, s.dv = bv - v0, s.dob = bo - o0;
     const int io0 = o0 < 0.0f ? 0 : f2i(o0);
-    code = (uint32_t)(f2i(v0) + 1) | (uint32_t)(f2i(u0) + 1) << 3 | (uint32_t)(io0 & (NO - 1)) << 6;
+    s.code = (uint32_t)(f2i(v0) + 1) | (uint32_t)(f2i(u0) + 1) << 3 | (uint32_t)(io0 & (NO - 1)) << 6;
     return true;
 }
 
-// A warp's 32 samples sorted into bins: list holds the products of the bins,
-// bin after bin, each bin's in sample order and padded with zeros to a multiple
-// of four (adding 0 changes no sum here: none is -0). off and any have a border
-// of one cell: a sample's products for rows and columns outside the 4 x 4 go to
-// the four places after the list.
-constexpr int kDescListMax = 4 * (256 + 3 * 128) / 4;  // 256 products, at most 3 zeros a bin
+// Its 8 products m wv wu wo, in the reference's order of factors: k's bits are the
+// upper row, column and orientation.
+__device__ __forceinline__ void desc_products(const DescSample &s, float (&out)[8]) {
+    const float pv[2] = {s.m * (1.0f - s.dv), s.m * s.dv}, wu[2] = {1.0f - s.du, s.du}, wo[2] = {1.0f - s.dob, s.dob};
+#pragma unroll
+    for (int k = 0; k < 8; ++k) out[k] = pv[k >> 2] * wu[(k >> 1) & 1] * wo[k & 1];
+}
+
+// A warp's samples, SETS times 32 of them, sorted into bins: list holds the
+// products of the bins, bin after bin, each bin's in sample order and padded with
+// zeros to a multiple of four (adding 0 changes no sum here: none is -0). off and any
+// have a border of one cell: a sample's products for rows and columns outside the
+// 4 x 4 go to the place after the list.
+template <int SETS>
 struct __align__(16) DescGroup {
-    float list[kDescListMax + 4];
+    static constexpr int kMax = 256 * SETS + 3 * 128;  // products, at most 3 zeros a bin
+    float list[kMax + 4];
     uint16_t off[6 * 6 * 8];  // first place of bin (row, column, orientation) at ((row + 1) * 6 + column + 1) * 8 + o
-    uint32_t any[6 + 6 + 8];  // samples that touch row -1..4, column -1..4, orientation 0..7
+    uint32_t any[SETS][6 + 6 + 8];  // samples of a set that touch row -1..4, column -1..4, orientation 0..7
 };
 
-__device__ __forceinline__ void desc_group_init(DescGroup &G, int lane) {
-    for (int e = lane; e < 6 * 6 * 8; e += 32) G.off[e] = kDescListMax;
-    if (lane < 20) G.any[lane] = 0;
+template <int SETS>
+__device__ __forceinline__ void desc_group_init(DescGroup<SETS> &G, int lane) {
+    for (int e = lane; e < 6 * 6 * 8; e += 32) G.off[e] = DescGroup<SETS>::kMax;
+    for (int e = lane; e < 20 * SETS; e += 32) G.any[0][e] = 0;
     __syncwarp();
 }
 
-// Fills G from each lane's sample (its 8 products and its code, desc_sample).
-// The bits of the codes by ballot give the mask of the samples that touch a
-// row, column or orientation (a lane makes one word); a bin's samples are the
-// AND of three, a sample's place in it the number of earlier ones. Lane l lays
-// out bins (iv, iu, io), (iv, iu, io + 4), (iv + 2, iu, io) and (iv + 2, iu, io +
-// 4) with iv = l / 16, iu = l / 4 % 4, io = l % 4, one after the other: quads
-// are their lengths in fours, start the first one's place / 4. Neighbouring
-// samples share cells and orientations, so the bins busy at one time lie in
-// different lanes.
-__device__ __forceinline__ void desc_group(const float (&prod)[8], uint32_t code, bool valid, int lane, DescGroup &G,
-                                           uint32_t (&quads)[4], uint32_t &start) {
-    uint32_t b[9];
-#pragma unroll
-    for (int k = 0; k < 9; ++k) b[k] = __ballot_sync(0xffffffffu, (code >> k) & 1u);
-    uint32_t lower = __ballot_sync(0xffffffffu, valid), upper = lower;
+// Fills G from each lane's samples, one a set (desc_sample); the sets come one after
+// the other in sample order. The bits of the codes by ballot give the mask of the
+// samples that touch a row, column or orientation (a lane makes one word); a bin's
+// samples are the AND of three, a sample's place in it the number of earlier ones.
+// Lane l lays out bins (iv, iu, io), (iv, iu, io + 4), (iv + 2, iu, io) and (iv + 2,
+// iu, io + 4) with iv = l / 16, iu = l / 4 % 4, io = l % 4, one after the other: quads
+// are their lengths in fours, start the first one's place / 4. Neighbouring samples
+// share cells and orientations, so the bins busy at one time lie in different lanes.
+template <int SETS>
+__device__ __forceinline__ void desc_group(const DescSample (&smp)[SETS], const bool (&valid)[SETS], int lane,
+                                           DescGroup<SETS> &G, uint32_t (&quads)[4], uint32_t &start) {
     // the codes of the samples whose lower / upper row, column or orientation this lane's word is for
     const int vu = lane < 8 ? lane & 3 : (lane + 7) & 7, vl = lane < 8 ? (lane & 3) + 1 : lane & 7;
 #pragma unroll
-    for (int k = 0; k < 3; ++k) {
-        const uint32_t t = lane < 4 ? b[k] : lane < 8 ? b[3 + k] : b[6 + k];
-        lower &= (vl >> k) & 1 ? t : ~t;
-        upper &= (vu >> k) & 1 ? t : ~t;
+    for (int s = 0; s < SETS; ++s) {
+        uint32_t b[9];
+#pragma unroll
+        for (int k = 0; k < 9; ++k) b[k] = __ballot_sync(0xffffffffu, (smp[s].code >> k) & 1u);
+        uint32_t lower = __ballot_sync(0xffffffffu, valid[s]), upper = lower;
+#pragma unroll
+        for (int k = 0; k < 3; ++k) {
+            const uint32_t t = lane < 4 ? b[k] : lane < 8 ? b[3 + k] : b[6 + k];
+            lower &= (vl >> k) & 1 ? t : ~t;
+            upper &= (vu >> k) & 1 ? t : ~t;
+        }
+        if (lane < 16) G.any[s][lane < 4 ? lane + 1 : lane < 8 ? lane + 3 : lane + 4] = lower | upper;
     }
-    if (lane < 16) G.any[lane < 4 ? lane + 1 : lane < 8 ? lane + 3 : lane + 4] = lower | upper;
     __syncwarp();
     const int p = lane >> 4, iu = (lane >> 2) & 3, q = lane & 3;
-    {
-        const uint32_t c = G.any[7 + iu], r0 = G.any[1 + p] & c, r2 = G.any[3 + p] & c;
-        const uint32_t o0 = G.any[12 + q], o4 = G.any[16 + q];
-        quads[0] = (__popc(r0 & o0) + 3) >> 2;
-        quads[1] = (__popc(r0 & o4) + 3) >> 2;
-        quads[2] = (__popc(r2 & o0) + 3) >> 2;
-        quads[3] = (__popc(r2 & o4) + 3) >> 2;
+    quads[0] = quads[1] = quads[2] = quads[3] = 3;
+#pragma unroll
+    for (int s = 0; s < SETS; ++s) {
+        const uint32_t *w = G.any[s], c = w[7 + iu], r0 = w[1 + p] & c, r2 = w[3 + p] & c, o0 = w[12 + q], o4 = w[16 + q];
+        quads[0] += __popc(r0 & o0);
+        quads[1] += __popc(r0 & o4);
+        quads[2] += __popc(r2 & o0);
+        quads[3] += __popc(r2 & o4);
     }
+#pragma unroll
+    for (int n = 0; n < 4; ++n) quads[n] >>= 2;
     const uint32_t mine = quads[0] + quads[1] + quads[2] + quads[3];
-    uint32_t s = mine;
+    uint32_t sum = mine;
 #pragma unroll
     for (int o = 1; o < 32; o <<= 1) {
-        const uint32_t t = __shfl_up_sync(0xffffffffu, s, o);
-        if (lane >= o) s += t;
+        const uint32_t t = __shfl_up_sync(0xffffffffu, sum, o);
+        if (lane >= o) sum += t;
     }
-    start = s - mine;
+    start = sum - mine;
     uint16_t *off = &G.off[((p + 1) * 6 + iu + 1) * 8 + q];
     off[0] = (uint16_t)(4 * start);
     off[4] = (uint16_t)(4 * (start + quads[0]));
     off[2 * 48] = (uint16_t)(4 * (start + quads[0] + quads[1]));
-    off[2 * 48 + 4] = (uint16_t)(4 * (s - quads[3]));
-    const uint32_t total = __shfl_sync(0xffffffffu, s, 31);
+    off[2 * 48 + 4] = (uint16_t)(4 * (sum - quads[3]));
+    const uint32_t total = __shfl_sync(0xffffffffu, sum, 31);
     for (uint32_t e = lane; e < total; e += 32)
         reinterpret_cast<float4 *>(G.list)[e] = make_float4(0.0f, 0.0f, 0.0f, 0.0f);
     __syncwarp();
-    if (valid) {
-        const uint32_t lt = (1u << lane) - 1, v0 = code & 7, u0 = (code >> 3) & 7, o0 = code >> 6, o1 = (o0 + 1) & 7;
-        const uint32_t t0 = G.any[12 + o0] & lt, t1 = G.any[12 + o1] & lt;
-        const uint16_t *at = &G.off[(v0 * 6 + u0) * 8];
 #pragma unroll
-        for (uint32_t d = 0; d < 4; ++d) {  // row v0 - 1 + d / 2, column u0 - 1 + d % 2
-            const uint32_t m = G.any[v0 + (d >> 1)] & G.any[6 + u0 + (d & 1)];
-            const uint16_t *w = at + (d >> 1) * 48 + (d & 1) * 8;
-            G.list[w[o0] + __popc(m & t0)] = prod[2 * d];
-            G.list[w[o1] + __popc(m & t1)] = prod[2 * d + 1];
+    for (int s = 0; s < SETS; ++s)
+        if (valid[s]) {
+            float prod[8];
+            desc_products(smp[s], prod);
+            const uint32_t code = smp[s].code, lt = (1u << lane) - 1;
+            const uint32_t v0 = code & 7, u0 = (code >> 3) & 7, o0 = code >> 6, o1 = (o0 + 1) & 7;
+            const uint32_t t0 = G.any[s][12 + o0] & lt, t1 = G.any[s][12 + o1] & lt;
+            const uint16_t *at = &G.off[(v0 * 6 + u0) * 8];
+#pragma unroll
+            for (uint32_t d = 0; d < 4; ++d) {  // row v0 - 1 + d / 2, column u0 - 1 + d % 2
+                const uint32_t iv = v0 + (d >> 1), iu1 = 6 + u0 + (d & 1);
+                const uint32_t m = G.any[s][iv] & G.any[s][iu1];
+                const uint16_t *w = at + (d >> 1) * 48 + (d & 1) * 8;
+                uint32_t a0 = w[o0] + __popc(m & t0), a1 = w[o1] + __popc(m & t1);
+#pragma unroll
+                for (int e = 0; e < s; ++e) {  // the earlier sets' samples of the bin
+                    const uint32_t me = G.any[e][iv] & G.any[e][iu1];
+                    a0 += __popc(me & G.any[e][12 + o0]);
+                    a1 += __popc(me & G.any[e][12 + o1]);
+                }
+                G.list[a0] = prod[2 * d];
+                G.list[a1] = prod[2 * d + 1];
+            }
         }
-    }
 }
 
 // n2 of a histogram in index order (features.rs:575-580)
@@ -798,12 +827,15 @@ __device__ __forceinline__ float desc_norm(const float *sq) {
 // sum over the window's samples in raster order: a serial chain, and on smooth
 // images few chains are busy at a time (32 neighbours share cells and nearly an
 // orientation: 22 adds in a row for the 136 of a group). So the work around the
-// adds is kept small: samples are sorted into bins 32 at a time (desc_group),
-// and a bin's owner then runs through its list.
+// adds is kept small: samples are sorted into bins 64 at a time (desc_group),
+// and a bin's owner then runs through its list. (32 at a time, the scan, the
+// clearing and the layout are paid twice: 2.49 ms for a call of 24 views, now 2.39,
+// and 0.58 for 1500 large windows, now 0.52; with 96 or 128 fewer warps fit: 2.47
+// and 2.72.)
 //   one warp a feature (windows of up to kDescWarpSide rows: everything the
 //   detector makes), four bins a lane. No barriers.
 //   one CTA of 8 warps a feature (larger windows, and all when there are few
-//   features: the first n_large jobs): the warps sort 32 samples each, then the
+//   features: the first n_large jobs): the warps sort 64 samples each, then the
 //   threads of four of them, one a bin, take their own first group with
 //   samples, then the next, so that cells far apart in a row progress together;
 //   busy bins are spread over the four warps. (Four warps in all: the 1500
@@ -815,14 +847,15 @@ __device__ __forceinline__ float desc_norm(const float *sq) {
 constexpr int kDescWarps = kDescThreads / 32;
 constexpr int kDescCtaWarps = 8, kDescCtaThreads = 32 * kDescCtaWarps;  // of a large window
 
+constexpr int kDescSets = 2, kDescCtaSets = 2;  // of 32 samples a warp sorts at a time: its own feature's, a CTA's
 struct __align__(16) DescWarpSmem {  // one per warp, side by side: list is read as float4
-    DescGroup g;
+    DescGroup<kDescSets> g;
     uint32_t first[kDescWarpSide + 1];
     int16_t left[kDescWarpSide + 1];
 };
-static_assert(sizeof(DescWarpSmem) % 16 == 0 && sizeof(DescGroup) % 16 == 0, "alignment of the vector accesses");
+static_assert(sizeof(DescWarpSmem) % 16 == 0 && sizeof(DescGroup<kDescCtaSets>) % 16 == 0 && sizeof(DescGroup<kDescSets>) % 16 == 0, "alignment of the vector accesses");
 struct __align__(16) DescCtaSmem {
-    DescGroup g[2][kDescCtaWarps];
+    DescGroup<kDescCtaSets> g[2][kDescCtaWarps];
     uint32_t wsum[kDescCtaWarps];
     float norm;
 };
@@ -852,17 +885,22 @@ __device__ void describe_warp(const DescribeArgs &a, uint32_t k, DescWarpSmem &S
     desc_group_init(S.g, lane);
     float acc[4] = {0.0f, 0.0f, 0.0f, 0.0f};  // this lane's bins (desc_group)
     int row = 0;
-    for (uint32_t base = 0; base < total; base += 32) {
-        const uint32_t t = base + lane;
-        uint32_t code = 0, n[4], at;
-        float prod[8];
-        bool valid = false;
-        if (t < total) {
-            while (t >= S.first[row + 1]) ++row;
-            const int px = W.xi + S.left[row] + (int)(t - S.first[row]), py = W.yi + row - W.r;
-            valid = desc_sample(W, px, py, prod, code);
+    for (uint32_t base = 0; base < total; base += 32 * kDescSets) {
+        DescSample smp[kDescSets];
+        bool valid[kDescSets];
+        uint32_t n[4], at;
+#pragma unroll
+        for (int e = 0; e < kDescSets; ++e) {
+            const uint32_t t = base + 32 * e + lane;
+            valid[e] = false;
+            smp[e].code = 0;
+            if (t < total) {
+                while (t >= S.first[row + 1]) ++row;
+                const int px = W.xi + S.left[row] + (int)(t - S.first[row]), py = W.yi + row - W.r;
+                valid[e] = desc_sample(W, px, py, smp[e]);
+            }
         }
-        desc_group(prod, code, valid, lane, S.g, n, at);
+        desc_group<kDescSets>(smp, valid, lane, S.g, n, at);
         __syncwarp();
         // the lane's bins lie one after the other; each run of four is one bin's
         const float4 *l = reinterpret_cast<const float4 *>(S.g.list) + at;
@@ -947,30 +985,40 @@ __device__ void describe_cta(const DescribeArgs &a, uint32_t k, DescCtaSmem &S, 
     const uint32_t place = ((iv + 1) * 6 + iu + 1) * 8 + io;
     float acc = 0.0f;  // bin (iv, iu, io)
     int row = 0, par = 0;
-    for (uint32_t base = 0; base < total; base += kDescCtaThreads, par ^= 1) {
-        const uint32_t t = base + tid;
-        uint32_t code = 0, n[4], at;
-        float prod[8];
-        bool valid = false;
-        if (t < total) {
-            while (t >= first[row + 1]) ++row;
-            const int px = W.xi + left[row] + (int)(t - first[row]), py = W.yi + row - W.r;
-            valid = desc_sample(W, px, py, prod, code);
+    for (uint32_t base = 0; base < total; base += kDescCtaThreads * kDescCtaSets, par ^= 1) {
+        uint32_t n[4], at;
+        DescSample smp[kDescCtaSets];
+        bool valid[kDescCtaSets];
+#pragma unroll
+        for (int e = 0; e < kDescCtaSets; ++e) {
+            const uint32_t t = base + 32 * (kDescCtaSets * warp + e) + lane;
+            valid[e] = false;
+            smp[e].code = 0;
+            if (t < total) {
+                while (t >= first[row + 1]) ++row;
+                const int px = W.xi + left[row] + (int)(t - first[row]), py = W.yi + row - W.r;
+                valid[e] = desc_sample(W, px, py, smp[e]);
+            }
         }
-        desc_group(prod, code, valid, lane, S.g[par][warp], n, at);
-        __syncthreads();  // one per 256 samples: the buffers take turns
+        desc_group<kDescCtaSets>(smp, valid, lane, S.g[par][warp], n, at);
+        __syncthreads();  // one for the warps' samples: the buffers take turns
         if (!owner) continue;
         uint32_t some = 0;
 #pragma unroll
         for (int g = 0; g < kDescCtaWarps; ++g) {
-            const DescGroup &G = S.g[par][g];
-            some |= (G.any[1 + iv] & G.any[7 + iu] & G.any[12 + io]) ? 1u << g : 0u;
+            const DescGroup<kDescCtaSets> &G = S.g[par][g];
+            uint32_t m = 0;
+#pragma unroll
+            for (int e = 0; e < kDescCtaSets; ++e) m |= G.any[e][1 + iv] & G.any[e][7 + iu] & G.any[e][12 + io];
+            some |= m ? 1u << g : 0u;
         }
         while (some) {
-            const DescGroup &G = S.g[par][__ffs(some) - 1];
+            const DescGroup<kDescCtaSets> &G = S.g[par][__ffs(some) - 1];
             some &= some - 1;
             const float4 *l = reinterpret_cast<const float4 *>(G.list + G.off[place]);
-            const int m = __popc(G.any[1 + iv] & G.any[7 + iu] & G.any[12 + io]);
+            int m = 0;
+#pragma unroll
+            for (int e = 0; e < kDescCtaSets; ++e) m += __popc(G.any[e][1 + iv] & G.any[e][7 + iu] & G.any[e][12 + io]);
             for (int i = 0; i < m; i += 4, ++l) {
                 const float4 f = *l;
                 acc += f.x;
