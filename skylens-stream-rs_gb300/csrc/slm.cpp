@@ -370,7 +370,7 @@ void plan_items(slm_plan *p) {
     if (row_tiles && row_tiles < want) split = (uint32_t)((want + row_tiles - 1) / row_tiles);
     ExactShapes shapes;
     for (uint32_t k = 0; k < p->np; ++k) shapes.add(p->meta[k].na, p->meta[k].nb);
-    const bool few = !p->tune.items_per_sm && shapes.few(std::max(1, p->ctx->sms));
+    const bool few = (!p->tune.items_per_sm || p->tune.items_per_sm == 4) && shapes.few(std::max(1, p->ctx->sms));
     const ExactShape shape = few ? shapes.best(std::max(1, p->ctx->sms)) : ExactShape{};
     p->items.clear();
     uint32_t part = 0;
