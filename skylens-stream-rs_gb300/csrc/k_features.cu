@@ -480,106 +480,153 @@ __global__ void __launch_bounds__(256) candidate_sigma_kernel(FeatCand *cands, c
 
 // --------------------------------------------------------------- orientations
 
-// One warp per candidate (orientations_with, features.rs:361-420): samples of
-// the (2r+1)^2 window in raster order, 32 at a time; lane b owns bins b and b +
-// 32 and adds the samples whose bin number's bits (by ballot) are its own, in
-// raster order (0.42 -> 0.19 ms for 24 views of 960 x 540, against passing all
-// 32 samples to every lane); then the lanes smooth and pick the peaks.
+// orientations_with (features.rs:361-420): samples of the (2r+1)^2 window in raster
+// order, 32 at a time; lane b owns bins b and b + 32 and adds the samples whose bin
+// number's bits (by ballot) are its own, in raster order (0.42 -> 0.19 ms for 24
+// views of 960 x 540, against passing all 32 samples to every lane); then the lanes
+// smooth and pick the peaks. One warp per candidate, or, while there are fewer
+// candidates than the SMs hold CTAs, one CTA: its warps take 32 samples each and
+// the first one adds them, set after set (one image's 700 candidates are a warp's
+// chain of 50 steps of 0.9 us each: 48 us, 30 with eight warps; with a CTA for each of
+// 3000 a call of 24 views takes 2.61 ms instead of 2.39).
+constexpr uint32_t kOriFew = 8;  // candidates a SM up to which each has a CTA
+struct OriWindow {
+    const float2 *grad;
+    int w, h, r, xi, yi, side, total;
+    float x, y, sw;
+};
+__device__ __forceinline__ OriWindow ori_window(const OrientArgs &a, uint32_t ci) {
+    const FeatCand c = a.cands[ci];
+    const OctaveGeom &G = a.geom[c.octave];
+    OriWindow W;
+    W.grad = a.grads + G.grad_off + ((uint64_t)c.img * a.s + (c.layer - 1)) * G.layer_stride;
+    W.w = G.w;
+    W.h = G.h;
+    W.x = c.x;
+    W.y = c.y;
+    W.sw = 1.5f * c.sig;
+    W.r = f2i(roundf(3.0f * W.sw));
+    W.xi = f2i(roundf(c.x));
+    W.yi = f2i(roundf(c.y));
+    W.side = 2 * W.r + 1;
+    W.total = W.side * W.side;
+    return W;
+}
+
+// Sample t's bin (63: none, no lane's bin) and value.
+__device__ __forceinline__ int ori_sample(const OriWindow &W, int t, float &val) {
+    val = 0.0f;
+    if (t >= W.total) return 63;
+    const int px = W.xi + (t % W.side) - W.r, py = W.yi + (t / W.side) - W.r;
+    if (px < 1 || py < 1 || px >= W.w - 1 || py >= W.h - 1) return 63;
+    const float2 gm = W.grad[(uint64_t)py * W.w + px];
+    const float fx = (float)px - W.x, fy = (float)py - W.y;
+    const float wgt = exp_cr(-(fx * fx + fy * fy) / (2.0f * W.sw * W.sw));
+    const float ang = rem_euclid(gm.y, kTwoPi);
+    const float bf = roundf(ang / kTwoPi * (float)kOriBins);
+    val = wgt * gm.x;
+    return (int)((unsigned)(bf < 0.0f ? 0 : f2i(bf)) % kOriBins);
+}
+
+// The lane's bins of 32 samples, whose values lie in vals (by a whole warp).
+__device__ __forceinline__ void ori_add(int bin, const float *vals, int lane, float &h0, float &h1) {
+    uint32_t low = ~0u;
+#pragma unroll
+    for (int k = 0; k < 5; ++k)  // the bits that make a bin number this lane's, and (lanes 0-3) this lane's + 32
+        low &= __ballot_sync(0xffffffffu, (bin >> k) & 1) ^ ((lane >> k) & 1 ? 0u : ~0u);
+    const uint32_t high = __ballot_sync(0xffffffffu, bin >> 5);
+    for (uint32_t m = low & ~high; m; m &= m - 1) h0 += vals[__ffs(m) - 1];
+    if (lane < kOriBins - 32)
+        for (uint32_t m = low & high; m; m &= m - 1) h1 += vals[__ffs(m) - 1];
+}
+
+// Smooths the histogram and writes its peaks (by a whole warp).
+__device__ __forceinline__ void ori_peaks(const OrientArgs &a, uint32_t ci, float *hist, int lane, float h0, float h1) {
+    // six [1,1,1]/3 smoothings, lane b computing bins b and b + 32 (each bin
+    // from the previous pass's three, ((l + c) + r) / 3 as the reference)
+    const int b1 = lane + 32;
+    const bool has1 = b1 < kOriBins;
+    for (int it = 0; it < 6; ++it) {
+        hist[lane] = h0;
+        if (has1) hist[b1] = h1;
+        __syncwarp();
+        const float n0 = (hist[(lane + kOriBins - 1) % kOriBins] + h0 + hist[(lane + 1) % kOriBins]) / 3.0f;
+        const float n1 = has1 ? (hist[(b1 + kOriBins - 1) % kOriBins] + h1 + hist[(b1 + 1) % kOriBins]) / 3.0f : 0.0f;
+        __syncwarp();
+        h0 = n0;
+        h1 = n1;
+    }
+    hist[lane] = h0;
+    if (has1) hist[b1] = h1;
+    __syncwarp();
+    // fold(0.0, f32::max): fmaxf is order-free (NaN ignored either way)
+    float mx = fmaxf(h0, has1 ? h1 : 0.0f);
+#pragma unroll
+    for (int o = 16; o; o >>= 1) mx = fmaxf(mx, __shfl_xor_sync(0xffffffffu, mx, o));
+    mx = fmaxf(0.0f, mx);
+    // peaks in bin order: bins 0..31 by lane, then 32..35
+    float *out = a.angles + (uint64_t)ci * kMaxAngles;
+    int na = 0;
+    if (mx > 0.0f) {
+#pragma unroll
+        for (int half = 0; half < 2; ++half) {
+            const int i = half ? b1 : lane;
+            bool peak = false;
+            float ang = 0.0f;
+            if (i < kOriBins) {
+                const float l = hist[(i + kOriBins - 1) % kOriBins], cc = hist[i], rr = hist[(i + 1) % kOriBins];
+                if (cc >= 0.8f * mx && cc > l && cc > rr) {
+                    const float off = 0.5f * (l - rr) / (l - 2.0f * cc + rr);
+                    ang = rem_euclid(((float)i + off) / (float)kOriBins * kTwoPi, kTwoPi);
+                    peak = true;
+                }
+            }
+            const unsigned m = __ballot_sync(0xffffffffu, peak);
+            if (peak) out[na + __popc(m & ((1u << lane) - 1u))] = ang;
+            na += __popc(m);
+        }
+    }
+    if (lane == 0) a.nang[ci] = (uint8_t)na;
+}
+
 __global__ void __launch_bounds__(256) orient_kernel(OrientArgs a) {
     __shared__ float hs[8][kOriBins];
-    __shared__ float vals[8][32];
+    __shared__ float vals[2][8][32];
+    __shared__ uint8_t bins[2][8][32];
     const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
     grid_wait();
     grid_go();
     const uint32_t n = min(*a.count, a.cap);
+    if (n <= a.few) {  // a CTA each
+        int par = 0;
+        for (uint32_t ci = blockIdx.x; ci < n; ci += gridDim.x) {
+            const OriWindow W = ori_window(a, ci);
+            float h0 = 0.0f, h1 = 0.0f;
+            for (int base = 0; base < W.total; base += 256, par ^= 1) {  // the buffers take turns
+                float v;
+                bins[par][warp][lane] = (uint8_t)ori_sample(W, base + threadIdx.x, v);
+                vals[par][warp][lane] = v;
+                __syncthreads();
+                if (warp == 0)
+                    for (int e = 0; e < 8 && base + 32 * e < W.total; ++e)
+                        ori_add(bins[par][e][lane], vals[par][e], lane, h0, h1);
+            }
+            if (warp == 0) ori_peaks(a, ci, hs[0], lane, h0, h1);
+        }
+        return;
+    }
     for (uint32_t ci = blockIdx.x * 8 + warp; ci < n; ci += gridDim.x * 8) {  // warp-uniform
-        const FeatCand c = a.cands[ci];
-        const OctaveGeom &G = a.geom[c.octave];
-        const float2 *grad = a.grads + G.grad_off + ((uint64_t)c.img * a.s + (c.layer - 1)) * G.layer_stride;
-        const int w = G.w, h = G.h;
-        const float sw = 1.5f * c.sig;
-        const int r = f2i(roundf(3.0f * sw));
-        const int xi = f2i(roundf(c.x)), yi = f2i(roundf(c.y));
-        const int side = 2 * r + 1;
-        const int total = side * side;
+        const OriWindow W = ori_window(a, ci);
         float h0 = 0.0f, h1 = 0.0f;
-        // the bits that make a bin number this lane's, and (lanes 0-3) this lane's + 32
-        uint32_t inv[5];
-#pragma unroll
-        for (int k = 0; k < 5; ++k) inv[k] = (lane >> k) & 1 ? 0u : ~0u;
-        for (int base = 0; base < total; base += 32) {
-            const int t = base + lane;
-            int bin = 63;  // none: no lane's bin
-            float val = 0.0f;
-            if (t < total) {
-                const int px = xi + (t % side) - r, py = yi + (t / side) - r;
-                if (!(px < 1 || py < 1 || px >= w - 1 || py >= h - 1)) {
-                    const float2 gm = grad[(uint64_t)py * w + px];
-                    const float fx = (float)px - c.x, fy = (float)py - c.y;
-                    const float wgt = exp_cr(-(fx * fx + fy * fy) / (2.0f * sw * sw));
-                    const float ang = rem_euclid(gm.y, kTwoPi);
-                    const float bf = roundf(ang / kTwoPi * (float)kOriBins);
-                    bin = (int)((unsigned)(bf < 0.0f ? 0 : f2i(bf)) % kOriBins);
-                    val = wgt * gm.x;
-                }
-            }
-            uint32_t low = ~0u;
-#pragma unroll
-            for (int k = 0; k < 5; ++k) low &= __ballot_sync(0xffffffffu, (bin >> k) & 1) ^ inv[k];
-            const uint32_t high = __ballot_sync(0xffffffffu, bin >> 5);
-            vals[warp][lane] = val;
+        for (int base = 0; base < W.total; base += 32) {
+            float v;
+            const int bin = ori_sample(W, base + lane, v);
+            vals[0][warp][lane] = v;
             __syncwarp();
-            for (uint32_t m = low & ~high; m; m &= m - 1) h0 += vals[warp][__ffs(m) - 1];
-            if (lane < kOriBins - 32)
-                for (uint32_t m = low & high; m; m &= m - 1) h1 += vals[warp][__ffs(m) - 1];
+            ori_add(bin, vals[0][warp], lane, h0, h1);
             __syncwarp();
         }
-        // six [1,1,1]/3 smoothings, lane b computing bins b and b + 32 (each bin
-        // from the previous pass's three, ((l + c) + r) / 3 as the reference)
-        float *hist = hs[warp];
-        const int b1 = lane + 32;
-        const bool has1 = b1 < kOriBins;
-        for (int it = 0; it < 6; ++it) {
-            hist[lane] = h0;
-            if (has1) hist[b1] = h1;
-            __syncwarp();
-            const float n0 = (hist[(lane + kOriBins - 1) % kOriBins] + h0 + hist[(lane + 1) % kOriBins]) / 3.0f;
-            const float n1 = has1 ? (hist[(b1 + kOriBins - 1) % kOriBins] + h1 + hist[(b1 + 1) % kOriBins]) / 3.0f : 0.0f;
-            __syncwarp();
-            h0 = n0;
-            h1 = n1;
-        }
-        hist[lane] = h0;
-        if (has1) hist[b1] = h1;
-        __syncwarp();
-        // fold(0.0, f32::max): fmaxf is order-free (NaN ignored either way)
-        float mx = fmaxf(h0, has1 ? h1 : 0.0f);
-#pragma unroll
-        for (int o = 16; o; o >>= 1) mx = fmaxf(mx, __shfl_xor_sync(0xffffffffu, mx, o));
-        mx = fmaxf(0.0f, mx);
-        // peaks in bin order: bins 0..31 by lane, then 32..35
-        float *out = a.angles + (uint64_t)ci * kMaxAngles;
-        int na = 0;
-        if (mx > 0.0f) {
-#pragma unroll
-            for (int half = 0; half < 2; ++half) {
-                const int i = half ? b1 : lane;
-                bool peak = false;
-                float ang = 0.0f;
-                if (i < kOriBins) {
-                    const float l = hist[(i + kOriBins - 1) % kOriBins], cc = hist[i], rr = hist[(i + 1) % kOriBins];
-                    if (cc >= 0.8f * mx && cc > l && cc > rr) {
-                        const float off = 0.5f * (l - rr) / (l - 2.0f * cc + rr);
-                        ang = rem_euclid(((float)i + off) / (float)kOriBins * kTwoPi, kTwoPi);
-                        peak = true;
-                    }
-                }
-                const unsigned m = __ballot_sync(0xffffffffu, peak);
-                if (peak) out[na + __popc(m & ((1u << lane) - 1u))] = ang;
-                na += __popc(m);
-            }
-        }
-        if (lane == 0) a.nang[ci] = (uint8_t)na;
+        ori_peaks(a, ci, hs[warp], lane, h0, h1);
     }
 }
 
@@ -1174,7 +1221,9 @@ void launch_candidate_sigma(FeatCand *cands, const uint32_t *count, uint32_t cap
 
 void launch_orient(const OrientArgs &a, int sms, cudaStream_t s) {
     const uint32_t grid = (a.cap + 7) / 8 < 16u * sms ? (a.cap + 7) / 8 : 16u * sms;
-    launch_next(orient_kernel, grid, 256, 0, s, a);
+    OrientArgs b = a;
+    b.few = kOriFew * (uint32_t)sms;
+    launch_next(orient_kernel, grid, 256, 0, s, b);
 }
 
 void launch_describe(const DescribeArgs &a, uint32_t njobs, cudaStream_t s) {

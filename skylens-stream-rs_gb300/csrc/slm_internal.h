@@ -253,6 +253,7 @@ struct OrientArgs {
     int s;
     float *angles;          // kMaxAngles per candidate
     uint8_t *nang;
+    uint32_t few;           // launch_orient's: up to so many candidates have a CTA each
 };
 
 struct DescJob {
