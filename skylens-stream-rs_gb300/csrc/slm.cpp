@@ -3632,13 +3632,17 @@ extern "C" slm_status slm_build_tracks_drop(slm_ctx *c, const uint32_t *n_featur
     for (uint32_t i = 0; i < n_images; ++i) off[i + 1] = off[i] + n_features[i];
     const uint64_t n = off[n_images];
     if (n >= 0xffffffffull) return fail(SLM_INVALID_ARG, "at most 2^32 - 2 features in all");
-    uint64_t n_match = 0;
+    uint64_t n_match = 0, n_edge = 0;  // matches in the array; edges they may make
     for (uint32_t p = 0; p < n_pairs; ++p) {
         if (pairs[p].count > ~0ull - pairs[p].first) return fail(SLM_INVALID_ARG, "a pair's match range overflows");
         n_match = std::max(n_match, pairs[p].first + pairs[p].count);
+        n_edge += std::min<uint64_t>(pairs[p].count, ~0ull - n_edge);
     }
+    // pairs may name the same matches: each makes edges of its own, so the edges
+    // are counted by pair, not by the array's length; no two are the same
+    n_edge = std::min<uint64_t>(n_edge, n ? n * (n - 1) / 2 : 0);
     if (n_match && !matches) return fail(SLM_INVALID_ARG, "NULL matches");
-    if (n_match > (1ull << 34)) return fail(SLM_INVALID_ARG, "more than 2^34 matches");
+    if (std::max(n_match, n_edge) > (1ull << 34)) return fail(SLM_INVALID_ARG, "more than 2^34 matches");
     SLM_TRY(ctx_check_device(c));
     // what the stream reads and writes outlives it
     std::vector<TrackPair> tp(n_pairs);
@@ -3657,8 +3661,8 @@ extern "C" slm_status slm_build_tracks_drop(slm_ctx *c, const uint32_t *n_featur
         ~Drain() { cudaStreamSynchronize(s); }
     } drain{s};
     uint64_t slots = 1024;
-    while (slots < 2 * n_match) slots <<= 1;
-    const uint64_t linked = std::min(n, 2 * n_match);  // nodes with an edge
+    while (slots < 2 * n_edge) slots <<= 1;
+    const uint64_t linked = std::min(n, 2 * n_edge);  // nodes with an edge
     const uint64_t comps = linked / 2;                 // of two nodes at least
     const uint64_t share = std::max<uint64_t>(1024, (n / 1024 + 256) / 256 * 256);
     const uint64_t o_pairs = 0, o_match = feat_align(sizeof(TrackPair) * (uint64_t)n_pairs),
@@ -3696,7 +3700,7 @@ extern "C" slm_status slm_build_tracks_drop(slm_ctx *c, const uint32_t *n_featur
         a.start = reinterpret_cast<uint32_t *>(d + o_start);
         a.members = reinterpret_cast<uint32_t *>(d + o_memb);
         a.spare = a.parent;
-        a.sorted = reinterpret_cast<uint2 *>(a.table);  // 16 n_match bytes or more
+        a.sorted = reinterpret_cast<uint2 *>(a.table);  // 16 n_edge bytes or more
         a.comps = reinterpret_cast<uint2 *>(d + o_comp);
         a.max_comps = comps;
         a.share = share;

@@ -1,0 +1,47 @@
+// Checks of the library's host code on the CPU: csrc/slm.cpp, over the fake runtime of
+// fake_cuda.h. Each check is a function of its own; `host_checks NAME` runs one
+// (tests/test_host_checks.py builds this file and runs them all).
+#include "fake_cuda.h"
+
+#include "slm.cpp"
+
+#define REQUIRE(x)                                                                                    \
+    do {                                                                                              \
+        if (!(x)) return std::printf("%s:%d: %s (last error: %s)\n", __FILE__, __LINE__, #x, slm_last_error()), 1; \
+    } while (0)
+
+// Scratch of slm_build_tracks_drop when pairs name the same matches: every pair's
+// matches are edges of their own.
+int tracks_that_share_matches() {
+    slm_ctx *c = nullptr;
+    REQUIRE(slm_ctx_create(nullptr, &c) == SLM_OK);
+    const uint32_t images = 64, features = 1000, np = images / 2;
+    std::vector<uint32_t> nf(images, features);
+    std::vector<slm_pair> m(features);
+    for (uint32_t k = 0; k < features; ++k) m[k] = slm_pair{k, k};
+    std::vector<slm_pair_matches> pairs(np);
+    for (uint32_t p = 0; p < np; ++p) pairs[p] = slm_pair_matches{2 * p, 2 * p + 1, 0, features};
+    uint64_t nt = 0, no = 0;
+    REQUIRE(slm_build_tracks_drop(c, nf.data(), images, pairs.data(), np, m.data(), 2, 100, nullptr, 0, nullptr, 0, &nt, &no,
+                                  nullptr) == SLM_OK);
+    const slm::TrackArgs &a = fake::tracks;
+    const uint64_t edges = uint64_t(np) * features, linked = 2 * edges;  // all distinct, no node shared
+    auto room = [](const void *from, const void *to) { return uint64_t(static_cast<const char *>(to) - static_cast<const char *>(from)); };
+    REQUIRE(a.table_mask + 1 >= edges);
+    REQUIRE(8 * (a.table_mask + 1) >= 8 * linked);  // `sorted` lies over the table
+    REQUIRE(room(a.members, a.comps) >= 4 * linked);
+    REQUIRE(a.max_comps >= edges);
+    REQUIRE(room(a.comps, a.sums) >= 8 * edges);
+    REQUIRE(room(a.track_off, a.obs) >= 8 * (edges + 1));
+    slm_ctx_destroy(c);
+    return 0;
+}
+
+int main(int argc, char **argv) {
+    const std::map<std::string, int (*)()> checks = {
+        {"tracks_that_share_matches", tracks_that_share_matches},
+    };
+    if (argc == 2 && checks.count(argv[1])) return checks.at(argv[1])();
+    for (const auto &k : checks) std::printf("%s\n", k.first.c_str());
+    return argc > 1;
+}

@@ -163,3 +163,29 @@ def test_long_components(matcher, length, twist):
 def test_every_match_invalid(matcher):
     assert both(matcher, [0, 0], [(0, 1, [(0, 0), (1, 0)])])[1]["invalid_matches"] == 2
     assert both(matcher, [], [(0, 1, [(0, 0)])])[1]["invalid_matches"] == 1
+
+
+@pytest.mark.parametrize("share", ["all", "overlap"])
+def test_pairs_that_share_matches(matcher, share):
+    # pairs naming the same matches of the flat array, or ranges that overlap:
+    # more edges than the array has matches
+    rng = np.random.default_rng(11)
+    n_images, n = 60, 400
+    nf = [n] * n_images
+    flat = np.stack([rng.permutation(n), rng.permutation(n)], 1).astype(np.uint32)
+    spec = [(a, a + 1, 0 if share == "all" else 3 * a, n if share == "all" else 100) for a in range(n_images - 1)]
+    pairs = [(a, b, flat[f:f + c]) for a, b, f, c in spec]
+    arr = (T.SlmPairMatches * len(spec))(*[T.SlmPairMatches(a, b, f, c) for a, b, f, c in spec])
+    want = O.build_tracks_drop(nf, pairs)
+    P = ctypes.POINTER
+    nfa = np.asarray(nf, np.uint32)
+    cap = sum(len(p[2]) for p in pairs)
+    toff, obs = np.zeros(cap + 1, np.uint64), np.zeros((2 * cap, 2), np.uint32)
+    nt, no, st = ctypes.c_uint64(), ctypes.c_uint64(), T.SlmTrackStats()
+    assert matcher._L.slm_build_tracks_drop(matcher.handle, nfa.ctypes.data_as(P(ctypes.c_uint32)), n_images, arr, len(spec),
+                                            flat.ctypes.data_as(P(T.SlmPair)), 3, 100000,
+                                            toff.ctypes.data_as(P(ctypes.c_uint64)), cap, obs.ctypes.data_as(P(T.SlmPair)),
+                                            2 * cap, ctypes.byref(nt), ctypes.byref(no), ctypes.byref(st)) == 0
+    got = [[(int(i), int(f)) for i, f in obs[int(toff[t]):int(toff[t + 1])]] for t in range(nt.value)]
+    assert got == want[0] and st.as_dict() == want[1]
+    assert st.as_dict()["edges"] > len(flat)
