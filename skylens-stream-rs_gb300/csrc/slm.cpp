@@ -311,6 +311,7 @@ struct slm_plan {
     uint64_t top_parts = 0;
     DevBuf d_topmm, d_topj, d_olist, d_ulist, d_ugroups;
     bool dump = false;
+    uint64_t raw_epoch = 0;          // the store's epoch whose a_raw0 and b_raw0 `meta` holds
     uint32_t min_matches = 0;        // pairs with fewer matches report none
     cudaGraphExec_t exec = nullptr;
     cudaGraph_t graph = nullptr;
@@ -713,6 +714,7 @@ slm_status plan_build(slm_plan *p, const slm_pair *pairs) {
         dist += (uint64_t)m.na * m.nb;
     }
     p->slot_off[p->np] = slot;
+    p->raw_epoch = st->epoch;
     p->n_cols = col;
     p->n_slots = slot;
     p->distances = dist;
@@ -1436,9 +1438,36 @@ slm_status plan_init(slm_plan *p, slm_ctx *c, slm_store *st, const slm_pair *pai
     return plan_build(p, pairs);
 }
 
+// A plan outlives slm_store_clear: it names views by their tiles, and those lie
+// where they lay when views of the same sizes are added again. Their row-major rows
+// have no padding, so they move when a view before them has another number of rows
+// within its tiles: looked up again, and uploaded, when the store was cleared.
+slm_status plan_sync_raw(slm_plan *p, cudaStream_t s) {
+    const slm_store *st = p->st;
+    if (p->prec == SLM_PREC_FP32 || p->raw_epoch == st->epoch) return SLM_OK;  // FP32 plans read tiles only
+    bool moved = false, found = true;
+    auto look = [&](uint32_t view, uint32_t row0, uint32_t &raw0) {
+        const bool there = view < st->row0.size() && st->row0[view] == row0;
+        found &= there;
+        if (!there || st->raw0[view] == raw0) return;
+        raw0 = st->raw0[view];  // at or below row0: in bounds for the plan's rows
+        moved = true;
+    };
+    for (uint32_t k = 0; k < p->np; ++k) {
+        PairMeta &m = p->meta[k];
+        look(p->spairs[k].view_a, m.a_row0, m.a_raw0);
+        look(p->spairs[k].view_b, m.b_row0, m.b_raw0);
+    }
+    if (moved)
+        SLM_CU(cudaMemcpyAsync(p->d_up.p, p->meta.data(), sizeof(PairMeta) * p->np, cudaMemcpyHostToDevice, s));
+    if (found) p->raw_epoch = st->epoch;  // else a view is still to be added: looked up at the next launch
+    return SLM_OK;
+}
+
 slm_status plan_launch_on(slm_plan *p, cudaStream_t s, bool use_graph) {
     if (p->prec != SLM_PREC_BF16) SLM_TRY(store_sync_fp32(p->st, s));
     SLM_TRY(store_sync_plan_images(p->st, p->prec, s));
+    SLM_TRY(plan_sync_raw(p, s));
     // a store buffer the captured graph reads may have moved: capture again
     if (p->exec && (p->st->tiled.p != p->graph_tiled || p->st->lowp[0].optiles.p != p->graph_optiles[0] ||
                     p->st->lowp[1].optiles.p != p->graph_optiles[1])) {

@@ -95,3 +95,36 @@ def test_more_views_than_one_copy_each(matcher, memory):
         assert np.array_equal(got[k], O.ratio_match_np(a, b, 0.8, True, threads=2)), (u, v)
     plan.close()
     st.close()
+
+
+@pytest.mark.parametrize("prec", ["fp32", "bf16", "fp8"])
+@pytest.mark.parametrize("use_graph", [1, 2])
+def test_plan_kept_while_the_views_are_exchanged(matcher, prec, use_graph):
+    """A plan names views by their place in the store: after a clear and new views
+    of the same sizes it matches those, also when a view it does not name has
+    another number of rows within the same tiles."""
+    rng = np.random.Generator(np.random.PCG64(44))
+    counts = [300, 700, 650, 90]
+    st = matcher.store(2000, 4)
+
+    def views(n0, n3):
+        base = synth.sift_like(rng, 700)
+        v = [synth.sift_like(rng, n0), base, np.concatenate([synth.noisy_copy(rng, base[rng.permutation(700)[:400]], 0.05),
+                                                             synth.sift_like(rng, 250)]), synth.sift_like(rng, n3)]
+        return v, st.add_views_packed(np.concatenate(v), np.concatenate([[0], np.cumsum([len(x) for x in v])[:-1]]),
+                                      [len(x) for x in v])
+
+    v, ids = views(counts[0], counts[3])
+    pairs = [(1, 2), (2, 1)]
+    plan = st.plan(pairs, 0.8, True, prec, use_graph=use_graph)
+    for n0, n3 in ((300, 90), (310, 90), (257, 128), (384, 1)):
+        st.clear()
+        v, ids = views(n0, n3)
+        plan.launch()
+        got = plan.per_pair()
+        for k, (a, b) in enumerate(pairs):
+            want = O.ratio_match_np(v[a], v[b], 0.8, True, threads=8)
+            assert len(want) > 100
+            assert np.array_equal(got[k], want), (n0, n3, a, b)
+    plan.close()
+    st.close()
