@@ -2648,7 +2648,10 @@ extern "C" slm_status slm_sampson_score(slm_ctx *c, const double *pts, const uin
         if (e == cudaSuccess && mask_off && mask_words)
             e = cudaMemcpyAsync(masks, d + o_mask, 4 * mask_words, cudaMemcpyDeviceToHost, s);
         if (e == cudaSuccess) e = cudaStreamSynchronize(s);
-        if (e != cudaSuccess) st = fail(SLM_CUDA_ERROR, std::string("slm_sampson_score: ") + cudaGetErrorString(e));
+        if (e != cudaSuccess) {
+            st = fail(SLM_CUDA_ERROR, std::string("slm_sampson_score: ") + cudaGetErrorString(e));
+            cudaStreamSynchronize(s);  // the kernel may still read the caller's arrays
+        }
     }
     ws_release(c, w);
     return st;

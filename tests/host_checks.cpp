@@ -37,9 +37,38 @@ int tracks_that_share_matches() {
     return 0;
 }
 
+// What a call's kernels may read in the caller's memory must be read when it returns,
+// also when a later step fails.
+size_t last(const char *what) {
+    for (size_t k = fake::log.size(); k; --k)
+        if (fake::log[k - 1] == what) return k;
+    return 0;
+}
+
+int sampson_waits_after_a_failure() {
+    slm_ctx *c = nullptr;
+    REQUIRE(slm_ctx_create(nullptr, &c) == SLM_OK);
+    std::vector<double> pts(4 * 10, 0.5), E(9 * 3, 0.25), th(1, 0.1);
+    const uint64_t off[2] = {0, 10}, mo[3] = {0, ~0ull, 1};
+    const uint32_t hp[3] = {0, 0, 0};
+    uint32_t counts[3], masks[2];
+    for (int nth = 1; nth <= 2; ++nth) {  // the counts' copy back, then the masks'
+        fake::log.clear();
+        fake::fail_d2h = nth;
+        REQUIRE(slm_sampson_score(c, pts.data(), off, 1, th.data(), E.data(), hp, 3, counts, mo, masks, 2) == SLM_CUDA_ERROR);
+        REQUIRE(fake::sampson.E == E.data());  // read where it lies
+        REQUIRE(last("sampson") && last("copy failed") > last("sampson"));
+        REQUIRE(last("sync") > last("copy failed"));
+    }
+    REQUIRE(slm_sampson_score(c, pts.data(), off, 1, th.data(), E.data(), hp, 3, counts, mo, masks, 2) == SLM_OK);
+    slm_ctx_destroy(c);
+    return 0;
+}
+
 int main(int argc, char **argv) {
     const std::map<std::string, int (*)()> checks = {
         {"tracks_that_share_matches", tracks_that_share_matches},
+        {"sampson_waits_after_a_failure", sampson_waits_after_a_failure},
     };
     if (argc == 2 && checks.count(argv[1])) return checks.at(argv[1])();
     for (const auto &k : checks) std::printf("%s\n", k.first.c_str());
