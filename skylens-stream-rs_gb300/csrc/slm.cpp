@@ -1787,10 +1787,15 @@ slm_status single_pair_enqueue(slm_ctx *c, Workspace *w, const float *a, uint32_
     return plan_launch_on(&w->plan, w->stream, false);
 }
 
+// Gives the workspace back. `drain`: first waits for its stream, for a call that may
+// have left work there which reads the caller's arrays or writes the host block
+// (one that fails half way).
 struct WsGuard {
     slm_ctx *c;
     Workspace *w;
+    bool drain = false;
     ~WsGuard() {
+        if (w && drain) cudaStreamSynchronize(w->stream);
         if (w) ws_release(c, w);
     }
 };
@@ -1887,8 +1892,12 @@ extern "C" slm_status slm_ratio_match(slm_ctx *c, const float *a, uint32_t na, c
     if (coalesce) return coalesce_call(c, a, na, b, nb, ratio, mutual, out, cap, n_out, st);
     Workspace *w = nullptr;
     SLM_TRY(ws_acquire(c, &w));
-    WsGuard guard{c, w};
-    if (prec == SLM_PREC_FP32) return single_pair_fp32(c, w, a, na, b, nb, ratio, mutual, out, cap, n_out, st);
+    WsGuard guard{c, w, true};
+    if (prec == SLM_PREC_FP32) {
+        const slm_status s = single_pair_fp32(c, w, a, na, b, nb, ratio, mutual, out, cap, n_out, st);
+        guard.drain = s != SLM_OK;
+        return s;
+    }
     SLM_TRY(single_pair_enqueue(c, w, a, na, b, nb, ratio, mutual, prec, false, st != nullptr));
     slm_plan *p = &w->plan;
     // the control words, the offsets and every slot the pairs may fill come
@@ -1900,6 +1909,7 @@ extern "C" slm_status slm_ratio_match(slm_ctx *c, const float *a, uint32_t na, c
     SLM_CU(cudaMemcpyAsync(h, p->d_ctl.p, head, cudaMemcpyDeviceToHost, w->stream));
     if (pair_bytes) SLM_CU(cudaMemcpyAsync(h + head, p->d_dense.p, pair_bytes, cudaMemcpyDeviceToHost, w->stream));
     SLM_CU(cudaStreamSynchronize(w->stream));
+    guard.drain = false;
     uint32_t ctl[16];
     std::memcpy(ctl, h, sizeof(ctl));
     SLM_TRY(status_of_word(ctl[1]));
@@ -2858,6 +2868,7 @@ void coal_loop(Coalescer *co) {
             }
             const slm_status is = coal_issue(co, &s, take);
             if (is != SLM_OK) {
+                cudaStreamSynchronize(s.w.stream);  // nothing still reads the callers' arrays
                 for (CoalReq *r : take) coal_finish(co, r, is, g_last_error);
                 co->cv_done.notify_all();
                 continue;
@@ -3635,7 +3646,10 @@ extern "C" slm_status slm_describe(slm_ctx *c, const float *img, uint32_t w, uin
         }
         if (e == cudaSuccess) e = cudaMemcpyAsync(desc, d + o_desc, 4ull * kDesc * n, cudaMemcpyDefault, st_);
         if (e == cudaSuccess) e = cudaStreamSynchronize(st_);
-        if (e != cudaSuccess) st = fail(SLM_CUDA_ERROR, std::string("slm_describe: ") + cudaGetErrorString(e));
+        if (e != cudaSuccess) {
+            st = fail(SLM_CUDA_ERROR, std::string("slm_describe: ") + cudaGetErrorString(e));
+            cudaStreamSynchronize(st_);  // a copy may still read or write the caller's arrays
+        }
     }
     ws_release(c, ws);
     return st;

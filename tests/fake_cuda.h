@@ -145,7 +145,7 @@ void launch_pack_fp32_tiles(const uint4 *, uint32_t, const float *, float *, cud
 void launch_pack_lowp(const uint4 *, uint32_t, const float *, int, uint8_t *, float *, float *, ViewStat *, cudaStream_t) {}
 void launch_gather(const uint2 *, const uint64_t *, const uint32_t *, const uint64_t *, uint32_t, uint2 *, uint64_t, cudaStream_t) {}
 void launch_copy_pairs(const uint2 *, const uint64_t *, slm_pair *, uint32_t, uint32_t *, cudaStream_t) {}
-void launch_gather_rows(const uint4 *, uint32_t, float *, cudaStream_t) {}
+void launch_gather_rows(const uint4 *, uint32_t, float *, cudaStream_t) { fake::note("gather rows"); }
 void launch_scatter_rows(const uint4 *, uint32_t, const float *, float *, cudaStream_t) {}
 void launch_scan_counts(const uint32_t *, uint32_t, uint64_t *, cudaStream_t) {}
 void launch_filter_counts(uint32_t *, uint32_t, uint32_t, cudaStream_t) {}

@@ -65,10 +65,48 @@ int sampson_waits_after_a_failure() {
     return 0;
 }
 
+int single_pair_waits_after_a_failure() {
+    slm_ctx *c = nullptr;
+    REQUIRE(slm_ctx_create(nullptr, &c) == SLM_OK);
+    void *a = nullptr;
+    REQUIRE(posix_memalign(&a, 16, 512 * 300) == 0);  // read where it lies
+    std::memset(a, 0, 512 * 300);
+    std::vector<slm_pair> out(300);
+    uint32_t n = 0;
+    for (const slm_precision prec : {SLM_PREC_BF16, SLM_PREC_FP8})
+        for (int nth = 1; nth <= 2; ++nth) {
+            fake::log.clear();
+            fake::fail_d2h = nth;
+            REQUIRE(slm_ratio_match(c, static_cast<float *>(a), 300, static_cast<float *>(a), 300, 0.8f, 1, prec, out.data(), 300, &n,
+                                    nullptr) == SLM_CUDA_ERROR);
+            REQUIRE(last("gather rows") && last("copy failed") > last("gather rows"));
+            REQUIRE(last("sync") > last("copy failed"));
+        }
+    // the same by way of the coalescer
+    REQUIRE(slm_ctx_set_coalescing(c, 0, 4) == SLM_OK);
+    fake::log.clear();
+    fake::fail_d2h = 1;
+    REQUIRE(slm_ratio_match(c, static_cast<float *>(a), 300, static_cast<float *>(a), 300, 0.8f, 1, SLM_PREC_AUTO, out.data(), 300, &n,
+                            nullptr) == SLM_CUDA_ERROR);
+    REQUIRE(last("gather rows") && last("sync") > last("copy failed"));
+    REQUIRE(slm_ctx_set_coalescing(c, 0, 0) == SLM_OK);
+    // and describe, whose image and keypoints are read by copies
+    const slm_keypoint kp{5, 5, 2, 0, 0};
+    std::vector<float> desc(128);
+    fake::log.clear();
+    fake::fail_d2h = 1;
+    REQUIRE(slm_describe(c, static_cast<float *>(a), 20, 20, &kp, 1, desc.data()) == SLM_CUDA_ERROR);
+    REQUIRE(last("sync") > last("copy failed"));
+    slm_ctx_destroy(c);
+    std::free(a);
+    return 0;
+}
+
 int main(int argc, char **argv) {
     const std::map<std::string, int (*)()> checks = {
         {"tracks_that_share_matches", tracks_that_share_matches},
         {"sampson_waits_after_a_failure", sampson_waits_after_a_failure},
+        {"single_pair_waits_after_a_failure", single_pair_waits_after_a_failure},
     };
     if (argc == 2 && checks.count(argv[1])) return checks.at(argv[1])();
     for (const auto &k : checks) std::printf("%s\n", k.first.c_str());
