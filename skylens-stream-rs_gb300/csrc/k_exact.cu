@@ -59,6 +59,9 @@ __global__ void __launch_bounds__(256) pack_fp32_tiles_kernel(const uint4 *__res
 // (the only readers of FP32 tiles on that path), packed on the device once the
 // routed pairs are known; with nothing routed every CTA returns at once. A
 // view shared by several routed pairs is packed once per pair (same values).
+// The tiles are dealt to the CTAs in turn over all pairs: dealt pair by pair, the
+// first few CTAs packed everything, and dependent launches put those on a few SMs
+// (392 pairs of 1200 x 1200: 4.6 ms, or 1.3 where they lie on different ones).
 __global__ void __launch_bounds__(256) pack_routed_kernel(const PairMeta *pairs,
                                                           const uint32_t *xlist,
                                                           const uint32_t *count,
@@ -66,14 +69,28 @@ __global__ void __launch_bounds__(256) pack_routed_kernel(const PairMeta *pairs,
     grid_wait();
     grid_go();
     __shared__ float sm[32][kDesc + 1];
+    __shared__ uint32_t tiles[256];  // of the next 256 pairs
     const uint32_t n = *count;
-    for (uint32_t k = 0; k < n; ++k) {
-        const PairMeta pm = pairs[xlist[k]];
-        const uint32_t ta = (pm.na + kTile - 1) / kTile, tb = (pm.nb + kTile - 1) / kTile;
-        for (uint32_t t = blockIdx.x; t < ta + tb; t += gridDim.x) {
-            const bool is_a = t < ta;
-            pack_view_tile(raw, tiled, is_a ? pm.a_raw0 : pm.b_raw0, is_a ? pm.a_row0 : pm.b_row0,
-                           is_a ? pm.na : pm.nb, is_a ? t : t - ta, sm);
+    uint64_t at = blockIdx.x;  // the CTA's next tile, from pair k's first on
+    for (uint32_t k0 = 0; k0 < n; k0 += 256) {
+        __syncthreads();
+        if (k0 + threadIdx.x < n) {
+            const PairMeta pm = pairs[xlist[k0 + threadIdx.x]];
+            tiles[threadIdx.x] = (pm.na + kTile - 1) / kTile + (pm.nb + kTile - 1) / kTile;
+        }
+        __syncthreads();
+        for (uint32_t k = 0; k < 256 && k0 + k < n; ++k) {  // block-uniform
+            const uint32_t all = tiles[k];
+            if (at < all) {
+                const PairMeta pm = pairs[xlist[k0 + k]];
+                const uint32_t ta = (pm.na + kTile - 1) / kTile;
+                for (; at < all; at += gridDim.x) {
+                    const bool is_a = at < ta;
+                    pack_view_tile(raw, tiled, is_a ? pm.a_raw0 : pm.b_raw0, is_a ? pm.a_row0 : pm.b_row0,
+                                   is_a ? pm.na : pm.nb, (uint32_t)(is_a ? at : at - ta), sm);
+                }
+            }
+            at -= all;
         }
     }
 }

@@ -1037,7 +1037,10 @@ SLM_DEV void block_argmin(float &d, uint32_t &idx, float *sd, uint32_t *si) {
 }
 
 // One CTA per entry of the scan queue: exact full scans, 32 distances at a
-// time (8 lanes each).
+// time (8 lanes each). Entries of pairs that were routed meanwhile (the exact
+// kernel settled those) are left out 32 at a time: when every pair is, the queue
+// holds an eighth and more of all rows, and one by one, each a chain of loads,
+// 470 K of them took 0.7 ms.
 __global__ void __launch_bounds__(256) sl_scan_kernel(SlArgs g) {
     grid_wait();
     grid_go();
@@ -1046,11 +1049,15 @@ __global__ void __launch_bounds__(256) sl_scan_kernel(SlArgs g) {
     const uint32_t lane = threadIdx.x & 31, grp = threadIdx.x >> 3;  // 32 groups of 8 lanes
     const uint32_t qn = min(g.ctl[kCtlScanLen], g.queue_cap);
     const float kInf = __int_as_float(0x7f800000);
-    for (uint32_t e = blockIdx.x; e < qn; e += gridDim.x) {
-        const SlQueue qe = g.queue[e];
+    const auto live = [&](uint64_t e0) {  // of the entries e0, e0 + gridDim.x, ..: the same in every warp
+        const uint64_t e = e0 + (uint64_t)lane * gridDim.x;
+        return __ballot_sync(0xffffffffu, e < qn && !g.spairs[g.queue[e].pair].routed);
+    };
+    for (uint64_t e0 = blockIdx.x; e0 < qn; e0 += 32ull * gridDim.x)
+    for (uint32_t todo = live(e0); todo; todo &= todo - 1) {
+        const SlQueue qe = g.queue[e0 + (uint64_t)(__ffs(todo) - 1) * gridDim.x];
         const PairMeta pm = g.pairs[qe.pair];
         const SlPair sp = g.spairs[qe.pair];
-        if (sp.routed) continue;  // block-uniform: the exact kernel settled the whole pair
         if (threadIdx.x == 0) atomicAdd(&g.ctl[qe.kind == 0 ? kCtlQueueRows : kCtlQueueCols], 1u);
         const float *A = g.raw + (size_t)pm.a_raw0 * kDesc;
         const float *B = g.raw + (size_t)pm.b_raw0 * kDesc;

@@ -144,3 +144,31 @@ def test_fp8_item_with_a_rescued_and_a_routed_pair(matcher):
         assert s["pairs_routed"] == 1
     plan.close()
     st.close()
+
+
+@pytest.mark.parametrize("n_views,step", [(24, 1), (20, 3)])
+def test_many_routed_pairs_beside_others(matcher, n_views, step):
+    """Hundreds of routed pairs of uneven sizes (their FP32 tiles are packed by all
+    CTAs in turn, 256 pairs at a time) beside pairs the BF16 bound settles and
+    columns that are scanned: every list is the oracle's."""
+    rng = np.random.Generator(np.random.PCG64(n_views))
+    base = synth.sift_like(rng, 500)
+    views = []
+    for v in range(n_views):
+        n = int(rng.integers(1, 420))
+        x = np.concatenate([synth.noisy_copy(rng, base[rng.permutation(500)[:n // 2]], 0.03), synth.sift_like(rng, n - n // 2)])
+        views.append(x * (100.0 if v % step == 0 else 1.0))  # norms above 64: routed before the pass
+    views = [np.ascontiguousarray(v, dtype=np.float32) for v in views]
+    st = matcher.store(sum(len(v) for v in views), n_views)
+    for v in views:
+        st.add_view(v)
+    pairs = [(a, b) for a in range(n_views) for b in range(n_views) if a != b]
+    plan = st.plan(pairs, 0.97, True, "bf16")
+    plan.launch()
+    got = plan.per_pair()
+    for k, (a, b) in enumerate(pairs):
+        assert np.array_equal(got[k], O.ratio_match_np(views[a], views[b], 0.97, True, threads=16)), (a, b)
+    routed = sum(a % step == 0 or b % step == 0 for a, b in pairs)
+    assert routed > 150 and plan.stats["pairs_routed"] == routed
+    plan.close()
+    st.close()
