@@ -219,9 +219,9 @@ uint32_t slm_store_num_views(slm_store *st);
 /* Tuning knobs; zero fields take the autotuned or default values. */
 typedef struct {
     uint32_t items_per_sm;  /* FP32, FP8: target work items per SM when splitting columns */
-    uint32_t shortlist_k;   /* shortlist capacity, 1..32 (0: 16). BF16: a row whose bounds decide
-                               nothing is rescored over up to 2 shortlist_k columns; FP8: records
-                               of 4-column hit groups per row, column range and column half */
+    uint32_t shortlist_k;   /* shortlist capacity, 1..32. BF16: a row whose bounds decide nothing
+                               is rescored over up to 4 shortlist_k columns (0: 128); FP8: records
+                               of 4-column hit groups per row, column range and column half (0: 16) */
     uint32_t use_graph;     /* 1: replay a captured CUDA graph (default), 2: plain launches */
     uint32_t variant;       /* FP32: 0 packed f32x2 arithmetic (default), 1 all
                                scalar; both IEEE, bit-exact.

@@ -36,15 +36,6 @@ namespace slm {
 
 // ------------------------------------------------------------------ pack
 
-// Tile `tile` of the view whose tiles start at store row `row0` and whose n rows
-// start at raw0: raw rows -> tile[slot][row]. Called by all 256 threads of a CTA alike.
-SLM_DEV void pack_view_tile(const float *__restrict__ raw, float *__restrict__ tiled, uint32_t raw0, uint32_t row0,
-                            uint32_t n, uint32_t tile, float (&sm)[32][kDesc + 1]) {
-    const float *src = raw + (size_t)raw0 * kDesc;
-    float *dst = tiled + (size_t)(row0 / kTile + tile) * kTileFloats;
-    for (int g = 0; g < 4; ++g) pack_group(src, n, dst, tile, g, sm);
-}
-
 // Many views at once: one CTA per 32-row group (blockIdx.y) of each entry of
 // a tile table {first row-major row, rows from it on, store tile, view}.
 __global__ void __launch_bounds__(256) pack_fp32_tiles_kernel(const uint4 *__restrict__ tab,
@@ -53,51 +44,6 @@ __global__ void __launch_bounds__(256) pack_fp32_tiles_kernel(const uint4 *__res
     __shared__ float sm[32][kDesc + 1];
     const uint4 e = tab[blockIdx.x];
     pack_group(raw + (size_t)e.x * kDesc, e.y, tiled + (size_t)e.z * kTileFloats, 0u, blockIdx.y, sm);
-}
-
-// The FP32 tiles of both views of every routed pair of a low-precision batch
-// (the only readers of FP32 tiles on that path), packed on the device once the
-// routed pairs are known; with nothing routed every CTA returns at once. A
-// view shared by several routed pairs is packed once per pair (same values).
-// The tiles are dealt to the CTAs in turn over all pairs: dealt pair by pair, the
-// first few CTAs packed everything, and dependent launches put those on a few SMs
-// (392 pairs of 1200 x 1200: 4.6 ms, or 1.3 where they lie on different ones).
-__global__ void __launch_bounds__(256) pack_routed_kernel(const PairMeta *pairs,
-                                                          const uint32_t *xlist,
-                                                          const uint32_t *count,
-                                                          const float *raw, float *tiled) {
-    grid_wait();
-    grid_go();
-    __shared__ float sm[32][kDesc + 1];
-    __shared__ uint32_t tiles[256];  // of the next 256 pairs
-    const uint32_t n = *count;
-    uint64_t at = blockIdx.x;  // the CTA's next tile, from pair k's first on
-    for (uint32_t k0 = 0; k0 < n; k0 += 256) {
-        __syncthreads();
-        if (k0 + threadIdx.x < n) {
-            const PairMeta pm = pairs[xlist[k0 + threadIdx.x]];
-            tiles[threadIdx.x] = (pm.na + kTile - 1) / kTile + (pm.nb + kTile - 1) / kTile;
-        }
-        __syncthreads();
-        for (uint32_t k = 0; k < 256 && k0 + k < n; ++k) {  // block-uniform
-            const uint32_t all = tiles[k];
-            if (at < all) {
-                const PairMeta pm = pairs[xlist[k0 + k]];
-                const uint32_t ta = (pm.na + kTile - 1) / kTile;
-                for (; at < all; at += gridDim.x) {
-                    const bool is_a = at < ta;
-                    pack_view_tile(raw, tiled, is_a ? pm.a_raw0 : pm.b_raw0, is_a ? pm.a_row0 : pm.b_row0,
-                                   is_a ? pm.na : pm.nb, (uint32_t)(is_a ? at : at - ta), sm);
-                }
-            }
-            at -= all;
-        }
-    }
-}
-
-void launch_pack_routed(const PairMeta *pairs, const uint32_t *xlist, const uint32_t *count, const float *raw,
-                        float *tiled, int grid, cudaStream_t s) {
-    launch_next(pack_routed_kernel, grid, 256, 0, s, pairs, xlist, count, raw, tiled);
 }
 
 void launch_pack_fp32_tiles(const uint4 *tab, uint32_t ntiles, const float *raw, float *tiled, cudaStream_t s) {

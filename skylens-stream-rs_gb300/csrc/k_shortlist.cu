@@ -31,6 +31,7 @@
 
 #include <cstdint>
 
+#include "pack.cuh"
 #include "shortlist.cuh"
 
 namespace slm {
@@ -1240,8 +1241,24 @@ __global__ void __launch_bounds__(1024) sl_route_plan_kernel(SlArgs g) {
     }
 }
 
+// Tile `tile` of the view whose tiles start at store row `row0` and whose n rows
+// start at raw0: raw rows -> tile[slot][row]. Called by all 256 threads of a CTA alike.
+SLM_DEV void pack_view_tile(const float *raw, float *tiled, uint32_t raw0, uint32_t row0, uint32_t n, uint32_t tile,
+                            float (&sm)[32][kDesc + 1]) {
+    const float *src = raw + (size_t)raw0 * kDesc;
+    float *dst = tiled + (size_t)(row0 / kTile + tile) * kTileFloats;
+    for (int g = 0; g < 4; ++g) pack_group(src, n, dst, tile, g, sm);
+}
+
 // Writes the exact work items of the routed pairs and resets their column
-// minima keys (one CTA per routed pair at a time).
+// minima keys (one CTA per routed pair at a time). PACK: also the FP32 tiles of
+// both their views, for a batch whose store does not keep them (the exact kernel
+// is their only reader on that path); a view shared by several routed pairs is
+// packed once per pair (same values). The tiles are dealt to the CTAs in turn over
+// all pairs: dealt pair by pair, the first few CTAs packed everything, and dependent
+// launches put those on a few SMs (392 pairs of 1200 x 1200: 4.6 ms, or 1.3 where they
+// lie on different ones). With nothing routed every CTA returns at once.
+template <bool PACK>
 __global__ void __launch_bounds__(256) sl_route_apply_kernel(SlArgs g) {
     grid_wait();
     grid_go();
@@ -1267,6 +1284,33 @@ __global__ void __launch_bounds__(256) sl_route_apply_kernel(SlArgs g) {
         }
         if (g.mutual)
             for (uint32_t j = threadIdx.x; j < pm.nb; j += blockDim.x) g.colbest[pm.col_base + j] = ~0ull;
+    }
+    if constexpr (PACK) {
+        __shared__ float sm[32][kDesc + 1];
+        __shared__ uint32_t tiles[256];  // of the next 256 pairs
+        float *tiled = const_cast<float *>(g.tiled);
+        uint64_t at = blockIdx.x;  // the CTA's next tile, from pair k's first on
+        for (uint32_t k0 = 0; k0 < n; k0 += 256) {
+            __syncthreads();
+            if (k0 + threadIdx.x < n) {
+                const PairMeta pm = g.pairs[g.xlist[k0 + threadIdx.x]];
+                tiles[threadIdx.x] = (pm.na + kTile - 1) / kTile + (pm.nb + kTile - 1) / kTile;
+            }
+            __syncthreads();
+            for (uint32_t k = 0; k < 256 && k0 + k < n; ++k) {  // block-uniform
+                const uint32_t all = tiles[k];
+                if (at < all) {
+                    const PairMeta pm = g.pairs[g.xlist[k0 + k]];
+                    const uint32_t ta = (pm.na + kTile - 1) / kTile;
+                    for (; at < all; at += gridDim.x) {
+                        const bool is_a = at < ta;
+                        pack_view_tile(g.raw, tiled, is_a ? pm.a_raw0 : pm.b_raw0, is_a ? pm.a_row0 : pm.b_row0,
+                                       is_a ? pm.na : pm.nb, (uint32_t)(is_a ? at : at - ta), sm);
+                    }
+                }
+                at -= all;
+            }
+        }
     }
 }
 
@@ -1449,7 +1493,13 @@ int launch_shortlist_tail(const SlArgs &a, int sms, cudaStream_t s) {
     const dim3 per_block(a.npairs, a.row_blocks);  // CTA per pair and row block
     // routed pairs: plan, exact kernel over all their rows and columns, decisions
     launch_next(sl_route_plan_kernel, 1, 1024, 0, s, a);
-    launch_next(sl_route_apply_kernel, rgrid, 256, 0, s, a);
+    // (BF16 batches rarely route a pair: their FP32 tiles are packed then, for the routed
+    // pairs' views only; FP8 batches, which route most pairs of unit descriptors, keep
+    // the store's packed tiles)
+    if (a.fp8)
+        launch_next(sl_route_apply_kernel<false>, rgrid, 256, 0, s, a);
+    else
+        launch_next(sl_route_apply_kernel<true>, 2 * sms, 256, 0, s, a);
     ExactArgs x{};
     x.tiled = a.tiled;
     x.items = a.xitems;
@@ -1462,17 +1512,12 @@ int launch_shortlist_tail(const SlArgs &a, int sms, cudaStream_t s) {
     x.err = a.ctl + 1;
     x.mutual = a.mutual;
     x.x2 = 1;
-    // BF16 batches rarely route a pair: the FP32 tiles the exact kernel reads
-    // are packed here for the routed pairs' views only (FP8 batches, which
-    // route most pairs of unit descriptors, keep the store's packed tiles)
-    if (!a.fp8)
-        launch_pack_routed(a.pairs, a.xlist, a.ctl + kCtlRoutedPairs, a.raw, const_cast<float *>(a.tiled), 2 * sms, s);
     launch_exact(x, sms, s);
     launch_next(sl_route_finalize_kernel, dim3(rgrid, a.row_blocks), 256, 0, s, a);
     if (a.fp8) launch_next(sl_rescore_kernel, 5 * sms, 256, 0, s, a);  // 40 warps per SM: latency-bound gathers
     launch_next(sl_scan_kernel, 2 * sms, 256, 0, s, a);
     launch_next(sl_compact_kernel, per_block, 256, 0, s, a);
-    return 7;
+    return a.fp8 ? 7 : 6;
 }
 
 }  // namespace slm

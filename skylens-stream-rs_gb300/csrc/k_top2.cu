@@ -425,12 +425,14 @@ SLM_DEV uint32_t mutual_from_top2(const SlArgs &g, uint32_t p, const SlPair &sp,
 }
 
 // Row i of pair p joins the undecided rows of its b view; whoever starts a new
-// run of 16 there registers that run as a group for sl_resolve_kernel.
+// run of 16 or 128 there registers that run as a group for the resolve kernels.
 SLM_DEV void list_undecided(const SlArgs &g, const SlPair &sp, uint32_t p, uint32_t i) {
     const uint32_t k = atomicAdd(&g.ucnt[sp.ubucket], 1u);
     g.ulist[sp.ubase + k] = make_uint2(p, i);
-    if (k % kResolveRows == 0)
+    if (k % kGroupRows == 0)
         g.ugroups[atomicAdd(&g.ctl[kCtlGroups], 1u)] = make_uint4(sp.ubase + k, sp.ubucket, k, 0u);
+    if (k % kTileRows == 0)
+        g.utiles[atomicAdd(&g.ctl[kCtlTiles], 1u)] = make_uint4(sp.ubase + k, sp.ubucket, k, 0u);
 }
 
 // A row whose ratio test the estimates leave open, its nearest column j certain
@@ -564,6 +566,54 @@ __global__ void __launch_bounds__(256) sl_nearest_kernel(SlArgs g) {
 
 // --------------------------------------------------------------- resolve
 
+// Undecided rows: the estimates against every column of their b view once more, the
+// columns within the window m2 + 2 eps, the exact distances of those, and the
+// reference's row rule (matching.rs:182-187, 204-206). Rows are grouped by b view over
+// all pairs, since reading the view is the cost: in tens of us by sl_resolve_kernel
+// where they are few, by sl_resolve_tile_kernel in groups of 128 where they are many,
+// whichever the estimate of the two finds shorter (both are launched, one returns).
+// With groups of 16 alone a 32768 x 32768 pair with every row undecided took 4.0 ms, or
+// 7.7 with shortlists of 32 columns, whose overflows are scanned; with groups of 128
+// alone 30 pairs of 500 to 4000 rows took 134 us instead of 126, and one pair of 8192
+// rows 172 instead of 161, from the larger CTAs' start.
+// us, measured: a group of 16 takes its share of a read of the view; a group of 128 about
+// 15 and 0.6 a tile of the CTA's, in rounds of the launch's CTAs or of their clusters.
+SLM_DEV float tiles_us(const SlArgs &g, uint32_t cluster) {
+    const float rounds = ceilf((float)g.ctl[kCtlTiles] * (float)cluster / (float)g.res_ctas);
+    return rounds * (15.f + 0.6f * g.mean_tiles / (float)cluster);
+}
+SLM_DEV bool resolve_by_tiles(const SlArgs &g) {
+    const float few = 0.005f * (float)g.ctl[kCtlGroups] * g.mean_tiles;
+    return few > 10.f + 1.2f * fminf(tiles_us(g, 1), tiles_us(g, g.res_cluster));
+}
+
+// A row with more columns in its window than a shortlist holds is scanned exactly; a
+// pair with more than 1/8 such rows goes to the exact kernel.
+SLM_DEV void scan_instead(const SlArgs &g, uint32_t p, const PairMeta &pm, uint32_t i) {
+    push_scan(g, p, 0, i, 0);
+    const uint32_t was = atomicAdd(&g.pairctl[4 * (size_t)p + kPcOver], 1u);
+    if (was * 8 <= pm.na && (was + 1) * 8 > pm.na) {
+        g.spairs[p].routed = 1;
+        atomicAdd(&g.ctl[kCtlRouteMarks], 1u);
+    }
+}
+
+// A row's decision from its exact two smallest distances.
+SLM_DEV void decide_exact(const SlArgs &g, uint32_t p, const SlPair &sp, uint32_t i, float e1, float e2, uint32_t ej) {
+    uint32_t dec = kDecNone;
+    if (ej != 0xffffffffu && e2 < __int_as_float(0x7f800000) && !(e1 >= __fmul_rn(g.ratio2, e2)))
+        dec = g.mutual ? mutual_from_top2(g, p, sp, i, ej, e1) : ej;
+    g.rowdec[sp.rbase + i] = dec;
+}
+
+SLM_DEV void merge_exact(float &e1, float &e2, uint32_t &ej, float o1, float o2, uint32_t oj) {
+    e2 = fminf(fminf(e2, o2), fmaxf(e1, o1));
+    if (o1 < e1 || (o1 == e1 && oj < ej)) {
+        e1 = o1;
+        ej = oj;
+    }
+}
+
 SLM_DEV void mma_16816(float (&c)[4], uint32_t a0, uint32_t a1, uint32_t a2, uint32_t a3, uint32_t b0, uint32_t b1) {
     asm volatile(
         "mma.sync.aligned.m16n8k16.row.col.f32.bf16.bf16.f32 {%0,%1,%2,%3}, {%4,%5,%6,%7}, {%8,%9}, {%0,%1,%2,%3};"
@@ -577,13 +627,9 @@ SLM_DEV uint4 op_chunk(const SlArgs &g, uint32_t r, uint32_t c) {
     return *reinterpret_cast<const uint4 *>(t + (((c & 7) ^ (r & 7)) * 16));
 }
 
-// One cluster per group of 16 undecided rows (about 1 in 200 of a zone's) of
-// one b view: their estimates against every column once more, the columns
-// within the window m2 + 2 eps, the exact distances of those, and the
-// reference's row rule (matching.rs:182-187, 204-206). The group's rows lie
-// scattered over views, which no shared-memory descriptor of tcgen05 can
-// address without staging, and 16 rows are a warp-level tile exactly: m16n8k16
-// with both operands straight from the operand image. The sum over k may run in
+// Few undecided rows: one cluster per group of 16 of one b view. The group's rows
+// lie scattered over views, and 16 are a warp-level tile exactly: m16n8k16 with both
+// operands straight from the operand image, without staging. The sum over k may run in
 // any order, so lane t of four takes the 16-byte chunks 4 q + t of its row, on
 // both sides, and each chunk is the operand words of two steps.
 // Reading the b view (256 bytes a column) is the cost, so rows are grouped by b
@@ -595,13 +641,14 @@ SLM_DEV uint4 op_chunk(const SlArgs &g, uint32_t r, uint32_t c) {
 __global__ void __launch_bounds__(256) sl_resolve_kernel(SlArgs g) {
     grid_wait();
     grid_go();
-    constexpr uint32_t kCap = 2 * kSlHalfRecsMax;
-    __shared__ uint32_t cand_s[kResolveRows][kCap];
-    __shared__ float cval_s[kResolveRows][kCap];
-    __shared__ uint32_t cnt_s[kResolveRows];
-    __shared__ uint2 rows[kResolveRows];
-    __shared__ uint32_t arow[kResolveRows];
-    __shared__ float win[kResolveRows], nrm[kResolveRows];
+    if (resolve_by_tiles(g)) return;
+    constexpr uint32_t kCap = kResolveCols;
+    __shared__ uint32_t cand_s[kGroupRows][kCap];
+    __shared__ float cval_s[kGroupRows][kCap];
+    __shared__ uint32_t cnt_s[kGroupRows];
+    __shared__ uint2 rows[kGroupRows];
+    __shared__ uint32_t arow[kGroupRows];
+    __shared__ float win[kGroupRows], nrm[kGroupRows];
     const cooperative_groups::cluster_group cl = cooperative_groups::this_cluster();
     const uint32_t rank = cl.block_rank(), ncta = cl.num_blocks();
     uint32_t (*cand)[kCap] = cl.map_shared_rank(cand_s, 0);
@@ -616,9 +663,9 @@ __global__ void __launch_bounds__(256) sl_resolve_kernel(SlArgs g) {
     float w_err = 0.f;
     for (uint32_t e = blockIdx.x / ncta; e < ng; e += gridDim.x / ncta) {
         const uint4 ug = g.ugroups[e];
-        const uint32_t n = min(kResolveRows, g.ucnt[ug.y] - ug.z);
+        const uint32_t n = min(kGroupRows, g.ucnt[ug.y] - ug.z);
         const PairMeta pb = g.pairs[g.ulist[ug.x].x];  // every pair of the group has this b view
-        if (tid < kResolveRows) {
+        if (tid < kGroupRows) {
             // rows past the list's end repeat its first row and admit nothing
             const uint2 r = g.ulist[ug.x + (tid < n ? tid : 0)];
             const SlPair sp = g.spairs[r.x];
@@ -680,7 +727,7 @@ __global__ void __launch_bounds__(256) sl_resolve_kernel(SlArgs g) {
         cl.sync();
         // exact distances, 2 lanes a column: a warp per row where the cluster has
         // 16 warps, else 8 lanes per row, four rows of a warp side by side
-        const uint32_t width = nwarp >= kResolveRows ? 32 : 8, sub = lane & (width - 1);
+        const uint32_t width = nwarp >= kGroupRows ? 32 : 8, sub = lane & (width - 1);
         const uint32_t per = 32 / width, cols = width / 2;
         for (uint32_t r0 = gwarp * per; r0 < n; r0 += nwarp * per) {  // warp-uniform
             const uint32_t r = min(r0 + lane / width, n - 1);
@@ -722,18 +769,10 @@ __global__ void __launch_bounds__(256) sl_resolve_kernel(SlArgs g) {
             }
             if (have && sub == 0) {
                 if (over) {
-                    push_scan(g, p, 0, i, 0);
-                    const uint32_t was = atomicAdd(&g.pairctl[4 * (size_t)p + kPcOver], 1u);
-                    if (was * 8 <= pm.na && (was + 1) * 8 > pm.na) {
-                        g.spairs[p].routed = 1;
-                        atomicAdd(&g.ctl[kCtlRouteMarks], 1u);
-                    }
+                    scan_instead(g, p, pm, i);
                 } else {
                     ++w_rows;
-                    uint32_t dec = kDecNone;
-                    if (ej != 0xffffffffu && e2 < kInf && !(e1 >= __fmul_rn(g.ratio2, e2)))
-                        dec = g.mutual ? mutual_from_top2(g, p, sp, i, ej, e1) : ej;
-                    g.rowdec[sp.rbase + i] = dec;
+                    decide_exact(g, p, sp, i, e1, e2, ej);
                 }
             }
         }
@@ -748,12 +787,283 @@ __global__ void __launch_bounds__(256) sl_resolve_kernel(SlArgs g) {
     }
 }
 
+constexpr uint32_t kResVals = 15;         // of a row's shortlist, with their estimates (for the largest error seen)
+constexpr uint32_t kResRunTiles = 512;    // column tiles between two looks at the lists: 16 bits a column
+struct ResSmem {
+    uint8_t A[kBf16TileStride];
+    uint8_t B[kTopStages][kStageBytes];
+    uint16_t cand[kTileRows][kResolveCols];
+    float cval[kTileRows][kResVals];
+    float4 part[2][kTileRows];  // by turns: a row's two smallest exact distances here, the column of the first, columns in the window
+    uint2 rows[kTileRows];
+    float thr[kTileRows];
+    uint32_t cnt[kTileRows];
+    uint64_t a_full;
+    uint64_t b_full[kTopStages];
+    uint64_t t_full[kTopStages], t_empty[kTopStages];  // t_full: also the b tiles are free again
+    uint32_t tmem_base;
+    uint32_t abort_flag;
+};
+constexpr size_t kResSmemBytes = sizeof(ResSmem) + 1024;  // slack for 1024-byte alignment
+static_assert(kResSmemBytes <= 232448, "shared memory of one CTA");
+static_assert(kTileRows == kTile && kTopStages == 2, "a group is one a tile, a stage's accumulator half of TMEM");
+
+SLM_DEV void epilogue_sync() { asm volatile("bar.sync 1, 512;" ::: "memory"); }
+
+// Many undecided rows: one cluster per group of up to 128 of one b view. The epilogue's
+// warps gather the rows, which lie scattered over views, from the operand image into one
+// a tile, and the group is then a tile of the pass: sl_top2_kernel's roles, M = 128, N =
+// 256. A cluster's CTAs share the view's tiles where there are few groups, else each has
+// its own. Each lists its columns within the window (in its own shared memory: appending
+// to one list over the cluster made a tile of 12 hits 2.6 us), takes their exact
+// distances, and the rows' two smallest meet at the end.
+__global__ void __maxnreg__(96) sl_resolve_tile_kernel(SlArgs g) {
+    grid_wait();
+    grid_go();
+    if (!resolve_by_tiles(g)) return;
+    extern __shared__ uint8_t res_smem_raw[];
+    const uint32_t pad = (1024u - (smem_u32(res_smem_raw) & 1023u)) & 1023u;
+    ResSmem &S = *reinterpret_cast<ResSmem *>(res_smem_raw + pad);
+    const cooperative_groups::cluster_group cl = cooperative_groups::this_cluster();
+    const bool shared = cl.num_blocks() > 1 && tiles_us(g, g.res_cluster) < tiles_us(g, 1);
+    const uint32_t rank = shared ? cl.block_rank() : 0, ncta = shared ? cl.num_blocks() : 1;
+    const uint32_t ng = g.ctl[kCtlTiles], e0 = blockIdx.x / ncta, step = gridDim.x / ncta;
+    if (e0 >= ng) return;  // all that share a group
+    const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
+    uint32_t *err = g.ctl + 1;
+    volatile uint32_t *abort_flag = &S.abort_flag;
+    if (threadIdx.x == 0) {
+        mbar_init(&S.a_full, kTopEpWarps);
+        for (int s = 0; s < kTopStages; ++s) {
+            mbar_init(&S.b_full[s], 1);
+            mbar_init(&S.t_full[s], 1);
+            mbar_init(&S.t_empty[s], kTopEpWarps);
+        }
+        S.abort_flag = 0;
+        fence_mbar_init();
+    }
+    if (warp == 1) {
+        tmem_alloc(&S.tmem_base, 512);
+        tmem_relinquish();
+        tc_fence_before();
+    }
+    __syncthreads();
+    tc_fence_after();
+    const uint32_t tmem = S.tmem_base;
+    const float kInf = __int_as_float(0x7f800000);
+    uint32_t st = 0, sph = 0, iter = 0;  // stage and its phase; groups
+    uint32_t w_rows = 0;
+    float w_err = 0.f;
+    // Every role goes through every group and its cluster barrier; after a wait that gave
+    // up it only does that, so that no CTA waits for, or reads in, one that left.
+    for (uint32_t e = e0; e < ng; e += step, ++iter) {
+        const uint4 ug = g.utiles[e];
+        const PairMeta pb = g.pairs[g.ulist[ug.x].x];  // every pair of the group has this b view
+        const uint32_t n = min(kTileRows, g.ucnt[ug.y] - ug.z);
+        const uint32_t nt = (pb.nb + kTile - 1) / kTile;
+        const uint32_t t0 = (uint32_t)((uint64_t)nt * rank / ncta), t1 = (uint32_t)((uint64_t)nt * (rank + 1) / ncta);
+        // columns of the stage from tile t on, rounded up to the MMA's and the loads' 16
+        const auto columns = [&](uint32_t t) { return (min(min(t1 - t, 2u) * kTile, pb.nb - t * kTile) + 15) & ~15u; };
+        if (warp == 0) {
+            // ------------------------------------------------------ producer
+            for (uint32_t t = t0; t < t1; t += 2) {
+                if (lane == 0 && !*abort_flag && sl_wait(&S.t_full[st], sph ^ 1, abort_flag, err)) {
+                    const uint32_t m = min(2u, t1 - t);
+                    mbar_arrive_expect_tx(&S.b_full[st], m * kBf16TileStride);
+                    for (uint32_t u = 0; u < m; ++u) {
+                        const uint8_t *src = g.optiles + (size_t)(pb.b_row0 / kTile + t + u) * kBf16TileStride;
+                        bulk_g2s(S.B[st] + u * kKb, src, kKb, &S.b_full[st]);
+                        bulk_g2s(S.B[st] + (2 + u) * kKb, src + kKb, kKb, &S.b_full[st]);
+                        bulk_g2s(S.B[st] + kStageExt + u * kBf16ExtBytes, src + 2 * kKb, kBf16ExtBytes, &S.b_full[st]);
+                    }
+                }
+                __syncwarp();
+                if (++st == kTopStages) st = 0, sph ^= 1;
+            }
+        } else if (warp == 1) {
+            // ---------------------------------------------------- MMA issue (as sl_top2_kernel's)
+            const uint64_t ad = umma_desc(smem_u32(S.A)), ax = umma_desc_plain(smem_u32(S.A) + 2 * kKb, 0, 256);
+            const uint64_t bd0 = umma_desc(smem_u32(S.B[0])), bx0 = umma_desc_plain(smem_u32(S.B[0]) + kStageExt + 128, 0, 256);
+            bool ok = !*abort_flag && sl_wait(&S.a_full, iter & 1, abort_flag, err);
+            for (uint32_t t = t0; t < t1 && ok; t += 2) {
+                ok = sl_wait(&S.b_full[st], sph, abort_flag, err) && sl_wait(&S.t_empty[st], sph ^ 1, abort_flag, err);
+                if (!ok) break;
+                tc_fence_after();
+                if (lane == 0) {
+                    const uint32_t cols = columns(t);
+                    const uint32_t d = tmem + st * 256, idesc = top_idesc(cols, false), idesc_neg = top_idesc(cols, true);
+                    const uint64_t stage = (uint64_t)(st * (kStageBytes >> 4));
+#pragma unroll
+                    for (int k = 0; k < 8; ++k)
+                        mma_f16(d, ad + (k >> 2) * (kKb >> 4) + (k & 3) * 2,
+                                bd0 + stage + (k >> 2) * (2 * kKb >> 4) + (k & 3) * 2, idesc_neg, k > 0);
+                    mma_f16(d, ax, bx0 + stage, idesc, true);
+                    mma_commit(&S.t_full[st]);
+                }
+                __syncwarp();
+                if (++st == kTopStages) st = 0, sph ^= 1;
+            }
+            __syncwarp();
+        } else {
+            // ------------------------------------------------------ epilogue
+            {  // four threads a row: its operand image (128 bytes of each K block, the norm extension)
+                const uint32_t et = threadIdx.x - 64, row = et >> 2, part = et & 3;
+                // rows past the list's end repeat its first row and admit nothing
+                const uint2 r = g.ulist[ug.x + (row < n ? row : 0)];
+                const uint32_t ar = g.pairs[r.x].a_row0 + r.y, rr = ar % kTile;
+                const uint8_t *src = g.optiles + (size_t)(ar / kTile) * kBf16TileStride;
+                uint4 v[4];
+#pragma unroll
+                for (uint32_t k = 0; k < 4; ++k) {
+                    const uint32_t c = part * 4 + k;
+                    v[k] = *reinterpret_cast<const uint4 *>(src + (c >> 3) * kKb + rr * 128 + (((c & 7) ^ (rr & 7)) * 16));
+                }
+                epilogue_sync();  // the group before: its MMAs are done, its rows were read until here
+#pragma unroll
+                for (uint32_t k = 0; k < 4; ++k) {
+                    const uint32_t c = part * 4 + k;
+                    *reinterpret_cast<uint4 *>(S.A + (c >> 3) * kKb + row * 128 + (((c & 7) ^ (row & 7)) * 16)) = v[k];
+                }
+                if (part == 0) {
+                    *reinterpret_cast<uint4 *>(S.A + 2 * kKb + (row >> 3) * 256 + (row & 7) * 16) =
+                        *reinterpret_cast<const uint4 *>(src + 2 * kKb + (rr >> 3) * 256 + (rr & 7) * 16);
+                } else if (part == 1) {
+                    S.rows[row] = r;
+                    S.cnt[row] = 0;
+                    S.part[iter & 1][row] = make_float4(kInf, kInf, __uint_as_float(0xffffffffu), 0.f);
+                } else if (part == 2) {
+                    const SlPair sp = g.spairs[r.x];
+                    float m1, m2;
+                    uint32_t j;
+                    row_top2(g, sp.tblk_a, r.y, m1, m2, j);
+                    S.thr[row] = row < n ? 0.5f * window_up(m2, sp.eps) : -kInf;  // of d~ / 2
+                }
+                fence_proxy_async();  // the MMAs read what this thread wrote
+                __syncwarp();
+                if (lane == 0) mbar_arrive(&S.a_full);
+            }
+            for (uint32_t run = t0; run < t1; run += kResRunTiles) {
+                epilogue_sync();  // the lists are empty
+                const int q = warp & 3, cg = (warp - 2) >> 2, row = q * 32 + lane;
+                const uint32_t lane_addr = (uint32_t)(q * 32) << 16;
+                const float thr = S.thr[row];
+                for (uint32_t t = run; t < min(run + kResRunTiles, t1); t += 2) {
+                    if (*abort_flag || !sl_wait(&S.t_full[st], sph, abort_flag, err)) break;
+                    tc_fence_after();
+                    const uint32_t tcol = tmem + lane_addr + st * 256, nch = columns(t) / 16;
+                    for (uint32_t c = cg; c < nch; c += 4) {
+                        uint32_t v[16], mn;
+                        tmem_ld16_min(tcol + c * 16, v, mn);
+                        asm volatile("tcgen05.wait::ld.sync.aligned;" : "+r"(mn)::"memory");
+                        tmem_tie16(v);
+                        if (__uint_as_float(mn) <= thr) {  // columns past nb have NaN estimates: never admitted
+                            uint32_t hits = 0;
+#pragma unroll
+                            for (int k = 0; k < 16; ++k) hits |= __uint_as_float(v[k]) <= thr ? 1u << k : 0u;
+                            // a lone hit's estimate is the chunk's minimum; of several, none is kept
+                            const float val = (hits & (hits - 1)) ? __int_as_float(0x7fc00000) : 2.f * __uint_as_float(mn);
+                            uint32_t s = atomicAdd(&S.cnt[row], (uint32_t)__popc(hits));
+                            const uint32_t j = (t - run) * kTile + c * 16 - 1;
+                            for (; hits; hits &= hits - 1, ++s) {
+                                if (s < kResolveCols) S.cand[row][s] = (uint16_t)(j + __ffs(hits));
+                                if (s < kResVals) S.cval[row][s] = val;
+                            }
+                        }
+                        __syncwarp();
+                    }
+                    tc_fence_before();
+                    __syncwarp();
+                    if (lane == 0) mbar_arrive(&S.t_empty[st]);
+                    if (++st == kTopStages) st = 0, sph ^= 1;
+                }
+                epilogue_sync();
+                // exact distances of this CTA's columns, 2 lanes each: four rows of a warp side by
+                // side, or all its lanes on one where there are as many warps
+                const uint32_t width = n <= kTopEpWarps ? 32 : n <= 2 * kTopEpWarps ? 16 : 8, sub = lane & (width - 1);
+                const uint32_t per = 32 / width, cols = width / 2;
+                for (uint32_t r0 = (warp - 2) * per; r0 < n; r0 += kTopEpWarps * per) {  // warp-uniform
+                    const uint32_t r = min(r0 + lane / width, n - 1), m = S.cnt[r];
+                    const bool have = r0 + lane / width < n;
+                    const PairMeta pm = g.pairs[S.rows[r].x];
+                    const float *a = g.raw + (size_t)(pm.a_raw0 + S.rows[r].y) * kDesc;
+                    const float *B = g.raw + (size_t)(pm.b_raw0 + (uint64_t)run * kTile) * kDesc;
+                    const uint32_t mine_n = have && m <= g.cand_cap ? m : 0;
+                    const uint32_t most = __reduce_max_sync(0xffffffffu, mine_n);
+                    float e1 = kInf, e2 = kInf;
+                    uint32_t ej = 0xffffffffu;
+                    for (uint32_t s = 0; s < most; s += cols) {
+                        const uint32_t mine = s + (sub >> 1);
+                        const uint32_t j = mine < mine_n ? S.cand[r][mine] : 0;
+                        const float d = dist2<8>(a, B + (size_t)j * kDesc);
+                        if (mine < mine_n) {
+                            if (mine < kResVals) w_err = fmaxf(w_err, fabsf(d - S.cval[r][mine]));
+                            merge_exact(e1, e2, ej, d, kInf, run * kTile + j);
+                        }
+                    }
+                    // over the row's lane pairs (no column occurs twice)
+                    for (uint32_t o = 2; o < width; o <<= 1)
+                        merge_exact(e1, e2, ej, __shfl_xor_sync(0xffffffffu, e1, o), __shfl_xor_sync(0xffffffffu, e2, o),
+                                    __shfl_xor_sync(0xffffffffu, ej, o));
+                    if (have && sub == 0) {
+                        float4 &p = S.part[iter & 1][r];  // with the runs before
+                        merge_exact(e1, e2, ej, p.x, p.y, __float_as_uint(p.z));
+                        p = make_float4(e1, e2, __uint_as_float(ej), __uint_as_float(__float_as_uint(p.w) + m));
+                        S.cnt[r] = 0;
+                    }
+                }
+            }
+            __syncwarp();
+        }
+        if (shared)
+            cl.sync();
+        else if (warp >= 2)
+            epilogue_sync();
+        if (warp >= 2) {
+            // the group's rows, dealt to its CTAs: a thread each
+            const uint32_t r = rank + ncta * (threadIdx.x - 64);
+            if (r < n) {
+                float e1 = kInf, e2 = kInf;
+                uint32_t ej = 0xffffffffu, m = 0;
+                for (uint32_t k = 0; k < ncta; ++k) {
+                    const float4 v = shared ? *cl.map_shared_rank(&S.part[iter & 1][r], k) : S.part[iter & 1][r];
+                    merge_exact(e1, e2, ej, v.x, v.y, __float_as_uint(v.z));
+                    m += __float_as_uint(v.w);
+                }
+                const uint32_t p = S.rows[r].x, i = S.rows[r].y;
+                if (m > g.cand_cap) {
+                    scan_instead(g, p, g.pairs[p], i);
+                } else {
+                    ++w_rows;
+                    decide_exact(g, p, g.spairs[p], i, e1, e2, ej);
+                }
+            }
+        }
+    }
+    if (shared) cl.sync();  // no CTA leaves while its results are read
+    if (warp >= 2) {
+#pragma unroll
+        for (int o = 16; o; o >>= 1) w_err = fmaxf(w_err, __shfl_xor_sync(0xffffffffu, w_err, o));
+        w_rows = __reduce_add_sync(0xffffffffu, w_rows);
+        if (lane == 0) {
+            if (w_rows) atomicAdd(&g.ctl[kCtlRescored], w_rows);
+            if (w_err > 0.f) atomicMax(&g.ctl[kCtlMaxErr], __float_as_uint(w_err));  // non-negative: bits order as values
+        }
+    }
+    tc_fence_before();
+    __syncthreads();
+    if (warp == 1) {
+        tc_fence_after();
+        tmem_dealloc(tmem, 512);
+    }
+}
+
 }  // namespace
 
 cudaError_t init_top2_kernels() {
     const cudaFuncAttribute at = cudaFuncAttributeMaxDynamicSharedMemorySize;
     cudaError_t e = cudaFuncSetAttribute(sl_top2_kernel<false>, at, (int)kTopSmemBytes);
     if (e == cudaSuccess) e = cudaFuncSetAttribute(sl_top2_kernel<true>, at, (int)kTopSmemBytes);
+    if (e == cudaSuccess) e = cudaFuncSetAttribute(sl_resolve_tile_kernel, at, (int)kResSmemBytes);
     return e;
 }
 
@@ -779,28 +1089,38 @@ int launch_top2_decide(const SlArgs &a, int sms, cudaStream_t s) {
 
 int launch_top2_resolve(const SlArgs &a, int sms, cudaStream_t s) {
     if (!a.npairs || !a.max_na) return 0;
-    // A group is a chain of dependent loads. With many groups (1 undecided row
-    // in 100 assumed) they cover each other: four warps a group, four groups a
-    // SM. With few, eight warps a CTA and the largest portable cluster that does
-    // not exceed the GPU (zone: 136 us against 365 with clusters of 4; one 8192
-    // pair: 24 us against 93 with one CTA).
-    const uint64_t est = a.n_rows / (100 * kResolveRows) + 1;
-    const bool many = est >= (uint64_t)sms;
-    uint32_t c = 1;
-    while (!many && c < 8 && 2 * c * est <= 2ull * sms) c *= 2;
+    SlArgs b = a;
+    // Tiles of 128 rows: a CTA a SM, and the largest portable cluster that leaves every
+    // group one of its own if one row in 100 is undecided.
+    b.res_cluster = 1;
+    while (b.res_cluster < 8 && 2 * b.res_cluster * (a.n_rows / (100 * kTileRows) + 1) <= (uint64_t)sms) b.res_cluster *= 2;
+    b.res_ctas = (uint32_t)sms / b.res_cluster * b.res_cluster;
     cudaLaunchConfig_t cfg{};
     cudaLaunchAttribute at[2]{};
     at[0].id = cudaLaunchAttributeClusterDimension;
-    at[0].val.clusterDim = {c, 1, 1};
     at[1].id = cudaLaunchAttributeProgrammaticStreamSerialization;
     at[1].val.programmaticStreamSerializationAllowed = 1;
-    cfg.gridDim = dim3((unsigned)((many ? 4 : 2) * sms) / c * c);
-    cfg.blockDim = dim3(many ? 128 : 256);
     cfg.stream = s;
     cfg.attrs = at;
     cfg.numAttrs = 2;
-    cudaLaunchKernelEx(&cfg, sl_resolve_kernel, a);
-    return 1;
+    // A group of 16 is a chain of dependent loads. With many groups (1 undecided row
+    // in 100 assumed) they cover each other: four warps a group, four groups a
+    // SM. With few, eight warps a CTA and the largest portable cluster that does
+    // not exceed the GPU (one 8192 pair: 24 us against 93 with one CTA).
+    const uint64_t est = a.n_rows / (100 * kGroupRows) + 1;
+    const bool many = est >= (uint64_t)sms;
+    uint32_t c = 1;
+    while (!many && c < 8 && 2 * c * est <= 2ull * sms) c *= 2;
+    at[0].val.clusterDim = {c, 1, 1};
+    cfg.gridDim = dim3((unsigned)((many ? 4 : 2) * sms) / c * c);
+    cfg.blockDim = dim3(many ? 128 : 256);
+    cudaLaunchKernelEx(&cfg, sl_resolve_kernel, b);
+    at[0].val.clusterDim = {b.res_cluster, 1, 1};
+    cfg.gridDim = dim3(b.res_ctas);
+    cfg.blockDim = dim3(kTopThreads);
+    cfg.dynamicSmemBytes = kResSmemBytes;
+    cudaLaunchKernelEx(&cfg, sl_resolve_tile_kernel, b);
+    return 2;
 }
 
 }  // namespace slm

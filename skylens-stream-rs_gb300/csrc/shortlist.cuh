@@ -236,11 +236,12 @@ SLM_DEV float dist8(const float *__restrict__ p, const float *__restrict__ r) {
 // components 8c + 4h .. 8c + 4h + 3; the even lane adds its four in order and
 // hands the sum to the odd lane, which adds its own. p and r (16-byte aligned)
 // may differ per pair of lanes; the result is valid in both.
+template <int U = 16>
 SLM_DEV float dist2(const float *__restrict__ p, const float *__restrict__ r) {
     const uint32_t h = threadIdx.x & 1;
     const float4 *p4 = reinterpret_cast<const float4 *>(p) + h, *r4 = reinterpret_cast<const float4 *>(r) + h;
     float acc[4] = {0.f, 0.f, 0.f, 0.f};
-#pragma unroll
+#pragma unroll U
     for (int c = 0; c < 16; ++c) {
         const float4 x = p4[2 * c], y = r4[2 * c];
         const float xs[4] = {x.x, x.y, x.z, x.w}, ys[4] = {y.x, y.y, y.z, y.w};

@@ -300,7 +300,7 @@ struct slm_plan {
     uint32_t half_recs = kSlHalfRecs;  // records per candidate row and column half
     uint64_t rows_pad = 0, cand_rows_pad = 0, cols_pad = 0, sl_parts = 0, queue_cap = 0, xitem_cap = 0, row_blocks_total = 0;
     uint32_t row_blocks = 1;  // the most row blocks of any pair
-    DevBuf d_rowpart, d_rownear, d_colmin, d_rowthr, d_colthr, d_rowcnt, d_rowrec, d_rowrecj, d_colcnt,
+    DevBuf d_rowpart, d_rownear, d_colmin, d_rowthr, d_colthr, d_rowcnt, d_rowrec, d_rowrecj,
         d_rowdec, d_queue, d_rqueue, d_dump, d_xlist, d_xitems, d_xparts, d_blkcnt;
     // BF16 pass: segments in the order the CTAs run them, each CTA's first one,
     // each block's parts; then its results and the undecided rows
@@ -308,7 +308,8 @@ struct slm_plan {
     std::vector<uint32_t> tstart;
     std::vector<uint2> tblk;
     uint32_t tshift = 8, max_na = 0, buckets = 0;
-    uint64_t top_parts = 0;
+    uint64_t top_parts = 0, n_groups = 0;
+    double mean_tiles = 0;
     DevBuf d_topmm, d_topj, d_olist, d_ulist, d_ugroups;
     bool dump = false;
     uint64_t raw_epoch = 0;          // the store's epoch whose a_raw0 and b_raw0 `meta` holds
@@ -334,9 +335,9 @@ struct slm_plan {
 
 // Every device buffer of a plan: all are used on the plan's stream only, and
 // allocated ordered on it (DevBuf::order_on).
-std::array<DevBuf *, 28> plan_buffers(slm_plan *p) {
+std::array<DevBuf *, 27> plan_buffers(slm_plan *p) {
     return {&p->d_up, &p->d_parts, &p->d_colbest, &p->d_slots, &p->d_ctl, &p->d_dense, &p->d_rowpart, &p->d_rownear,
-            &p->d_colmin, &p->d_rowthr, &p->d_colthr, &p->d_rowcnt, &p->d_rowrec, &p->d_rowrecj, &p->d_colcnt,
+            &p->d_colmin, &p->d_rowthr, &p->d_colthr, &p->d_rowcnt, &p->d_rowrec, &p->d_rowrecj,
             &p->d_rowdec, &p->d_queue, &p->d_rqueue, &p->d_dump, &p->d_xlist, &p->d_xitems, &p->d_xparts, &p->d_blkcnt,
             &p->d_topmm, &p->d_topj, &p->d_olist, &p->d_ulist, &p->d_ugroups};
 }
@@ -598,10 +599,9 @@ slm_status plan_fp8_items(slm_plan *p, const slm_pair *pairs) {
     SLM_TRY(p->d_colmin.ensure(c, sizeof(uint32_t) * p->cols_pad));
     SLM_TRY(p->d_rowthr.ensure(c, sizeof(float) * p->rows_pad));
     SLM_TRY(p->d_colthr.ensure(c, sizeof(float) * p->cols_pad));
-    SLM_TRY(p->d_rowcnt.ensure(c, 2 * sizeof(uint32_t) * p->cand_rows_pad));
+    SLM_TRY(p->d_rowcnt.ensure(c, sizeof(uint32_t) * (2 * p->cand_rows_pad + p->cols_pad)));  // colcnt behind
     SLM_TRY(p->d_rowrec.ensure(c, sizeof(float4) * 2 * p->half_recs * p->cand_rows_pad));
     SLM_TRY(p->d_rowrecj.ensure(c, sizeof(uint32_t) * 2 * p->half_recs * p->cand_rows_pad));
-    SLM_TRY(p->d_colcnt.ensure(c, sizeof(uint32_t) * p->cols_pad));
     SLM_TRY(p->d_rqueue.ensure(c, sizeof(SlQueue) * p->queue_cap));
     return SLM_OK;
 }
@@ -619,6 +619,7 @@ slm_status plan_build_shortlist(slm_plan *p, const slm_pair *pairs) {
     uint64_t rb = 0, row_tiles = 0, blk = 0;
     p->row_blocks = 1;
     p->max_na = p->buckets = 0;
+    p->mean_tiles = 0;
     // undecided rows are listed by b view: each view's share of the list holds
     // every row that meets it
     std::vector<uint32_t> bucket(p->st->n.size(), 0xffffffffu);
@@ -639,19 +640,21 @@ slm_status plan_build_shortlist(slm_plan *p, const slm_pair *pairs) {
         }
         sp.ubucket = bk;
         bucket_rows[bk] += m.na;
+        p->mean_tiles += (double)m.na * ((m.nb + kTile - 1) / kTile) / std::max<double>(1, (double)p->n_slots);
         sp.rbase = (uint32_t)rb;
         sp.view_a = pairs[k].i;
         sp.view_b = pairs[k].j;
         rb += pad_rows(m.na);
     }
-    uint64_t groups = 0;
+    uint64_t groups = 0, tiles = 0;
     {
         uint64_t at = 0;
         for (uint64_t &r : bucket_rows) {
             const uint64_t n = r;
             r = at;
             at += n;
-            groups += (n + kResolveRows - 1) / kResolveRows;
+            groups += (n + kGroupRows - 1) / kGroupRows;
+            tiles += (n + kTileRows - 1) / kTileRows;
         }
         for (SlPair &sp : p->spairs) sp.ubase = (uint32_t)bucket_rows[sp.ubucket];
     }
@@ -667,7 +670,8 @@ slm_status plan_build_shortlist(slm_plan *p, const slm_pair *pairs) {
     SLM_TRY(p->d_topj.ensure(c, sizeof(uint32_t) * std::max<uint64_t>(1, p->top_parts << p->tshift)));
     SLM_TRY(p->d_olist.ensure(c, sizeof(uint4) * std::max<uint64_t>(1, p->n_slots)));
     SLM_TRY(p->d_ulist.ensure(c, sizeof(uint2) * std::max<uint64_t>(1, p->n_slots)));
-    SLM_TRY(p->d_ugroups.ensure(c, sizeof(uint4) * std::max<uint64_t>(1, groups)));
+    SLM_TRY(p->d_ugroups.ensure(c, sizeof(uint4) * std::max<uint64_t>(1, groups + tiles)));
+    p->n_groups = groups;
     SLM_TRY(p->d_blkcnt.ensure(c, sizeof(uint32_t) * std::max<uint64_t>(1, blk)));
     SLM_TRY(p->d_xlist.ensure(c, sizeof(uint32_t) * std::max<size_t>(1, p->np)));
     SLM_TRY(p->d_xitems.ensure(c, sizeof(Item) * p->xitem_cap));
@@ -743,8 +747,7 @@ slm_status plan_enqueue(slm_plan *p, cudaStream_t s) {
         const bool fp8 = p->prec == SLM_PREC_FP8;
         if (fp8) {
             launch_fill_u32(p->d_colmin.as<uint32_t>(), p->cols_pad, 0xff800000u, s);  // encodes +inf
-            SLM_CU(cudaMemsetAsync(p->d_rowcnt.p, 0, 2 * sizeof(uint32_t) * p->cand_rows_pad, s));
-            SLM_CU(cudaMemsetAsync(p->d_colcnt.p, 0, sizeof(uint32_t) * p->cols_pad, s));
+            SLM_CU(cudaMemsetAsync(p->d_rowcnt.p, 0, sizeof(uint32_t) * (2 * p->cand_rows_pad + p->cols_pad), s));
         }
         SlArgs a{};
         const slm_store::LowpImage &im = st->lowp[p->prec == SLM_PREC_FP8 ? 1 : 0];
@@ -770,7 +773,7 @@ slm_status plan_enqueue(slm_plan *p, cudaStream_t s) {
         a.rowrec = p->d_rowrec.as<float4>();
         a.half_recs = p->half_recs;
         a.rowrecj = p->d_rowrecj.as<uint32_t>();
-        a.colcnt = p->d_colcnt.as<float>();
+        a.colcnt = reinterpret_cast<float *>(a.rowcnt + 2 * p->cand_rows_pad);
         a.rowdec = p->d_rowdec.as<uint32_t>();
         a.queue = p->d_queue.as<SlQueue>();
         a.rqueue = p->d_rqueue.as<SlQueue>();
@@ -803,10 +806,12 @@ slm_status plan_enqueue(slm_plan *p, cudaStream_t s) {
         a.max_na = p->max_na;
         a.n_rows = p->n_slots;
         a.olist = p->d_olist.as<uint4>();
-        a.cand_cap = 2 * (p->tune.shortlist_k ? p->tune.shortlist_k : (uint32_t)kSlHalfRecs);
+        a.cand_cap = p->tune.shortlist_k ? 4 * p->tune.shortlist_k : kResolveCols;
         a.ulist = p->d_ulist.as<uint2>();
         a.ucnt = reinterpret_cast<uint32_t *>(p->d_ctl.as<unsigned char>() + p->o_ucnt);
         a.ugroups = p->d_ugroups.as<uint4>();
+        a.utiles = a.ugroups + p->n_groups;
+        a.mean_tiles = (float)p->mean_tiles;
         int nk = fp8 ? 1 : 0;  // the colmin fill
         if (p->timed) SLM_CU(record_event(p->ev0, s));
         nk += launch_shortlist_eps(a, s);

@@ -19,7 +19,7 @@
 //                       their ratio test get their exact d1; those still open
 //                       are listed by b view, other columns queued for an
 //                       exact scan.
-//   resolve             the listed rows, 16 of a b view at a time: every column
+//   resolve             the listed rows, 16 or 128 of a b view at a time: every column
 //                       with d~ <= m2 + 2 eps, and their exact distances.
 //   scan                one CTA per queued row or column: exact full scans.
 //
@@ -88,7 +88,8 @@ constexpr int kSlEpWarps = 16;     // epilogue warps
 constexpr int kSlThreads = 32 * (2 + kSlEpWarps);  // producer, MMA, epilogue
 constexpr int kTopEpWarps = 16;
 constexpr int kTopThreads = 32 * (2 + kTopEpWarps);
-constexpr uint32_t kResolveRows = 16;  // undecided rows per CTA of the resolve kernel
+constexpr uint32_t kGroupRows = 16, kTileRows = 128;  // undecided rows per cluster of the two resolve kernels
+constexpr uint32_t kResolveCols = 128;                // columns a row's shortlist there may hold
 
 // Operand tile sizes per 128 descriptors.
 //
@@ -200,7 +201,8 @@ struct SlQueue {
 // Counters in the plan's control block (word 1: the error word).
 enum : int { kCtlGroups = 0, kCtlRescored = 2, kCtlQueueRows = 3, kCtlQueueCols = 4, kCtlMaxErr = 5, kCtlScanLen = 6,
              kCtlRescoreLen = 7, kCtlXItems = 8, kCtlXWork = 9, kCtlRoutedPairs = 10, kCtlRoutedRows = 11,
-             kCtlRoutedCols = 12, kCtlRouteMarks = 13, kCtlRescuedPairs = 14, kCtlRescuedRows = 15, kCtlOpen = 16 };
+             kCtlRoutedCols = 12, kCtlRouteMarks = 13, kCtlRescuedPairs = 14, kCtlRescuedRows = 15, kCtlOpen = 16,
+             kCtlTiles = 17 };
 constexpr size_t kCtlBytes = 128;
 
 // Routed pairs: at most this many column chunks per 128-row tile; the exact
@@ -270,7 +272,9 @@ struct SlArgs {
     uint32_t cand_cap;           // resolve: columns a row's shortlist holds
     uint2 *ulist;                // undecided rows {pair, row}, by b view (from SlPair::ubase)
     uint32_t *ucnt;              // and their number per b view (SlPair::ubucket)
-    uint4 *ugroups;              // {first entry in ulist, bucket, entry within the bucket}, kResolveRows rows each
+    uint4 *ugroups, *utiles;     // {first entry in ulist, bucket, entry within the bucket}: kGroupRows, kTileRows rows each
+    float mean_tiles;            // column tiles of a row's b view, on average
+    uint32_t res_cluster, res_ctas;  // launch of sl_resolve_tile_kernel
 };
 
 // Whether a pair takes part in this tier's per-pair kernels (pass 2, finalize,
