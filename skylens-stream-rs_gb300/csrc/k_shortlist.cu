@@ -1037,26 +1037,59 @@ SLM_DEV void block_argmin(float &d, uint32_t &idx, float *sd, uint32_t *si) {
         }
 }
 
+// After exact_kernel: the routed pairs' row decisions in their row block `block`, as
+// finalize_kernel makes them (matching.rs:204-214), into rowdec.
+SLM_DEV void route_finalize(const SlArgs &g, uint32_t cta, uint32_t ctas, uint32_t block) {
+    const uint32_t n = g.ctl[kCtlRoutedPairs];
+    const float kInf = __int_as_float(0x7f800000);
+    for (uint32_t k = cta; k < n; k += ctas) {
+        const uint32_t p = g.xlist[k];
+        const PairMeta pm = g.pairs[p];
+        const SlPair sp = g.spairs[p];
+        const uint32_t r1 = min(block * kSlRowBlock + kSlRowBlock, pm.na);  // this CTA's row block
+        for (uint32_t i = block * kSlRowBlock + threadIdx.x; i < r1; i += blockDim.x) {
+            const uint32_t rt = i / kTile;
+            float d1 = kInf, d2 = kInf;
+            uint32_t j1 = 0xffffffffu;
+            for (uint32_t c = 0; c < sp.xchunk; ++c) {
+                const uint32_t part = sp.xpart + rt * sp.xchunk + c;
+                if (part < g.xitem_cap) merge_rowpart(g.xparts[(size_t)part * kTile + (i % kTile)], d1, d2, j1);
+            }
+            uint32_t dec = kDecNone;
+            if (j1 != 0xffffffffu && d2 < kInf && !(d1 >= __fmul_rn(g.ratio2, d2)))
+                if (!g.mutual || static_cast<uint32_t>(g.colbest[pm.col_base + j1]) == i) dec = j1;
+            g.rowdec[sp.rbase + i] = dec;
+        }
+    }
+}
+
 // One CTA per entry of the scan queue: exact full scans, 32 distances at a
 // time (8 lanes each). Entries of pairs that were routed meanwhile (the exact
 // kernel settled those) are left out 32 at a time: when every pair is, the queue
 // holds an eighth and more of all rows, and one by one, each a chain of loads,
 // 470 K of them took 0.7 ms.
-__global__ void __launch_bounds__(256) sl_scan_kernel(SlArgs g) {
+// The CTAs from scan_ctas on make the routed pairs' decisions (rgrid a row block): other
+// pairs' rows, so one launch for both, which mostly find nothing.
+__global__ void __launch_bounds__(256) sl_scan_kernel(SlArgs g, uint32_t scan_ctas, uint32_t rgrid) {
     grid_wait();
     grid_go();
+    if (blockIdx.x >= scan_ctas) {  // block-uniform
+        const uint32_t cta = blockIdx.x - scan_ctas;
+        route_finalize(g, cta % rgrid, rgrid, cta / rgrid);
+        return;
+    }
     __shared__ float sd[8], s2[8];
     __shared__ uint32_t si[8];
     const uint32_t lane = threadIdx.x & 31, grp = threadIdx.x >> 3;  // 32 groups of 8 lanes
     const uint32_t qn = min(g.ctl[kCtlScanLen], g.queue_cap);
     const float kInf = __int_as_float(0x7f800000);
-    const auto live = [&](uint64_t e0) {  // of the entries e0, e0 + gridDim.x, ..: the same in every warp
-        const uint64_t e = e0 + (uint64_t)lane * gridDim.x;
+    const auto live = [&](uint64_t e0) {  // of the entries e0, e0 + scan_ctas, ..: the same in every warp
+        const uint64_t e = e0 + (uint64_t)lane * scan_ctas;
         return __ballot_sync(0xffffffffu, e < qn && !g.spairs[g.queue[e].pair].routed);
     };
-    for (uint64_t e0 = blockIdx.x; e0 < qn; e0 += 32ull * gridDim.x)
+    for (uint64_t e0 = blockIdx.x; e0 < qn; e0 += 32ull * scan_ctas)
     for (uint32_t todo = live(e0); todo; todo &= todo - 1) {
-        const SlQueue qe = g.queue[e0 + (uint64_t)(__ffs(todo) - 1) * gridDim.x];
+        const SlQueue qe = g.queue[e0 + (uint64_t)(__ffs(todo) - 1) * scan_ctas];
         const PairMeta pm = g.pairs[qe.pair];
         const SlPair sp = g.spairs[qe.pair];
         if (threadIdx.x == 0) atomicAdd(&g.ctl[qe.kind == 0 ? kCtlQueueRows : kCtlQueueCols], 1u);
@@ -1314,34 +1347,6 @@ __global__ void __launch_bounds__(256) sl_route_apply_kernel(SlArgs g) {
     }
 }
 
-// After exact_kernel: the routed pairs' row decisions, as finalize_kernel
-// makes them (matching.rs:204-214), into rowdec.
-__global__ void __launch_bounds__(256) sl_route_finalize_kernel(SlArgs g) {
-    grid_wait();
-    grid_go();
-    const uint32_t n = g.ctl[kCtlRoutedPairs];
-    const float kInf = __int_as_float(0x7f800000);
-    for (uint32_t k = blockIdx.x; k < n; k += gridDim.x) {
-        const uint32_t p = g.xlist[k];
-        const PairMeta pm = g.pairs[p];
-        const SlPair sp = g.spairs[p];
-        const uint32_t r1 = min(blockIdx.y * kSlRowBlock + kSlRowBlock, pm.na);  // this CTA's row block
-        for (uint32_t i = blockIdx.y * kSlRowBlock + threadIdx.x; i < r1; i += blockDim.x) {
-            const uint32_t rt = i / kTile;
-            float d1 = kInf, d2 = kInf;
-            uint32_t j1 = 0xffffffffu;
-            for (uint32_t c = 0; c < sp.xchunk; ++c) {
-                const uint32_t part = sp.xpart + rt * sp.xchunk + c;
-                if (part < g.xitem_cap) merge_rowpart(g.xparts[(size_t)part * kTile + (i % kTile)], d1, d2, j1);
-            }
-            uint32_t dec = kDecNone;
-            if (j1 != 0xffffffffu && d2 < kInf && !(d1 >= __fmul_rn(g.ratio2, d2)))
-                if (!g.mutual || static_cast<uint32_t>(g.colbest[pm.col_base + j1]) == i) dec = j1;
-            g.rowdec[sp.rbase + i] = dec;
-        }
-    }
-}
-
 // -------------------------------------------------------------- compact
 
 // Matches of a pair's row block in ascending i, at the block's slot range
@@ -1491,7 +1496,7 @@ int launch_shortlist_tail(const SlArgs &a, int sms, cudaStream_t s) {
     if (!a.npairs) return 0;
     const unsigned rgrid = (unsigned)(a.npairs < (uint32_t)(4 * sms) ? a.npairs : (uint32_t)(4 * sms));
     const dim3 per_block(a.npairs, a.row_blocks);  // CTA per pair and row block
-    // routed pairs: plan, exact kernel over all their rows and columns, decisions
+    // routed pairs: plan, exact kernel over all their rows and columns (their decisions: with the scan)
     launch_next(sl_route_plan_kernel, 1, 1024, 0, s, a);
     // (BF16 batches rarely route a pair: their FP32 tiles are packed then, for the routed
     // pairs' views only; FP8 batches, which route most pairs of unit descriptors, keep
@@ -1513,11 +1518,10 @@ int launch_shortlist_tail(const SlArgs &a, int sms, cudaStream_t s) {
     x.mutual = a.mutual;
     x.x2 = 1;
     launch_exact(x, sms, s);
-    launch_next(sl_route_finalize_kernel, dim3(rgrid, a.row_blocks), 256, 0, s, a);
     if (a.fp8) launch_next(sl_rescore_kernel, 5 * sms, 256, 0, s, a);  // 40 warps per SM: latency-bound gathers
-    launch_next(sl_scan_kernel, 2 * sms, 256, 0, s, a);
+    launch_next(sl_scan_kernel, 2 * sms + rgrid * a.row_blocks, 256, 0, s, a, (uint32_t)(2 * sms), (uint32_t)rgrid);
     launch_next(sl_compact_kernel, per_block, 256, 0, s, a);
-    return a.fp8 ? 7 : 6;
+    return a.fp8 ? 6 : 5;
 }
 
 }  // namespace slm
