@@ -297,7 +297,7 @@ __global__ void __maxnreg__(kSlMaxRegs) sl_pass_kernel(SlArgs g) {
     if (warp == 0) {
         // ---------------------------------------------------------- producer
         if (lane == 0) {
-            uint32_t st = 0, sph = 0, iter = 0;  // iter: items processed (routed pairs skip pass 2)
+            uint32_t st = 0, sph = 0, iter = 0, a_loads = 0, issued = 0;  // iter: items processed (routed pairs skip pass 2)
             for (uint32_t it = blockIdx.x; it < g.n_items; it += gridDim.x) {
                 const SlItem item = g.items[it];
                 if (item_off(g, item)) continue;
@@ -310,6 +310,7 @@ __global__ void __maxnreg__(kSlMaxRegs) sl_pass_kernel(SlArgs g) {
                 if (PASS == 2) bytes += item.nat * 512;
                 bytes += item.nat * 1024;  // norms and scales
                 mbar_arrive_expect_tx(&S.a_full, bytes);
+                ++a_loads;
 #pragma unroll
                 for (uint32_t a = 0; a < 2; ++a) {  // static indices keep the item in registers
                     if (a >= item.nat) break;
@@ -326,6 +327,7 @@ __global__ void __maxnreg__(kSlMaxRegs) sl_pass_kernel(SlArgs g) {
                     const uint32_t brow = pm.b_row0 + t * kTile;
                     uint32_t bb = kOp + (PASS == 2 ? (two ? 1024 : 512) : 0) + 1024;
                     mbar_arrive_expect_tx(&S.b_full[st], bb);
+                    ++issued;
                     bulk_g2s(S.B[st], g.optiles + (size_t)(brow / kTile) * kOp, kOp, &S.b_full[st]);
                     bulk_g2s(S.bnorm[st], g.norms + brow, 512, &S.b_full[st]);
                     if (PASS == 2) {
@@ -338,6 +340,8 @@ __global__ void __maxnreg__(kSlMaxRegs) sl_pass_kernel(SlArgs g) {
                 ++iter;
                 if (*abort_flag) break;
             }
+            drain_loads(S.b_full, kStg, issued);
+            drain_loads(&S.a_full, 1, a_loads);
         }
     } else if (warp == 1) {
         // ---------------------------------------------------------- MMA issue
@@ -1063,14 +1067,122 @@ SLM_DEV void route_finalize(const SlArgs &g, uint32_t cta, uint32_t ctas, uint32
     }
 }
 
-// One CTA per entry of the scan queue: exact full scans, 32 distances at a
-// time (8 lanes each). Entries of pairs that were routed meanwhile (the exact
-// kernel settled those) are left out 32 at a time: when every pair is, the queue
-// holds an eighth and more of all rows, and one by one, each a chain of loads,
-// 470 K of them took 0.7 ms.
+// One entry of the scan queue by a CTA: exact full scans, 64 distances at a time (8
+// lanes for two of them), the entry's own row in registers. Bound by the rows' latency:
+// 32 at a time, its own row read again for each, the 302 K columns of a zone at ratio
+// 0.99 took 31.6 ms of 38.3; the call now takes 30.7. Ends with a barrier.
+SLM_DEV void scan_entry(const SlArgs &g, const SlQueue qe, const PairMeta pm, const SlPair sp, float *sd, float *s2,
+                        uint32_t *si) {
+    const uint32_t lane = threadIdx.x & 31, grp = threadIdx.x >> 3;  // 32 groups of 8 lanes
+    const float kInf = __int_as_float(0x7f800000);
+    if (threadIdx.x == 0) atomicAdd(&g.ctl[qe.kind == 0 ? kCtlQueueRows : kCtlQueueCols], 1u);
+    const float *A = g.raw + (size_t)pm.a_raw0 * kDesc;
+    const float *B = g.raw + (size_t)pm.b_raw0 * kDesc;
+    uint32_t dec = kDecNone, col = qe.j;
+    bool check_col = qe.kind == 1;
+    if (qe.kind == 0) {
+        float d1 = kInf, d2 = kInf;
+        uint32_t j1 = 0xffffffffu;
+        float own[16];
+        load8(A + (size_t)qe.i * kDesc, own);
+        for (uint32_t j0 = 0; j0 < pm.nb; j0 += 64) {
+            const uint32_t j[2] = {j0 + grp, j0 + 32 + grp};
+            float x[2][16];
+#pragma unroll
+            for (int u = 0; u < 2; ++u) load8(B + (size_t)(j[u] < pm.nb ? j[u] : 0) * kDesc, x[u]);
+#pragma unroll
+            for (int u = 0; u < 2; ++u) {
+                const float d = dist8(own, x[u]);
+                if (j[u] < pm.nb) {
+                    if (d < d1) {
+                        d2 = d1;
+                        d1 = d;
+                        j1 = j[u];
+                    } else if (d < d2) {
+                        d2 = d;
+                    }
+                }
+            }
+        }
+        // merge (d1, j1, d2) across the 32 groups (lanes within a group agree)
+        float m2 = d2;
+        float b1 = d1;
+        uint32_t bj = j1;
+#pragma unroll
+        for (int o = 8; o < 32; o <<= 1) {
+            const float o1 = __shfl_xor_sync(0xffffffffu, b1, o);
+            const float o2 = __shfl_xor_sync(0xffffffffu, m2, o);
+            const uint32_t oj = __shfl_xor_sync(0xffffffffu, bj, o);
+            const float n2 = fminf(fminf(m2, o2), fmaxf(b1, o1));
+            if (o1 < b1 || (o1 == b1 && oj < bj)) {
+                b1 = o1;
+                bj = oj;
+            }
+            m2 = n2;
+        }
+        const int w = threadIdx.x >> 5;
+        __syncthreads();
+        if (lane == 0) {
+            sd[w] = b1;
+            s2[w] = m2;
+            si[w] = bj;
+        }
+        __syncthreads();
+        b1 = sd[0];
+        m2 = s2[0];
+        bj = si[0];
+        for (int q = 1; q < 8; ++q) {
+            const float n2 = fminf(fminf(m2, s2[q]), fmaxf(b1, sd[q]));
+            if (sd[q] < b1 || (sd[q] == b1 && si[q] < bj)) {
+                b1 = sd[q];
+                bj = si[q];
+            }
+            m2 = n2;
+        }
+        if (bj != 0xffffffffu && m2 < kInf && !(b1 >= __fmul_rn(g.ratio2, m2))) {
+            if (g.mutual) {
+                check_col = true;
+                col = bj;
+            } else {
+                dec = bj;
+            }
+        }
+    }
+    if (check_col) {
+        float bd = kInf;
+        uint32_t bi = 0xffffffffu;
+        float own[16];
+        load8(B + (size_t)col * kDesc, own);
+        for (uint32_t r0 = 0; r0 < pm.na; r0 += 64) {
+            const uint32_t r[2] = {r0 + grp, r0 + 32 + grp};
+            float x[2][16];
+#pragma unroll
+            for (int u = 0; u < 2; ++u) load8(A + (size_t)(r[u] < pm.na ? r[u] : 0) * kDesc, x[u]);
+#pragma unroll
+            for (int u = 0; u < 2; ++u) {
+                const float d = dist8(x[u], own);
+                if (r[u] < pm.na && (d < bd || (d == bd && r[u] < bi))) {
+                    bd = d;
+                    bi = r[u];
+                }
+            }
+        }
+        block_argmin(bd, bi, sd, si);
+        dec = bi == qe.i ? col : kDecNone;
+    }
+    if (threadIdx.x == 0) g.rowdec[sp.rbase + qe.i] = dec;
+    __syncthreads();
+}
+
+// The scan queue, a CTA an entry at a time. Entries of pairs that were routed meanwhile
+// (the exact kernel settled those) are left out 32 at a time: when every pair is, the
+// queue holds an eighth and more of all rows, and one by one, each a chain of loads,
+// 470 K of them took 0.7 ms. (Taken as the CTAs go, by tickets, the
+// entries of views of unlike sizes even out, but a call that scans 237 columns of 2000
+// rows took 157 us instead of 146.)
 // The CTAs from scan_ctas on make the routed pairs' decisions (rgrid a row block): other
 // pairs' rows, so one launch for both, which mostly find nothing.
-__global__ void __launch_bounds__(256) sl_scan_kernel(SlArgs g, uint32_t scan_ctas, uint32_t rgrid) {
+__global__ void __launch_bounds__(256, 2) sl_scan_kernel(SlArgs g, uint32_t scan_ctas, uint32_t rgrid) {
     grid_wait();
     grid_go();
     if (blockIdx.x >= scan_ctas) {  // block-uniform
@@ -1080,99 +1192,14 @@ __global__ void __launch_bounds__(256) sl_scan_kernel(SlArgs g, uint32_t scan_ct
     }
     __shared__ float sd[8], s2[8];
     __shared__ uint32_t si[8];
-    const uint32_t lane = threadIdx.x & 31, grp = threadIdx.x >> 3;  // 32 groups of 8 lanes
-    const uint32_t qn = min(g.ctl[kCtlScanLen], g.queue_cap);
-    const float kInf = __int_as_float(0x7f800000);
-    const auto live = [&](uint64_t e0) {  // of the entries e0, e0 + scan_ctas, ..: the same in every warp
+    const uint32_t lane = threadIdx.x & 31, qn = min(g.ctl[kCtlScanLen], g.queue_cap);
+    for (uint64_t e0 = blockIdx.x; e0 < qn; e0 += 32ull * scan_ctas) {
         const uint64_t e = e0 + (uint64_t)lane * scan_ctas;
-        return __ballot_sync(0xffffffffu, e < qn && !g.spairs[g.queue[e].pair].routed);
-    };
-    for (uint64_t e0 = blockIdx.x; e0 < qn; e0 += 32ull * scan_ctas)
-    for (uint32_t todo = live(e0); todo; todo &= todo - 1) {
-        const SlQueue qe = g.queue[e0 + (uint64_t)(__ffs(todo) - 1) * scan_ctas];
-        const PairMeta pm = g.pairs[qe.pair];
-        const SlPair sp = g.spairs[qe.pair];
-        if (threadIdx.x == 0) atomicAdd(&g.ctl[qe.kind == 0 ? kCtlQueueRows : kCtlQueueCols], 1u);
-        const float *A = g.raw + (size_t)pm.a_raw0 * kDesc;
-        const float *B = g.raw + (size_t)pm.b_raw0 * kDesc;
-        uint32_t dec = kDecNone, col = qe.j;
-        bool check_col = qe.kind == 1;
-        if (qe.kind == 0) {
-            float d1 = kInf, d2 = kInf;
-            uint32_t j1 = 0xffffffffu;
-            for (uint32_t j0 = 0; j0 < pm.nb; j0 += 32) {
-                const uint32_t j = j0 + grp;
-                const float d = dist8(A + (size_t)qe.i * kDesc, B + (size_t)(j < pm.nb ? j : 0) * kDesc);
-                if (j < pm.nb) {
-                    if (d < d1) {
-                        d2 = d1;
-                        d1 = d;
-                        j1 = j;
-                    } else if (d < d2) {
-                        d2 = d;
-                    }
-                }
-            }
-            // merge (d1, j1, d2) across the 32 groups (lanes within a group agree)
-            float m2 = d2;
-            float b1 = d1;
-            uint32_t bj = j1;
-#pragma unroll
-            for (int o = 8; o < 32; o <<= 1) {
-                const float o1 = __shfl_xor_sync(0xffffffffu, b1, o);
-                const float o2 = __shfl_xor_sync(0xffffffffu, m2, o);
-                const uint32_t oj = __shfl_xor_sync(0xffffffffu, bj, o);
-                const float n2 = fminf(fminf(m2, o2), fmaxf(b1, o1));
-                if (o1 < b1 || (o1 == b1 && oj < bj)) {
-                    b1 = o1;
-                    bj = oj;
-                }
-                m2 = n2;
-            }
-            const int w = threadIdx.x >> 5;
-            __syncthreads();
-            if (lane == 0) {
-                sd[w] = b1;
-                s2[w] = m2;
-                si[w] = bj;
-            }
-            __syncthreads();
-            b1 = sd[0];
-            m2 = s2[0];
-            bj = si[0];
-            for (int q = 1; q < 8; ++q) {
-                const float n2 = fminf(fminf(m2, s2[q]), fmaxf(b1, sd[q]));
-                if (sd[q] < b1 || (sd[q] == b1 && si[q] < bj)) {
-                    b1 = sd[q];
-                    bj = si[q];
-                }
-                m2 = n2;
-            }
-            if (bj != 0xffffffffu && m2 < kInf && !(b1 >= __fmul_rn(g.ratio2, m2))) {
-                if (g.mutual) {
-                    check_col = true;
-                    col = bj;
-                } else {
-                    dec = bj;
-                }
-            }
+        uint32_t todo = __ballot_sync(0xffffffffu, e < qn && !g.spairs[g.queue[e].pair].routed);  // the same in every warp
+        for (; todo; todo &= todo - 1) {
+            const SlQueue qe = g.queue[e0 + (uint64_t)(__ffs(todo) - 1) * scan_ctas];
+            scan_entry(g, qe, g.pairs[qe.pair], g.spairs[qe.pair], sd, s2, si);
         }
-        if (check_col) {
-            float bd = kInf;
-            uint32_t bi = 0xffffffffu;
-            for (uint32_t r0 = 0; r0 < pm.na; r0 += 32) {
-                const uint32_t r = r0 + grp;
-                const float d = dist8(A + (size_t)(r < pm.na ? r : 0) * kDesc, B + (size_t)col * kDesc);
-                if (r < pm.na && (d < bd || (d == bd && r < bi))) {
-                    bd = d;
-                    bi = r;
-                }
-            }
-            block_argmin(bd, bi, sd, si);
-            dec = bi == qe.i ? col : kDecNone;
-        }
-        if (threadIdx.x == 0) g.rowdec[sp.rbase + qe.i] = dec;
-        __syncthreads();
     }
 }
 

@@ -43,6 +43,7 @@
 #include <cooperative_groups.h>
 #include <cuda_runtime.h>
 
+#include <algorithm>
 #include <cstdint>
 
 #include "shortlist.cuh"
@@ -576,15 +577,14 @@ __global__ void __launch_bounds__(256) sl_nearest_kernel(SlArgs g) {
 // 7.7 with shortlists of 32 columns, whose overflows are scanned; with groups of 128
 // alone 30 pairs of 500 to 4000 rows took 134 us instead of 126, and one pair of 8192
 // rows 172 instead of 161, from the larger CTAs' start.
-// us, measured: a group of 16 takes its share of a read of the view; a group of 128 about
-// 15 and 0.6 a tile of the CTA's, in rounds of the launch's CTAs or of their clusters.
-SLM_DEV float tiles_us(const SlArgs &g, uint32_t cluster) {
-    const float rounds = ceilf((float)g.ctl[kCtlTiles] * (float)cluster / (float)g.res_ctas);
-    return rounds * (15.f + 0.6f * g.mean_tiles / (float)cluster);
-}
+// us, measured: groups of 16 take about 18 and 1.3 a tile of a CTA of their cluster, in
+// rounds of the launch's clusters; groups of 128 about 15 and 0.6 a tile, in rounds of CTAs,
+// and 20 to start.
 SLM_DEV bool resolve_by_tiles(const SlArgs &g) {
-    const float few = 0.005f * (float)g.ctl[kCtlGroups] * g.mean_tiles;
-    return few > 10.f + 1.2f * fminf(tiles_us(g, 1), tiles_us(g, g.res_cluster));
+    const float few = ceilf((float)g.ctl[kCtlGroups] * (float)g.few_cluster / (float)g.few_ctas) *
+                      (18.f + 1.3f * g.mean_tiles / (float)g.few_cluster);
+    const float many = ceilf((float)g.ctl[kCtlTiles] / (float)g.res_ctas) * (15.f + 0.6f * g.mean_tiles);
+    return few > 20.f + 1.2f * many;
 }
 
 // A row with more columns in its window than a shortlist holds is scanned exactly; a
@@ -794,7 +794,7 @@ struct ResSmem {
     uint8_t B[kTopStages][kStageBytes];
     uint16_t cand[kTileRows][kResolveCols];
     float cval[kTileRows][kResVals];
-    float4 part[2][kTileRows];  // by turns: a row's two smallest exact distances here, the column of the first, columns in the window
+    float4 part[kTileRows];  // a row's two smallest exact distances, the column of the first, columns in the window
     uint2 rows[kTileRows];
     float thr[kTileRows];
     uint32_t cnt[kTileRows];
@@ -810,13 +810,14 @@ static_assert(kTileRows == kTile && kTopStages == 2, "a group is one a tile, a s
 
 SLM_DEV void epilogue_sync() { asm volatile("bar.sync 1, 512;" ::: "memory"); }
 
-// Many undecided rows: one cluster per group of up to 128 of one b view. The epilogue's
+// Many undecided rows: one CTA per group of up to 128 of one b view. The epilogue's
 // warps gather the rows, which lie scattered over views, from the operand image into one
 // a tile, and the group is then a tile of the pass: sl_top2_kernel's roles, M = 128, N =
-// 256. A cluster's CTAs share the view's tiles where there are few groups, else each has
-// its own. Each lists its columns within the window (in its own shared memory: appending
-// to one list over the cluster made a tile of 12 hits 2.6 us), takes their exact
-// distances, and the rows' two smallest meet at the end.
+// 256. What is within a row's window is listed in shared memory, its exact distances
+// taken once the view (or 65536 columns of it) is through. 0.55 us a tile of 128 columns,
+// bound by the MMAs (0.36 in the pass, whose b tiles serve two a tiles); with many hits,
+// which a warp appends by the chunk, up to 0.9. (N = 128: 0.95. A cluster's CTAs sharing
+// the view's tiles and one list: 2.6 us for a tile of 12 hits.)
 __global__ void __maxnreg__(96) sl_resolve_tile_kernel(SlArgs g) {
     grid_wait();
     grid_go();
@@ -824,11 +825,8 @@ __global__ void __maxnreg__(96) sl_resolve_tile_kernel(SlArgs g) {
     extern __shared__ uint8_t res_smem_raw[];
     const uint32_t pad = (1024u - (smem_u32(res_smem_raw) & 1023u)) & 1023u;
     ResSmem &S = *reinterpret_cast<ResSmem *>(res_smem_raw + pad);
-    const cooperative_groups::cluster_group cl = cooperative_groups::this_cluster();
-    const bool shared = cl.num_blocks() > 1 && tiles_us(g, g.res_cluster) < tiles_us(g, 1);
-    const uint32_t rank = shared ? cl.block_rank() : 0, ncta = shared ? cl.num_blocks() : 1;
-    const uint32_t ng = g.ctl[kCtlTiles], e0 = blockIdx.x / ncta, step = gridDim.x / ncta;
-    if (e0 >= ng) return;  // all that share a group
+    const uint32_t ng = g.ctl[kCtlTiles];
+    if (blockIdx.x >= ng) return;
     const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
     uint32_t *err = g.ctl + 1;
     volatile uint32_t *abort_flag = &S.abort_flag;
@@ -854,21 +852,19 @@ __global__ void __maxnreg__(96) sl_resolve_tile_kernel(SlArgs g) {
     uint32_t st = 0, sph = 0, iter = 0;  // stage and its phase; groups
     uint32_t w_rows = 0;
     float w_err = 0.f;
-    // Every role goes through every group and its cluster barrier; after a wait that gave
-    // up it only does that, so that no CTA waits for, or reads in, one that left.
-    for (uint32_t e = e0; e < ng; e += step, ++iter) {
+    // (after a wait that gave up every role still goes through its groups, without waiting)
+    for (uint32_t e = blockIdx.x; e < ng; e += gridDim.x, ++iter) {
         const uint4 ug = g.utiles[e];
         const PairMeta pb = g.pairs[g.ulist[ug.x].x];  // every pair of the group has this b view
         const uint32_t n = min(kTileRows, g.ucnt[ug.y] - ug.z);
         const uint32_t nt = (pb.nb + kTile - 1) / kTile;
-        const uint32_t t0 = (uint32_t)((uint64_t)nt * rank / ncta), t1 = (uint32_t)((uint64_t)nt * (rank + 1) / ncta);
         // columns of the stage from tile t on, rounded up to the MMA's and the loads' 16
-        const auto columns = [&](uint32_t t) { return (min(min(t1 - t, 2u) * kTile, pb.nb - t * kTile) + 15) & ~15u; };
+        const auto columns = [&](uint32_t t) { return (min(2u * kTile, pb.nb - t * kTile) + 15) & ~15u; };
         if (warp == 0) {
             // ------------------------------------------------------ producer
-            for (uint32_t t = t0; t < t1; t += 2) {
+            for (uint32_t t = 0; t < nt; t += 2) {
                 if (lane == 0 && !*abort_flag && sl_wait(&S.t_full[st], sph ^ 1, abort_flag, err)) {
-                    const uint32_t m = min(2u, t1 - t);
+                    const uint32_t m = min(2u, nt - t);
                     mbar_arrive_expect_tx(&S.b_full[st], m * kBf16TileStride);
                     for (uint32_t u = 0; u < m; ++u) {
                         const uint8_t *src = g.optiles + (size_t)(pb.b_row0 / kTile + t + u) * kBf16TileStride;
@@ -885,7 +881,7 @@ __global__ void __maxnreg__(96) sl_resolve_tile_kernel(SlArgs g) {
             const uint64_t ad = umma_desc(smem_u32(S.A)), ax = umma_desc_plain(smem_u32(S.A) + 2 * kKb, 0, 256);
             const uint64_t bd0 = umma_desc(smem_u32(S.B[0])), bx0 = umma_desc_plain(smem_u32(S.B[0]) + kStageExt + 128, 0, 256);
             bool ok = !*abort_flag && sl_wait(&S.a_full, iter & 1, abort_flag, err);
-            for (uint32_t t = t0; t < t1 && ok; t += 2) {
+            for (uint32_t t = 0; t < nt && ok; t += 2) {
                 ok = sl_wait(&S.b_full[st], sph, abort_flag, err) && sl_wait(&S.t_empty[st], sph ^ 1, abort_flag, err);
                 if (!ok) break;
                 tc_fence_after();
@@ -930,7 +926,7 @@ __global__ void __maxnreg__(96) sl_resolve_tile_kernel(SlArgs g) {
                 } else if (part == 1) {
                     S.rows[row] = r;
                     S.cnt[row] = 0;
-                    S.part[iter & 1][row] = make_float4(kInf, kInf, __uint_as_float(0xffffffffu), 0.f);
+                    S.part[row] = make_float4(kInf, kInf, __uint_as_float(0xffffffffu), 0.f);
                 } else if (part == 2) {
                     const SlPair sp = g.spairs[r.x];
                     float m1, m2;
@@ -942,12 +938,12 @@ __global__ void __maxnreg__(96) sl_resolve_tile_kernel(SlArgs g) {
                 __syncwarp();
                 if (lane == 0) mbar_arrive(&S.a_full);
             }
-            for (uint32_t run = t0; run < t1; run += kResRunTiles) {
+            for (uint32_t run = 0; run < nt; run += kResRunTiles) {
                 epilogue_sync();  // the lists are empty
                 const int q = warp & 3, cg = (warp - 2) >> 2, row = q * 32 + lane;
                 const uint32_t lane_addr = (uint32_t)(q * 32) << 16;
                 const float thr = S.thr[row];
-                for (uint32_t t = run; t < min(run + kResRunTiles, t1); t += 2) {
+                for (uint32_t t = run; t < min(run + kResRunTiles, nt); t += 2) {
                     if (*abort_flag || !sl_wait(&S.t_full[st], sph, abort_flag, err)) break;
                     tc_fence_after();
                     const uint32_t tcol = tmem + lane_addr + st * 256, nch = columns(t) / 16;
@@ -1005,41 +1001,28 @@ __global__ void __maxnreg__(96) sl_resolve_tile_kernel(SlArgs g) {
                         merge_exact(e1, e2, ej, __shfl_xor_sync(0xffffffffu, e1, o), __shfl_xor_sync(0xffffffffu, e2, o),
                                     __shfl_xor_sync(0xffffffffu, ej, o));
                     if (have && sub == 0) {
-                        float4 &p = S.part[iter & 1][r];  // with the runs before
+                        float4 &p = S.part[r];  // with the runs before
                         merge_exact(e1, e2, ej, p.x, p.y, __float_as_uint(p.z));
                         p = make_float4(e1, e2, __uint_as_float(ej), __uint_as_float(__float_as_uint(p.w) + m));
                         S.cnt[r] = 0;
                     }
                 }
             }
-            __syncwarp();
-        }
-        if (shared)
-            cl.sync();
-        else if (warp >= 2)
             epilogue_sync();
-        if (warp >= 2) {
-            // the group's rows, dealt to its CTAs: a thread each
-            const uint32_t r = rank + ncta * (threadIdx.x - 64);
+            const uint32_t r = threadIdx.x - 64;  // a thread a row
             if (r < n) {
-                float e1 = kInf, e2 = kInf;
-                uint32_t ej = 0xffffffffu, m = 0;
-                for (uint32_t k = 0; k < ncta; ++k) {
-                    const float4 v = shared ? *cl.map_shared_rank(&S.part[iter & 1][r], k) : S.part[iter & 1][r];
-                    merge_exact(e1, e2, ej, v.x, v.y, __float_as_uint(v.z));
-                    m += __float_as_uint(v.w);
-                }
+                const float4 v = S.part[r];
                 const uint32_t p = S.rows[r].x, i = S.rows[r].y;
-                if (m > g.cand_cap) {
+                if (__float_as_uint(v.w) > g.cand_cap) {
                     scan_instead(g, p, g.pairs[p], i);
                 } else {
                     ++w_rows;
-                    decide_exact(g, p, g.spairs[p], i, e1, e2, ej);
+                    decide_exact(g, p, g.spairs[p], i, v.x, v.y, __float_as_uint(v.z));
                 }
             }
+            __syncwarp();
         }
     }
-    if (shared) cl.sync();  // no CTA leaves while its results are read
     if (warp >= 2) {
 #pragma unroll
         for (int o = 16; o; o >>= 1) w_err = fmaxf(w_err, __shfl_xor_sync(0xffffffffu, w_err, o));
@@ -1090,11 +1073,7 @@ int launch_top2_decide(const SlArgs &a, int sms, cudaStream_t s) {
 int launch_top2_resolve(const SlArgs &a, int sms, cudaStream_t s) {
     if (!a.npairs || !a.max_na) return 0;
     SlArgs b = a;
-    // Tiles of 128 rows: a CTA a SM, and the largest portable cluster that leaves every
-    // group one of its own if one row in 100 is undecided.
-    b.res_cluster = 1;
-    while (b.res_cluster < 8 && 2 * b.res_cluster * (a.n_rows / (100 * kTileRows) + 1) <= (uint64_t)sms) b.res_cluster *= 2;
-    b.res_ctas = (uint32_t)sms / b.res_cluster * b.res_cluster;
+    b.res_ctas = (uint32_t)std::min<uint64_t>(sms, a.n_tiles);
     cudaLaunchConfig_t cfg{};
     cudaLaunchAttribute at[2]{};
     at[0].id = cudaLaunchAttributeClusterDimension;
@@ -1112,14 +1091,12 @@ int launch_top2_resolve(const SlArgs &a, int sms, cudaStream_t s) {
     uint32_t c = 1;
     while (!many && c < 8 && 2 * c * est <= 2ull * sms) c *= 2;
     at[0].val.clusterDim = {c, 1, 1};
-    cfg.gridDim = dim3((unsigned)((many ? 4 : 2) * sms) / c * c);
+    b.few_cluster = c;
+    b.few_ctas = (uint32_t)((many ? 4 : 2) * sms) / c * c;
+    cfg.gridDim = dim3(b.few_ctas);
     cfg.blockDim = dim3(many ? 128 : 256);
     cudaLaunchKernelEx(&cfg, sl_resolve_kernel, b);
-    at[0].val.clusterDim = {b.res_cluster, 1, 1};
-    cfg.gridDim = dim3(b.res_ctas);
-    cfg.blockDim = dim3(kTopThreads);
-    cfg.dynamicSmemBytes = kResSmemBytes;
-    cudaLaunchKernelEx(&cfg, sl_resolve_tile_kernel, b);
+    launch_next(sl_resolve_tile_kernel, b.res_ctas, kTopThreads, kResSmemBytes, s, b);
     return 2;
 }
 

@@ -137,6 +137,13 @@ SLM_DEV bool sl_wait(uint64_t *bar, uint32_t parity, volatile uint32_t *abort_fl
     }
 }
 
+// The loads into a ring of `stages` (`issued` were started in all) land before the CTA
+// ends, also when a wait gave up and nobody took them. Bounded like that wait.
+SLM_DEV void drain_loads(uint64_t *full, uint32_t stages, uint32_t issued) {
+    for (uint32_t q = 0; q < stages && q < issued; ++q)
+        mbar_wait(&full[(issued - 1 - q) % stages], ((issued - 1 - q) / stages) & 1, nullptr);
+}
+
 // ------------------------------------------------------------ error bound
 
 // The per-pair error bound of this launch's precision (g.fp8) from the two
@@ -224,6 +231,25 @@ SLM_DEV float dist8(const float *__restrict__ p, const float *__restrict__ r) {
 #pragma unroll
     for (int c = 0; c < 16; ++c) {
         const float t = __fsub_rn(p[8 * c + k], r[8 * c + k]);
+        acc = __fadd_rn(acc, __fmul_rn(t, t));
+    }
+    float s = 0.f;
+#pragma unroll
+    for (int q = 0; q < 8; ++q) s = __fadd_rn(s, __shfl_sync(0xffffffffu, acc, base + q));
+    return s;
+}
+
+// The same from one row to many: the row's share of a lane (components 8c + k) is kept.
+SLM_DEV void load8(const float *p, float (&own)[16]) {
+#pragma unroll
+    for (int c = 0; c < 16; ++c) own[c] = p[8 * c + (threadIdx.x & 7)];
+}
+SLM_DEV float dist8(const float (&own)[16], const float (&other)[16]) {
+    const uint32_t base = threadIdx.x & 24;  // the group's first lane
+    float acc = 0.f;
+#pragma unroll
+    for (int c = 0; c < 16; ++c) {
+        const float t = __fsub_rn(own[c], other[c]);
         acc = __fadd_rn(acc, __fmul_rn(t, t));
     }
     float s = 0.f;

@@ -308,7 +308,7 @@ struct slm_plan {
     std::vector<uint32_t> tstart;
     std::vector<uint2> tblk;
     uint32_t tshift = 8, max_na = 0, buckets = 0;
-    uint64_t top_parts = 0, n_groups = 0;
+    uint64_t top_parts = 0, n_groups = 0, n_tiles = 0;
     double mean_tiles = 0;
     DevBuf d_topmm, d_topj, d_olist, d_ulist, d_ugroups;
     bool dump = false;
@@ -672,6 +672,7 @@ slm_status plan_build_shortlist(slm_plan *p, const slm_pair *pairs) {
     SLM_TRY(p->d_ulist.ensure(c, sizeof(uint2) * std::max<uint64_t>(1, p->n_slots)));
     SLM_TRY(p->d_ugroups.ensure(c, sizeof(uint4) * std::max<uint64_t>(1, groups + tiles)));
     p->n_groups = groups;
+    p->n_tiles = tiles;
     SLM_TRY(p->d_blkcnt.ensure(c, sizeof(uint32_t) * std::max<uint64_t>(1, blk)));
     SLM_TRY(p->d_xlist.ensure(c, sizeof(uint32_t) * std::max<size_t>(1, p->np)));
     SLM_TRY(p->d_xitems.ensure(c, sizeof(Item) * p->xitem_cap));
@@ -811,6 +812,7 @@ slm_status plan_enqueue(slm_plan *p, cudaStream_t s) {
         a.ucnt = reinterpret_cast<uint32_t *>(p->d_ctl.as<unsigned char>() + p->o_ucnt);
         a.ugroups = p->d_ugroups.as<uint4>();
         a.utiles = a.ugroups + p->n_groups;
+        a.n_tiles = p->n_tiles;
         a.mean_tiles = (float)p->mean_tiles;
         int nk = fp8 ? 1 : 0;  // the colmin fill
         if (p->timed) SLM_CU(record_event(p->ev0, s));

@@ -88,7 +88,7 @@ constexpr int kSlEpWarps = 16;     // epilogue warps
 constexpr int kSlThreads = 32 * (2 + kSlEpWarps);  // producer, MMA, epilogue
 constexpr int kTopEpWarps = 16;
 constexpr int kTopThreads = 32 * (2 + kTopEpWarps);
-constexpr uint32_t kGroupRows = 16, kTileRows = 128;  // undecided rows per cluster of the two resolve kernels
+constexpr uint32_t kGroupRows = 16, kTileRows = 128;  // undecided rows a group of the two resolve kernels
 constexpr uint32_t kResolveCols = 128;                // columns a row's shortlist there may hold
 
 // Operand tile sizes per 128 descriptors.
@@ -274,7 +274,8 @@ struct SlArgs {
     uint32_t *ucnt;              // and their number per b view (SlPair::ubucket)
     uint4 *ugroups, *utiles;     // {first entry in ulist, bucket, entry within the bucket}: kGroupRows, kTileRows rows each
     float mean_tiles;            // column tiles of a row's b view, on average
-    uint32_t res_cluster, res_ctas;  // launch of sl_resolve_tile_kernel
+    uint64_t n_tiles;            // the most utiles there may be
+    uint32_t res_ctas, few_ctas, few_cluster;  // grids of sl_resolve_tile_kernel and sl_resolve_kernel
 };
 
 // Whether a pair takes part in this tier's per-pair kernels (pass 2, finalize,
