@@ -188,7 +188,7 @@ __global__ void __maxnreg__(96) sl_top2_kernel(SlArgs g) {
     if (warp == 0) {
         // ---------------------------------------------------------- producer
         if (lane == 0) {
-            uint32_t st = 0, sph = 0, loads = 0, cur = 0xffffffffu;
+            uint32_t st = 0, sph = 0, loads = 0, issued = 0, cur = 0xffffffffu;
             bool ok = true;
             for (uint32_t it = it0; it < it1 && ok; ++it) {
                 const TopItem item = g.titems[it];
@@ -206,6 +206,7 @@ __global__ void __maxnreg__(96) sl_top2_kernel(SlArgs g) {
                     if (!(ok = sl_wait(&S.b_empty[st], sph ^ 1, abort_flag, err))) break;
                     const uint32_t n = min(2u, item.nt - t);
                     mbar_arrive_expect_tx(&S.b_full[st], n * kBf16TileStride);
+                    ++issued;
                     for (uint32_t u = 0; u < n; ++u) {
                         const uint8_t *src = g.optiles + (size_t)(item.b_tile + t + u) * kBf16TileStride;
                         bulk_g2s(S.B[st] + u * kKb, src, kKb, &S.b_full[st]);
@@ -215,6 +216,8 @@ __global__ void __maxnreg__(96) sl_top2_kernel(SlArgs g) {
                     if (++st == kTopStages) st = 0, sph ^= 1;
                 }
             }
+            drain_loads(S.b_full, kTopStages, issued);
+            drain_loads(&S.a_full, 1, loads);
         }
     } else if (warp == 1) {
         // ---------------------------------------------------------- MMA issue
@@ -850,6 +853,7 @@ __global__ void __maxnreg__(96) sl_resolve_tile_kernel(SlArgs g) {
     const uint32_t tmem = S.tmem_base;
     const float kInf = __int_as_float(0x7f800000);
     uint32_t st = 0, sph = 0, iter = 0;  // stage and its phase; groups
+    uint32_t issued = 0;                 // stages loaded
     uint32_t w_rows = 0;
     float w_err = 0.f;
     // (after a wait that gave up every role still goes through its groups, without waiting)
@@ -866,6 +870,7 @@ __global__ void __maxnreg__(96) sl_resolve_tile_kernel(SlArgs g) {
                 if (lane == 0 && !*abort_flag && sl_wait(&S.t_full[st], sph ^ 1, abort_flag, err)) {
                     const uint32_t m = min(2u, nt - t);
                     mbar_arrive_expect_tx(&S.b_full[st], m * kBf16TileStride);
+                    ++issued;
                     for (uint32_t u = 0; u < m; ++u) {
                         const uint8_t *src = g.optiles + (size_t)(pb.b_row0 / kTile + t + u) * kBf16TileStride;
                         bulk_g2s(S.B[st] + u * kKb, src, kKb, &S.b_full[st]);
@@ -1023,6 +1028,8 @@ __global__ void __maxnreg__(96) sl_resolve_tile_kernel(SlArgs g) {
             __syncwarp();
         }
     }
+    if (warp == 0 && lane == 0) drain_loads(S.b_full, kTopStages, issued);
+    __syncwarp();
     if (warp >= 2) {
 #pragma unroll
         for (int o = 16; o; o >>= 1) w_err = fmaxf(w_err, __shfl_xor_sync(0xffffffffu, w_err, o));
