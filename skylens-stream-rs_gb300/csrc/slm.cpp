@@ -93,7 +93,15 @@ struct slm_ctx {
     std::vector<Workspace *> all;
     std::map<uint64_t, slm_tune> tuned;  // autotuned settings by batch shape
 
+    // Gives back the device memory that workspaces not in use hold (they keep it between
+    // calls); true when there was any.
+    bool reclaim();
     slm_status alloc(void **p, size_t bytes) {
+        slm_status s = try_alloc(p, bytes);
+        if (s != SLM_OK && reclaim()) s = try_alloc(p, bytes);
+        return s;
+    }
+    slm_status try_alloc(void **p, size_t bytes) {
         *p = nullptr;
         if (bytes == 0) return SLM_OK;
         uint64_t now = used.fetch_add(bytes) + bytes;
@@ -121,6 +129,11 @@ struct slm_ctx {
     // grows does not stall the work of other streams (serving slots).
     cudaMemPool_t pool = nullptr;
     slm_status alloc_ordered(void **p, size_t bytes, cudaStream_t s) {
+        slm_status r = try_alloc_ordered(p, bytes, s);
+        if (r != SLM_OK && reclaim()) r = try_alloc_ordered(p, bytes, s);
+        return r;
+    }
+    slm_status try_alloc_ordered(void **p, size_t bytes, cudaStream_t s) {
         *p = nullptr;
         if (bytes == 0) return SLM_OK;
         uint64_t now = used.fetch_add(bytes) + bytes;
@@ -962,6 +975,39 @@ void ws_release(slm_ctx *c, Workspace *w) {
     std::lock_guard<std::mutex> g(c->mu);
     c->idle.push_back(w);
 }
+
+}  // namespace
+
+// A call that ran in parts, or at another size, leaves every workspace it used with
+// buffers of its own: a later call within the budget must not fail for them.
+bool slm_ctx::reclaim() {
+    std::vector<Workspace *> take;
+    {
+        std::lock_guard<std::mutex> g(mu);
+        take.swap(idle);
+    }
+    const uint64_t before = used.load();
+    for (Workspace *w : take) {
+        cudaStreamSynchronize(w->stream);  // slm_ratio_match_device leaves work pending
+        for (DevBuf *b : {&w->single, &w->score, &w->feat_in, &w->feat_up, &w->feat_pyr, &w->feat_desc[0], &w->feat_desc[1],
+                          &w->store.raw, &w->store.tiled, &w->store.tiletab, &w->store.staging})
+            b->reset();
+        for (auto &im : w->store.lowp)
+            for (DevBuf *b : {&im.optiles, &im.norms, &im.qscale, &im.vstats}) b->reset();
+        w->store.max_rows = 0;
+        plan_release(&w->plan);
+        cudaStreamSynchronize(w->stream);  // the plan's frees are ordered on it
+    }
+    if (pool && !take.empty()) cudaMemPoolTrimTo(pool, 0);
+    cudaGetLastError();
+    {
+        std::lock_guard<std::mutex> g(mu);
+        idle.insert(idle.end(), take.begin(), take.end());
+    }
+    return used.load() < before;
+}
+
+namespace {
 
 // Reserve room for rows in a store (grows the device buffers if needed).
 slm_status store_reserve(slm_store *st, uint64_t rows) {
@@ -3087,7 +3133,7 @@ slm_status feat_core(slm_ctx *c, Workspace *ws, const float *d_img, uint32_t n, 
     }
     if (out.geom.empty() || n == 0) return SLM_OK;
     const uint64_t wh0 = out.geom[0].layer_stride;
-    const uint64_t wh1 = out.geom.size() > 1 ? out.geom[1].layer_stride : 0;
+    const uint64_t wh1 = out.geom.size() > 1 ? out.geom[1].layer_stride : 0;  // at most wh0 / 4
     uint64_t ngrad = 0;
     for (const OctaveGeom &g : out.geom) ngrad += (uint64_t)n * s * g.layer_stride;
     uint32_t cap = std::max<uint32_t>(4096, std::min<uint64_t>(uint64_t(n) * 16384, 1u << 26));
@@ -3106,13 +3152,15 @@ slm_status feat_core(slm_ctx *c, Workspace *ws, const float *d_img, uint32_t n, 
     }
     for (int attempt = 0; attempt < 2; ++attempt) {
         const uint64_t o_geom = 0, o_gauss = feat_align(o_geom + sizeof(OctaveGeom) * out.geom.size()),
-                       o_odd = feat_align(o_gauss + 4 * (uint64_t)n * ng * wh0),  // odd octaves' layers
-                       o_dog = feat_align(o_odd + 4 * (uint64_t)n * ng * wh1),
+                       o_dog = feat_align(o_gauss + 4 * (uint64_t)n * ng * wh0),
                        o_tmp = feat_align(o_dog + 4 * (uint64_t)n * (ng - 1) * wh0),
                        o_grad = feat_align(o_tmp + 4 * (uint64_t)n * wh0),
                        o_cand = feat_align(o_grad + 8 * ngrad), o_cnt = feat_align(o_cand + sizeof(FeatCand) * cap),
                        o_ang = feat_align(o_cnt + 16), o_nang = feat_align(o_ang + 4ull * kMaxAngles * cap),
-                       bytes = feat_align(o_nang + cap);
+                       bytes = feat_align(o_nang + cap),
+                       // odd octaves' layers: at the end of the first octave's DoG layers, of which
+                       // the later octaves use less than a quarter
+                       o_odd = (o_tmp - 4 * (uint64_t)n * ng * wh1) & ~uint64_t(255);
         SLM_TRY(pyr.ensure(c, bytes));
         unsigned char *d = pyr.as<unsigned char>();
         float *dog = reinterpret_cast<float *>(d + o_dog), *tmp = reinterpret_cast<float *>(d + o_tmp);
@@ -3452,7 +3500,7 @@ slm_status feat_emit(const FeatOut &fo, uint32_t n, const uint64_t *off, slm_key
 // two images in each of twelve parts the 24 take 2.78. Features come out in
 // image order whatever the split.
 constexpr uint32_t kFeatParts = 8;
-slm_status feat_call(slm_ctx *c, const void *imgs, bool rgb, uint32_t n, uint32_t w, uint32_t h,
+slm_status feat_parts(slm_ctx *c, const void *imgs, bool rgb, uint32_t n, uint32_t w, uint32_t h,
                      const slm_detector_config &cfg, slm_keypoint *kps, float *desc, uint64_t cap, uint64_t *off) {
     const uint64_t wh = (uint64_t)w * h;
     const uint32_t parts = n < 4 ? 1 : std::max(std::min(n / 2, 4u), std::min(n / 3, kFeatParts));
@@ -3545,6 +3593,15 @@ slm_status feat_call(slm_ctx *c, const void *imgs, bool rgb, uint32_t n, uint32_
             st = fail(SLM_CUDA_ERROR, std::string("slm_detect_and_describe: ") + cudaGetErrorString(e));
         ws_release(c, ws[p]);
     }
+    return st;
+}
+
+// Without room for it: once more with the memory that the workspaces keep given back (the
+// parts' own hold what calls of other sizes left there).
+slm_status feat_call(slm_ctx *c, const void *imgs, bool rgb, uint32_t n, uint32_t w, uint32_t h,
+                     const slm_detector_config &cfg, slm_keypoint *kps, float *desc, uint64_t cap, uint64_t *off) {
+    slm_status st = feat_parts(c, imgs, rgb, n, w, h, cfg, kps, desc, cap, off);
+    if (st == SLM_OOM && c->reclaim()) st = feat_parts(c, imgs, rgb, n, w, h, cfg, kps, desc, cap, off);
     return st;
 }
 

@@ -95,6 +95,7 @@ cudaError_t cudaMalloc(void **p, size_t n) { return fake::alloc(p, n); }
 cudaError_t cudaFree(void *p) { return fake::release(p); }
 cudaError_t cudaMemPoolCreate(cudaMemPool_t *p, const cudaMemPoolProps *) { return *p = fake::handle<cudaMemPool_t>(), cudaSuccess; }
 cudaError_t cudaMemPoolSetAttribute(cudaMemPool_t, cudaMemPoolAttr, void *) { return cudaSuccess; }
+cudaError_t cudaMemPoolTrimTo(cudaMemPool_t, size_t) { return cudaSuccess; }
 cudaError_t cudaMemPoolDestroy(cudaMemPool_t) { return cudaSuccess; }
 cudaError_t cudaMallocFromPoolAsync(void **p, size_t n, cudaMemPool_t, cudaStream_t) { return fake::alloc(p, n); }
 cudaError_t cudaFreeAsync(void *p, cudaStream_t) { return fake::release(p); }

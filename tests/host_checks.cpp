@@ -102,11 +102,71 @@ int single_pair_waits_after_a_failure() {
     return 0;
 }
 
+// Device memory of a detection call: the layers of an octave at a time, every octave's
+// gradient tables, the candidates and the images, with the buffers' slack of a quarter,
+// whatever parts the batch goes in.
+uint64_t detection_bytes(uint64_t n, uint64_t w, uint64_t h) {
+    const uint64_t s = 3, ng = s + 3, wh0 = w * h, wh1 = (w / 2) * (h / 2);
+    uint64_t grads = 0;
+    for (int o = 0; o < 4; ++o) grads += 8 * s * (w >> o) * (h >> o);
+    const uint64_t image = 4 * (ng * wh0 + (ng - 1) * wh0 + wh0 + wh1) + grads + 16384 * (sizeof(slm::FeatCand) + 4 * slm::kMaxAngles + 1) + 7 * wh0;
+    return (n * image + (64 << 10)) * 5 / 4;
+}
+
+int detect(slm_ctx *c, uint32_t n, uint32_t w, uint32_t h) {
+    slm_detector_config cfg;
+    slm_detector_config_default(&cfg);
+    std::vector<uint8_t> img(size_t(3) * n * w * h);
+    std::vector<uint64_t> off(n + 1);
+    return slm_detect_and_describe_rgb8(c, img.data(), n, w, h, &cfg, nullptr, nullptr, 0, off.data());
+}
+
+int detection_within_its_budget() {
+    for (const uint32_t n : {1u, 3u, 4u, 8u, 15u, 24u, 31u}) {
+        slm_opts o{};
+        o.hbm_budget = detection_bytes(n, 960, 540);
+        slm_ctx *c = nullptr;
+        REQUIRE(slm_ctx_create(&o, &c) == SLM_OK);
+        REQUIRE(detect(c, n, 960, 540) == SLM_OK);
+        slm_ctx_destroy(c);
+        REQUIRE(fake::device_bytes == 0);
+    }
+    return 0;
+}
+
+// A batch leaves its workspaces with memory; a later call of another shape may need it.
+int idle_workspaces_give_memory_back() {
+    slm_opts o{};
+    o.hbm_budget = detection_bytes(24, 960, 540) * 13 / 10;
+    slm_ctx *c = nullptr;
+    REQUIRE(slm_ctx_create(&o, &c) == SLM_OK);
+    for (int k = 0; k < 2; ++k) {
+        REQUIRE(detect(c, 24, 960, 540) == SLM_OK);
+        REQUIRE(detect(c, 1, 4500, 2700) == SLM_OK);  // as many pixels in one image
+    }
+    void *a = nullptr;  // and a pair of another kind
+    REQUIRE(posix_memalign(&a, 16, 512 * 300) == 0);
+    std::memset(a, 0, 512 * 300);
+    std::vector<slm_pair> out(300);
+    uint32_t n = 0;
+    REQUIRE(slm_ratio_match(c, static_cast<float *>(a), 300, static_cast<float *>(a), 300, 0.8f, 1, SLM_PREC_BF16, out.data(), 300, &n,
+                            nullptr) == SLM_OK);
+    REQUIRE(detect(c, 24, 960, 540) == SLM_OK);
+    REQUIRE(detect(c, 60, 960, 540) == SLM_OOM);  // what does not fit at all is refused, and the context stays usable
+    REQUIRE(detect(c, 24, 960, 540) == SLM_OK);
+    slm_ctx_destroy(c);
+    REQUIRE(fake::device_bytes == 0);
+    std::free(a);
+    return 0;
+}
+
 int main(int argc, char **argv) {
     const std::map<std::string, int (*)()> checks = {
         {"tracks_that_share_matches", tracks_that_share_matches},
         {"sampson_waits_after_a_failure", sampson_waits_after_a_failure},
         {"single_pair_waits_after_a_failure", single_pair_waits_after_a_failure},
+        {"detection_within_its_budget", detection_within_its_budget},
+        {"idle_workspaces_give_memory_back", idle_workspaces_give_memory_back},
     };
     if (argc == 2 && checks.count(argv[1])) return checks.at(argv[1])();
     for (const auto &k : checks) std::printf("%s\n", k.first.c_str());
