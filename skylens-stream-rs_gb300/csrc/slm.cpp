@@ -1724,8 +1724,10 @@ extern "C" slm_status slm_plan_device_results(slm_plan *p, const uint32_t **d_co
 }
 
 extern "C" uint64_t slm_plan_bytes(slm_plan *p) {
-    if (!p) return 0;
-    return p->d_up.bytes + p->d_parts.bytes + p->d_colbest.bytes + p->d_slots.bytes + p->d_ctl.bytes + p->d_dense.bytes;
+    uint64_t n = 0;
+    if (p)
+        for (const DevBuf *b : plan_buffers(p)) n += b->bytes;
+    return n;
 }
 
 // A plan that is launched once: plain launches. Capturing, instantiating and
@@ -2221,36 +2223,77 @@ struct slm_server {
 
 namespace {
 
-// Scratch a batch needs (matches plan_build_shortlist's and plan_build's
-// allocations; used for admission).
+// Device memory a batch's plan holds at the default tuning: what plan_build and
+// plan_build_shortlist allocate for these pairs, or a little more (a CPU check compares
+// the two), with the buffers' growth slack; for admission.
 uint64_t batch_bytes(const slm_store *st, const std::vector<uint32_t> &vn, const std::vector<slm_pair> &pairs,
-                     slm_precision prec) {
-    uint64_t rows = 0, cols = 0, na = 0, items = 0, supers = 0, cand_rows = 0;
+                     slm_precision prec, int mutual) {
+    const uint64_t sms = (uint64_t)std::max(1, st->ctx->sms), np = pairs.size();
+    auto tiles = [](uint64_t n) { return (n + kTile - 1) / kTile; };
+    auto size = [&](uint32_t v) -> uint64_t { return v < vn.size() ? vn[v] : 0; };
+    uint64_t distances = 0, rows = 0, cols = 0, na = 0, row_tiles = 0, supers = 0, steps = 0, blk = 0;
+    ExactShapes shapes;
     for (const slm_pair &p : pairs) {
-        const uint64_t a = p.i < vn.size() ? vn[p.i] : 0, b = p.j < vn.size() ? vn[p.j] : 0;
-        if (b) supers += (a + 2 * kTile - 1) / (2 * kTile);
+        const uint64_t a = size(p.i), b = size(p.j);
+        distances += a * b;
+        rows += pad_rows(a), cols += pad_rows(b), na += a;
+        row_tiles += tiles(a);
+        if (b) supers += (tiles(a) + 1) / 2;
+        steps += ((tiles(a) + 1) / 2) * ((tiles(b) + 1) / 2) * (mutual ? 2 : 1);
+        blk += (a + kSlRowBlock - 1) / kSlRowBlock;
+        shapes.add((uint32_t)a, (uint32_t)b);
     }
-    // column ranges per pair as plan_build_shortlist splits them (default items per SM)
-    const uint64_t want = (uint64_t)std::max(1, st->ctx->sms) * 3;
-    const uint64_t split = supers && supers < want ? (want + supers - 1) / supers : 1;
+    prec = resolve_prec(prec, distances);
+    // every plan: columns' keys, slots, the dense list, control words, the pairs' table
+    const uint64_t pad = 4096;  // the sections of one upload start at 256 bytes
+    uint64_t bytes = pad + cols * 8 + na * 16 + np * (sizeof(PairMeta) + 8 + 8 + 4);
+    if (prec == SLM_PREC_FP32) {
+        const bool few = shapes.few((int)sms);
+        const ExactShape shape = few ? shapes.best((int)sms) : ExactShape{};
+        const uint64_t split = row_tiles && row_tiles < 4 * sms ? (4 * sms + row_tiles - 1) / row_tiles : 1;
+        for (const slm_pair &p : pairs) {
+            const uint64_t a = size(p.i), b = size(p.j);
+            const uint64_t chunks = few ? ExactShapes::chunks_of((uint32_t)b, shape.cols)
+                                        : std::max<uint64_t>(1, std::min(split, tiles(b)));
+            bytes += tiles(a) * chunks * (sizeof(RowPart) * kTile + sizeof(Item) * (4 / shape.rows));
+        }
+        return bytes + bytes / 4;
+    }
+    // BF16 pass: blocks of 256 or 128 rows, cut where a CTA's share ends, up to twice a
+    // CTA (to whole steps), and no finer than steps
+    const uint64_t per = steps <= sms ? 1 : 2;
+    uint64_t blocks = 0, nsteps = 0;
     for (const slm_pair &p : pairs) {
-        const uint64_t a = p.i < vn.size() ? vn[p.i] : 0, b = p.j < vn.size() ? vn[p.j] : 0;
-        rows += pad_rows(a);
-        cols += pad_rows(b);
-        na += a;
-        items += (pad_rows(a) / kTile + 1) * 4;
-        cand_rows += pad_rows(a) *
-                     std::max<uint64_t>(1, std::min<uint64_t>(std::min<uint64_t>(split, pad_rows(b) / kTile), kSlMaxRanges));
+        const uint64_t ta = tiles(size(p.i)), tb = tiles(size(p.j));
+        if (!ta || !tb) continue;
+        const uint64_t ba = (ta + per - 1) / per, bb = mutual ? (tb + per - 1) / per : 0;
+        blocks += ba + bb, nsteps += ba * ((tb + 1) / 2) + bb * ((ta + 1) / 2);
     }
-    uint64_t bytes = 64 + pairs.size() * (sizeof(PairMeta) + 16 + 8) + na * 16 + cols * 8;
-    if (prec == SLM_PREC_FP32)
-        bytes += items * (sizeof(Item) + sizeof(RowPart) * kTile);
-    else
-        bytes += rows * 3 * 4 + cand_rows * (2 * 4 + 2 * kSlHalfRecs * 20) + cols * 12 + na * 2 * sizeof(SlQueue) +
-                 items * 256 * 12 +
-                 pairs.size() * (4 + 16) + (rows / kSlRowBlock + pairs.size()) * 4 +
-                 (rows / kTile + 4ull * (uint64_t)std::max(1, st->ctx->sms)) * (sizeof(Item) + sizeof(RowPart) * kTile);
-    return bytes + bytes / 4;  // DevBuf growth slack
+    const uint64_t parts = std::min(blocks + 2 * sms, nsteps), rows_pad = rows + 2 * kTile, items = row_tiles + 4 * sms;
+    bytes += parts * (12 * per * kTile + sizeof(TopItem)) + blocks * 8 + 4 * (sms + 2);
+    bytes += np * (sizeof(SlPair) + 16 + 4 + 4) + blk * 4 + rows_pad * 4 + (na + 64) * sizeof(SlQueue);
+    bytes += na * 24 + (na / kGroupRows + na / kTileRows + 2 * np) * 16;     // open and undecided rows, their groups
+    bytes += items * (sizeof(Item) + sizeof(RowPart) * kTile);               // of routed pairs
+    if (prec == SLM_PREC_FP8) {
+        const uint64_t split = supers && supers < 3 * sms ? (3 * sms + supers - 1) / supers : 1, cols_pad = cols + kTile;
+        uint64_t cand = 2 * kTile, sl_parts = 0, sitems = 0;
+        for (const slm_pair &p : pairs) {
+            const uint64_t a = size(p.i), b = size(p.j);
+            const uint64_t chunks = std::max<uint64_t>(1, std::min<uint64_t>(std::min(split, tiles(b)), kSlMaxRanges));
+            cand += pad_rows(a) * chunks;
+            if (a && b) sl_parts += (tiles(a) + 1) / 2 * chunks;
+            if (a * b >= kSlSampleMin) {
+                const uint64_t n = (std::min<uint64_t>(tiles(b), kSlSampleTiles) + kSlSampleItemTiles - 1) / kSlSampleItemTiles;
+                sl_parts += n, sitems += n;
+                bytes += sizeof(SlSample);
+            }
+        }
+        sitems += sl_parts;
+        bytes += sl_parts * 256 * 12 + sitems * sizeof(SlItem);
+        bytes += cols_pad * (4 + 4 + 4) + rows_pad * 4;                      // minima, thresholds, window counts
+        bytes += cand * (8 + 2 * kSlHalfRecs * (sizeof(float4) + 4)) + (na + 64) * sizeof(SlQueue);
+    }
+    return bytes + bytes / 4;
 }
 
 void serve_fail_request(ServeRequest *r, slm_status s, const std::string &error) {
@@ -2375,7 +2418,7 @@ void serve_loop(slm_server *srv) {
                     if (!pairs.empty() && pairs.size() + r->pairs.size() > srv->opts.max_batch_pairs) break;
                     std::vector<slm_pair> trial = pairs;
                     trial.insert(trial.end(), r->pairs.begin(), r->pairs.end());
-                    if (!pairs.empty() && batch_bytes(srv->store, srv->view_n, trial, srv->opts.prec) > srv->slot_budget)
+                    if (!pairs.empty() && batch_bytes(srv->store, srv->view_n, trial, srv->opts.prec, srv->opts.mutual) > srv->slot_budget)
                         break;
                     pairs.swap(trial);
                 }
@@ -2396,8 +2439,15 @@ void serve_loop(slm_server *srv) {
             if (ps == SLM_OK && !pairs.empty()) {
                 slm_tune t{};
                 t.use_graph = 2;
-                ps = plan_init(&s->plan, srv->ctx, srv->store, pairs.data(), (uint32_t)pairs.size(), srv->opts.ratio,
-                               srv->opts.mutual, srv->opts.prec, &t, s->stream);
+                auto plan = [&] {
+                    return plan_init(&s->plan, srv->ctx, srv->store, pairs.data(), (uint32_t)pairs.size(), srv->opts.ratio,
+                                     srv->opts.mutual, srv->opts.prec, &t, s->stream);
+                };
+                ps = plan();
+                if (ps == SLM_OOM) {  // each buffer is as large as any batch before made it: this batch's only
+                    plan_release(&s->plan);
+                    ps = plan();
+                }
                 s->plan.timed = false;
                 if (ps == SLM_OK) ps = plan_launch_on(&s->plan, s->stream, false);
             }

@@ -5,6 +5,7 @@
 // the log.
 #pragma once
 #include <cuda_runtime.h>
+#include <sys/mman.h>
 
 #include <cstdint>
 #include <cstdio>
@@ -36,8 +37,8 @@ inline void note(const char *what) {
 }
 inline cudaError_t alloc(void **p, size_t n) {
     std::lock_guard<std::mutex> g(mu);
-    if (posix_memalign(p, 256, n ? n : 1)) return cudaErrorMemoryAllocation;
-    std::memset(*p, 0, n);
+    *p = mmap(nullptr, n ? n : 1, PROT_READ | PROT_WRITE, MAP_PRIVATE | MAP_ANONYMOUS | MAP_NORESERVE, -1, 0);  // zeros
+    if (*p == MAP_FAILED) return *p = nullptr, cudaErrorMemoryAllocation;
     device[*p] = n;
     device_bytes += n;
     if (device_bytes > device_peak) device_peak = device_bytes;
@@ -48,8 +49,8 @@ inline cudaError_t release(void *p) {
     auto it = device.find(p);
     if (it == device.end()) return p ? cudaErrorInvalidValue : cudaSuccess;
     device_bytes -= it->second;
+    munmap(p, it->second ? it->second : 1);
     device.erase(it);
-    std::free(p);
     return cudaSuccess;
 }
 inline bool on_device(const void *p) {

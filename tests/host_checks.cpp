@@ -160,11 +160,96 @@ int idle_workspaces_give_memory_back() {
     return 0;
 }
 
+// What a batch is admitted by is what its plan allocates, and slm_plan_bytes counts that.
+// (The BF16 pass's parts are bounded, not counted: one more for each of 152 CTAs, of 3 KB
+// and the buffers' quarter.)
+int plans_hold_what_is_counted() {
+    std::vector<uint32_t> bad;
+    uint32_t seed = 1;
+    auto next = [&](uint32_t n) { return (seed = seed * 1664525u + 1013904223u) / 65536u % n; };
+    for (const slm_precision prec : {SLM_PREC_FP32, SLM_PREC_BF16, SLM_PREC_FP8})
+        for (int round = 0; round < 40; ++round) {
+            slm_ctx *c = nullptr;
+            REQUIRE(slm_ctx_create(nullptr, &c) == SLM_OK);
+            const uint32_t most = round % 4 == 0 ? 9000 : round % 4 == 1 ? 2000 : round % 4 == 2 ? 300 : 40000;
+            const uint32_t nv = 2 + next(most > 3000 ? 4 : 30), np = 1 + next(round % 3 ? 40 : 400);
+            std::vector<uint32_t> n(nv);
+            for (uint32_t &v : n) v = next(8) ? 1 + next(most) : next(3);
+            std::vector<float> rows(size_t(most + 3) * 128);
+            slm_store *st = nullptr;
+            REQUIRE(slm_store_create(c, size_t(nv) * (most + 3), nv, &st) == SLM_OK);
+            for (uint32_t v : n) REQUIRE(slm_store_add_view(st, rows.data(), v, nullptr) == SLM_OK);
+            std::vector<slm_pair> pairs(np);
+            for (slm_pair &p : pairs) p = slm_pair{next(nv), next(nv)};
+            const int mutual = round & 1;
+            slm_tune t{};
+            t.use_graph = 2;
+            slm_plan *warm = nullptr, *p = nullptr;  // the first builds the store's images
+            REQUIRE(slm_plan_create(c, st, pairs.data(), np, 0.8f, mutual, prec, &t, &warm) == SLM_OK);
+            const uint64_t before = slm_ctx_bytes_in_use(c);
+            REQUIRE(slm_plan_create(c, st, pairs.data(), np, 0.8f, mutual, prec, &t, &p) == SLM_OK);
+            const uint64_t held = slm_ctx_bytes_in_use(c) - before, counted = batch_bytes(st, n, pairs, prec, mutual);
+            REQUIRE(slm_plan_bytes(p) == held);
+            if (counted < held || counted > held + held / 4 + (768 << 10)) {
+                std::printf("precision %d, %u pairs of up to %u rows, mutual %d: holds %llu, counted %llu\n", (int)prec, np, most, mutual,
+                            (unsigned long long)held, (unsigned long long)counted);
+                bad.push_back(round);
+            }
+            slm_plan_destroy(p);
+            slm_plan_destroy(warm);
+            slm_store_destroy(st);
+            slm_ctx_destroy(c);
+        }
+    REQUIRE(bad.empty());
+    return 0;
+}
+
+// A server within a small budget: batches of unlike shapes one after the other in one
+// slot, whose buffers keep the size of the largest before.
+int serving_batches_of_unlike_shapes() {
+    for (const slm_precision prec : {SLM_PREC_FP32, SLM_PREC_BF16, SLM_PREC_FP8}) {
+        std::vector<float> rows(size_t(20000) * 128);
+        std::vector<uint32_t> n(12, 64);  // the first view's many rows now as rows, now as columns
+        n[0] = 20000;
+        uint64_t largest = 0, images = 0;
+        for (int pass = 0; pass < 2; ++pass) {  // the first finds what the batches need
+            slm_server_opts o{};
+            o.max_descs = 60000, o.max_views = 64, o.slots = 1, o.max_batch_pairs = 4096, o.tick_us = 50;
+            o.ratio = 0.8f, o.mutual = 1, o.prec = prec;
+            o.hbm_budget = pass ? images + largest + largest / 32 : 0;
+            slm_server *srv = nullptr;
+            REQUIRE(slm_server_create(&o, &srv) == SLM_OK);
+            images = srv->ctx->used.load();
+            std::vector<slm_pair> out(1), pairs;
+            for (uint32_t v = 0; v < n.size(); ++v) {
+                pairs.clear();
+                if (v % 2) pairs.assign(v % 3 ? 1 : 2, slm_pair{0, SLM_SELF});
+                if (v && v % 2 == 0) pairs.assign(prec == SLM_PREC_FP32 ? 2 : 4, slm_pair{SLM_SELF, 0});
+                std::vector<slm_pair> named = pairs;
+                for (slm_pair &p : named) p = slm_pair{p.i == SLM_SELF ? v : p.i, p.j == SLM_SELF ? v : p.j};
+                if (!pass) {
+                    std::vector<uint32_t> seen(n.begin(), n.begin() + v + 1);
+                    largest = std::max(largest, batch_bytes(srv->store, seen, named, prec, 1));
+                }
+                uint64_t ticket = 0;
+                std::vector<uint64_t> off(pairs.size() + 1);
+                REQUIRE(slm_server_submit(srv, rows.data(), n[v], pairs.data(), (uint32_t)pairs.size(), nullptr, &ticket) == SLM_OK);
+                REQUIRE(slm_server_wait(srv, ticket, 20000, out.data(), 0, off.data(), nullptr) == SLM_OK);
+            }
+            slm_server_destroy(srv);
+            REQUIRE(fake::device_bytes == 0);
+        }
+    }
+    return 0;
+}
+
 int main(int argc, char **argv) {
     const std::map<std::string, int (*)()> checks = {
         {"tracks_that_share_matches", tracks_that_share_matches},
         {"sampson_waits_after_a_failure", sampson_waits_after_a_failure},
         {"single_pair_waits_after_a_failure", single_pair_waits_after_a_failure},
+        {"plans_hold_what_is_counted", plans_hold_what_is_counted},
+        {"serving_batches_of_unlike_shapes", serving_batches_of_unlike_shapes},
         {"detection_within_its_budget", detection_within_its_budget},
         {"idle_workspaces_give_memory_back", idle_workspaces_give_memory_back},
     };
