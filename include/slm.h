@@ -218,7 +218,8 @@ uint32_t slm_store_num_views(slm_store *st);
 
 /* Tuning knobs; zero fields take the autotuned or default values. */
 typedef struct {
-    uint32_t items_per_sm;  /* FP32, FP8: target work items per SM when splitting columns */
+    uint32_t items_per_sm;  /* FP32, FP8: target work items per SM when splitting columns (0: 4 and 3;
+                               FP32 batches of few tiles also split tiles then) */
     uint32_t shortlist_k;   /* shortlist capacity, 1..32. BF16: a row whose bounds decide nothing
                                is rescored over up to 4 shortlist_k columns (0: 128); FP8: records
                                of 4-column hit groups per row, column range and column half (0: 16) */
@@ -233,7 +234,7 @@ typedef struct {
 } slm_tune;
 
 /* Time a grid of settings on this batch with CUDA events (FP32: items per SM
- * {2, 4, 8} x arithmetic variant; FP8: items per SM {2, 4, 8} x row tiles
+ * {2, 4, 8}, for few tiles also 0, x arithmetic variant; FP8: items per SM {2, 4, 8} x row tiles
  * per work item {1, 2} x shortlist_k {8, 12, 16}; BF16: the latter two) and return the fastest in
  * *best (and its time in *best_ms). The result is cached in the context under
  * the batch's shape (precision, mean rows per pair, pair count), which plans

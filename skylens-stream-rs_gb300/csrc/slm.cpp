@@ -385,7 +385,7 @@ void plan_items(slm_plan *p) {
     if (row_tiles && row_tiles < want) split = (uint32_t)((want + row_tiles - 1) / row_tiles);
     ExactShapes shapes;
     for (uint32_t k = 0; k < p->np; ++k) shapes.add(p->meta[k].na, p->meta[k].nb);
-    const bool few = (!p->tune.items_per_sm || p->tune.items_per_sm == 4) && shapes.few(std::max(1, p->ctx->sms));
+    const bool few = !p->tune.items_per_sm && shapes.few(std::max(1, p->ctx->sms));
     const ExactShape shape = few ? shapes.best(std::max(1, p->ctx->sms)) : ExactShape{};
     p->items.clear();
     uint32_t part = 0;
@@ -1583,16 +1583,22 @@ extern "C" slm_status slm_autotune(slm_ctx *c, slm_store *st, const slm_pair *pa
     SLM_TRY(validate_ratio(ratio));
     SLM_TRY(ctx_check_device(c));
     prec = resolve_prec(prec, prec == SLM_PREC_AUTO ? batch_distances(st, pairs, np) : 0);
-    // FP32: items per SM x arithmetic variant; BF16/FP8: items per SM x the
+    // FP32: items per SM (in a batch of few tiles also the default's smaller items) x
+    // arithmetic variant; BF16/FP8: items per SM x the
     // M tile shape (128-row a tiles per CTA work item, M = 128 or 256) x the
     // shortlist capacity (records of 4-column hit groups per row and column half)
     std::vector<slm_tune> grid;
-    const uint32_t ips[3] = {2, 4, 8};
+    ExactShapes shapes;
+    for (uint32_t k = 0; k < np && prec == SLM_PREC_FP32; ++k)
+        if (pairs[k].i < st->n.size() && pairs[k].j < st->n.size()) shapes.add(st->n[pairs[k].i], st->n[pairs[k].j]);
+    const bool few = prec == SLM_PREC_FP32 && shapes.few(std::max(1, c->sms));
+    const uint32_t ips[4] = {0, 2, 4, 8};
     const uint32_t ks[3] = {8, 12, 16};
     for (uint32_t a = 0; a < 2; ++a)
         for (uint32_t ki = 0; ki < (prec == SLM_PREC_FP32 ? 1u : 3u); ++ki)
             for (uint32_t ipsm : ips) {
                 if (prec == SLM_PREC_BF16 && ipsm != 4) continue;  // its pass is cut into equal shares
+                if (!ipsm && !few) continue;
                 slm_tune t{};
                 t.use_graph = 2;
                 t.items_per_sm = ipsm;

@@ -243,6 +243,36 @@ int serving_batches_of_unlike_shapes() {
     return 0;
 }
 
+// Items a SM asked for are whole tiles against ranges of whole tiles, four a SM too; only
+// the default cuts a batch of few tiles finer.
+int items_asked_for() {
+    slm_ctx *c = nullptr;
+    slm_store *st = nullptr;
+    REQUIRE(slm_ctx_create(nullptr, &c) == SLM_OK);
+    REQUIRE(slm_store_create(c, 2000, 2, &st) == SLM_OK);
+    std::vector<float> rows(size_t(1000) * 128);
+    REQUIRE(slm_store_add_view(st, rows.data(), 700, nullptr) == SLM_OK && slm_store_add_view(st, rows.data(), 900, nullptr) == SLM_OK);
+    const slm_pair pr{0, 1};
+    for (const uint32_t ips : {0u, 1u, 2u, 4u, 8u}) {
+        slm_tune t{};
+        t.items_per_sm = ips;
+        slm_plan *p = nullptr;
+        REQUIRE(slm_plan_create(c, st, &pr, 1, 0.8f, 1, SLM_PREC_FP32, &t, &p) == SLM_OK);
+        bool whole = true;
+        for (const slm::Item &it : p->items) whole &= it.g0 == 0 && it.g1 == 4 && it.q0 % 4 == 0 && (it.q1 % 4 == 0 || it.q1 == 29);
+        REQUIRE(whole == (ips != 0));
+        slm_plan_destroy(p);
+    }
+    // the autotuner looks at the default there too
+    slm_tune best{};
+    float ms = 0;
+    REQUIRE(slm_autotune(c, st, &pr, 1, 0.8f, 1, SLM_PREC_FP32, &best, &ms) == SLM_OK);
+    REQUIRE(best.items_per_sm == 0);  // the first of equals: every timing here is the same
+    slm_store_destroy(st);
+    slm_ctx_destroy(c);
+    return 0;
+}
+
 int main(int argc, char **argv) {
     const std::map<std::string, int (*)()> checks = {
         {"tracks_that_share_matches", tracks_that_share_matches},
@@ -250,6 +280,7 @@ int main(int argc, char **argv) {
         {"single_pair_waits_after_a_failure", single_pair_waits_after_a_failure},
         {"plans_hold_what_is_counted", plans_hold_what_is_counted},
         {"serving_batches_of_unlike_shapes", serving_batches_of_unlike_shapes},
+        {"items_asked_for", items_asked_for},
         {"detection_within_its_budget", detection_within_its_budget},
         {"idle_workspaces_give_memory_back", idle_workspaces_give_memory_back},
     };
