@@ -462,10 +462,10 @@ SLM_DEV bool settle_with_d1(const SlArgs &g, const SlPair &sp, uint32_t p, uint3
 // 13 in a kernel of its own).
 constexpr uint32_t kDecideThreads = 256;
 template <int R>
-__global__ void __launch_bounds__(kDecideThreads) sl_decide_kernel(SlArgs g) {
+__global__ void __launch_bounds__(kDecideThreads) sl_decide_kernel(SlArgs g, uint32_t block0) {
     grid_wait();
     grid_go();
-    const uint32_t p = blockIdx.x, row0 = blockIdx.y * (kDecideThreads * R);
+    const uint32_t p = blockIdx.x, row0 = (block0 + blockIdx.y) * (kDecideThreads * R);
     const PairMeta pm = g.pairs[p];
     if (row0 >= pm.na) return;  // block-uniform, as below
     const SlPair sp = g.spairs[p];
@@ -1066,15 +1066,17 @@ int launch_top2_pass(const SlArgs &a, cudaStream_t s) {
 int launch_top2_decide(const SlArgs &a, int sms, cudaStream_t s) {
     if (!a.npairs || !a.max_na) return 0;
     // four rows a thread once that still gives every SM its eight CTAs
-    if (a.n_rows < 8ull * sms * 4 * kDecideThreads) {
-        launch_next(sl_decide_kernel<1>, dim3(a.npairs, (a.max_na + kDecideThreads - 1) / kDecideThreads), kDecideThreads,
-                    0, s, a);
-        return 1;
+    const bool four = a.n_rows >= 8ull * sms * 4 * kDecideThreads;
+    const uint32_t rows = (four ? 4 : 1) * kDecideThreads, blocks = (uint32_t)(((uint64_t)a.max_na + rows - 1) / rows);
+    int n = 0;
+    for (uint32_t b = 0; b < blocks; b += 65535, ++n)  // a grid's second dimension: 67 M rows of one view
+        launch_next(four ? sl_decide_kernel<4> : sl_decide_kernel<1>, dim3(a.npairs, std::min(65535u, blocks - b)),
+                    kDecideThreads, 0, s, a, b);
+    if (four) {
+        launch_next(sl_nearest_kernel, 2 * sms, 256, 0, s, a);
+        ++n;
     }
-    launch_next(sl_decide_kernel<4>, dim3(a.npairs, (a.max_na + 4 * kDecideThreads - 1) / (4 * kDecideThreads)),
-                kDecideThreads, 0, s, a);
-    launch_next(sl_nearest_kernel, 2 * sms, 256, 0, s, a);
-    return 2;
+    return n;
 }
 
 int launch_top2_resolve(const SlArgs &a, int sms, cudaStream_t s) {
