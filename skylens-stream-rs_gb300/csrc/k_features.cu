@@ -1152,12 +1152,13 @@ cudaError_t init_feature_kernels() {
 }
 
 void launch_blur(const float *src, float *tmp, float *dst, const float *prev, float *dog, int w, int h, int nimg,
-                 uint64_t stride_src, uint64_t stride_dst, uint64_t stride_dog, const BlurTaps &t, cudaStream_t s) {
+                 uint64_t stride_src, uint64_t stride_dst, uint64_t stride_dog, const BlurTaps &t, int sms, cudaStream_t s) {
     if (t.r <= kFusedR && (!dog || (prev == src && stride_src == stride_dst))) {
-        // tall tiles (less halo) once they still give every SM four: 0.61 -> 0.58 ms
-        // for 24 views, where one photo's launches would leave SMs idle
+        // tall tiles (less halo) once they still give every SM four: 0.61 -> 0.58 ms for
+        // 24 views of 960 x 540 in one launch, where one photo's would leave SMs idle (a
+        // batch's parts have fewer tiles: the large images of a call are what takes them)
         const uint64_t tiles = (uint64_t)((w + kFX - 1) / kFX) * ((h + 63) / 64) * nimg;
-        const BlurFused f = blur_of_radius<1>(t.r, tiles >= 608);
+        const BlurFused f = blur_of_radius<1>(t.r, tiles >= 4ull * sms);
         const dim3 g((w + kFX - 1) / kFX, (h + f.rows - 1) / f.rows, nimg);
         launch_next(f.kernel, g, 256, f.smem, s, src, dst, dog, w, h, stride_src, stride_dst, stride_dog, t);
         return;
@@ -1198,11 +1199,11 @@ void launch_grad(const float *gauss, float2 *grad, int w, int h, int s_, uint64_
                 kGradThreads, 0, s, gauss, grad, w, h, s_, (uint64_t)w * h, img_stride, l0);
 }
 
-void launch_layers(const ExtremaArgs &a, const float *gauss, float2 *grad, uint64_t img_stride, int nimg,
+void launch_layers(const ExtremaArgs &a, const float *gauss, float2 *grad, uint64_t img_stride, int nimg, int sms,
                    cudaStream_t s) {
     // strips of 16 rows where that leaves every SM its 16 warps, else of 4
     const uint64_t warps = (uint64_t)((a.w + 27) / 30) * ((a.h + 13) / 16) * nimg * a.s;
-    const int rows = warps >= 16 * 152 ? kExtremaRows : 4, strip = kExtremaWarps * rows;
+    const int rows = warps >= 16ull * sms ? kExtremaRows : 4, strip = kExtremaWarps * rows;
     const uint32_t layers = (uint32_t)nimg * a.s;
     const uint3 gg = make_uint3((a.w + kGradThreads - 1) / kGradThreads, (a.h + kGradRows - 1) / kGradRows, layers);
     const uint3 eg = a.w < 3 || a.h < 3 ? make_uint3(1, 1, 0)

@@ -3235,7 +3235,8 @@ slm_status feat_core(slm_ctx *c, Workspace *ws, const float *d_img, uint32_t n, 
             // an octave's first layer comes from the one before it, so they alternate
             float *gauss = reinterpret_cast<float *>(d + (o & 1 ? o_odd : o_gauss));
             if (o == 0) {
-                launch_blur(d_img, tmp, gauss, nullptr, nullptr, G.w, G.h, (int)n, wh, ng * wh, 0, taps[0], st);
+                launch_blur(d_img, tmp, gauss, nullptr, nullptr, G.w, G.h, (int)n, wh, ng * wh, 0, taps[0],
+                            c->sms, st);
             } else {
                 const OctaveGeom &P = out.geom[o - 1];
                 const float *before = reinterpret_cast<const float *>(d + (o & 1 ? o_gauss : o_odd));
@@ -3243,7 +3244,7 @@ slm_status feat_core(slm_ctx *c, Workspace *ws, const float *d_img, uint32_t n, 
             }
             for (int i = 1; i < ng; ++i)
                 launch_blur(gauss + (i - 1) * wh, tmp, gauss + i * wh, gauss + (i - 1) * wh, dog + (i - 1) * wh, G.w,
-                            G.h, (int)n, ng * wh, ng * wh, (ng - 1) * wh, taps[i], st);
+                            G.h, (int)n, ng * wh, ng * wh, (ng - 1) * wh, taps[i], c->sms, st);
             ExtremaArgs ea{};
             ea.dog = dog;
             ea.layer_stride = wh;
@@ -3257,7 +3258,7 @@ slm_status feat_core(slm_ctx *c, Workspace *ws, const float *d_img, uint32_t n, 
             ea.cands = out.d_cands;
             ea.count = d_count;
             ea.cap = cap;
-            launch_layers(ea, gauss, out.d_grads + G.grad_off, ng * wh, (int)n, st);
+            launch_layers(ea, gauss, out.d_grads + G.grad_off, ng * wh, (int)n, c->sms, st);
         }
         OrientArgs oa{};
         oa.cands = out.d_cands;
@@ -3374,7 +3375,7 @@ slm_status feat_describe(slm_ctx *c, cudaStream_t st, DevBuf &buf, const FeatCor
     }
     // windows too large for one warp first
     const auto small = std::stable_partition(jobs.begin(), jobs.end(), [&](const DescJob &j) {
-        return describe_side(fc.cands[j.cand].sig) > describe_warp_side(list.size());
+        return describe_side(fc.cands[j.cand].sig) > describe_warp_side(list.size(), c->sms);
     });
     unsigned char *d = buf.as<unsigned char>();
     SLM_CU(cudaMemcpyAsync(d + o_jobs, jobs.data(), sizeof(DescJob) * jobs.size(), cudaMemcpyHostToDevice, st));
@@ -3752,7 +3753,7 @@ extern "C" slm_status slm_describe(slm_ctx *c, const float *img, uint32_t w, uin
             DescribeArgs da{};
             da.jobs = reinterpret_cast<const DescJob *>(d + o_jobs);
             da.cs = reinterpret_cast<float2 *>(d + o_cs);
-            while (da.n_large < n && describe_side(kps[jobs[da.n_large].cand].sigma) > describe_warp_side(n)) ++da.n_large;
+            while (da.n_large < n && describe_side(kps[jobs[da.n_large].cand].sigma) > describe_warp_side(n, c->sms)) ++da.n_large;
             da.max_side = describe_side(kps[jobs[0].cand].sigma);
             da.kps = reinterpret_cast<const slm_keypoint *>(d + o_kps);
             da.grads = reinterpret_cast<const float2 *>(d + o_grad);

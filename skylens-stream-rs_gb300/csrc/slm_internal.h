@@ -262,7 +262,7 @@ struct DescJob {
 struct DescribeArgs {
     const DescJob *jobs;
     float2 *cs;             // scratch: cos and sin of each job's angle
-    uint32_t n_large;       // the first jobs, those of more than kDescWarpSide window rows: a CTA each
+    uint32_t n_large;       // the first jobs, those above describe_warp_side (all, with few features): a CTA each
     int max_side;           // the most window rows of any job (describe_side of the largest sigma)
     const FeatCand *cands;  // null: keypoints kps (image pixels) on one table, grads, geom[0]
     const slm_keypoint *kps;
@@ -276,7 +276,7 @@ cudaError_t init_feature_kernels();  // kernel attributes, once per device
 // Both passes of a blur of nimg images (src -> tmp -> dst); with dog, also
 // dog = dst - prev (prev strided as dst). Strides are per image, in floats.
 void launch_blur(const float *src, float *tmp, float *dst, const float *prev, float *dog, int w, int h, int nimg,
-                 uint64_t stride_src, uint64_t stride_dst, uint64_t stride_dog, const BlurTaps &t, cudaStream_t s);
+                 uint64_t stride_src, uint64_t stride_dst, uint64_t stride_dog, const BlurTaps &t, int sms, cudaStream_t s);
 void launch_downsample(const float *src, float *dst, int w, int h, int nimg, uint64_t stride_src,
                        uint64_t stride_dst, cudaStream_t s);
 void launch_upsample2(const float *src, float *dst, int w, int h, int nimg, cudaStream_t s);
@@ -289,7 +289,7 @@ void launch_grad(const float *gauss, float2 *grad, int w, int h, int s_, uint64_
                  cudaStream_t s);
 // an octave's extrema, and the gradient tables of its layers 1 .. s (image k's layer
 // l at gauss + k * img_stride + l * layer_stride)
-void launch_layers(const ExtremaArgs &a, const float *gauss, float2 *grad, uint64_t img_stride, int nimg,
+void launch_layers(const ExtremaArgs &a, const float *gauss, float2 *grad, uint64_t img_stride, int nimg, int sms,
                    cudaStream_t s);
 void launch_candidate_sigma(FeatCand *cands, const uint32_t *count, uint32_t cap, float sigma0, float kstep, int sms,
                             cudaStream_t s);
@@ -297,9 +297,9 @@ void launch_orient(const OrientArgs &a, int sms, cudaStream_t s);
 constexpr int kDescWarpSide = 127;  // window rows one warp takes
 // The window rows from which a feature gets a CTA instead of a warp: those a
 // warp cannot take, or, with fewer features than four warps for each of the
-// GPU's 608 sub-partitions, all: the chain of one warp then decides (one 717 x
+// SMs' four sub-partitions, all: the chain of one warp then decides (one 717 x
 // 531 photo's 1026 features 0.39 ms as warps, 0.13 as CTAs).
-inline int describe_warp_side(size_t features) { return features < 2432 ? 0 : kDescWarpSide; }
+inline int describe_warp_side(size_t features, int sms) { return features < 16 * (size_t)sms ? 0 : kDescWarpSide; }
 // Window rows of a feature of scale sigma (features.rs:526-528), at least.
 inline int describe_side(float sigma) { return 2 * ((int)(3.0f * sigma * 1.41421356f * 2.5f + 0.5f) + 1) + 1; }
 void launch_describe(const DescribeArgs &a, uint32_t njobs, cudaStream_t s);

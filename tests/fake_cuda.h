@@ -166,9 +166,9 @@ int launch_shortlist_finalize(const SlArgs &, cudaStream_t) { return 1; }
 int launch_shortlist_rescue_prep(const SlArgs &, cudaStream_t) { return 1; }
 int launch_shortlist_tail(const SlArgs &, int, cudaStream_t) { return 1; }
 void launch_sampson(const SampsonArgs &a, cudaStream_t) { fake::note("sampson"), fake::sampson = a; }
-void launch_blur(const float *, float *, float *, const float *, float *, int, int, int, uint64_t, uint64_t, uint64_t, const BlurTaps &, cudaStream_t) {}
+void launch_blur(const float *, float *, float *, const float *, float *, int, int, int, uint64_t, uint64_t, uint64_t, const BlurTaps &, int, cudaStream_t) {}
 void launch_grad(const float *, float2 *, int, int, int, uint64_t, int, int, cudaStream_t) {}
-void launch_layers(const ExtremaArgs &, const float *, float2 *, uint64_t, int, cudaStream_t) {}
+void launch_layers(const ExtremaArgs &, const float *, float2 *, uint64_t, int, int, cudaStream_t) {}
 void launch_orient(const OrientArgs &, int, cudaStream_t) {}
 void launch_describe(const DescribeArgs &a, uint32_t, cudaStream_t) { fake::describes.push_back(a); }
 void launch_upsample2(const float *, float *, int, int, int, cudaStream_t) {}
