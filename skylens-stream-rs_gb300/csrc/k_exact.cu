@@ -91,11 +91,6 @@ SLM_DEV u64 f2_sub(u64 a, u64 b) {
     asm("sub.rn.f32x2 %0, %1, %2;" : "=l"(d) : "l"(a), "l"(b));
     return d;
 }
-SLM_DEV u64 f2_mul(u64 a, u64 b) {
-    u64 d;
-    asm("mul.rn.f32x2 %0, %1, %2;" : "=l"(d) : "l"(a), "l"(b));
-    return d;
-}
 SLM_DEV u64 f2_add(u64 a, u64 b) {
     u64 d;
     asm("add.rn.f32x2 %0, %1, %2;" : "=l"(d) : "l"(a), "l"(b));

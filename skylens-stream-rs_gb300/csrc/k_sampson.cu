@@ -19,8 +19,13 @@
 // come within the bound (a few matches in 10^5 of a wrong hypothesis, a few in
 // 10^3 of a near-true one), and only then is the f64 residual formed. The
 // counts and masks stay the f64 residual's, since a certain answer is its
-// answer whatever the roundings. The same call from host arrays went from 8.8
-// to 0.90 ms, most of which now is the upload of the 14 MB of hypotheses.
+// answer whatever the roundings. The same call from host arrays, with 100 masks
+// read back as Python arrays, went from 8.8 to 0.82 ms; the C call without them takes
+// 0.40 of it, the 14 MB of hypotheses read over the link where they lie. A
+// hypothesis beyond the FP32 test's range is f64 throughout and reads its
+// entries again, through the cache, for every 32 matches: a call of nothing
+// else takes 8.4 ms. (Its entries kept in shared memory: no faster, and the
+// usual call slower.)
 #include <cuda_runtime.h>
 
 #include <cstdint>

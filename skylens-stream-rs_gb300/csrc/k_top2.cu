@@ -39,7 +39,7 @@
 // measured BF16 rate with the padding of ragged tiles counted. The two passes
 // before (N = 128; row and column minima, then the candidates of each row
 // recomputed against a threshold) took 1.33 and 1.64 ms, and the zone's batch
-// with its lists read back 3.50 ms; now 2.10.
+// with its lists read back 3.50 ms; now 2.07.
 #include <cooperative_groups.h>
 #include <cuda_runtime.h>
 

@@ -2715,9 +2715,10 @@ extern "C" slm_status slm_sampson_score(slm_ctx *c, const double *pts, const uin
     SLM_TRY(ctx_check_device(c));
     Workspace *w = nullptr;
     SLM_TRY(ws_acquire(c, &w));
-    // The hypotheses are most of a call's bytes and each is read once, by one
-    // warp: the kernel reads them (and their pairs and mask offsets) where they
-    // lie if the device can read host memory, else they are copied first.
+    // The hypotheses are most of a call's bytes and each is one warp's: the kernel
+    // reads them (and their pairs and mask offsets) where they lie if the device
+    // can read host memory, else they are copied first. (Matches that FP32 does
+    // not decide read the entries again, mostly from the cache.)
     auto in_place = [&](const void *p, size_t align) {
         if (!c->host_direct || !p || (reinterpret_cast<uintptr_t>(p) & (align - 1))) return false;
         cudaPointerAttributes at{};

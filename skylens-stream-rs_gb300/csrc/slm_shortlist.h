@@ -179,9 +179,9 @@ __host__ __device__ inline uint32_t sl_cand_row(const SlPair &sp, uint32_t na, u
     return sp.crbase + c * ((na + kTile - 1) / kTile * kTile) + i;
 }
 
-// The per-pair kernels after pass 1 (mid, finalize, compact, route_finalize)
-// run one CTA per pair and block of this many rows (and columns), so that a
-// single large pair spreads over many CTAs.
+// The per-pair kernels after pass 1 (mid, finalize, compact, and route_finalize
+// in the scan's launch) run one CTA per pair and block of this many rows (and
+// columns), so that a single large pair spreads over many CTAs.
 constexpr uint32_t kSlRowBlock = 2048;
 
 // Per-pair counters of one launch (SlArgs::pairctl, 4 words per pair).
@@ -226,7 +226,7 @@ struct SlArgs {
     float *rowthr;               // mid -> pass 2
     float *colthr;               // mid -> pass 2
     uint32_t *rowcnt;            // pass 2: records per candidate row and column half
-    float4 *rowrec;              // pass 2: a record's 4 d~ values (BF16: d~ / 2), 2 half_recs per candidate row
+    float4 *rowrec;              // pass 2: a record's 4 d~ values, 2 half_recs per candidate row
     uint32_t *rowrecj;           // the record's first column
     float *colcnt;               // |C| per column (f32 counts: exact below 2^24)
     uint32_t *rowdec;            // finalize / rescore / scan
@@ -252,8 +252,8 @@ struct SlArgs {
     unsigned long long *colbest; // by PairMeta::col_base
     uint32_t want_items;         // exact items wanted to fill the GPU (4 x SMs)
     // FP8 plans: pairs the FP8 bound cannot settle (mid: too many wide rows) are
-    // rescued by a second, BF16 run of eps / pass 1 / mid / pass 2 / finalize
-    // over those pairs only (tier 1), instead of the exact kernel
+    // rescued by the BF16 steps (eps, the one pass, decide, resolve) over those
+    // pairs only (tier 1), instead of the exact kernel
     uint32_t half_recs;          // records per candidate row and column half (1..kSlHalfRecsMax)
     uint32_t tier;               // 0: the plan's precision; 1: the BF16 rescue of an FP8 plan
     const SlSample *samples;     // FP8: the sampled pairs; their items follow the pass's own

@@ -3,8 +3,8 @@
 Views made of dense clusters (copies of a few rows, apart by less than the bound)
 leave every row undecided, with as many columns in its window as a cluster has:
 counts of rows around a group's 128, columns around a tile's, shortlists below,
-at and above their capacity, in single pairs (a cluster of CTAs a group) and in
-batches (a CTA a group, rows of many pairs in one). Each list is the oracle's.
+at and above their capacity, in single pairs (fewer groups than SMs) and in
+batches (rows of many pairs in a group). Each list is the oracle's.
 """
 import numpy as np
 import pytest
